@@ -303,6 +303,12 @@ int mlh_probe_fast_math(int n, const double *x, const double *y, double *rcp, do
  * them bit for bit against IEEE products (subnormal results included). */
 int mlh_probe_scale2(int n, const double *x, double *half, double *quarter, double *twice);
 
+/* TEST HOOK.  The kernels' integer-pipe products and roots and their sums and
+ * products as fused multiply-adds, for n pairs of host values: out holds nine
+ * arrays of n, x y (integer pipe), x y, x + y, x - y, sqrt(x), x^(1/5),
+ * x^(-1/5), x^(1/7), x^(-1/7). */
+int mlh_probe_int_math(int n, const double *x, const double *y, double *out);
+
 /* TEST HOOK.  The grid barriers of the persistent binning wait for
  * `extra_arrivals` more blocks than the launch holds (nonzero: every wait runs
  * out, which no correct launch can make happen) and give up after

@@ -283,7 +283,7 @@ StepArgs make_args(mlh_ctx *c, double dt_max) {
     a.p.faces_cap = c->faces_cap > 0x7fffffff ? 0x7fffffff : (int)c->faces_cap;
     a.qcap = c->queue_cap > 0x7fffffff ? 0x7fffffff : (int)c->queue_cap;
     a.qcap2 = c->queue_cap2 > 0x7fffffff ? 0x7fffffff : (int)c->queue_cap2;
-    a.root5 = make_riemann_consts(c->p.gamma, c->p.rtol, c->p.rmaxit).root5;
+    a.root = make_riemann_consts(c->p.gamma, c->p.rtol, c->p.rmaxit).root;
     a.dt_max = dt_max;
     a.x = c->x; a.y = c->y; a.z = c->z; a.vx = c->vx; a.vy = c->vy; a.vz = c->vz; a.m = c->m; a.u = c->u;
     a.posf = c->posf;

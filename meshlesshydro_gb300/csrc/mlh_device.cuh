@@ -7,6 +7,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "mlh_intmath.cuh"
+
 namespace mlh {
 
 constexpr unsigned IMG_SHIFT = 29;
@@ -153,7 +155,7 @@ __device__ __forceinline__ double kernel_sigma(double h2) {
 // abs() as bound by the reference's limiter code (fabs, or int abs(int) with
 // x86 conversion semantics: NaN / out of range -> INT_MIN, abs(INT_MIN) = INT_MIN).
 __device__ __forceinline__ double ref_abs(double x, int int_abs) {
-    if (!int_abs) return fabs(x);
+    if (!int_abs) return abs_bits(x);
     if (!(x > -2147483649.0 && x < 2147483648.0)) return -2147483648.0;
     int t = (int)x;
     if (t == (int)0x80000000) return -2147483648.0;
@@ -229,39 +231,11 @@ __device__ __forceinline__ double image_coord(double xa, const GridInfo &g, int 
     return __dadd_rn(low ? g.hi[a] : g.lo[a], __dsub_rn(xa, low ? g.lo[a] : g.hi[a]));
 }
 
-// Reciprocal and reciprocal square root from the hardware estimates of PTX
-// rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64 (relative error e of the estimate
-// a few times 2^-23), each refined by one third-order step:
-//   1/x       = r (1 - e)^-1   = r (1 + e + e^2 + ...),         e = 1 - x r
-//   1/sqrt(x) = y (1 - e)^-1/2 = y (1 + e/2 + 3 e^2/8 + ...),   e = 1 - x y^2
-// whose dropped terms (e^3, 5 e^3 / 16) are below 2^-60: the result is within
-// about an ulp of the correctly rounded one (the probe mlh_probe_fast_math
-// measures it against exact values).  Three and five FP64 operations in a
-// dependent chain of the same length, against four and six for two
-// Newton-Raphson steps: these sit on the Riemann iteration's dependency
-// chain, and the face pass waits on that chain as well as on the pipe.
-// Cheaper on the FP64 pipe than IEEE division, which also guards subnormal,
-// zero and infinite operands: these are for normal, finite, nonzero operands
-// only.
-__device__ __forceinline__ double frcp(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.);
-    return fma(r, fma(e, e, e), r);
-}
-__device__ __forceinline__ double fdiv(double a, double b) { return a * frcp(b); }
-__device__ __forceinline__ double frsqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.);
-    return fma(y, e * fma(0.375, e, 0.5), y);
-}
-
 template <int D>
 __device__ __forceinline__ double dotD(const double *a, const double *b) {
-    double r = 0.;
+    double r = mulr(a[0], b[0]);
 #pragma unroll
-    for (int k = 0; k < D; ++k) r += a[k] * b[k];
+    for (int k = 1; k < D; ++k) r = fma(a[k], b[k], r);
     return r;
 }
 

@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
         geo[bi].V = frcp(bomega);
         const double irho = frcp(rho);   // also the face kernel's 1/rho_i
         geo[bi].irho = irho;
-        const double cs = sqrt(p.gamma * P * irho);
+        const double cs = fsqrt_rn(p.gamma * P * irho);
         geo[bi].c = cs;
         // velocity and sound speed in single precision, for the time step's
         // filter (k_gradients)
@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
                             }
                             pass = __double_as_longlong(d2) < __double_as_longlong(lim);
                             if (pass) {
-                                r = sqrt(d2);
+                                r = fsqrt_rn(d2);
                                 w = kernelW2(r, ih2_i, sigma_i, sigma4_i);
                             }
                         }
@@ -1131,7 +1131,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32) k_hsolve(
                                 double d2 = __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey));
                                 if (D == 3) { double ez = __dsub_rn(xj[2], xi[2]); d2 = __dadd_rn(d2, __dmul_rn(ez, ez)); }
                                 pass = __double_as_longlong(d2) < __double_as_longlong(mb.hsq);   // d2 < H^2, both >= 0
-                                if (pass) r = __dsqrt_rn(d2);
+                                if (pass) r = fsqrt_rn(d2);
                             }
                         }
                         const unsigned bal = __ballot_sync(0xffffffffu, pass);
@@ -1978,13 +1978,13 @@ __device__ __forceinline__ double pairwise_side(double phi0, double phi_i, doubl
     // one division by the Newton-Raphson reciprocal, and only where the
     // shift would change the sign; the same value to a few ulp, also for
     // |phi| = 0 and the int abs binding)
-    const double shifted = fma(i_lt_j ? -psi1 : psi1, ad, phi_i);
+    const double shifted = fma(flip_if(psi1, i_lt_j), ad, phi_i);
     double bound = shifted;
     if ((ord_key(shifted) >= 0) != (ord_key(phi_i) >= 0)) {
         const double ra = ref_abs(phi_i, int_abs);
-        bound = fdiv(phi_i * ra, fma(psi1, ad, ra));
+        bound = mulr(mulr(phi_i, ra), frcp(fma(psi1, ad, ra)));
     }
-    const double t = fma(i_lt_j ? psi2 : -psi2, ad, phi_ij);
+    const double t = fma(flip_if(psi2, !i_lt_j), ad, phi_ij);
     if (i_lt_j) {
         const double minPhiD2 = dlt(t, phi0) ? t : phi0;
         return dlt(minPhiD2, bound) ? bound : minPhiD2;
@@ -2001,19 +2001,24 @@ __device__ __forceinline__ double pairwise_side(double phi0, double phi_i, doubl
 // sides and is computed once; phi_ij on the j side, phi_j + rL (phi_i -
 // phi_j), is fma(rL, d, phi_j) with d = phi_i - phi_j.  Equal particle values
 // (neither phi_i < phi_j nor phi_i > phi_j) give the particle values back.
+template <bool MIDPOINT>
 __device__ __forceinline__ void pairwise_limiter(const Params &p, double &phi0R, double &phi0L, double phiR,
                                                  double phiL, double rR, double rL) {
     const long long kR = ord_key(phiR), kL = ord_key(phiL);
     if (kR == kL) { phi0R = phiR; phi0L = phiL; return; }
     const bool r_lt_l = kR < kL;
-    const double d = phiR - phiL;
+    const double d = subr(phiR, phiL);
     const double ad = ref_abs(d, p.int_abs);
-    phi0R = pairwise_side(phi0R, phiR, fma(rR, -d, phiR), ad, p.psi1, p.psi2, r_lt_l, p.int_abs);
-    phi0L = pairwise_side(phi0L, phiL, fma(rL, d, phiL), ad, p.psi1, p.psi2, !r_lt_l, p.int_abs);
+    // phi_ij on the two sides, phi_R + rR (phi_L - phi_R) and phi_L + rL (phi_R -
+    // phi_L): with rR = rL = 1/2 both are the mean, evaluated once
+    const double fR = fma(rR, -d, phiR);
+    const double fL = MIDPOINT ? fR : fma(rL, d, phiL);
+    phi0R = pairwise_side(phi0R, phiR, fR, ad, p.psi1, p.psi2, r_lt_l, p.int_abs);
+    phi0L = pairwise_side(phi0L, phiL, fL, ad, p.psi1, p.psi2, !r_lt_l, p.int_abs);
 }
 
 // Network inputs of a face, from its face-frame problem sorted as the
-// gamma = 5/3 solver sorts it (riemann5_begin): side A the one with the lower
+// root solver sorts it (riemann_root_begin): side A the one with the lower
 // pressure (particle i on ties), side B the other, the mirror image negating
 // both normal velocities, so that du = uB - uA is the same in both
 // orientations:  log(rhoB/rhoA), du/cA, log(pB/pA) >= 0, log(cB/cA), in single
@@ -2078,7 +2083,7 @@ __device__ __forceinline__ void face_normal(const double *A, const double *R, co
                                             double &unR, double &unL) {
     const double iAN = frsqrt(dotD<D>(A, A));
 #pragma unroll
-    for (int a = 0; a < D; ++a) hatA[a] = iAN * A[a];
+    for (int a = 0; a < D; ++a) hatA[a] = mulr(iAN, A[a]);
     unR = dotD<D>(hatA, R + 2);
     unL = dotD<D>(hatA, L + 2);
 }
@@ -2101,46 +2106,46 @@ __device__ __forceinline__ unsigned project_flux(const RiemannResult &rs, const 
     double vSol[3] = {0., 0., 0.};
     if (rs.flag == 1 || rs.flag == -1) {
         const double *side = rs.flag == 1 ? L : R;
-        const double du = rs.u - (rs.flag == 1 ? unL : unR);
+        const double du = subr(rs.u, rs.flag == 1 ? unL : unR);
 #pragma unroll
         for (int a = 0; a < D; ++a) vSol[a] = fma(du, hatA[a], side[2 + a]);
     } else {
         st = ST_VACUUM;
 #pragma unroll
-        for (int a = 0; a < D; ++a) vSol[a] = rs.u * hatA[a];
+        for (int a = 0; a < D; ++a) vSol[a] = mulr(rs.u, hatA[a]);
     }
     // F_m = rho* (A . v*), F_p = F_m v_lab + P* A,
     // F_E = (A . v*) (P*/(gamma-1) + rho*/2 |v_lab|^2) + P* (A . v_lab);
     // MESHLESS_FINITE_MASS keeps F_m and drops the advective terms
     const double rhoSol = rs.rho, PSol = rs.p;
-    const double pe = PSol * inv_gm1;
+    const double pe = xmul(PSol, inv_gm1);
     const double Av = dotD<D>(A, vSol);
     double vLab[3] = {0., 0., 0.};
 #pragma unroll
-    for (int a = 0; a < D; ++a) vLab[a] = vSol[a] + vf[a];
-    Fo[0] = rhoSol * Av;
+    for (int a = 0; a < D; ++a) vLab[a] = addr(vSol[a], vf[a]);
+    Fo[0] = mulr(rhoSol, Av);
     const double Avm = mfm ? 0. : Av;
-    const double mflux = rhoSol * Avm;
+    const double mflux = mfm ? 0. : Fo[0];
 #pragma unroll
-    for (int a = 0; a < D; ++a) Fo[2 + a] = fma(mflux, vLab[a], PSol * A[a]);
+    for (int a = 0; a < D; ++a) Fo[2 + a] = fma(mflux, vLab[a], mulr(PSol, A[a]));
     if (D == 2) Fo[4] = 0.;
     // pe + rho*/2 |v_lab|^2 as one fused multiply-add
-    Fo[1] = fma(Avm, fma(half_of(rhoSol), dotD<D>(vLab, vLab), pe), PSol * dotD<D>(A, vLab));
+    Fo[1] = fma(Avm, fma(half_of(rhoSol), dotD<D>(vLab, vLab), pe), mulr(PSol, dotD<D>(A, vLab)));
     return st;
 }
 
-// Register caps of the face kernels, per dimension: more warps per SM hide
-// more of the Riemann iteration's dependency latency, fewer registers spill
-// more.  Measured on the face passes: 3D (Sedov 128^3) 168 registers (12
-// warps per SM, a small spill) 21.60 ms, against 21.74 / 21.81 / 22.29 /
-// 21.80 ms at 152 / 144 / 136 / 128; 2D (the 256-member KH ensemble) 128
-// registers (16 warps) 19.34 ms, against 20.95 ms at 168 and 21.6-21.9 ms
-// at 136-152.  Blocks of up to 256 threads.
+// Register caps of the face kernels: with the roots and products on the integer
+// pipe the passes wait on latency at 16 warps per SM.  One pass over the Sedov
+// 128^3 faces at 128 / 104 / 96 / 80 registers (16 / 16 / 20 / 24 warps):
+// 14.3 / 14.2 / 13.9 / 14.2 ms; over those of 64 KH members at 128 / 96 / 80 /
+// 72 (28 warps): 2.96 / 2.87 / 2.83 / 2.85 ms.  The grid is a multiple of the blocks that
+// reside at once (face_blocks): at 96 registers 8 blocks per SM left the
+// second of two rounds 3/5 full, 16.4 ms.
 #ifndef MLH_FACE_MAXREG_3D
-#define MLH_FACE_MAXREG_3D 168
+#define MLH_FACE_MAXREG_3D 96
 #endif
 #ifndef MLH_FACE_MAXREG_2D
-#define MLH_FACE_MAXREG_2D 128
+#define MLH_FACE_MAXREG_2D 80
 #endif
 #define MLH_FACE_BOUNDS __maxnreg__(D == 3 ? MLH_FACE_MAXREG_3D : MLH_FACE_MAXREG_2D)
 // The face-frame Riemann problem of canonical face f (i < j): effective face
@@ -2149,10 +2154,14 @@ __device__ __forceinline__ unsigned project_flux(const RiemannResult &rs, const 
 // reconstructed, optionally pairwise-limited and half-step-predicted states
 // (compRiemannStatesLR, :1488-1733 / 2533-2683, including the vz[i] of
 // :1717,1719); the face normal and the normal velocity components
-// (face_normal).  R (particle i, the left state) and L: [rho, P, v..] with
+// (face_normal).  MID: the first-order quadrature point, the midpoint of x_i and
+// x_j (else x_i + h/4 (x_j - x_i)).  It is a parameter of the kernel, not a test:
+// the other point's few FP64 instructions under a test were issued with their
+// lanes off, which holds the FP64 pipe as long (27 of 260 warp instructions per
+// 32 faces in 3D), and out of line they cost registers.  R (particle i, the left state) and L: [rho, P, v..] with
 // unrotated velocities.  Returns false for a face without its links (the
 // status bit is set).
-template <int D>
+template <int D, bool MID>
 __device__ __forceinline__ bool face_states(const Params &p, const Member *__restrict__ members,
                                             const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
                                             const Prim *__restrict__ prim, const Geo *__restrict__ geo,
@@ -2170,8 +2179,6 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
     const int i = fr.i;
     const int mi = memberOf ? memberOf[i] : 0;
     const double dt = dtp[mi];
-    const double h = members[mi].h;
-    const double hq = p.adaptive_h ? p.hp[i] : h;   // quadrature-point radius
     const size_t si = (size_t)i * p.K + fr.slot;
     const uint32_t e = nbr[si];
     const int j = (int)(e & IDX_MASK);
@@ -2187,39 +2194,40 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
         if (fr.rslot >= 0) {
             const double *ps_j = psi + ((size_t)j * p.K + fr.rslot) * 3;
 #pragma unroll
-            for (int a = 0; a < D; ++a) A[a] = Vi * ps_i[a] - Vj * ps_j[a];
+            for (int a = 0; a < D; ++a) A[a] = fma(Vi, ps_i[a], -mulr(Vj, ps_j[a]));
         } else {
             st_local |= ST_ASYMMETRIC;
 #pragma unroll
-            for (int a = 0; a < D; ++a) A[a] = Vi * ps_i[a];
+            for (int a = 0; a < D; ++a) A[a] = mulr(Vi, ps_i[a]);
         }
     }
     // --- states at the face
     double xijxi[3], xjxi[3], xijxj[3];
+    const double hq = MID ? 0. : p.adaptive_h ? p.hp[i] : members[mi].h;   // quadrature-point radius
 #pragma unroll
     for (int a = 0; a < D; ++a) {
-        xjxi[a] = xj[a] - xi[a];
-        if (p.foqp) {
+        xjxi[a] = subr(xj[a], xi[a]);
+        if (MID) {
             // .5 (x_j - x_i) (on the integer pipe), and .5 (x_i - x_j) is its
             // exact negation
             xijxi[a] = half_of(xjxi[a]);
-            xijxj[a] = -xijxi[a];
+            xijxj[a] = flip_if(xijxi[a], true);
         } else {
-            double xij = xi[a] + hq / 4. * xjxi[a];
-            xijxi[a] = xij - xi[a];
-            xijxj[a] = xij - xj[a];
+            const double xij = fma(hq / 4., xjxi[a], xi[a]);
+            xijxi[a] = subr(xij, xi[a]);
+            xijxj[a] = subr(xij, xj[a]);
         }
     }
     const double vi[3] = {pi.vx, pi.vy, pi.vz}, vj[3] = {pj.vx, pj.vy, pj.vz};
     if (p.move) {
-        if (p.foqp) {
+        if (MID) {
 #pragma unroll
-            for (int a = 0; a < D; ++a) vf[a] = half_of(vi[a] + vj[a]);
+            for (int a = 0; a < D; ++a) vf[a] = half_of(addr(vi[a], vj[a]));
         } else {
-            double dotProd = dotD<D>(xijxi, xjxi);
-            double dSqr = dotD<D>(xjxi, xjxi);
+            const double dotProd = dotD<D>(xijxi, xjxi);
+            const double dSqr = dotD<D>(xjxi, xjxi);
 #pragma unroll
-            for (int a = 0; a < D; ++a) vf[a] = vi[a] + (vj[a] - vi[a]) * dotProd / dSqr;
+            for (int a = 0; a < D; ++a) vf[a] = addr(vi[a], mulr(subr(vj[a], vi[a]), dotProd) / dSqr);
         }
     }
     const double *Gi = grad[i].g, *Gj = grad[j].g;
@@ -2227,16 +2235,16 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
     R[0] = pi.rho; L[0] = pj.rho;
     R[1] = pi.P; L[1] = pj.P;
 #pragma unroll
-    for (int a = 0; a < D; ++a) { R[2 + a] = vi[a] - vf[a]; L[2 + a] = vj[a] - vf[a]; }
+    for (int a = 0; a < D; ++a) { R[2 + a] = subr(vi[a], vf[a]); L[2 + a] = subr(vj[a], vf[a]); }
     // W -= dt/2 (source + (v - v_frame) . grad W): the particle part,
     // source + v . grad W, comes with the gradients (Grad::t); the face adds
     // v_frame . grad W.  The reference uses vz[i] on the j side of the vx and
     // vy terms in 3D (Particles.cpp:1717,1719): (vz_i - vf_z) = (vz_j - vq_z)
     // with the shifted frame velocity vq_z = vf_z - (vz_i - vz_j).
-    const double hdt = half_of(dt);
+    const double hdt = half_of(dt), nhdt = flip_if(hdt, true);
     const double *Ti = grad[i].t, *Tj = grad[j].t;
     const int blk[5] = {0, 12, 3, 6, 9};   // gradient blocks: 0 rho, 3 vx, 6 vy, 9 vz, 12 P
-    const double vq2 = D == 3 ? vf[2] - (vi[2] - vj[2]) : 0.;
+    const double vq2 = D == 3 ? subr(vf[2], subr(vi[2], vj[2])) : 0.;
     if (D == 2 && !p.pairwise) {
         // no limiter between reconstruction and prediction: one FMA chain per
         // field and side, W - dt/2 T + grad W . (x_ij - x_side + dt/2 v_frame)
@@ -2252,9 +2260,9 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
         }
 #pragma unroll
         for (int f = 0; f < NV; ++f) {
-            R[f] = fma_dotD<D>(Gi + blk[f], yi, fma(-hdt, Ti[f], R[f]));
+            R[f] = fma_dotD<D>(Gi + blk[f], yi, fma(nhdt, Ti[f], R[f]));
             const double *yy = (D == 3 && (f == 2 || f == 3)) ? yq : yj;
-            L[f] = fma_dotD<D>(Gj + blk[f], yy, fma(-hdt, Tj[f], L[f]));
+            L[f] = fma_dotD<D>(Gj + blk[f], yy, fma(nhdt, Tj[f], L[f]));
         }
     } else {
         double Rb[5], Lb[5];
@@ -2269,32 +2277,31 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
         if (p.pairwise && (!img || p.img_pw)) {   // image faces skip it (Particles.cpp:2533-2683)
             // |x_ij - x_i| / |x_j - x_i| and |x_ij - x_j| / |x_j - x_i|: with the
             // first-order quadrature point x_ij - x_i = (x_j - x_i) / 2 exactly,
-            // so both norms are exactly half of |x_j - x_i| (scaling by 1/2 and
-            // 1/4 is exact) and both quotients are exactly 0.5
+            // so both quotients are exactly 0.5
             double ri = .5, rj = .5;
-            if (!p.foqp) {
+            if (!MID) {
                 double xijxi_abs = 0., xijxj_abs = 0., xjxi_abs = 0.;
 #pragma unroll
                 for (int a = 0; a < D; ++a) {
-                    xijxi_abs += xijxi[a] * xijxi[a];
-                    xijxj_abs += xijxj[a] * xijxj[a];
-                    xjxi_abs += xjxi[a] * xjxi[a];
+                    xijxi_abs = fma(xijxi[a], xijxi[a], xijxi_abs);
+                    xijxj_abs = fma(xijxj[a], xijxj[a], xijxj_abs);
+                    xjxi_abs = fma(xjxi[a], xjxi[a], xjxi_abs);
                 }
                 xjxi_abs = sqrt(xjxi_abs);
                 ri = sqrt(xijxi_abs) / xjxi_abs;
                 rj = sqrt(xijxj_abs) / xjxi_abs;
             }
 #pragma unroll
-            for (int k = 0; k < NV; ++k) pairwise_limiter(p, R[k], L[k], Rb[k], Lb[k], ri, rj);
+            for (int k = 0; k < NV; ++k) pairwise_limiter<MID>(p, R[k], L[k], Rb[k], Lb[k], ri, rj);
         }
         // the prediction, one FMA chain per field and side from the limited value
-        const double nvf[3] = {-vf[0], -vf[1], -vf[2]};
-        const double nvq[3] = {-vf[0], -vf[1], -vq2};
+        const double nvf[3] = {flip_if(vf[0], true), flip_if(vf[1], true), flip_if(vf[2], true)};
+        const double nvq[3] = {nvf[0], nvf[1], flip_if(vq2, true)};
 #pragma unroll
         for (int f = 0; f < NV; ++f) {
-            R[f] = fma(-hdt, fma_dotD<D>(nvf, Gi + blk[f], Ti[f]), R[f]);
+            R[f] = fma(nhdt, fma_dotD<D>(nvf, Gi + blk[f], Ti[f]), R[f]);
             const double *nj = (D == 3 && (f == 2 || f == 3)) ? nvq : nvf;
-            L[f] = fma(-hdt, fma_dotD<D>(nj, Gj + blk[f], Tj[f]), L[f]);
+            L[f] = fma(nhdt, fma_dotD<D>(nj, Gj + blk[f], Tj[f]), L[f]);
         }
     }
     if (dneg(R[1]) || dneg(L[1])) st_local |= ST_NEG_PRESSURE;
@@ -2303,8 +2310,8 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
     return true;
 }
 
-template <int D, bool ROOT5, int MODE>
-__global__ void MLH_FACE_BOUNDS k_faces(Params p, const Member *__restrict__ members,
+template <int D, int ROOT, int MODE, bool MID>
+__global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member *__restrict__ members,
                                                const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
                                                const Prim *__restrict__ prim, const Geo *__restrict__ geo,
                                                const Grad *__restrict__ grad, const uint32_t *__restrict__ nbr,
@@ -2320,7 +2327,6 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, const Member *__restrict__ mem
         const int qn = *qa.count < qa.cap ? *qa.count : qa.cap;
         nf = qn < nf ? qn : nf;
     }
-    const RiemannConsts rc = make_riemann_consts(p.gamma, p.rtol, p.rmaxit);
     const double gamma = p.gamma;
     unsigned long long iters_local = 0, fallback_local = 0, deferred_local = 0;
     unsigned st_local = 0;
@@ -2340,7 +2346,7 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, const Member *__restrict__ mem
             unR = dotD<D>(hatA, R + 2);
             unL = dotD<D>(hatA, L + 2);
         } else {
-        if (!face_states<D>(p, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, f, st_local, R, L, A,
+        if (!face_states<D, MID>(p, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, f, st_local, R, L, A,
                             vf, hatA, unR, unL))
             continue;
         }   // !QUEUED
@@ -2353,7 +2359,7 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, const Member *__restrict__ mem
         if (MODE == 4) guess = ptr_q;
         // MODE 1 defers faces whose two-rarefaction guess says strong shock
         const double defer = MODE == 1 ? PSTAR_HARD * (dlt(L[1], R[1]) ? L[1] : R[1]) : 0.;   // min on the keys
-        RiemannResult rs = ROOT5 ? riemann_exact5(rc, R[0], unR, R[1], L[0], unL, L[1], guess, defer,
+        RiemannResult rs = ROOT ? riemann_exact_root<ROOT ? ROOT : 5>(rc, R[0], unR, R[1], L[0], unL, L[1], guess, defer,
                                                   (MODE == 3 || (MODE == 1 && p.face_split)) ? 1 : 0)
                                  : riemann_exact(rc, R[0], unR, R[1], L[0], unL, L[1], guess, defer);
         // deferred faces: strong shocks of MODE 1 (unsolved, iters 0) go to
@@ -2377,12 +2383,12 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, const Member *__restrict__ mem
             }
             // queue full: finish here, from the iterate or from p_TR
             const int done = rs.iters;
-            rs = ROOT5 ? riemann_exact5(rc, R[0], unR, R[1], L[0], unL, L[1], strong ? -1. : rs.pstar, 0.)
+            rs = ROOT ? riemann_exact_root<ROOT ? ROOT : 5>(rc, R[0], unR, R[1], L[0], unL, L[1], strong ? -1. : rs.pstar, 0.)
                        : riemann_exact(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.);
             if (rs.iters >= 0) rs.iters += done;
         }
         if (MODE == 0 && hv.stride > 0 && (hv.strong || f % hv.stride == 0)) {
-            const double ptr = two_rarefaction_guess<ROOT5>(rc, R[0], unR, R[1], L[0], unL, L[1]);
+            const double ptr = two_rarefaction_guess<ROOT>(rc, R[0], unR, R[1], L[0], unL, L[1]);
             if (rs.iters >= 0 && rs.pstar > 0. && ptr > 0.) {
                 if (hv.strong) {
                     // the faces the learned step hands to the network
@@ -2445,7 +2451,7 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, const Member *__restrict__ mem
 // the block's round sets up its problem and takes the first Newton step
 // from p_TR, and leaves its solver state (sorted sides, iterate) in shared
 // memory; the block's unfinished faces are listed and continued, densely, by
-// its first threads (the iteration riemann_exact5 runs from the iterate as a
+// its first threads (the iteration riemann_exact_root runs from the iterate as a
 // guess, on the stored sides: the same arithmetic as the two-pass split);
 // then every face samples its solution and projects its flux, with all
 // lanes busy.  The loop runs in block-wide rounds so that every thread
@@ -2465,7 +2471,7 @@ constexpr int FB_T = 128;   // threads per block of k_faces_block
 // warp runs the MMAs (rows beyond ns are zero inputs whose outputs are
 // dropped).  Out of line, so that the rare branch that calls it does not shape
 // the register allocation of the face pass.
-__device__ __noinline__ void block_network_guess(const PackedMlp *__restrict__ w, Solve5 *sv, const int *slist,
+__device__ __noinline__ void block_network_guess(const PackedMlp *__restrict__ w, RootSolve *sv, const int *slist,
                                                  int ns, float gamma) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int base = warp * 16; base < ns; base += FB_T / 2) {
@@ -2473,19 +2479,19 @@ __device__ __noinline__ void block_network_guess(const PackedMlp *__restrict__ w
         const bool mine = lane < 16 && row < ns;
         float4 xi = make_float4(0.f, 0.f, 0.f, 0.f);
         if (mine) {
-            const Solve5 &q = sv[slist[row]];
+            const RootSolve &q = sv[slist[row]];
             xi = pstar_features_sorted(q.A.rho, q.A.p, q.B.rho, q.B.p, q.du, gamma);
         }
         const float y = mlp_rows<1>(w, xi);
         if (mine && isfinite(y) && fabsf(y) > PSTAR_GATE && fabsf(y) < 30.f) {
-            Solve5 &q = sv[slist[row]];
+            RootSolve &q = sv[slist[row]];
             q.p = q.p * (double)__expf(y);
         }
     }
 }
 
-template <int D, bool LEARNED>
-__global__ void MLH_FACE_BOUNDS k_faces_block(Params p, const Member *__restrict__ members,
+template <int D, int ROOT, bool LEARNED>
+__global__ void MLH_FACE_BOUNDS k_faces_block(Params p, RiemannConsts rc, const Member *__restrict__ members,
                                               const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
                                               const Prim *__restrict__ prim, const Geo *__restrict__ geo,
                                               const Grad *__restrict__ grad, const uint32_t *__restrict__ nbr,
@@ -2493,12 +2499,11 @@ __global__ void MLH_FACE_BOUNDS k_faces_block(Params p, const Member *__restrict
                                               const FaceRef *__restrict__ faces, const double *__restrict__ dtp,
                                               double *__restrict__ Fface, unsigned long long *__restrict__ newtonSum,
                                               unsigned *__restrict__ status, const PackedMlp *__restrict__ mlp) {
-    __shared__ Solve5 sv[FB_T];
+    __shared__ RootSolve sv[FB_T];
     __shared__ int todo[FB_T];
     __shared__ int slist[LEARNED ? FB_T : 1];
     __shared__ int wcount[FB_T / 32];
     const int nf = *faceTotal < p.faces_cap ? *faceTotal : p.faces_cap;
-    const RiemannConsts rc = make_riemann_consts(p.gamma, p.rtol, p.rmaxit);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long iters_local = 0, fallback_local = 0, learned_local = 0;
     unsigned st_local = 0;
@@ -2508,14 +2513,14 @@ __global__ void MLH_FACE_BOUNDS k_faces_block(Params p, const Member *__restrict
         double unR = 0., unL = 0.;
         bool valid = f < nf;
         if (valid)
-            valid = face_states<D>(p, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, f, st_local, R,
+            valid = face_states<D, true>(p, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, f, st_local, R,
                                    L, A, vf, hatA, unR, unL);
         bool unfinished = false, strong = false;
         if (valid) {
             // strong shocks of the learned step stop before their first
             // Newton step: p_TR > PSTAR_HARD min(pL, pR) (min on the keys)
             const double defer = LEARNED ? PSTAR_HARD * (dlt(L[1], R[1]) ? L[1] : R[1]) : 0.;
-            const Solve5 s0 = riemann5_begin(rc, R[0], unR, R[1], L[0], unL, L[1], -1., defer, 1);
+            const RootSolve s0 = riemann_root_begin<ROOT>(rc, R[0], unR, R[1], L[0], unL, L[1], -1., defer, 1);
             sv[threadIdx.x] = s0;
             unfinished = s0.stage == 2;
             strong = LEARNED && s0.stage == 3;
@@ -2545,9 +2550,9 @@ __global__ void MLH_FACE_BOUNDS k_faces_block(Params p, const Member *__restrict
         // --- continue them on the first nu threads
         if ((int)threadIdx.x < nu) {
             const int slot = todo[threadIdx.x];
-            Solve5 c = sv[slot];
+            RootSolve c = sv[slot];
             const bool from_net = LEARNED && c.stage == 3;
-            riemann5_continue(rc, c);
+            riemann_root_continue<ROOT>(rc, c);
             if (from_net) {
                 ++learned_local;
                 if (c.iters > rc.max_iter) ++fallback_local;
@@ -2557,12 +2562,12 @@ __global__ void MLH_FACE_BOUNDS k_faces_block(Params p, const Member *__restrict
         __syncthreads();
         // --- sample and project, every face of the round
         if (valid) {
-            const Solve5 s = sv[threadIdx.x];
+            const RootSolve s = sv[threadIdx.x];
             RiemannResult rs;
             if (s.stage == 0) {
                 rs.rho = 0.; rs.u = 0.; rs.p = 0.; rs.pstar = 0.; rs.flag = 0; rs.iters = 0;
             } else {
-                rs = riemann5_finish(rc, s);
+                rs = riemann_root_finish<ROOT>(rc, s);
             }
             if (unfinished) iters_local += 1;   // the first step, counted as the two-pass split counts it
             if (rs.iters < 0) st_local |= ST_NEWTON;
@@ -2599,7 +2604,7 @@ __global__ void MLH_FACE_BOUNDS k_faces_block(Params p, const Member *__restrict
 // velocity and A_ij; one thread per face, the same device functions as
 // k_faces.  F: [mass, energy, momentum] per face; iters: Newton iterations
 // (-1 when the iteration did not converge).
-template <int D, bool ROOT5>
+template <int D, int ROOT>
 __global__ void __launch_bounds__(256) k_riemann_batch(int n, RiemannConsts rc, int mfm,
                                                        const double *__restrict__ Wi, const double *__restrict__ Wj,
                                                        const double *__restrict__ vFrame,
@@ -2616,7 +2621,7 @@ __global__ void __launch_bounds__(256) k_riemann_batch(int n, RiemannConsts rc, 
         for (int a = 0; a < D; ++a) { A[a] = Aij[(size_t)f * D + a]; vf[a] = vFrame[(size_t)f * D + a]; }
         if (R[1] < 0. || L[1] < 0.) st |= ST_NEG_PRESSURE;
         face_normal<D>(A, R, L, hatA, unR, unL);
-        const RiemannResult rs = ROOT5 ? riemann_exact5(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.)
+        const RiemannResult rs = ROOT ? riemann_exact_root<ROOT ? ROOT : 5>(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.)
                                        : riemann_exact(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.);
         if (rs.iters < 0) st |= ST_NEWTON;
         double Fo[5];
@@ -2634,8 +2639,8 @@ void riemann_batch(int dim, int n, double gamma, double rtol, int max_iter, int 
     const RiemannConsts rc = make_riemann_consts(gamma, rtol, max_iter);
     const int blocks = n > 0 ? (n + 255) / 256 : 1;
 #define MLH_RB(DD, R5) k_riemann_batch<DD, R5><<<blocks, 256, 0, s>>>(n, rc, mfm, Wi, Wj, vFrame, Aij, F, iters, status)
-    if (dim == 2) { if (rc.root5) MLH_RB(2, true); else MLH_RB(2, false); }
-    else { if (rc.root5) MLH_RB(3, true); else MLH_RB(3, false); }
+    if (dim == 2) { if (rc.root) MLH_RB(2, 5); else MLH_RB(2, 0); }
+    else { if (rc.root) MLH_RB(3, 5); else MLH_RB(3, 0); }
 #undef MLH_RB
 }
 
@@ -2826,6 +2831,19 @@ void launch_hsolve(StepArgs &a) {
                                                      a.cellStart, a.cellList, a.hp, a.hpf, a.neff, a.hstat, a.status);
 }
 
+// Blocks of a face pass: the tuned number per SM, raised to a multiple of the
+// blocks that an SM holds at once (the register cap's threads), and no more
+// than the faces that the table can hold need.
+int face_blocks(int dim, int threads, const StepArgs &a) {
+    const int cap = dim == 3 ? MLH_FACE_MAXREG_3D : MLH_FACE_MAXREG_2D;
+    int resident = 65536 / cap / threads;
+    if (resident < 1) resident = 1;
+    const int per_sm = (a.tune.face_blocks_per_sm + resident - 1) / resident * resident;
+    const size_t most = (a.faces_cap + threads - 1) / threads;
+    const size_t want = (size_t)a.sm_count * per_sm;
+    return (int)(want < most ? want : most);
+}
+
 template <int D>
 void launch_step(StepArgs &a) {
     const Params &p = a.p;
@@ -2924,45 +2942,55 @@ void launch_step(StepArgs &a) {
     }
 
     tick(KT_FACES);
-    const int fT = a.tune.face_threads, fB = a.sm_count * a.tune.face_blocks_per_sm;
+    const int fT = a.tune.face_threads, fB = face_blocks(D, fT, a), fBb = face_blocks(D, FB_T, a);
     Params pf = p;   // the face passes see the tuned split
-    pf.face_split = a.tune.face_split;
+    const RiemannConsts rc = make_riemann_consts(p.gamma, p.rtol, p.rmaxit);
     const FaceQueue qa{a.fstate, a.queueFace, a.queueCount, a.qcap};
     const FaceQueue qb{a.fstate2, a.queueFace2, a.queueCount2, a.qcap2};
-#define MLH_FACES(R5, MODE, QA, QB)                                                                              \
-    k_faces<D, R5, MODE><<<fB, fT, 0, s>>>(pf, a.members, a.memberOf, a.grids, a.prim, a.geo, a.grad, a.nbr, a.psi, \
-                                           a.faceOff + p.n, a.faces, a.dt, a.Fface, a.newtonSum, a.status, QA,   \
-                                           QB, a.feat, a.yguess, a.harvest)
+#define MLH_FACES(ROOT, MODE, MID, QA, QB)                                                                        \
+    k_faces<D, ROOT, MODE, MID><<<fB, fT, 0, s>>>(pf, rc, a.members, a.memberOf, a.grids, a.prim, a.geo, a.grad,  \
+                                                  a.nbr, a.psi, a.faceOff + p.n, a.faces, a.dt, a.Fface,          \
+                                                  a.newtonSum, a.status, QA, QB, a.feat, a.yguess, a.harvest)
+#define MLH_FACES_MID(ROOT, MODE, QA, QB)                     \
+    do {                                                      \
+        if (p.foqp) MLH_FACES(ROOT, MODE, true, QA, QB);      \
+        else MLH_FACES(ROOT, MODE, false, QA, QB);            \
+    } while (0)
+    // the structures that regroup unfinished faces (face_split 1, 2) are built
+    // for the midpoint quadrature point; with the other one a step runs the one
+    // pass (the same bits)
+    const int split = p.foqp ? a.tune.face_split : 0;
+    pf.face_split = split;
     if (a.learned) {
         // strong shocks: network guess (queue A); the rest as the plain step
         cudaMemsetAsync(a.queueCount, 0, sizeof(int), s);
         if (a.queueCount2) cudaMemsetAsync(a.queueCount2, 0, sizeof(int), s);
-        if (a.root5 && a.tune.face_split == 2) {
+        if (a.root && split == 2) {
             // unfinished faces continued inside the block, strong shocks from
             // the network's guess evaluated there
-            k_faces_block<D, true><<<fB, FB_T, 0, s>>>(pf, a.members, a.memberOf, a.grids, a.prim, a.geo, a.grad,
+            k_faces_block<D, 5, true><<<fBb, FB_T, 0, s>>>(pf, rc, a.members, a.memberOf, a.grids, a.prim, a.geo, a.grad,
                                                        a.nbr, a.psi, a.faceOff + p.n, a.faces, a.dt, a.Fface,
                                                        a.newtonSum, a.status, (const PackedMlp *)a.mlp_packed);
         } else {
-            if (a.root5) MLH_FACES(true, 1, qa, qb);
-            else MLH_FACES(false, 1, qa, qb);
+            if (a.root) MLH_FACES_MID(5, 1, qa, qb); else MLH_FACES_MID(0, 1, qa, qb);
             pstar_infer_dev(a.feat, a.queueCount, (int)a.faces_cap, a.mlp_packed, a.yguess, a.sm_count, s);
-            if (a.root5) MLH_FACES(true, 2, qa, qb); else MLH_FACES(false, 2, qa, qb);
-            if (a.root5 && a.fstate2 && a.tune.face_split == 1) MLH_FACES(true, 4, qb, qb);
+            if (a.root) MLH_FACES(5, 2, true, qa, qb); else MLH_FACES(0, 2, true, qa, qb);
+            if (a.root && a.fstate2 && split == 1) MLH_FACES(5, 4, true, qb, qb);
         }
-    } else if (a.root5 && a.harvest.stride == 0 && a.tune.face_split == 2) {
+    } else if (a.root && a.harvest.stride == 0 && split == 2) {
         // unconverged faces after one Newton step continued inside the block
-        k_faces_block<D, false><<<fB, FB_T, 0, s>>>(pf, a.members, a.memberOf, a.grids, a.prim, a.geo, a.grad, a.nbr,
+        k_faces_block<D, 5, false><<<fBb, FB_T, 0, s>>>(pf, rc, a.members, a.memberOf, a.grids, a.prim, a.geo, a.grad, a.nbr,
                                                     a.psi, a.faceOff + p.n, a.faces, a.dt, a.Fface, a.newtonSum,
                                                     a.status, nullptr);
-    } else if (a.root5 && a.fstate && a.harvest.stride == 0 && a.tune.face_split) {
+    } else if (a.root && a.fstate && a.harvest.stride == 0 && split) {
         // unconverged faces after one Newton step go to a second, dense pass
         cudaMemsetAsync(a.queueCount, 0, sizeof(int), s);
-        MLH_FACES(true, 3, qa, qb);
-        MLH_FACES(true, 4, qa, qb);
+        MLH_FACES(5, 3, true, qa, qb);
+        MLH_FACES(5, 4, true, qa, qb);
     } else {
-        if (a.root5) MLH_FACES(true, 0, qa, qb); else MLH_FACES(false, 0, qa, qb);
+        if (a.root) MLH_FACES_MID(5, 0, qa, qb); else MLH_FACES_MID(0, 0, qa, qb);
     }
+#undef MLH_FACES_MID
 #undef MLH_FACES
     tock(KT_FACES);
 

@@ -12,10 +12,10 @@ enum KernelTimerId { KT_GRID = 0, KT_NNS, KT_DT, KT_GRAD, KT_LINK, KT_FACES, KT_
 // Launch shapes chosen by the autotuner (mlh_autotune).
 struct Tuning {
     int face_threads = 128;        // threads per block of k_faces
-    int face_blocks_per_sm = 8;    // grid of the grid-stride face loop
+    int face_blocks_per_sm = 32;   // grid of the grid-stride face loop (32 against 8: -0.5 % on Sedov 128^3, -9 % on 16 blasts in 48^3, whose shocks fill a few blocks)
     int grad_threads = 128;        // threads per block of k_gradients
     int nns_warps_per_sm = 64;     // warps (= particles in flight) of k_neighbours
-    int face_split = 1;            // plain gamma = 5/3 step: 1 second Newton pass over a queue, 2 in-block, 0 none
+    int face_split = 0;            // plain root-solver step: 1 second Newton pass over a queue, 2 in-block, 0 none
     int link_overlap = 1;          // face links on the second stream beside the time step and gradients
     int persistent_binning = 0;    // the binning as one persistent cooperative kernel (k_binning)
     int fp32_filters = 3;          // bits: 1 slope-limiter extrema, 2 time step (FP64 only where a single-precision bound reaches the result)
@@ -36,7 +36,7 @@ struct StepArgs {
     cudaEvent_t ev_fork, ev_join;
     int face_blocks;
     int sm_count;
-    int root5;              // gamma = 5/3 fast path of the Riemann solver
+    int root;               // RiemannConsts::root: 5 runs the root solver, 0 the general one
     size_t faces_cap;
     double dt_max;
     // state (structure of arrays)

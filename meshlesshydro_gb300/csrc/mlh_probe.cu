@@ -104,6 +104,16 @@ __global__ void k_fast_math(int n, const double *__restrict__ x, const double *_
     }
 }
 
+__global__ void k_int_math(int n, const double *__restrict__ x, const double *__restrict__ y,
+                           double *__restrict__ o) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double a = x[i], b = y[i];
+        const double v[9] = {mlh::xmul(a, b), mlh::mulr(a, b), mlh::addr(a, b), mlh::subr(a, b), mlh::fsqrt_rn(a),
+                             mlh::root<5>(a), mlh::rroot<5>(a), mlh::root<7>(a), mlh::rroot<7>(a)};
+        for (int k = 0; k < 9; ++k) o[(size_t)k * n + i] = v[k];
+    }
+}
+
 __global__ void k_scale2(int n, const double *__restrict__ x, double *__restrict__ half, double *__restrict__ quarter,
                          double *__restrict__ twice) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -135,8 +145,27 @@ extern "C" int mlh_probe_scale2(int n, const double *x, double *half, double *qu
     return e == cudaSuccess ? 0 : MLH_ERR_CUDA;
 }
 
+// The products, sums and roots of mlh_intmath.cuh of host values (9 arrays of n
+// in out), for checking them against IEEE operations and exact roots.
+extern "C" int mlh_probe_int_math(int n, const double *x, const double *y, double *out) {
+    if (n < 0 || (n > 0 && (!x || !y || !out))) return MLH_ERR_INVALID;
+    if (n == 0) return 0;
+    double *d = nullptr;
+    if (cudaMalloc(&d, sizeof(double) * 11 * (size_t)n) != cudaSuccess) return MLH_ERR_CUDA;
+    const size_t b = sizeof(double) * (size_t)n;
+    cudaError_t e = cudaMemcpy(d, x, b, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + n, y, b, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_int_math<<<(n + 255) / 256, 256>>>(n, d, d + n, d + 2 * (size_t)n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 9 * b, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? 0 : MLH_ERR_CUDA;
+}
+
 // The library's reciprocal, quotient and reciprocal square root
-// (mlh_device.cuh: frcp, fdiv, frsqrt) of host arrays, for checking them
+// (mlh_intmath.cuh: frcp, fdiv, frsqrt) of host arrays, for checking them
 // against exact values: rcp = 1/x, quot = y/x, rsqrt = 1/sqrt(x).
 extern "C" int mlh_probe_fast_math(int n, const double *x, const double *y, double *rcp, double *quot,
                                    double *rsqrt) {

@@ -16,10 +16,13 @@ struct RiemannConsts {
     double gamma, g1, g2, g3, g4, g5, g6, g7, inv_gamma, inv_gm1, tol;
     double tol_half;   // tol / 2 (exact): 2 |dp| <= tol s  <=>  |dp| <= (tol / 2) s
     double ig5;   // 1 / g5 = (gamma + 1) / 2
+    double g6ig5; // g6 ig5 = (gamma - 1) / 2
     int max_iter;
-    // gamma = 5/3: g1 = 1/5, g3 = 5, g4 = 3 and 1/gamma = 3 g1, so every
-    // power in the solver is a fifth root or an integer power
-    int root5;
+    // 2 gamma / (gamma - 1) where it is 5 (gamma = 5/3) or 7 (gamma = 7/5), else
+    // 0.  With N = 2 gamma / (gamma - 1): g1 = 1/N, g3 = N, g4 = N - 2 and
+    // 1/gamma = (N - 2) g1, so every power in the solver is an N-th root or an
+    // integer power
+    int root;
 };
 
 __host__ __device__ inline RiemannConsts make_riemann_consts(double gamma, double tol, int max_iter) {
@@ -31,6 +34,7 @@ __host__ __device__ inline RiemannConsts make_riemann_consts(double gamma, doubl
     c.g4 = 2. / (gamma - 1.);
     c.g5 = 2. / (gamma + 1.);
     c.ig5 = (gamma + 1.) / 2.;
+    c.g6ig5 = (gamma - 1.) / 2.;
     c.g6 = (gamma - 1.) / (gamma + 1.);
     c.g7 = (gamma - 1.) / 2.;
     c.inv_gamma = 1. / gamma;
@@ -38,7 +42,9 @@ __host__ __device__ inline RiemannConsts make_riemann_consts(double gamma, doubl
     c.tol = tol;
     c.tol_half = tol / 2.;
     c.max_iter = max_iter;
-    c.root5 = (fabs(1. / c.g1 - 5.) < 1e-12 && fabs(c.g4 - 3.) < 1e-12) ? 1 : 0;
+    c.root = 0;
+    for (int n = 5; n <= 5; n += 2)
+        if (fabs(1. / c.g1 - n) < 1e-12 && fabs(c.g4 - (n - 2)) < 1e-12) c.root = n;
     return c;
 }
 
@@ -179,108 +185,91 @@ __device__ inline RiemannResult riemann_exact(const RiemannConsts &c, double rho
 // are ordered as the values.
 __device__ __forceinline__ bool nn_le(double a, double b) { return __double_as_longlong(a) <= __double_as_longlong(b); }
 
-// x^(-1/5) to a few ulp: a single-precision seed y (relative error e below
-// 3e-7) refined by one third-order step.  With r = 1 - x y^5,
-// x^(-1/5) = y (1 - r)^(-1/5) = y (1 + r/5 + 3 r^2/25 + O(r^3)), and
-// |r| ~ 5 e, so dropping the O(r^3) term (0.088 r^3 < 1e-18) leaves the
-// roundings of y^5, r and the last two operations: within a few ulp of the
-// correctly rounded value, in seven FP64 operations (two Newton steps, whose
-// error contracts as 3 e^2, took twelve).  Values outside the float range go
-// through pow.
-__device__ __forceinline__ double rroot5(double x) {
-    // 1e-30 < x < 1e30 on the bit patterns (the test is false for NaN and x <= 0)
-    const long long b = __double_as_longlong(x);
-    if (!(b > 0x39B4484BFEEBC2A0ll && b < 0x46293E5939A08CEAll)) return pow(x, -0.2);
-    // double -> float and back on the bit patterns (integer pipe): rebias the
-    // exponent (1023 - 127 = 896) and keep the top 23 mantissa bits; x and
-    // the seed are positive and normal in both formats in this range
-    const float xf = __int_as_float((int)((b >> 29) - (896ll << 23)));
-    const float yf = exp2f(-0.2f * __log2f(xf));
-    const double y = __longlong_as_double(((long long)__float_as_int(yf) + (896ll << 23)) << 29);
-    const double y2 = y * y;
-    const double r = fma(-x, y2 * y2 * y, 1.);
-    return fma(y, r * fma(0.12, r, 0.2), y);
-}
-// x^(1/5) = x * (x^(-1/5))^4
-__device__ __forceinline__ double root5(double x) {
-    double y = rroot5(x);
-    double y2 = y * y;
-    return x * (y2 * y2);
+// The multiplies, adds and fused multiply-adds of the fast path are written
+// out (mulr, addr, subr, fma): left to the compiler, their fusing would depend
+// on the basic blocks around them and so on the kernel that inlines the
+// solver, whose variants have to give the same bits.
+
+// x^N and x^(N-2) for N = 5, 7
+template <int N>
+__device__ __forceinline__ double pow_n(double x, double &xm2) {
+    const double x2 = mulr(x, x), x3 = mulr(x2, x), x5 = mulr(x3, x2);
+    if (N == 5) { xm2 = x3; return x5; }
+    xm2 = x5;
+    return mulr(x5, x2);
 }
 
 // Two-rarefaction estimate of p* (Toro eq. 4.46), the default starting point
-// of both solvers; ROOT5 takes the gamma = 5/3 powers.  Not positive when the
-// states generate vacuum.
-template <bool ROOT5>
+// of both solvers; ROOT takes the roots of its gamma (0: any gamma).  Not
+// positive when the states generate vacuum.
+template <int ROOT>
 __device__ __forceinline__ double two_rarefaction_guess(const RiemannConsts &k, double rhoL, double uL, double pL,
                                                         double rhoR, double uR, double pR) {
     const double cL = sqrt(k.gamma * pL / rhoL), cR = sqrt(k.gamma * pR / rhoR);
     const double num = cL + cR - k.g7 * (uR - uL);
     if (!(num > 0.)) return -1.;
-    if (ROOT5) {
-        const double t = fdiv(num, cL * rroot5(pL) + cR * rroot5(pR));
-        const double t2 = t * t;
-        return t2 * t2 * t;
+    if (ROOT) {
+        constexpr int N = ROOT ? ROOT : 5;
+        const double t = fdiv(num, cL * rroot<N>(pL) + cR * rroot<N>(pR));
+        double tm2;
+        return pow_n<N>(t, tm2);
     }
     return pow(num / (cL / pow(pL, k.g1) + cR / pow(pR, k.g1)), k.g3);
 }
 
+// A side of the problem: a = 1 / A_K = rho / g5, b = B_K a (so that
+// (B_K + p) / A_K = a p + b), C = c / gamma, g4c = g4 c.
 struct RiemannSide {
-    double rho, u, p, c, invp, C, iak, bk, g4c;   // iak = 1 / A_K = rho / g5
+    double rho, u, p, c, invp, C, a, b, g4c;
 };
 
 __device__ __forceinline__ RiemannSide make_side(const RiemannConsts &k, double rho, double u, double p) {
     RiemannSide s;
     s.rho = rho; s.u = u; s.p = p;
-    // one reciprocal square root for c and 1/p: with g = gamma p and
-    // y = 1/sqrt(g rho), c = sqrt(g / rho) = g y and 1/p = gamma rho y^2
-    // (each within a few ulp)
-    const double gp = k.gamma * p;
-    const double y = frsqrt(gp * rho);
-    s.c = gp * y;
-    s.invp = (k.gamma * rho) * (y * y);
-    s.C = s.c * k.inv_gamma;     // pK / (rhoK cK) = cK / gamma: f' = (p/pK)^g1 C / p
-    s.iak = rho * k.ig5;
-    s.bk = k.g6 * p;
-    s.g4c = k.g4 * s.c;
+    const double rp = xmul(rho, p);
+    // c = sqrt(gamma p / rho) = gamma p / sqrt(gamma p rho)
+    s.c = xmul(xmul(k.gamma, p), frsqrt(xmul(k.gamma, rp)));
+    s.invp = frcp(p);
+    s.C = xmul(s.c, k.inv_gamma);     // pK / (rhoK cK) = cK / gamma: f' = (p/pK)^g1 C / p
+    s.a = xmul(rho, k.ig5);
+    s.b = xmul(rp, k.g6ig5);
+    s.g4c = xmul(k.g4, s.c);
     return s;
 }
 
 // f_K, f_K' at p (1/p given); q = (p/pK)^g1 on the rarefaction branch
-__device__ __forceinline__ void pressure_fn5(const RiemannSide &s, double p, double invp, double &f, double &fd,
-                                             double &q, bool &rare) {
+template <int N>
+__device__ __forceinline__ void pressure_fn_root(const RiemannSide &s, double p, double invp, double &f, double &fd,
+                                                 double &q, bool &rare) {
     if (nn_le(p, s.p)) {
-        q = root5(p * s.invp);
-        f = s.g4c * (q - 1.);
-        fd = q * s.C * invp;
+        q = root<N>(xmul(p, s.invp));
+        f = fma(s.g4c, q, -s.g4c);
+        fd = xmul(xmul(q, s.C), invp);
         rare = true;
     } else {
         // qrt = sqrt(A_K / (B_K + p)) and t = 1 / (B_K + p) from one
         // reciprocal square root: qrt = 1/sqrt((B_K + p) / A_K), t = qrt^2 / A_K
-        const double bp = s.bk + p;
-        const double qrt = frsqrt(bp * s.iak);
+        const double qrt = frsqrt(fma(s.a, p, s.b));
         // t / 2 = qrt^2 A_K^-1 / 2, halved through the operand (exact), so
         // that nothing on the iteration's dependency chain waits on it
-        const double t2 = (qrt * qrt) * half_of(s.iak);
-        f = (p - s.p) * qrt;
-        fd = __dmul_rn(fma(-(p - s.p), t2, 1.), qrt);
+        const double t2 = xmul(xmul(qrt, qrt), half_of(s.a));
+        const double d = subr(p, s.p);
+        f = mulr(d, qrt);
+        fd = xmul(fma(-d, t2, 1.), qrt);
         q = 0.;
         rare = false;
     }
 }
 
-// x with its sign bit flipped when f (integer pipe; exact negation)
-__device__ __forceinline__ double flip_if(double x, bool f) {
-    return __longlong_as_double(__double_as_longlong(x) ^ ((long long)f << 63));
-}
-
-// Same solution as riemann_exact for gamma = 5/3 with cheaper arithmetic:
-// fifth roots instead of pow, integer powers for g3, g4 and 1/gamma,
-// reciprocals by Newton-Raphson (frcp), f_K(p*) from the last Newton
-// evaluation plus its derivative times the final (<= tol relative) step,
-// which differs from re-evaluating f at p* by O(tol^2) relative, and sign
-// and order tests on the integer pipe; halvings and doublings on the
-// integer pipe too (half_of, twice).
+// Same solution as riemann_exact for N = 2 gamma / (gamma - 1) = 5 or 7 with
+// cheaper arithmetic: N-th roots instead of pow, integer powers for g3, g4 and
+// 1/gamma, f_K(p*) from the last Newton evaluation plus its derivative times
+// the final (<= tol relative) step, which differs from re-evaluating f at p*
+// by O(tol^2) relative, and sign and order tests, halvings, reciprocals, roots
+// and most products on the integer pipe (mlh_intmath.cuh).  A product goes
+// there (xmul) where both factors are positive in every physical state, so
+// that its range test never fails; products that can be zero, and sums, stay
+// on the FP64 pipe.
 // first_iters > 0: when Newton from the two-rarefaction guess has not
 // converged after that many steps, return unsolved (flag 2, pstar = the
 // current iterate, iters = steps run); solving again with that iterate as
@@ -305,9 +294,9 @@ __device__ __forceinline__ double flip_if(double x, bool f) {
 // speed it stands for, and the ties at zero are resolved as the right-side
 // tests resolve them, so the sampled state is the one of the two-sided
 // sampling (Toro section 4.5).
-// State of the gamma = 5/3 solver between its phases: the sorted sides, the
-// Newton iterate and, once converged, f_K(p*) and (p*/p_K)^(1/5).
-struct Solve5 {
+// State of the root solver between its phases: the sorted sides, the Newton
+// iterate and, once converged, f_K(p*) and (p*/p_K)^(1/N).
+struct RootSolve {
     RiemannSide A, B;
     double du, pfloor, p, fAs, fBs, qAs, qBs;
     int iters;   // Newton steps run (a restart from p_TR counts max_iter first); -1: no convergence
@@ -315,11 +304,23 @@ struct Solve5 {
     bool mir;
 };
 
+// p_TR (Toro eq. 4.46) of the sorted problem.
+template <int N>
+__device__ __forceinline__ double root_guess(const RiemannConsts &k, const RiemannSide &A, const RiemannSide &B,
+                                             double du) {
+    const double num = fma(-k.g7, du, addr(A.c, B.c));
+    const double den = fma(A.c, rroot<N>(A.p), xmul(B.c, rroot<N>(B.p)));
+    const double t = mulr(num, frcp(den));
+    const double t2 = xmul(t, t), t4 = xmul(t2, t2);
+    return N == 5 ? xmul(t4, t) : xmul(xmul(t4, t2), t);
+}
+
 // Newton from p0 (raised to the floor) on the sorted problem; with
 // tried_guess, a start that does not converge is retried from p_TR.
 // first_iters > 0 (not with tried_guess): stop unfinished after that many
 // steps (stage 2, s.p the iterate).
-__device__ __forceinline__ void riemann5_newton(const RiemannConsts &k, Solve5 &s, double p0, bool tried_guess,
+template <int N>
+__device__ __forceinline__ void riemann_root_newton(const RiemannConsts &k, RootSolve &s, double p0, bool tried_guess,
                                                 int first_iters) {
     const RiemannSide &A = s.A, &B = s.B;
     const double du = s.du, pfloor = s.pfloor;
@@ -330,31 +331,27 @@ __device__ __forceinline__ void riemann5_newton(const RiemannConsts &k, Solve5 &
         if (attempt == 1) {
             if (!tried_guess) break;
             extra = k.max_iter;
-            double num = A.c + B.c - k.g7 * du;
-            double den = A.c * rroot5(A.p) + B.c * rroot5(B.p);
-            double t = fdiv(num, den);
-            double t2 = t * t;
-            p0 = t2 * t2 * t;
+            p0 = root_guess<N>(k, A, B, du);
         }
         p = nn_le(p0, pfloor) ? pfloor : p0;
         for (int it = 1; it <= k.max_iter; ++it) {
             double invp = frcp(p);
             double fA, fdA, qA, fB, fdB, qB;
             bool rA, rB;
-            pressure_fn5(A, p, invp, fA, fdA, qA, rA);
-            pressure_fn5(B, p, invp, fB, fdB, qB, rB);
-            double pnew = p - (fA + fB + du) * frcp(fdA + fdB);
+            pressure_fn_root<N>(A, p, invp, fA, fdA, qA, rA);
+            pressure_fn_root<N>(B, p, invp, fB, fdB, qB, rB);
+            double pnew = fma(-addr(addr(fA, fB), du), frcp(addr(fdA, fdB)), p);
             {   // !(pnew > 0): zero, negative or NaN (bit patterns)
                 const long long pb = __double_as_longlong(pnew);
                 if (pb <= 0 || pb > 0x7FF0000000000000ll) pnew = pfloor;
             }
-            double dp = pnew - p;
-            if (nn_le(fabs(dp), k.tol_half * (pnew + p))) {
-                s.fAs = fA + fdA * dp;
-                s.fBs = fB + fdB * dp;
-                double rel = dp * invp;
-                s.qAs = rA ? qA + qA * (k.g1 * rel) : -1.;
-                s.qBs = rB ? qB + qB * (k.g1 * rel) : -1.;
+            const double dp = subr(pnew, p);
+            if (nn_le(abs_bits(dp), mulr(k.tol_half, addr(pnew, p)))) {
+                s.fAs = fma(fdA, dp, fA);
+                s.fBs = fma(fdB, dp, fB);
+                const double rel = mulr(k.g1, mulr(dp, invp));
+                s.qAs = rA ? fma(qA, rel, qA) : -1.;
+                s.qBs = rB ? fma(qB, rel, qB) : -1.;
                 p = pnew;
                 iters = it;
                 break;
@@ -372,53 +369,53 @@ __device__ __forceinline__ void riemann5_newton(const RiemannConsts &k, Solve5 &
 }
 
 // The sides, the vacuum test, the start (the given guess, or p_TR) and the
-// Newton iteration of riemann_exact5, up to its optional stops.
-__device__ __forceinline__ Solve5 riemann5_begin(const RiemannConsts &k, double rhoL, double uL, double pL,
+// Newton iteration of riemann_exact_root, up to its optional stops.
+template <int N>
+__device__ __forceinline__ RootSolve riemann_root_begin(const RiemannConsts &k, double rhoL, double uL, double pL,
                                                  double rhoR, double uR, double pR, double guess,
                                                  double defer_above, int first_iters) {
-    Solve5 s;
+    RootSolve s;
     s.mir = dlt(pR, pL);
     const bool mir = s.mir;
     s.A = make_side(k, mir ? rhoR : rhoL, mir ? flip_if(uR, true) : uL, mir ? pR : pL);
     s.B = make_side(k, mir ? rhoL : rhoR, mir ? flip_if(uL, true) : uR, mir ? pL : pR);
     s.fAs = 0.; s.fBs = 0.; s.qAs = -1.; s.qBs = -1.; s.iters = 0; s.p = 0.;
-    if (!dlt(s.B.u - s.A.u, k.g4 * (s.A.c + s.B.c))) {   // g4 (cL + cR) <= uR - uL: vacuum
+    s.du = subr(s.B.u, s.A.u);
+    if (!dlt(s.du, addr(s.A.g4c, s.B.g4c))) {   // g4 cL + g4 cR <= uR - uL: vacuum
         s.stage = 0;
         return s;
     }
-    s.du = s.B.u - s.A.u;
-    s.pfloor = 1e-12 * s.B.p;                   // 1e-12 max(pL, pR)
+    s.pfloor = xmul(1e-12, s.B.p);              // 1e-12 max(pL, pR)
     double p0;
     const bool tried_guess = __double_as_longlong(guess) > 0;   // guess > 0 (-1: none)
     if (tried_guess) p0 = guess;
     else {
-        double num = s.A.c + s.B.c - k.g7 * s.du;
-        double den = s.A.c * rroot5(s.A.p) + s.B.c * rroot5(s.B.p);
-        double t = fdiv(num, den);
-        double t2 = t * t;
-        p0 = t2 * t2 * t;
+        p0 = root_guess<N>(k, s.A, s.B, s.du);
         // defer_above > 0 and p0 > defer_above, on the keys (see riemann_exact)
         if (ord_key(defer_above) > 0 && dlt(defer_above, p0)) {
             s.p = p0; s.stage = 3;
             return s;
         }
     }
-    riemann5_newton(k, s, p0, tried_guess, first_iters);
+    riemann_root_newton<N>(k, s, p0, tried_guess, first_iters);
     return s;
 }
 
 // Continue a solve stopped unfinished (stage 2) from its iterate: the same
-// iteration as restarting riemann_exact5 with the iterate as the guess.
-__device__ __forceinline__ void riemann5_continue(const RiemannConsts &k, Solve5 &s) {
-    riemann5_newton(k, s, s.p, true, 0);
+// iteration as restarting riemann_exact_root with the iterate as the guess.
+template <int N>
+__device__ __forceinline__ void riemann_root_continue(const RiemannConsts &k, RootSolve &s) {
+    riemann_root_newton<N>(k, s, s.p, true, 0);
 }
 
-__device__ inline RiemannResult riemann5_finish(const RiemannConsts &k, const Solve5 &s);
+template <int N>
+__device__ inline RiemannResult riemann_root_finish(const RiemannConsts &k, const RootSolve &s);
 
-__device__ inline RiemannResult riemann_exact5(const RiemannConsts &k, double rhoL, double uL, double pL,
+template <int N>
+__device__ inline RiemannResult riemann_exact_root(const RiemannConsts &k, double rhoL, double uL, double pL,
                                                double rhoR, double uR, double pR, double guess = -1.,
                                                double defer_above = 0., int first_iters = 0) {
-    const Solve5 s = riemann5_begin(k, rhoL, uL, pL, rhoR, uR, pR, guess, defer_above, first_iters);
+    const RootSolve s = riemann_root_begin<N>(k, rhoL, uL, pL, rhoR, uR, pR, guess, defer_above, first_iters);
     RiemannResult res;
     if (s.stage == 0) {
         res.rho = 0.; res.u = 0.; res.p = 0.; res.pstar = 0.; res.flag = 0; res.iters = 0;
@@ -428,11 +425,12 @@ __device__ inline RiemannResult riemann_exact5(const RiemannConsts &k, double rh
         res.rho = 0.; res.u = 0.; res.p = 0.; res.pstar = s.p; res.flag = 2; res.iters = s.stage == 2 ? s.iters : 0;
         return res;
     }
-    return riemann5_finish(k, s);
+    return riemann_root_finish<N>(k, s);
 }
 
 // u* and the sampled state of a converged (or given-up) solve.
-__device__ inline RiemannResult riemann5_finish(const RiemannConsts &k, const Solve5 &s) {
+template <int N>
+__device__ inline RiemannResult riemann_root_finish(const RiemannConsts &k, const RootSolve &s) {
     RiemannResult res;
     const RiemannSide &A = s.A, &B = s.B;
     const bool mir = s.mir;
@@ -443,8 +441,8 @@ __device__ inline RiemannResult riemann5_finish(const RiemannConsts &k, const So
     if (s.iters < 0) {
         double invp = frcp(pstar), fdA, fdB, qA, qB;
         bool rA, rB;
-        pressure_fn5(A, pstar, invp, fAs, fdA, qA, rA);
-        pressure_fn5(B, pstar, invp, fBs, fdB, qB, rB);
+        pressure_fn_root<N>(A, pstar, invp, fAs, fdA, qA, rA);
+        pressure_fn_root<N>(B, pstar, invp, fBs, fdB, qB, rB);
         qAs = rA ? qA : -1.;
         qBs = rB ? qB : -1.;
     }
@@ -452,7 +450,7 @@ __device__ inline RiemannResult riemann5_finish(const RiemannConsts &k, const So
     // u* of the given problem (the sorted one's, negated when mirrored)
     // .5 (uA + uB) + .5 (fB - fA) = .5 ((uA + uB) + (fB - fA)): halving is
     // exact, so one rounding of the sum, halved on the integer pipe
-    const double ustar = flip_if(half_of((A.u + B.u) + (fBs - fAs)), mir);
+    const double ustar = flip_if(half_of(addr(addr(A.u, B.u), subr(fBs, fAs))), mir);
     // --- sampling at S = 0: side s of the contact, as the left side
     const bool right = dneg(ustar);               // u* < 0: the right state
     const bool useB = right != mir;               // where side s sits in the sorted problem
@@ -467,23 +465,27 @@ __device__ inline RiemannResult riemann5_finish(const RiemannConsts &k, const So
         const double sh = __dsub_rn(u_s, c_s);    // head speed
         if (!dneg(sh)) { rho = rho_s; u = u_s; pp = p_s; }
         else {
-            const double q = !dneg(q_s) ? q_s : root5(pstar * invp_s);
+            const double q = !dneg(q_s) ? q_s : root<N>(xmul(pstar, invp_s));
             const double st = __fma_rn(-c_s, q, ustar_s);   // tail speed
             // tail < 0 puts S = 0 in the star region (left side); the right
             // side's test, tail >= 0 there, reads tail <= 0 mirrored
             const long long kst = ord_key(st);
-            if (right ? kst <= 0 : kst < 0) { rho = rho_s * (q * q * q); u = ustar_s; pp = pstar; }
-            else {
-                const double cf = k.g5 * __fma_rn(k.g7, u_s, c_s);
-                const double r = fdiv(cf, c_s), r3 = r * r * r;
-                u = cf; rho = rho_s * r3; pp = p_s * (r3 * r * r);
+            if (right ? kst <= 0 : kst < 0) {
+                const double q2 = xmul(q, q), q3 = xmul(q2, q);
+                rho = xmul(rho_s, N == 5 ? q3 : xmul(q3, q2));   // q^(N-2)
+                u = ustar_s; pp = pstar;
+            } else {
+                const double cf = mulr(k.g5, __fma_rn(k.g7, u_s, c_s));
+                double rm2;
+                const double rn = pow_n<N>(mulr(cf, frcp(c_s)), rm2);
+                u = cf; rho = mulr(rho_s, rm2); pp = mulr(p_s, rn);
             }
         }
     } else {                                      // shock on side s
-        const double pm = pstar * invp_s;
-        const double sl = __fma_rn(-c_s, sqrt(k.g2 * pm + k.g1), u_s);   // shock speed
+        const double pm = xmul(pstar, invp_s);
+        const double sl = __fma_rn(-c_s, fsqrt_rn(fma(k.g2, pm, k.g1)), u_s);   // shock speed
         if (!dneg(sl)) { rho = rho_s; u = u_s; pp = p_s; }
-        else { rho = rho_s * fdiv(pm + k.g6, pm * k.g6 + 1.); u = ustar_s; pp = pstar; }
+        else { rho = xmul(rho_s, xmul(addr(pm, k.g6), frcp(fma(pm, k.g6, 1.)))); u = ustar_s; pp = pstar; }
     }
     res.flag = right ? 1 : -1;
     res.rho = rho; res.u = flip_if(u, right); res.p = pp;
