@@ -231,6 +231,17 @@ __device__ __forceinline__ double image_coord(double xa, const GridInfo &g, int 
     return __dadd_rn(low ? g.hi[a] : g.lo[a], __dsub_rn(xa, low ? g.lo[a] : g.hi[a]));
 }
 
+// position of neighbour entry e (an image: shifted by the ghost rule)
+template <int D>
+__device__ __forceinline__ void neighbour_pos(uint32_t e, const Prim &pj, const GridInfo &g, double *xj) {
+    xj[0] = pj.x; xj[1] = pj.y; if (D == 3) xj[2] = pj.z;
+    if (e >> IMG_SHIFT) {
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+            if (e & (1u << (IMG_SHIFT + a))) xj[a] = image_coord(xj[a], g, a);
+    }
+}
+
 template <int D>
 __device__ __forceinline__ double dotD(const double *a, const double *b) {
     double r = mulr(a[0], b[0]);

@@ -36,7 +36,7 @@ struct StepArgs {
     cudaEvent_t ev_fork, ev_join;
     int face_blocks;
     int sm_count;
-    int root;               // RiemannConsts::root: 5 runs the root solver, 0 the general one
+    int root;               // RiemannConsts::root: 5 or 7 runs the root solver, 0 the general one
     size_t faces_cap;
     double dt_max;
     // state (structure of arrays)
