@@ -78,7 +78,7 @@ struct mlh_ctx {
     int *cell = nullptr, *cellCount = nullptr, *cellStart = nullptr, *cellFill = nullptr, *cellList = nullptr;
     // neighbours (capacity K slots per particle)
     uint32_t *nbr = nullptr;
-    double *rr = nullptr, *ww = nullptr, *psi = nullptr;
+    double *ww = nullptr, *psi = nullptr;   // W and, per slot, x_j - x_i (search) then V_i psi~ (gradients)
     size_t faces_cap = 0;
     size_t queue_cap = 0, queue_cap2 = 0;
     int *noi = nullptr, *noiImg = nullptr, *faceCnt = nullptr, *faceOff = nullptr, *faceOf = nullptr;
@@ -134,13 +134,13 @@ namespace {
 int round_slots(int k) { return (k + 3) & ~3; }
 
 void free_neighbour_buffers(mlh_ctx *c) {
-    cudaFree(c->nbr); cudaFree(c->rr); cudaFree(c->ww); cudaFree(c->psi); cudaFree(c->faceOf); cudaFree(c->faces);
+    cudaFree(c->nbr); cudaFree(c->ww); cudaFree(c->psi); cudaFree(c->faceOf); cudaFree(c->faces);
     cudaFree(c->Fface);
     cudaFree(c->fstate); cudaFree(c->feat); cudaFree(c->yguess); cudaFree(c->queueFace); cudaFree(c->queueCount);
     cudaFree(c->fstate2); cudaFree(c->queueFace2); cudaFree(c->queueCount2);
     c->queueFace = nullptr; c->queueCount = nullptr;
     c->fstate2 = nullptr; c->queueFace2 = nullptr; c->queueCount2 = nullptr;
-    c->nbr = nullptr; c->rr = nullptr; c->ww = nullptr; c->psi = nullptr; c->faceOf = nullptr; c->faces = nullptr;
+    c->nbr = nullptr; c->ww = nullptr; c->psi = nullptr; c->faceOf = nullptr; c->faces = nullptr;
     c->Fface = nullptr; c->fstate = nullptr; c->feat = nullptr; c->yguess = nullptr;
 }
 
@@ -157,7 +157,6 @@ int alloc_neighbour_buffers(mlh_ctx *c) {
         return MLH_ERR_CAPACITY;
     }
     CK(dalloc(&c->nbr, slots));
-    CK(dalloc(&c->rr, slots));
     CK(dalloc(&c->ww, slots));
     CK(dalloc(&c->psi, slots * 3));
     c->faces_cap = faces;
@@ -293,7 +292,7 @@ StepArgs make_args(mlh_ctx *c, double dt_max) {
     a.grids = c->grids; a.cellTotal = c->cellTotal; a.boundsPart = c->boundsPart;
     a.cell = c->cell; a.cellCount = c->cellCount; a.cellStart = c->cellStart; a.cellFill = c->cellFill;
     a.cellList = c->cellList;
-    a.nbr = c->nbr; a.rr = c->rr; a.ww = c->ww; a.psi = c->psi;
+    a.nbr = c->nbr; a.ww = c->ww; a.psi = c->psi;
     a.noi = c->noi; a.noiImg = c->noiImg; a.faceCnt = c->faceCnt; a.faceOff = c->faceOff; a.faceOf = c->faceOf;
     a.faces = c->faces;
     a.prim = c->prim; a.geo = c->geo; a.grad = c->grad; a.gradRaw = c->debug_arrays ? c->gradRaw : nullptr;

@@ -238,21 +238,20 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
     const int j = (int)(e & IDX_MASK);
     const bool img = (e >> IMG_SHIFT) != 0;
     const Prim pi = prim[i], pj = prim[j];
-    const double Vi = geo[i].V, Vj = geo[j].V;
     double xi[3] = {pi.x, pi.y, pi.z}, xj[3];
     if (img) neighbour_pos<D>(e, pj, grids[mi], xj);
     else { xj[0] = pj.x; xj[1] = pj.y; xj[2] = pj.z; }
-    // --- effective face
+    // --- effective face, from V_i psi~_j(x_i) of both slots
     {
         const double *ps_i = psi + si * 3;
         if (fr.rslot >= 0) {
             const double *ps_j = psi + ((size_t)j * p.K + fr.rslot) * 3;
 #pragma unroll
-            for (int a = 0; a < D; ++a) A[a] = fma(Vi, ps_i[a], -mulr(Vj, ps_j[a]));
+            for (int a = 0; a < D; ++a) A[a] = subr(ps_i[a], ps_j[a]);
         } else {
             st_local |= ST_ASYMMETRIC;
 #pragma unroll
-            for (int a = 0; a < D; ++a) A[a] = mulr(Vi, ps_i[a]);
+            for (int a = 0; a < D; ++a) A[a] = ps_i[a];
         }
     }
     // --- states at the face

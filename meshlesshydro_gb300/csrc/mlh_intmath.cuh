@@ -271,13 +271,10 @@ __device__ __forceinline__ double fsqrt_rn(double x) {
     return __hiloint2double(hi_word(r) + (uint32_t)((1022 + o.q) << 20), (uint32_t)r);
 }
 
-// a b, the IEEE product bit for bit: the 106-bit product, one place to the
-// left where its top bit is clear, and rounded to nearest even with the carry
-// running into the exponent field.  Both exponent fields in [767, 1278]
-// (2^-256 to 2^256), which keeps the product normal; else the FP64 product.
-__device__ __forceinline__ double xmul(double a, double b) {
-    const uint32_t ah = __double2hiint(a), al = __double2loint(a), bh = __double2hiint(b), bl = __double2loint(b);
-    if ((((ah & 0x7fffffffu) - 0x2ff00000u) | ((bh & 0x7fffffffu) - 0x2ff00000u)) & 0xe0000000u) return mul_fp64(a, b);
+// the 106-bit product of two normal doubles, one place to the left where its
+// top bit is clear, and rounded to nearest even with the carry running into
+// the exponent field
+__device__ __forceinline__ double mul_mantissas(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl) {
     const uint32_t mah = __funnelshift_l(al, ah, 11) | 0x80000000u, mal = al << 11, mbh = (bh & 0xfffffu) | 0x100000u;
     const uint64_t t = mul_wide(mal, bl), u = mul_wide(mah, bl) + hi_word(t);
     const uint64_t v = mul_wide(mal, mbh) + (uint32_t)u, w = mul_wide(mah, mbh) + hi_word(u) + hi_word(v);
@@ -296,6 +293,36 @@ __device__ __forceinline__ double xmul(double a, double b) {
     asm("{\n\t.reg .u32 drop;\n\tadd.cc.u32 drop, %2, %3;\n\taddc.cc.u32 %0, %4, 0;\n\taddc.u32 %1, %5, %6;\n\t}"
         : "=r"(rl), "=r"(rh) : "r"(rem), "r"(half), "r"(wl), "r"(wh), "r"(ex));
     return __hiloint2double(rh, rl);
+}
+// not 0 in the top bits unless the exponent field is in [767, 1278] (2^-256 to
+// 2^256): products and quotients of two such numbers are normal
+__device__ __forceinline__ uint32_t out_of_window(uint32_t h) { return (h & 0x7fffffffu) - 0x2ff00000u; }
+
+// a b, the IEEE product bit for bit; outside the window the FP64 product
+__device__ __forceinline__ double xmul(double a, double b) {
+    const uint32_t ah = __double2hiint(a), al = __double2loint(a), bh = __double2hiint(b), bl = __double2loint(b);
+    if ((out_of_window(ah) | out_of_window(bh)) & 0xe0000000u) return mul_fp64(a, b);
+    return mul_mantissas(ah, al, bh, bl);
+}
+// the same where a may be zero (an offset along an axis of a lattice): zeros
+// stay on the straight path
+__device__ __forceinline__ double xmul_z(double a, double b) {
+    const uint32_t ah = __double2hiint(a), al = __double2loint(a), bh = __double2hiint(b), bl = __double2loint(b);
+    const bool zero = ((ah << 1) | al) == 0u;
+    if (((zero ? 0u : out_of_window(ah)) | out_of_window(bh)) & 0xe0000000u) return mul_fp64(a, b);
+    const double r = mul_mantissas(ah, al, bh, bl);
+    return zero ? __hiloint2double((ah ^ bh) & 0x80000000u, 0) : r;
+}
+
+static __device__ __noinline__ double div_fp64(double a, double b) { return a / b; }
+// a / b: the quotient by the reciprocal and its remainder's correction, three
+// FP64 instructions (90 SM cycles per warp for a / b); zero, subnormal,
+// infinite and NaN operands and those outside the window by a / b
+__device__ __forceinline__ double fdiv_rn(double a, double b) {
+    const uint32_t ah = __double2hiint(a), bh = __double2hiint(b);
+    if ((out_of_window(ah) | out_of_window(bh)) & 0xe0000000u) return div_fp64(a, b);
+    const double r = frcp(b), q = mulr(a, r);
+    return fma(fma(-q, b, a), r, q);
 }
 
 }  // namespace mlh

@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(PB_T) k_binning(const double *__restrict__ x, 
 // above h^2, survivors compacted with a ballot into the particle's shared
 // list in stencil order.  Then, particle by particle, phase 2: the lanes take
 // the survivors 32 at a time and apply the reference's FP64 test exactly (d^2
-// = (dx*dx + dy*dy) + dz*dz < h*h, no fused multiply-add), compute r and
+// = (dx*dx + dy*dy) + dz*dz < h*h, no fused multiply-add), compute
 // W(r), and append real neighbours (in order) to the slot list and images to
 // a shared list, which is then placed behind the real neighbours sorted by
 // parent index.  The single-precision test only decides which candidates
@@ -537,8 +537,8 @@ struct NnsCells {
 // shared memory of k_neighbours: NNS_WARPS NnsCells, then per warp the
 // staged chunk (NNS_CH float4 positions and entries), NNS_PB candidate lists
 // (K + 32 uint32 each), four NNS_PB int arrays (candidate counts, offsets in
-// the batch's sequence, real and image neighbour counts), image r and W (K
-// doubles each) and image entries (K uint32), each rounded up to 16 bytes
+// the batch's sequence, real and image neighbour counts), image W (K doubles)
+// and image entries (K uint32), each rounded up to 16 bytes
 __host__ __device__ constexpr size_t nns_cells_bytes() {
     return (sizeof(NnsCells) * NNS_WARPS + 15) / 16 * 16;
 }
@@ -548,7 +548,7 @@ __host__ __device__ constexpr size_t nns_r16(size_t b) { return (b + 15) / 16 * 
 // of the SM's shared memory at K = 64, for 3 blocks per SM)
 __host__ __device__ constexpr size_t nns_warp_bytes(int K, bool adaptive = false) {
     return (size_t)NNS_CH * 4 + (size_t)NNS_CH * 16 + nns_r16((size_t)NNS_PB * (K + 32) * 4) +
-           nns_r16((size_t)4 * NNS_PB * 4) + (size_t)K * 16 + nns_r16((size_t)K * 4) +
+           nns_r16((size_t)4 * NNS_PB * 4) + nns_r16((size_t)K * 8) + nns_r16((size_t)K * 4) +
            (adaptive ? (size_t)NNS_CH * 4 : 0);
 }
 
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
     const double *__restrict__ z, const float4 *__restrict__ posf, const double *__restrict__ vx,
     const double *__restrict__ vy, const double *__restrict__ vz, const double *__restrict__ m,
     const double *__restrict__ u, const int *__restrict__ cellTotal, const int *__restrict__ cellStart,
-    const int *__restrict__ cellList, uint32_t *__restrict__ nbr, double *__restrict__ rr,
+    const int *__restrict__ cellList, uint32_t *__restrict__ nbr, double *__restrict__ dd,
     double *__restrict__ ww, int *__restrict__ noi, int *__restrict__ noiImg, int *__restrict__ faceCnt,
     Prim *__restrict__ prim, Geo *__restrict__ geo, float4 *__restrict__ velf, unsigned *__restrict__ status) {
     const int K = p.K;
@@ -644,8 +644,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
     uint32_t *candq = stE + NNS_CH;                                                   // NNS_PB lists of CAP
     int *ncq = reinterpret_cast<int *>(wbase + (size_t)NNS_CH * 20 + nns_r16((size_t)NNS_PB * CAP * 4));
     int *offq = ncq + NNS_PB, *nrq = offq + NNS_PB, *niq = nrq + NNS_PB;
-    double *imgR = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(ncq) + nns_r16((size_t)4 * NNS_PB * 4));
-    double *imgW = imgR + K;
+    double *imgW = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(ncq) + nns_r16((size_t)4 * NNS_PB * 4));
     uint32_t *imgE = reinterpret_cast<uint32_t *>(imgW + K);
     float *stH = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(imgE) + nns_r16((size_t)K * 4));   // staged h_j
 
@@ -825,7 +824,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
                     const double sigma4_i = __shfl_sync(0xffffffffu, mySig4, q);
                     bool pass = false, img = false;
                     uint32_t e = 0;
-                    double r = 0., w = 0.;
+                    double w = 0., ed[3] = {0., 0., 0.};
                     if (valid) {
                         e = candq[(size_t)q * CAP + (gi - offq[q])];
                         const int j = (int)(e & IDX_MASK);
@@ -842,9 +841,10 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
                             }
                         }
                         if (ok) {
-                            double ex = __dsub_rn(xj[0], xi[0]), ey = __dsub_rn(xj[1], xi[1]);
-                            double d2 = __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey));
-                            if (D == 3) { double ez = __dsub_rn(xj[2], xi[2]); d2 = __dadd_rn(d2, __dmul_rn(ez, ez)); }
+#pragma unroll
+                            for (int a = 0; a < D; ++a) ed[a] = subr(xj[a], xi[a]);
+                            double d2 = addr(mulr(ed[0], ed[0]), mulr(ed[1], ed[1]));
+                            if (D == 3) d2 = addr(d2, mulr(ed[2], ed[2]));
                             // d2, h^2 >= 0: compared as bit patterns on the integer pipe
                             double lim = mb.hsq;
                             if (p.adaptive_h) {
@@ -853,10 +853,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
                                 lim = __double_as_longlong(hsq_i) < __double_as_longlong(hsq_j) ? hsq_j : hsq_i;
                             }
                             pass = __double_as_longlong(d2) < __double_as_longlong(lim);
-                            if (pass) {
-                                r = fsqrt_rn(d2);
-                                w = kernelW2(r, ih2_i, sigma_i, sigma4_i);
-                            }
+                            if (pass) w = kernelW2(fsqrt_rn(d2), ih2_i, sigma_i, sigma4_i);
                         }
                     }
                     // lanes of the same particle, and their ranks among its passes
@@ -867,11 +864,16 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
                     const size_t base = (size_t)i * K;
                     if (pass && !img) {
                         const int pos = nr0 + __popc(balR & lt_mask);
-                        if (pos < K) { nbr[base + pos] = e; rr[base + pos] = r; ww[base + pos] = w; }
+                        if (pos < K) {
+                            nbr[base + pos] = e;
+                            ww[base + pos] = w;
+#pragma unroll
+                            for (int a = 0; a < D; ++a) dd[(base + pos) * 3 + a] = ed[a];
+                        }
                     }
                     if (pass && img) {
                         const int pos = ni0 + __popc(balI & lt_mask);
-                        if (pos < K) { nbr[base + K - 1 - pos] = e; rr[base + K - 1 - pos] = r; ww[base + K - 1 - pos] = w; }
+                        if (pos < K) { nbr[base + K - 1 - pos] = e; ww[base + K - 1 - pos] = w; }
                     }
                     __syncwarp();
                     if (valid && (grp & lt_mask) == 0) {   // first lane of each particle's group
@@ -896,19 +898,25 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
                 // images from the back of the row, in candidate order
                 for (int t = lane; t < ni; t += 32) {
                     imgE[t] = nbr[base + K - 1 - t];
-                    imgR[t] = rr[base + K - 1 - t];
                     imgW[t] = ww[base + K - 1 - t];
                 }
                 __syncwarp();
                 // --- images behind the real neighbours, ordered by parent index
+                // (their offsets are formed again: few particles have images, and
+                // a copy beside imgE and imgW would cost a resident block)
                 for (int t = lane; t < ni; t += 32) {
                     const uint32_t e = imgE[t];
                     const uint32_t id = e & IDX_MASK;
                     int rank = 0;
                     for (int u = 0; u < ni; ++u) rank += (imgE[u] & IDX_MASK) < id;
                     nbr[base + nr + rank] = e;
-                    rr[base + nr + rank] = imgR[t];
                     ww[base + nr + rank] = imgW[t];
+#pragma unroll
+                    for (int a = 0; a < D; ++a) {
+                        double xa = X[a][id];
+                        if (e & (1u << (IMG_SHIFT + a))) xa = image_coord(xa, g, a);
+                        dd[(base + nr + rank) * 3 + a] = __dsub_rn(xa, X[a][i]);
+                    }
                 }
                 __syncwarp();
                 // canonical faces among the stored slots (neighbour or parent > i);
@@ -1250,6 +1258,20 @@ size_t nns_smem_bytes(int K, bool adaptive) {
 
 // ------------------------------------------------------------------ dt
 
+// c_i + c_j - min(0, v_ij . x_ij / r) as one fused multiply-add: 1/r only when
+// the dot product dv = v_ij . x_ij is negative, 0 otherwise; r as the neighbour
+// search takes it
+template <int D>
+__device__ __forceinline__ double signal_speed(double dv, const double *xij, double csum) {
+    double ir = 0.;
+    if (dneg(dv)) {
+        double d2 = addr(mulr(xij[0], xij[0]), mulr(xij[1], xij[1]));
+        if (D == 3) d2 = addr(d2, mulr(xij[2], xij[2]));
+        ir = frcp(fsqrt_rn(d2));
+    }
+    return fma(-dv, ir, csum);
+}
+
 // Particles::compGlobalTimestep (Particles.cpp:1446-1485): real neighbours
 // only, v_sig starting at numeric_limits<double>::min().  The minimum over
 // particles is order independent, so an atomicMin on the bit pattern of the
@@ -1258,7 +1280,7 @@ template <int D>
 __global__ void __launch_bounds__(256) k_timestep(Params p, const Member *__restrict__ members,
                                                   const int *__restrict__ memberOf, const Prim *__restrict__ prim,
                                                   const Geo *__restrict__ geo, const uint32_t *__restrict__ nbr,
-                                                  const double *__restrict__ rr, const int *__restrict__ noi,
+                                                  const int *__restrict__ noi,
                                                   unsigned long long *__restrict__ dtbits,
                                                   const float *__restrict__ dtlo, const unsigned *__restrict__ dtcap) {
     const int lane = threadIdx.x & 31;
@@ -1289,11 +1311,8 @@ __global__ void __launch_bounds__(256) k_timestep(Params p, const Member *__rest
                 const double cj = geo[j].c;
                 double xij[3] = {pi.x - pj.x, pi.y - pj.y, pi.z - pj.z};
                 double vij[3] = {pi.vx - pj.vx, pi.vy - pj.vy, pi.vz - pj.vz};
-                // c_i + c_j - min(0, v_ij . x_ij / r) as one fused multiply-add:
-                // 1/r only when the dot product is negative, 0 otherwise
                 const double dv = dotD<D>(vij, xij);
-                const double ir = dneg(dv) ? frcp(rr[base + s]) : 0.;
-                const double vs = fma(-dv, ir, ci + cj);
+                const double vs = signal_speed<D>(dv, xij, ci + cj);
                 vSig = dlt(vSig, vs) ? vs : vSig;
             }
             dti = (p.adaptive_h ? p.cfl * p.hp[i] : members[mi].cfl_h) / vSig;
@@ -1446,30 +1465,34 @@ __global__ void __launch_bounds__(256) k_link(Params p, const uint32_t *__restri
 // Particles::gradient (:1257-1270, 2457-2502) for rho, vx, vy, (vz), P with
 // psi~_j(x_i) = B_i (x_j - x_i) W_ij / omega_i; Particles::slopeLimiter
 // (:1313-1444) with the face midpoint x_ij = (x_i + x_j)/2.
+// inverse of the symmetric matrix A (closed form; the upper triangle is read,
+// every entry written)
 template <int D>
-__device__ __forceinline__ void invert_closed_form(double *A) {
+__device__ __forceinline__ void invert_symmetric(double *A) {
     if (D == 2) {
-        double a = A[0], b = A[1], c = A[2], d = A[3];
-        double det = a * d - b * c;
-        double id = 1. / det;
-        A[0] = d * id; A[1] = -b * id; A[2] = -c * id; A[3] = a * id;
+        const double a = A[0], b = A[1], d = A[3];
+        const double id = frcp(fma(a, d, -mulr(b, b)));
+        A[0] = mulr(d, id); A[1] = A[2] = -mulr(b, id); A[3] = mulr(a, id);
     } else {
-        double a00 = A[0], a01 = A[1], a02 = A[2], a10 = A[3], a11 = A[4], a12 = A[5], a20 = A[6], a21 = A[7], a22 = A[8];
-        double c00 = a11 * a22 - a12 * a21;
-        double c01 = a12 * a20 - a10 * a22;
-        double c02 = a10 * a21 - a11 * a20;
-        double det = a00 * c00 + a01 * c01 + a02 * c02;
-        double id = 1. / det;
-        A[0] = c00 * id;
-        A[1] = (a02 * a21 - a01 * a22) * id;
-        A[2] = (a01 * a12 - a02 * a11) * id;
-        A[3] = c01 * id;
-        A[4] = (a00 * a22 - a02 * a20) * id;
-        A[5] = (a02 * a10 - a00 * a12) * id;
-        A[6] = c02 * id;
-        A[7] = (a01 * a20 - a00 * a21) * id;
-        A[8] = (a00 * a11 - a01 * a10) * id;
+        const double a = A[0], b = A[1], c = A[2], d = A[4], e = A[5], f = A[8];
+        const double c00 = fma(d, f, -mulr(e, e)), c01 = fma(e, c, -mulr(b, f)), c02 = fma(b, e, -mulr(d, c));
+        const double id = frcp(fma(a, c00, fma(b, c01, mulr(c, c02))));
+        A[0] = mulr(c00, id);
+        A[1] = A[3] = mulr(c01, id);
+        A[2] = A[6] = mulr(c02, id);
+        A[4] = mulr(fma(a, f, -mulr(c, c)), id);
+        A[5] = A[7] = mulr(fma(c, b, -mulr(a, e)), id);
+        A[8] = mulr(fma(a, d, -mulr(b, b)), id);
     }
+}
+
+// x in single precision, the mantissa truncated (error below 2^-23 |x|, or
+// 2^-126 where it flushes to zero), on the integer pipe
+__device__ __forceinline__ float trunc_f32(double x) {
+    const uint32_t h = __double2hiint(x), l = __double2loint(x);
+    const uint32_t m = (h & 0x7fffffffu) - (896u << 20);      // rebased exponent and the mantissa's top
+    const uint32_t v = __funnelshift_l(l, m, 3);
+    return __uint_as_float(((int)m < (1 << 20) ? 0u : (int)m >= (255 << 20) ? 0x7f800000u : v & 0x7fffffffu) | (h & 0x80000000u));
 }
 
 template <int D>
@@ -1489,19 +1512,20 @@ __device__ __forceinline__ double field_of(const Prim &q, int f) {
 // numeric_limits<double>::min(), the same expressions), on the positions and
 // velocities that pass loads anyway; the per-particle dt goes into the
 // per-member minimum (warp reduction, then one atomicMin on its bit pattern).
-// Register caps of the gradients kernel, per dimension.  It waits on
-// dependent gathers as much as on the FP64 pipe (Sedov 64^3: FP64 pipe 73 %
-// active, 17 % of the warp slots occupied at 146 registers), so warps per SM
-// matter: in 3D 128 registers (16 warps per SM, a small spill) took the Sedov
-// 128^3 gradients from 11.1-11.4 to 10.1 ms (112: 10.4, 120: +0.2 ms, 136:
-// +0.5 ms); in 2D (the KH ensemble, 110 registers uncapped) 96 registers
-// gave 7.19 ms against 7.45 at 104 and 7.59 at 128.  Blocks of up to 256
-// threads.
+// Bound: the FP64 pipe (79 % active on Sedov 64^3, 1625 instructions per
+// particle, 41 per neighbour) and, at 12 warps per SM, the latency of the
+// gathers.  One gather of the neighbours' records instead of three, the next
+// one's in flight while one is summed: Sedov 128^3 8.29 -> 6.98 ms, 64 KH
+// members 1.55 -> 1.27 ms, KH 100^2 93 -> 78 us (with the time step's kernel).
+// Register caps, Sedov 128^3: 7.64 ms at 144 and 7.48 at 128 registers (a spill
+// that 16 warps do not make up for), 7.82 at 200.  The products of the offsets
+// on the integer pipe (xmul) made it slower, 7.34 ms: the chain per neighbour
+// gets longer.  Blocks of up to 256 threads.
 #ifndef MLH_GRAD_MAXREG
-#define MLH_GRAD_MAXREG 128
+#define MLH_GRAD_MAXREG 168
 #endif
 #ifndef MLH_GRAD_MAXREG_2D
-#define MLH_GRAD_MAXREG_2D 96
+#define MLH_GRAD_MAXREG_2D 128
 #endif
 #define MLH_GRAD_BOUNDS __maxnreg__(D == 3 ? MLH_GRAD_MAXREG : MLH_GRAD_MAXREG_2D)
 template <int D>
@@ -1509,14 +1533,13 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                                                    const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
                                                    const Prim *__restrict__ prim, Geo *__restrict__ geo,
                                                    const uint32_t *__restrict__ nbr, const double *__restrict__ ww,
-                                                   const double *__restrict__ rr,
                                                    const int *__restrict__ noi, const int *__restrict__ noiImg,
                                                    Grad *__restrict__ grad, Grad *__restrict__ gradRaw,
-                                                   double *__restrict__ psiOut,
+                                                   double *__restrict__ psi,
                                                    unsigned long long *__restrict__ dtbits,
                                                    const int *__restrict__ faceOff, int *__restrict__ faceOf,
                                                    FaceRef *__restrict__ faces, unsigned *__restrict__ status,
-                                                   const float4 *__restrict__ posf, int fp32_filters,
+                                                   int fp32_filters,
                                                    const float4 *__restrict__ velf, float *__restrict__ dtlo,
                                                    unsigned *__restrict__ dtcap) {
     constexpr int NF = D + 2;
@@ -1533,11 +1556,8 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
         // hides, and whose registers are free again before the passes below
         if (faceOff) link_particle(i, p, nbr, noi, noiImg, faceOff, faceOf, faces, status);
         mi = memberOf ? memberOf[i] : 0;
-        const GridInfo g = grids[mi];
-        const double h = members[mi].h;
-        const double hq = p.adaptive_h ? p.hp[i] : h;   // quadrature-point radius
+        const double hq = p.adaptive_h ? p.hp[i] : members[mi].h;   // quadrature-point radius
         const Prim pi = prim[i];
-        const double xi[3] = {pi.x, pi.y, pi.z};
         const size_t base = (size_t)i * p.K;
         const int nr = noi[i];
         const int tot = nr + noiImg[i];
@@ -1546,58 +1566,63 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
         double vSig = DBL_MIN_;
         // the time step's single-precision filter (dtlo): bounds on v_sig
         // = max_j (c_i + c_j - min(0, v_ij . x_ij / r_ij)) over the real
-        // neighbours from the packed positions, velocities and sound speeds
+        // neighbours from their offsets and the packed velocities and sound speeds
         const bool want_dtf = dtlo != nullptr;
-        float4 vif = make_float4(0.f, 0.f, 0.f, 0.f), xif4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        float vlo = 0.f, vhi = 0.f, xbf = 0.f;
+        float4 vif = make_float4(0.f, 0.f, 0.f, 0.f);
+        float vlo = 0.f, vhi = 0.f;
         bool dt_exact = false;   // no usable bound: the particle is always a candidate
-        if (want_dtf) {
-            vif = velf[i];
-            xif4 = posf[i];
-            double xb = 0.;
-#pragma unroll
-            for (int a = 0; a < D; ++a) xb = fmax(xb, fmax(fabs(g.lo[a]), fabs(g.hi[a])));
-            xbf = __double2float_ru(xb);
-        }
-        // E_i = V_i E' with E' = sum_j (x_j - x_i)(x_j - x_i)^T W_ij, so that
-        // psi~_j(x_i) = E_i^-1 (x_j - x_i) W_ij V_i = E'^-1 (x_j - x_i) W_ij:
-        // V_i cancels and neither pass multiplies by it
+        if (want_dtf) vif = velf[i];
+        // One gather of every neighbour's record: E' = sum_j d d^T W with d =
+        // x_j - x_i from the search (psi holds it), and S_f = sum_j (f_j - f_i)
+        // d W, of which the gradient is E'^-1 S_f: psi~_j(x_i) = E_i^-1 d W V_i =
+        // E'^-1 d W (E_i = V_i E': V_i cancels), so that neither the second
+        // gather nor the weighting of every neighbour by psi~ is needed.
         double E[9] = {0., 0., 0., 0., 0., 0., 0., 0., 0.};
+        double gr[NF][3], fi[NF];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) { fi[f] = field_of<D>(pi, f); gr[f][0] = gr[f][1] = gr[f][2] = 0.; }
+        // the next neighbour's record is on its way while this one is summed
+        uint32_t en = tot > 0 ? nbr[base] : 0u, en2 = tot > 1 ? nbr[base + 1] : 0u;
+        Prim pn = prim[en & IDX_MASK];
+        float4 vn = want_dtf ? velf[en & IDX_MASK] : vif;
         for (int s = 0; s < tot; ++s) {
-            const uint32_t e = nbr[base + s];
-            const Prim pj = prim[e & IDX_MASK];
-            double xj[3];
-            neighbour_pos<D>(e, pj, g, xj);
+            const uint32_t e = en;
+            const Prim pj = pn;
+            const float4 vj = vn;
+            en = en2;
+            pn = prim[en & IDX_MASK];
+            if (want_dtf) vn = velf[en & IDX_MASK];
+            en2 = s + 2 < tot ? nbr[base + s + 2] : 0u;
             const double wij = ww[base + s];
+            const double *ds = psi + (base + s) * 3;
             double d[3], dp[3];
 #pragma unroll
-            for (int a = 0; a < D; ++a) { d[a] = xj[a] - xi[a]; dp[a] = d[a] * wij; }
+            for (int a = 0; a < D; ++a) { d[a] = ds[a]; dp[a] = mulr(d[a], wij); }
 #pragma unroll
             for (int a = 0; a < D; ++a)
 #pragma unroll
                 for (int b = a; b < D; ++b) E[D * a + b] = fma(d[a], dp[b], E[D * a + b]);
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                const double df = subr(field_of<D>(pj, f), fi[f]);
+#pragma unroll
+                for (int a = 0; a < D; ++a) gr[f][a] = fma(df, dp[a], gr[f][a]);
+            }
             if (want_dt && s < nr) {
-                // v_sig = c_i + c_j - min(0, v_ij . x_ij / r) as one fused
-                // multiply-add (1/r only when the dot product is negative);
                 // x_ij = x_i - x_j is the exact negation of d
                 const double cj = geo[e & IDX_MASK].c;
                 const double xij[3] = {-d[0], -d[1], D == 3 ? -d[2] : 0.};
-                const double vij[3] = {pi.vx - pj.vx, pi.vy - pj.vy, pi.vz - pj.vz};
-                const double dv = dotD<D>(vij, xij);
-                const double ir = dneg(dv) ? frcp(rr[base + s]) : 0.;
-                const double vs = fma(-dv, ir, ci + cj);
+                const double vij[3] = {subr(pi.vx, pj.vx), subr(pi.vy, pj.vy), subr(pi.vz, pj.vz)};
+                const double vs = signal_speed<D>(dotD<D>(vij, xij), xij, addr(ci, cj));
                 vSig = dlt(vSig, vs) ? vs : vSig;
             }
             if (want_dtf && s < nr) {
-                // |vs - vs64| <= B: the inputs' roundings (eps |c|, eps |v|,
-                // 3 eps X on each coordinate difference), the estimate's own
-                // and the FP64 expression's, at most eps (2 (c_i + c_j) +
-                // 2 vs + V (7 X / r + 8)) with V = |v_i|_1 + |v_j|_1; B is
-                // twice that
-                const int j = (int)(e & IDX_MASK);
-                const float4 vj = velf[j], xj4 = posf[j];
-                const float dx = __fsub_rn(xj4.x, xif4.x), dy = __fsub_rn(xj4.y, xif4.y),
-                            dz = D == 3 ? __fsub_rn(xj4.z, xif4.z) : 0.f;
+                // |vs - vs64| <= B: the inputs' roundings (eps |c|, eps |v|, 2 eps |d|
+                // per offset), the estimate's own and the FP64 expression's, at
+                // most eps (2 (c_i + c_j) + 2 vs + 12 V) with V = |v_i|_1 + |v_j|_1
+                // (an offset that flushes to zero is below 2^-126, and r above 1e-30);
+                // B is twice eps (2 (c_i + c_j) + 2 vs + 16 V)
+                const float dx = trunc_f32(d[0]), dy = trunc_f32(d[1]), dz = D == 3 ? trunc_f32(d[2]) : 0.f;
                 const float wx = __fsub_rn(vif.x, vj.x), wy = __fsub_rn(vif.y, vj.y),
                             wz = D == 3 ? __fsub_rn(vif.z, vj.z) : 0.f;
                 const float dvd = __fmaf_rn(wz, dz, __fmaf_rn(wy, dy, __fmul_rn(wx, dx)));   // v_ij . (x_j - x_i)
@@ -1607,8 +1632,8 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 const float vs = __fadd_rn(__fadd_rn(vif.w, vj.w), T);
                 const float V = fabsf(vif.x) + fabsf(vif.y) + fabsf(vif.z) + fabsf(vj.x) + fabsf(vj.y) + fabsf(vj.z);
                 constexpr float EPS32 = 5.9604645e-8f;
-                const float B = 2.f * EPS32 * (2.f * (vif.w + vj.w) + 2.f * vs + V * (7.f * __fdiv_ru(xbf, r) + 8.f));
-                dt_exact = dt_exact || !(r > 0.f) || !(B < 1e30f);
+                const float B = 2.f * EPS32 * (2.f * (vif.w + vj.w) + 2.f * vs + 16.f * V);
+                dt_exact = dt_exact || !(r > 1e-15f) || !(r < 1e15f) || !(B < 1e30f);
                 vlo = fmaxf(vlo, vs - B);
                 vhi = fmaxf(vhi, vs + B);
             }
@@ -1629,40 +1654,18 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
             dtlo[i] = dt_exact ? 0.f : lo;
             if (dt_exact) dthi = FLT_INF_;
         }
+        invert_symmetric<D>(E);
 #pragma unroll
-        for (int a = 0; a < D; ++a)
+        for (int f = 0; f < NF; ++f) {
+            double S[3];
 #pragma unroll
-            for (int b = 0; b < a; ++b) E[D * a + b] = E[D * b + a];
-        invert_closed_form<D>(E);
-        double gr[NF][3];
-        double fi[NF];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) { fi[f] = field_of<D>(pi, f); gr[f][0] = gr[f][1] = gr[f][2] = 0.; }
-        for (int s = 0; s < tot; ++s) {
-            const uint32_t e = nbr[base + s];
-            const Prim pj = prim[e & IDX_MASK];
-            double xj[3];
-            neighbour_pos<D>(e, pj, g, xj);
-            const double wij = ww[base + s];
-            double d[3], ps[3];
-#pragma unroll
-            for (int a = 0; a < D; ++a) d[a] = xj[a] - xi[a];
+            for (int a = 0; a < D; ++a) S[a] = gr[f][a];
 #pragma unroll
             for (int a = 0; a < D; ++a) {
-                double t = E[D * a] * d[0];
+                double t = mulr(E[D * a], S[0]);
 #pragma unroll
-                for (int b = 1; b < D; ++b) t = fma(E[D * a + b], d[b], t);
-                ps[a] = t * wij;
-            }
-            // psi~_j(x_i) of this slot, reused by the face kernel for A_ij
-            double *po = psiOut + (base + s) * 3;
-#pragma unroll
-            for (int a = 0; a < D; ++a) po[a] = ps[a];
-#pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                const double df = field_of<D>(pj, f) - fi[f];
-#pragma unroll
-                for (int a = 0; a < D; ++a) gr[f][a] += df * ps[a];
+                for (int b = 1; b < D; ++b) t = fma(E[D * a + b], S[b], t);
+                gr[f][a] = t;
             }
         }
         if (gradRaw) {
@@ -1677,13 +1680,32 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
             }
             gradRaw[i] = graw;
         }
-        // B_i = E_i^-1 = E'^-1 / V_i = E'^-1 omega_i (kept for inspection; E
-        // is not needed after the gradient pass)
+        // B_i = E_i^-1 = E'^-1 / V_i = E'^-1 omega_i (kept for inspection); then
+        // E'^-1 V_i, of which V_i psi~_j(x_i) = (E'^-1 V_i) d W
         {
-            const double omega_i = geo[i].omega;
+            const double omega_i = geo[i].omega, V_i = geo[i].V;
 #pragma unroll
-            for (int k = 0; k < D * D; ++k) geo[i].B[k] = E[k] * omega_i;
+            for (int k = 0; k < D * D; ++k) geo[i].B[k] = mulr(E[k], omega_i);
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+#pragma unroll
+                for (int b = a; b < D; ++b) E[D * a + b] = E[D * b + a] = mulr(E[D * a + b], V_i);
         }
+        // V_i psi~_j(x_i) of a slot, for the face kernel's A_ij, over its offset
+        auto store_psi = [&](int s, const double *d) {
+            double *po = psi + (base + s) * 3;
+            const double wij = ww[base + s];
+            double dp[3];
+#pragma unroll
+            for (int a = 0; a < D; ++a) dp[a] = mulr(d[a], wij);
+#pragma unroll
+            for (int a = 0; a < D; ++a) {
+                double t = mulr(E[D * a], dp[0]);
+#pragma unroll
+                for (int b = 1; b < D; ++b) t = fma(E[D * a + b], dp[b], t);
+                po[a] = t;
+            }
+        };
         if (p.slope) {
             // running extrema as integer keys (ord_key): the comparisons of
             // the reference's if (max < f) max = f stay off the FP64 pipe
@@ -1709,14 +1731,8 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
 #pragma unroll
                     for (int a = 0; a < D; ++a) gr[f][a] *= cq;
             }
-            // one neighbour's f_ij of every field, into the extrema
-            auto exact_slot = [&](int s) {
-                const uint32_t e = nbr[base + s];
-                const Prim pj = prim[e & IDX_MASK];
-                double xj[3], d[3];
-                neighbour_pos<D>(e, pj, g, xj);
-#pragma unroll
-                for (int a = 0; a < D; ++a) d[a] = xj[a] - xi[a];
+            // one neighbour's f_ij of every field, into the extrema (its offset d)
+            auto exact_slot = [&](const double *d) {
 #pragma unroll
                 for (int f = 0; f < NF; ++f) {
                     double fij = fma(gr[f][0], d[0], fi[f]);
@@ -1736,53 +1752,33 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                         if (mxN[f] < kj) mxN[f] = kj;
                         if (mnN[f] > kj) mnN[f] = kj;
                     }
-                    exact_slot(s);
+                    const double *ds = psi + (base + s) * 3;
+                    const double d[3] = {ds[0], ds[1], D == 3 ? ds[2] : 0.};
+                    exact_slot(d);
+                    store_psi(s, d);
                 }
             } else {
                 // Single-precision filter (the FP64 pipe is the step's
                 // bound; the FP32 pipe is 64 times wider).  The increment
                 // q_j = (c grad f) . (x_j - x_i) is estimated in single
-                // precision from the packed positions; |f_ij - (f_i + q_j)|
-                // <= B_f for every neighbour, B_f bounding the estimate's
-                // rounding (positions, gradients, the chain) and the FP64
-                // chain's own.  The neighbour with the largest f_ij then has
-                // q_j >= max_k q_k - 2 B_f (and the smallest q_j <= min_k q_k
-                // + 2 B_f), so the FP64 chain runs only over the neighbours
-                // inside those windows (a handful; every lane of a warp walks
-                // its own list): the same extrema, bit for bit.  A field whose
-                // gradient is zero has f_ij = f_i at every neighbour.
-                float gf[NF][3], xif[3];
+                // precision from the offsets; |f_ij - (f_i + q_j)| <= B_f for
+                // every neighbour, B_f bounding the estimate's rounding
+                // (offsets, gradients, the chain) and the FP64 chain's own.  The
+                // neighbour with the largest f_ij then has q_j >= max_k q_k -
+                // 2 B_f (and the smallest q_j <= min_k q_k + 2 B_f), so the FP64
+                // chain runs only over the neighbours inside those windows (a
+                // handful; every lane of a warp walks its own list): the same
+                // extrema, bit for bit.  A field whose gradient is zero has
+                // f_ij = f_i at every neighbour.
+                float gf[NF][3];
 #pragma unroll
                 for (int f = 0; f < NF; ++f)
 #pragma unroll
                     for (int a = 0; a < 3; ++a) gf[f][a] = a < D ? __double2float_rn(gr[f][a]) : 0.f;
+                auto offset_f = [&](int s, float *df, double *d) {
+                    const double *ds = psi + (base + s) * 3;
 #pragma unroll
-                for (int a = 0; a < 3; ++a) xif[a] = a < D ? __double2float_rn(xi[a]) : 0.f;
-                // bound on |coordinate| of any neighbour or image: the box (the
-                // grid spans every particle) and one box length for images
-                double xb = 0.;
-#pragma unroll
-                for (int a = 0; a < D; ++a) {
-                    const double ext = fmax(fabs(g.lo[a]), fabs(g.hi[a])) + (p.periodic ? g.hi[a] - g.lo[a] : 0.);
-                    xb = fmax(xb, ext);
-                }
-                // x_j - x_i in single precision: the packed position, or the
-                // image coordinate (double) rounded once
-                auto offset_f = [&](uint32_t e, const Prim *pjp, float *d) {
-                    const int j = (int)(e & IDX_MASK);
-                    float xj[3];
-                    if (e >> IMG_SHIFT) {
-                        const Prim pj = pjp ? *pjp : prim[j];
-                        double xd[3];
-                        neighbour_pos<D>(e, pj, g, xd);
-#pragma unroll
-                        for (int a = 0; a < 3; ++a) xj[a] = a < D ? __double2float_rn(xd[a]) : 0.f;
-                    } else {
-                        const float4 q = posf[j];
-                        xj[0] = q.x; xj[1] = q.y; xj[2] = q.z;
-                    }
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) d[a] = a < D ? __fsub_rn(xj[a], xif[a]) : 0.f;
+                    for (int a = 0; a < D; ++a) { d[a] = ds[a]; df[a] = trunc_f32(d[a]); }
                 };
                 auto incr = [&](int f, const float *d) {
                     float q = __fmul_rn(gf[f][0], d[0]);
@@ -1794,33 +1790,35 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
 #pragma unroll
                 for (int f = 0; f < NF; ++f) { hiQ[f] = -FLT_MAX_; loQ[f] = FLT_MAX_; }
                 for (int s = 0; s < tot; ++s) {
-                    const uint32_t e = nbr[base + s];
-                    const Prim pj = prim[e & IDX_MASK];
+                    const Prim pj = prim[nbr[base + s] & IDX_MASK];
 #pragma unroll
                     for (int f = 0; f < NF; ++f) {
                         const long long kj = ord_key(field_of<D>(pj, f));
                         if (mxN[f] < kj) mxN[f] = kj;
                         if (mnN[f] > kj) mnN[f] = kj;
                     }
-                    float d[3];
-                    offset_f(e, &pj, d);
+                    float df[3];
+                    double d[3];
+                    offset_f(s, df, d);
 #pragma unroll
-                    for (int a = 0; a < D; ++a) dmax = fmaxf(dmax, fabsf(d[a]));
+                    for (int a = 0; a < D; ++a) dmax = fmaxf(dmax, fabsf(df[a]));
 #pragma unroll
                     for (int f = 0; f < NF; ++f) {
-                        const float q = incr(f, d);
+                        const float q = incr(f, df);
                         hiQ[f] = fmaxf(hiQ[f], q);
                         loQ[f] = fminf(loQ[f], q);
                     }
                 }
-                // B_f = 12 eps32 S R + 12 u64 (|f_i| + S R) with S = sum |c grad f|
-                // and R = max|x| + max|x_j - x_i|: twice the sum of the
-                // single-precision error, at most (6 |x|max + 5 |d|max) eps32 S,
-                // and the FP64 chain's, at most 4 u64 (|f_i| + S (|d|max + eps |x|max))
+                // B_f = 16 eps32 S (dmax + 1e-30) + 12 u64 (|f_i| + S dmax) with S = sum
+                // |c grad f| and dmax = max |x_j - x_i|: more than twice the sum of the
+                // single-precision error, at most 6 eps32 S dmax (2 from the offset's
+                // truncation, 1 from the gradient, 3 from the chain) and 2^-126 S for
+                // offsets flushed to zero, and the FP64 chain's, at most 4 u64 (|f_i| +
+                // S dmax)
                 constexpr float EPS32 = 5.9604645e-8f, U64 = 1.1102230e-16f;
-                const float R = __double2float_ru(xb) + dmax;
+                const float R = dmax * (1.f + 4.f * EPS32) + 1e-30f;
                 float thHi[NF], thLo[NF];
-                bool ok = true, flat[NF];
+                bool ok = dmax < 1e30f, flat[NF];
 #pragma unroll
                 for (int f = 0; f < NF; ++f) {
                     bool z = true;
@@ -1833,33 +1831,43 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                     flat[f] = z;
                     const float fa = fabsf(__double2float_rn(fi[f]));
                     const float SR = S * R;
-                    ok = ok && SR < 1e36f && fa < 1e36f;   // false for NaN and infinity
-                    const float B = 12.f * EPS32 * SR + 12.f * U64 * (fa + SR) + 1e-36f;
+                    ok = ok && SR < 1e36f && S < 1e36f && fa < 1e36f;   // false for NaN and infinity
+                    const float B = 16.f * EPS32 * SR + 12.f * U64 * (fa + SR) + 1e-36f;
                     thHi[f] = z ? FLT_INF_ : hiQ[f] - 2.f * B;
                     thLo[f] = z ? -FLT_INF_ : loQ[f] + 2.f * B;
                 }
-                const int t64 = tot < 64 ? tot : 64;
-                unsigned long long cand = t64 == 64 ? ~0ull : ((1ull << t64) - 1ull);
-                if (ok) {
-                    cand = 0ull;
-                    for (int s = 0; s < t64; ++s) {
-                        float d[3];
-                        offset_f(nbr[base + s], nullptr, d);
-                        bool c = false;
+                // the candidates as a bit mask, every lane walking its own afterwards
+                // (taken where they stand, some lane of the warp would want nearly
+                // every slot); slots from the 65th on are all candidates
+                unsigned long long cand = 0ull;
+                for (int s = 0; s < tot; ++s) {
+                    float df[3];
+                    double d[3];
+                    offset_f(s, df, d);
+                    bool c = !ok;
 #pragma unroll
-                        for (int f = 0; f < NF; ++f) {
-                            const float q = incr(f, d);
-                            c = c || q >= thHi[f] || q <= thLo[f];
-                        }
-                        cand |= (unsigned long long)c << s;
+                    for (int f = 0; f < NF; ++f) {
+                        const float q = incr(f, df);
+                        c = c || q >= thHi[f] || q <= thLo[f];
                     }
+                    cand |= (unsigned long long)(c && s < 64) << (s & 63);
+                    if (s >= 64) exact_slot(d);
+                    store_psi(s, d);
                 }
+                // psi holds V_i psi~ now: the few candidates' offsets from the records
+                const GridInfo &g = grids[mi];
                 while (cand) {
                     const int s = __ffsll((long long)cand) - 1;
                     cand &= cand - 1ull;
-                    exact_slot(s);
+                    const uint32_t e = nbr[base + s];
+                    const Prim pj = prim[e & IDX_MASK];
+                    double xj[3], d[3];
+                    neighbour_pos<D>(e, pj, g, xj);
+                    const double xi[3] = {pi.x, pi.y, pi.z};
+#pragma unroll
+                    for (int a = 0; a < D; ++a) d[a] = subr(xj[a], xi[a]);
+                    exact_slot(d);
                 }
-                for (int s = 64; s < tot; ++s) exact_slot(s);
                 if (tot > 0) {
 #pragma unroll
                     for (int f = 0; f < NF; ++f)
@@ -1881,8 +1889,8 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
             for (int f = 0; f < NF; ++f) {
                 const double xN = key_double(mxN[f]), nN = key_double(mnN[f]);
                 const double xM = key_double(mxM[f]), nM = key_double(mnM[f]);
-                double aMax = ref_abs((xN - fi[f]) / (xM - fi[f]), p.int_abs);
-                double aMin = ref_abs((fi[f] - nN) / (fi[f] - nM), p.int_abs);
+                double aMax = ref_abs(fdiv_rn(subr(xN, fi[f]), subr(xM, fi[f])), p.int_abs);
+                double aMin = ref_abs(fdiv_rn(subr(fi[f], nN), subr(fi[f], nM)), p.int_abs);
                 if (aMin <= aMax && p.beta * aMin < 1.) {
 #pragma unroll
                     for (int a = 0; a < D; ++a) gr[f][a] *= aMin;
@@ -1890,6 +1898,13 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
 #pragma unroll
                     for (int a = 0; a < D; ++a) gr[f][a] *= aMax;
                 }
+            }
+        }
+        else {
+            for (int s = 0; s < tot; ++s) {
+                const double *ds = psi + (base + s) * 3;
+                const double d[3] = {ds[0], ds[1], D == 3 ? ds[2] : 0.};
+                store_psi(s, d);
             }
         }
         Grad go;
@@ -2180,7 +2195,7 @@ void launch_step(StepArgs &a) {
             cudaFuncSetAttribute(k_neighbours<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_neighbours<D><<<blocks, NNS_WARPS * 32, smem, s>>>(
             p, a.members, a.memberOf, a.grids, a.x, a.y, a.z, a.posf, a.vx, a.vy, a.vz, a.m, a.u, a.cellTotal,
-            a.cellStart, a.cellList, a.nbr, a.rr, a.ww, a.noi, a.noiImg, a.faceCnt, a.prim, a.geo, a.velf, a.status);
+            a.cellStart, a.cellList, a.nbr, a.psi, a.ww, a.noi, a.noiImg, a.faceCnt, a.prim, a.geo, a.velf, a.status);
     }
     tock(KT_NNS);
 
@@ -2219,8 +2234,8 @@ void launch_step(StepArgs &a) {
     if (dt_filter) cudaMemsetAsync(a.dtcap, 0x7f, sizeof(unsigned) * (size_t)a.nmembers, s);
     if (a.separate_dt) {
         tick(KT_DT);
-        k_timestep<D><<<(p.n + 255) / 256, 256, 0, s>>>(p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.rr,
-                                                        a.noi, a.dtbits, nullptr, nullptr);
+        k_timestep<D><<<(p.n + 255) / 256, 256, 0, s>>>(p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.noi,
+                                                        a.dtbits, nullptr, nullptr);
         tock(KT_DT);
     }
     tick(KT_GRAD);
@@ -2229,14 +2244,14 @@ void launch_step(StepArgs &a) {
         cudaMemsetAsync(a.faces, 0xff, sizeof(FaceRef) * a.faces_cap, s);
     }
     k_gradients<D><<<(p.n + gT - 1) / gT, gT, 0, s>>>(p, a.members, a.memberOf, a.grids, a.prim, a.geo, a.nbr, a.ww,
-                                                      a.rr, a.noi, a.noiImg, a.grad, a.gradRaw, a.psi,
+                                                      a.noi, a.noiImg, a.grad, a.gradRaw, a.psi,
                                                       (p.adaptive && !a.separate_dt && !dt_filter) ? a.dtbits : nullptr,
                                                       fused ? a.faceOff : nullptr, a.faceOf, a.faces, a.status,
-                                                      a.posf, a.tune.fp32_filters, a.velf, dt_filter ? a.dtlo : nullptr,
+                                                      a.tune.fp32_filters, a.velf, dt_filter ? a.dtlo : nullptr,
                                                       a.dtcap);
     if (dt_filter)
-        k_timestep<D><<<(p.n + 255) / 256, 256, 0, s>>>(p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.rr,
-                                                        a.noi, a.dtbits, a.dtlo, a.dtcap);
+        k_timestep<D><<<(p.n + 255) / 256, 256, 0, s>>>(p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.noi,
+                                                        a.dtbits, a.dtlo, a.dtcap);
     k_dt_final<<<(a.nmembers + 127) / 128, 128, 0, s>>>(p, a.nmembers, a.dtbits, a.dt_max, a.dt);
     tock(KT_GRAD);
     if (a.stop_after_gradients) return;

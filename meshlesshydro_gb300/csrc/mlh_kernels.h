@@ -60,7 +60,7 @@ struct StepArgs {
     int *cell, *cellCount, *cellStart, *cellFill, *cellList;
     // neighbours
     uint32_t *nbr;
-    double *rr, *ww, *psi;
+    double *ww, *psi;          // W; per slot x_j - x_i from the search, then V_i psi~ from the gradients
     int *noi, *noiImg, *faceCnt, *faceOff, *faceOf;
     FaceRef *faces;
     // per particle
