@@ -1350,7 +1350,17 @@ __global__ void k_dt_final(Params p, int nmembers, const unsigned long long *__r
 // copied with the opposite sign), face -> (i, slot, reverse slot).  The
 // reverse slot of a non-canonical slot is the first entry of j's list (real
 // part or image part) that refers to i, as in the reference's searches.
-// The face links of particle i (see k_link).
+// The face links of particle i by one thread.  A slot with j < i finds i in j's
+// list (real part or image part) and the face's rank in j's list from j's
+// canonical entries (index > j) on one side of it: searching forward, the rank
+// is the count before i; searching backward from the end of j's list, it is
+// faceCnt[j] - 1 - the count after i, faceCnt[j] = faceOff[j + 1] - faceOff[j]
+// being the number of canonical entries of j's list.  The stencils of i and j
+// mirror each other, so j early in i's list puts i late in j's list: those
+// searches and the image searches (images sit at the end of the list) go
+// backward.  The own list is read four slots per load (K is a multiple of 4)
+// and the searches of those four slots advance together, one 4-entry load of
+// each list per round, so that a thread has up to four loads in flight.
 __device__ __forceinline__ void link_particle(int i, const Params &p, const uint32_t *__restrict__ nbr,
                                               const int *__restrict__ noi, const int *__restrict__ noiImg,
                                               const int *__restrict__ faceOff, int *__restrict__ faceOf,
@@ -1436,26 +1446,86 @@ __device__ __forceinline__ void link_particle(int i, const Params &p, const uint
     }
 }
 
+// The face links as two kernels.  k_link_own, a warp per particle and a lane
+// per slot: a slot with j > i owns face faceOff[i] + its rank among i's
+// canonical slots (a ballot); the other slots are set to 0 until their face
+// finds them.
+__global__ void __launch_bounds__(256) k_link_own(Params p, const uint32_t *__restrict__ nbr,
+                                                  const int *__restrict__ noi, const int *__restrict__ noiImg,
+                                                  const int *__restrict__ faceOff, int *__restrict__ faceOf,
+                                                  FaceRef *__restrict__ faces, unsigned *__restrict__ status) {
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    bool full = false;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < p.n; i += nw) {
+        const size_t base = (size_t)i * p.K;
+        const int tot = noi[i] + noiImg[i];
+        int rank = faceOff[i];
+        for (int s0 = 0; s0 < tot; s0 += 32) {
+            const int s = s0 + lane;
+            const bool canon = s < tot && (int)(nbr[base + s] & IDX_MASK) > i;
+            const unsigned cm = __ballot_sync(0xffffffffu, canon);
+            const int f = rank + __popc(cm & ((1u << lane) - 1u));
+            const bool fits = canon && f < p.faces_cap;
+            if (s < tot) faceOf[base + s] = fits ? f + 1 : 0;
+            if (fits) { faces[f].i = i; faces[f].slot = s; }
+            full = full || (canon && !fits);
+            rank += __popc(cm);
+        }
+    }
+    if (full) flag(status, ST_CAPACITY);
+}
+
+// k_link, a thread per face: finds i in j's list (real part or image part) and
+// links that slot, faceOf = -(face + 1) and the face's rslot; each slot with
+// j < i is found by the one face it belongs to (one that no face finds keeps 0
+// and is reported by the flux gather).  The stencils of i and j mirror each
+// other, so slot s of i's real part puts i near slot noi[j] - 1 - s of j's: the
+// search starts at that 4-entry chunk and widens to both sides.  Images are
+// ordered by parent index: that part is searched from its start.  Sedov 64^3 /
+// 128^3 / 64 KH members, with the scan of the face counts: 130 / 1015 / 276 us; a thread
+// per particle, searching four lists in lockstep from their ends (link_particle,
+// which the gradients kernel runs with link_overlap 2), took 288 / 1771 / 446 us,
+// 700 warp instructions per particle with 13 of 32 lanes active.
 __global__ void __launch_bounds__(256) k_link(Params p, const uint32_t *__restrict__ nbr, const int *__restrict__ noi,
-                                              const int *__restrict__ noiImg, const int *__restrict__ faceOff,
+                                              const int *__restrict__ noiImg, const int *__restrict__ faceTotal,
                                               int *__restrict__ faceOf, FaceRef *__restrict__ faces,
                                               unsigned *__restrict__ status) {
-    // faces[] was set to -1: the owner writes (i, slot), the slot on the other
-    // side writes rslot, so each field has exactly one writer.  A slot with
-    // j > i owns face faceOff[i] + (its rank among i's canonical slots).  A
-    // slot with j < i finds i in j's list (real part or image part) and the
-    // face's rank in j's list from j's canonical entries (index > j) on one
-    // side of it: searching forward, the rank is the count before i; searching
-    // backward from the end of j's list, it is faceCnt[j] - 1 - the count
-    // after i, faceCnt[j] = faceOff[j + 1] - faceOff[j] being the number of
-    // canonical entries of j's list.  The stencils of i and j mirror each
-    // other, so j early in i's list puts i late in j's list: those searches
-    // and the image searches (images sit at the end of the list) go backward.
-    // The own list is read four slots per load (K is a multiple of 4) and the
-    // searches of those four slots advance together, one 4-entry load of each
-    // list per round, so that a thread has up to four loads in flight.
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += gridDim.x * blockDim.x)
-        link_particle(i, p, nbr, noi, noiImg, faceOff, faceOf, faces, status);
+    const int nf = *faceTotal < p.faces_cap ? *faceTotal : p.faces_cap;
+    bool lost = false;
+    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
+        const int i = faces[f].i, s = faces[f].slot;
+        const uint32_t e = nbr[(size_t)i * p.K + s];
+        const int j = (int)(e & IDX_MASK);
+        const bool img = (e >> IMG_SHIFT) != 0u;
+        const int nrj = noi[j];
+        // the part of j's list that i is sought in, and the chunks that hold it
+        const int lo = img ? nrj : 0, hi = img ? nrj + noiImg[j] : nrj;
+        int at = -1;
+        if (hi > lo) {
+            const uint4 *row = reinterpret_cast<const uint4 *>(nbr + (size_t)j * p.K);
+            const int c_lo = lo >> 2, c_hi = (hi - 1) >> 2, guess = nrj - 1 - s;
+            int c = img ? c_lo : guess > 0 ? guess >> 2 : 0;
+            int up = c + 1, dn = c - 1;   // the next chunks on either side
+            bool go_up = true;
+            for (;;) {
+                const uint4 v = row[c];
+                const uint32_t ev[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int t = c * 4 + m;
+                    if ((int)(ev[m] & IDX_MASK) == i && t >= lo && t < hi) at = t;   // a part holds i once
+                }
+                const bool can_up = up <= c_hi, can_dn = dn >= c_lo;
+                if (at >= 0 || !(can_up || can_dn)) break;
+                c = can_up && (go_up || !can_dn) ? up++ : dn--;
+                go_up = !go_up;
+            }
+        }
+        faces[f].rslot = at;
+        if (at >= 0) faceOf[(size_t)j * p.K + at] = -(f + 1);
+        else lost = true;
+    }
+    if (lost) flag(status, ST_ASYMMETRIC);
 }
 
 // ------------------------------------------------------------------ gradients
@@ -2010,7 +2080,10 @@ __global__ void __launch_bounds__(256) k_update(Params p, const int *__restrict_
             for (int k = 0; k < 4; ++k) {
                 const int fo = fos[k];
                 const int af = fo > 0 ? fo : -fo;
-                if (!(s0 + k < tot && fo != 0 && af <= p.faces_cap)) continue;
+                if (!(s0 + k < tot && fo != 0 && af <= p.faces_cap)) {
+                    if (s0 + k < tot && fo == 0) st_local |= ST_ASYMMETRIC;   // a slot that no face found
+                    continue;
+                }
                 // the flux with the slot's sign: the sign bit flipped on the
                 // integer pipe for a copied face, so that both kinds of slot
                 // share one set of additions (x + (-f) is the same double as
@@ -2207,11 +2280,16 @@ void launch_step(StepArgs &a) {
     // 0: in order
     const bool fused = a.tune.link_overlap == 2 && !a.stop_after_gradients;
     const bool overlap = !fused && a.stream2 && !a.timer && !a.stop_after_gradients && a.tune.link_overlap == 1;
-    const int blocksLink = blocksN;
+    auto grid_of = [&](long long threads) {   // blocks of 256 threads, at most 8 rounds of a full GPU
+        const long long b = (threads + 255) / 256, most = a.sm_count * 64ll;
+        return (int)(b < 1 ? 1 : b < most ? b : most);
+    };
     auto launch_links = [&](cudaStream_t ls) {
         exclusive_scan(a.faceCnt, p.n, a.faceOff, a.scanTiles, a.scanTotal, ls);
-        cudaMemsetAsync(a.faces, 0xff, sizeof(FaceRef) * a.faces_cap, ls);
-        k_link<<<blocksLink, T, 0, ls>>>(p, a.nbr, a.noi, a.noiImg, a.faceOff, a.faceOf, a.faces, a.status);
+        k_link_own<<<grid_of(32ll * p.n), 256, 0, ls>>>(p, a.nbr, a.noi, a.noiImg, a.faceOff, a.faceOf, a.faces,
+                                                        a.status);
+        k_link<<<grid_of((long long)a.faces_cap), 256, 0, ls>>>(p, a.nbr, a.noi, a.noiImg, a.faceOff + p.n, a.faceOf,
+                                                                a.faces, a.status);
     };
     if (overlap) {
         cudaEventRecord(a.ev_fork, s);
