@@ -1298,24 +1298,34 @@ __global__ void __launch_bounds__(256) k_timestep(Params p, const Member *__rest
             const int m = memberOf ? memberOf[i] : 0;
             cand = dtlo[i] <= __uint_as_float(dtcap[m]);
         }
-        if (cand) {
-            mi = memberOf ? memberOf[i] : 0;
-            const Prim pi = prim[i];
-            const double ci = geo[i].c;
+        // the warp's candidates one after another, a lane per neighbour: a handful
+        // of candidates would leave a thread each to a chain of dependent loads
+        // (KH 100^2: 20.7 us with a thread per candidate, 6.5 so)
+        unsigned todo = __ballot_sync(0xffffffffu, cand);
+        if (cand) mi = memberOf ? memberOf[i] : 0;
+        while (todo) {
+            const int b = __ffs((int)todo) - 1, ib = i0 + b;
+            todo &= todo - 1u;
+            const Prim pi = prim[ib];
+            const double ci = geo[ib].c;
+            const size_t base = (size_t)ib * p.K;
+            const int nr = noi[ib];
             double vSig = DBL_MIN_;
-            const size_t base = (size_t)i * p.K;
-            const int nr = noi[i];
-            for (int s = 0; s < nr; ++s) {
+            for (int s = lane; s < nr; s += 32) {
                 const int j = (int)(nbr[base + s] & IDX_MASK);
                 const Prim pj = prim[j];
                 const double cj = geo[j].c;
-                double xij[3] = {pi.x - pj.x, pi.y - pj.y, pi.z - pj.z};
-                double vij[3] = {pi.vx - pj.vx, pi.vy - pj.vy, pi.vz - pj.vz};
-                const double dv = dotD<D>(vij, xij);
-                const double vs = signal_speed<D>(dv, xij, ci + cj);
+                const double xij[3] = {subr(pi.x, pj.x), subr(pi.y, pj.y), subr(pi.z, pj.z)};
+                const double vij[3] = {subr(pi.vx, pj.vx), subr(pi.vy, pj.vy), subr(pi.vz, pj.vz)};
+                const double vs = signal_speed<D>(dotD<D>(vij, xij), xij, addr(ci, cj));
                 vSig = dlt(vSig, vs) ? vs : vSig;
             }
-            dti = (p.adaptive_h ? p.cfl * p.hp[i] : members[mi].cfl_h) / vSig;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double t = __shfl_xor_sync(0xffffffffu, vSig, o);
+                vSig = dlt(vSig, t) ? t : vSig;
+            }
+            if (lane == b) dti = (p.adaptive_h ? p.cfl * p.hp[ib] : members[mi].cfl_h) / vSig;
         }
         // the minimum over particles does not depend on the order of the
         // atomicMin calls: a warp inside one simulation (the common case)
@@ -1584,18 +1594,19 @@ __device__ __forceinline__ double field_of(const Prim &q, int f) {
 // per-member minimum (warp reduction, then one atomicMin on its bit pattern).
 // Bound: the FP64 pipe (79 % active on Sedov 64^3, 1625 instructions per
 // particle, 41 per neighbour) and, at 12 warps per SM, the latency of the
-// gathers.  One gather of the neighbours' records instead of three, the next
-// one's in flight while one is summed: Sedov 128^3 8.29 -> 6.98 ms, 64 KH
-// members 1.55 -> 1.27 ms, KH 100^2 93 -> 78 us (with the time step's kernel).
-// Register caps, Sedov 128^3: 7.64 ms at 144 and 7.48 at 128 registers (a spill
-// that 16 warps do not make up for), 7.82 at 200.  The products of the offsets
+// gathers.  One gather of the neighbours' records instead of three (the sums and
+// the neighbours' extrema), the next one's in flight while one is summed: Sedov
+// 128^3 8.29 -> 6.51 ms, 64 KH members 1.55 -> 1.18 ms, KH 100^2 93 -> 64 us
+// (with the time step's kernel).  Register caps, Sedov 128^3: 6.62 ms at 160 and
+// 6.82 at 128 registers (a spill that 16 warps do not make up for), 7.21 at 200;
+// 64 KH members: 1.23 / 1.19 / 1.30 ms at 128 / 144 / 168.  The products of the offsets
 // on the integer pipe (xmul) made it slower, 7.34 ms: the chain per neighbour
 // gets longer.  Blocks of up to 256 threads.
 #ifndef MLH_GRAD_MAXREG
 #define MLH_GRAD_MAXREG 168
 #endif
 #ifndef MLH_GRAD_MAXREG_2D
-#define MLH_GRAD_MAXREG_2D 128
+#define MLH_GRAD_MAXREG_2D 144
 #endif
 #define MLH_GRAD_BOUNDS __maxnreg__(D == 3 ? MLH_GRAD_MAXREG : MLH_GRAD_MAXREG_2D)
 template <int D>
@@ -1651,6 +1662,13 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
         double gr[NF][3], fi[NF];
 #pragma unroll
         for (int f = 0; f < NF; ++f) { fi[f] = field_of<D>(pi, f); gr[f][0] = gr[f][1] = gr[f][2] = 0.; }
+        // extrema of the neighbours' values for the slope limiter, as integer
+        // keys (ord_key): the comparisons of the reference's if (max < f) max = f
+        // stay off the FP64 pipe
+        long long mxN[NF], mnN[NF];
+        const long long kmin = ord_key(DBL_MIN_), kmax = ord_key(DBL_MAX_);
+#pragma unroll
+        for (int f = 0; f < NF; ++f) { mxN[f] = kmin; mnN[f] = kmax; }
         // the next neighbour's record is on its way while this one is summed
         uint32_t en = tot > 0 ? nbr[base] : 0u, en2 = tot > 1 ? nbr[base + 1] : 0u;
         Prim pn = prim[en & IDX_MASK];
@@ -1674,9 +1692,12 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 for (int b = a; b < D; ++b) E[D * a + b] = fma(d[a], dp[b], E[D * a + b]);
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
-                const double df = subr(field_of<D>(pj, f), fi[f]);
+                const double fj = field_of<D>(pj, f), df = subr(fj, fi[f]);
 #pragma unroll
                 for (int a = 0; a < D; ++a) gr[f][a] = fma(df, dp[a], gr[f][a]);
+                const long long kj = ord_key(fj);
+                if (mxN[f] < kj) mxN[f] = kj;
+                if (mnN[f] > kj) mnN[f] = kj;
             }
             if (want_dt && s < nr) {
                 // x_ij = x_i - x_j is the exact negation of d
@@ -1777,12 +1798,10 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
             }
         };
         if (p.slope) {
-            // running extrema as integer keys (ord_key): the comparisons of
-            // the reference's if (max < f) max = f stay off the FP64 pipe
-            long long mxN[NF], mnN[NF], mxM[NF], mnM[NF];
-            const long long kmin = ord_key(DBL_MIN_), kmax = ord_key(DBL_MAX_);
+            // extrema of the face-point values, as integer keys
+            long long mxM[NF], mnM[NF];
 #pragma unroll
-            for (int f = 0; f < NF; ++f) { mxN[f] = kmin; mnN[f] = kmax; mxM[f] = kmin; mnM[f] = kmax; }
+            for (int f = 0; f < NF; ++f) { mxM[f] = kmin; mnM[f] = kmax; }
             // face point x_ij = x_i + c (x_j - x_i): c = 1/2 (first-order
             // quadrature point) or h/4 (the reference's other choice);
             // f_ij = f_i + grad f . (x_ij - x_i) as one FMA chain from f_i, with
@@ -1815,13 +1834,6 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
             };
             if (!(fp32_filters & MLH_FILTER_SLOPE)) {
                 for (int s = 0; s < tot; ++s) {
-                    const Prim pj = prim[nbr[base + s] & IDX_MASK];
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) {
-                        const long long kj = ord_key(field_of<D>(pj, f));
-                        if (mxN[f] < kj) mxN[f] = kj;
-                        if (mnN[f] > kj) mnN[f] = kj;
-                    }
                     const double *ds = psi + (base + s) * 3;
                     const double d[3] = {ds[0], ds[1], D == 3 ? ds[2] : 0.};
                     exact_slot(d);
@@ -1860,13 +1872,6 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
 #pragma unroll
                 for (int f = 0; f < NF; ++f) { hiQ[f] = -FLT_MAX_; loQ[f] = FLT_MAX_; }
                 for (int s = 0; s < tot; ++s) {
-                    const Prim pj = prim[nbr[base + s] & IDX_MASK];
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) {
-                        const long long kj = ord_key(field_of<D>(pj, f));
-                        if (mxN[f] < kj) mxN[f] = kj;
-                        if (mnN[f] > kj) mnN[f] = kj;
-                    }
                     float df[3];
                     double d[3];
                     offset_f(s, df, d);
