@@ -74,6 +74,7 @@ struct mlh_ctx {
     // grids (one per member)
     GridInfo *grids = nullptr;
     int *cellTotal = nullptr;
+    long long cells_est = 0;
     double *boundsPart = nullptr;
     int *cell = nullptr, *cellCount = nullptr, *cellStart = nullptr, *cellFill = nullptr, *cellList = nullptr;
     // neighbours (capacity K slots per particle)
@@ -203,10 +204,11 @@ int alloc_cell_buffers(mlh_ctx *c) {
     return 0;
 }
 
-long long estimate_cells(const mlh_config &cfg, const mlh_particles_view *v, const Member &mb) {
+// the cells of a simulation's grid, with room for an expanding bounding box; *now: without
+long long estimate_cells(const mlh_config &cfg, const mlh_particles_view *v, const Member &mb, long long *now) {
     double lo[3], hi[3];
     const double *X[3] = {v->x, v->y, v->z};
-    long long total = 1;
+    long long total = 1, exact = 1;
     for (int a = 0; a < cfg.dim; ++a) {
         if (cfg.periodic) { lo[a] = mb.box_lo[a]; hi[a] = mb.box_hi[a]; }
         else {
@@ -218,9 +220,11 @@ long long estimate_cells(const mlh_config &cfg, const mlh_particles_view *v, con
         }
         double c = std::floor((hi[a] - lo[a]) / mb.h);
         long long ci = c >= 1. ? (long long)c : 1;
+        exact *= ci;
         if (!cfg.periodic) ci = ci + ci / 4 + 4;   // room for an expanding bounding box
         total *= ci;
     }
+    *now += exact;
     return total;
 }
 
@@ -289,7 +293,7 @@ StepArgs make_args(mlh_ctx *c, double dt_max) {
     a.velf = c->velf; a.dtlo = c->dtlo; a.dtcap = c->dtcap;
     a.nmembers = c->nmembers; a.bpm = c->bpm;
     a.members = c->members; a.memberOf = c->memberOf;
-    a.grids = c->grids; a.cellTotal = c->cellTotal; a.boundsPart = c->boundsPart;
+    a.grids = c->grids; a.cellTotal = c->cellTotal; a.cells_est = c->cells_est; a.boundsPart = c->boundsPart;
     a.cell = c->cell; a.cellCount = c->cellCount; a.cellStart = c->cellStart; a.cellFill = c->cellFill;
     a.cellList = c->cellList;
     a.nbr = c->nbr; a.ww = c->ww; a.psi = c->psi;
@@ -436,7 +440,7 @@ static int create_impl(const mlh_config *cfg, int nmembers, const mlh_member *md
     // starts on a 16-byte boundary (read as uint4 by k_link)
     c->p.K = round_slots(cfg->max_neighbours > 0 ? cfg->max_neighbours : (cfg->dim == 2 ? 40 : 64));
     long long nc = 0;
-    for (const Member &mb : mem) nc += estimate_cells(*cfg, init, mb);
+    for (const Member &mb : mem) nc += estimate_cells(*cfg, init, mb, &c->cells_est);
     if (nc > (1ll << 30)) { delete c; g_last_error = "grid too large"; return MLH_ERR_CAPACITY; }
     c->p.ncells_cap = (int)nc;
     int rc = 0;

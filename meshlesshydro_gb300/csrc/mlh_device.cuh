@@ -134,15 +134,15 @@ struct Harvest {
 __device__ __forceinline__ double kernelW2(double r, double ih2, double sigma, double sigma4) {
     // r >= 0, so q >= 0 and the range tests compare bit patterns (integer
     // pipe): q <= 1 and q < 2
-    const double q = __dmul_rn(r, ih2);
+    const double q = mulr(r, ih2);
     const long long qb = __double_as_longlong(q);
     const bool inner = qb <= 0x3FF0000000000000ll;
     const double t = __fma_rn(inner ? -0.5 : -1., q, inner ? 1. : 2.);
-    const double y = __dmul_rn(inner ? 1.5 : t, inner ? q : t);
-    const double z = __dmul_rn(y, inner ? q : t);
+    const double y = mulr(inner ? 1.5 : t, inner ? q : t);
+    const double z = mulr(y, inner ? q : t);
     const double zs = __longlong_as_double(__double_as_longlong(z) ^ (inner ? (long long)0x8000000000000000ull : 0ll));
     const double w = __fma_rn(zs, inner ? t : 1., inner ? 1. : 0.);
-    const double W = __dmul_rn(inner ? sigma : sigma4, w);
+    const double W = mulr(inner ? sigma : sigma4, w);
     return qb < 0x4000000000000000ll ? W : 0.;
 }
 // Particles.cpp:10-15 (the value of the kernel at r = 0 is sigma)

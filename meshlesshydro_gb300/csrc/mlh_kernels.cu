@@ -504,28 +504,36 @@ __global__ void __launch_bounds__(PB_T) k_binning(const double *__restrict__ x, 
 // Then Particles::compDensity/compOmega (Particles.cpp:1151-1184, 2262-2290)
 // and compPressure (:1272-1288) for the particle.
 //
-// One warp per cell: the particles of a cell share the candidate sequence
-// (the stencil cells of their cell, in order), so the warp stages it in
-// shared memory once, 128 candidates at a time (index with image bits, and
-// the single-precision position with the image shift applied), and filters
-// every chunk for a batch of up to NNS_PB particles of the cell against the
-// staged copy: a single-precision distance test against a bound slightly
-// above h^2, survivors compacted with a ballot into the particle's shared
-// list in stencil order.  Then, particle by particle, phase 2: the lanes take
-// the survivors 32 at a time and apply the reference's FP64 test exactly (d^2
-// = (dx*dx + dy*dy) + dz*dz < h*h, no fused multiply-add), compute
-// W(r), and append real neighbours (in order) to the slot list and images to
-// a shared list, which is then placed behind the real neighbours sorted by
-// parent index.  The single-precision test only decides which candidates
-// phase 2 sees; it passes every neighbour (its error is far below the bound's
-// margin), so the lists are those of the FP64 test alone.
+// One warp per cell (or per part of one, `nsplit` of them, where the cells are
+// too few to fill the GPU): the particles of a cell share the candidate sequence
+// (the stencil cells of their cell, in order).  Phase 1: the lanes hold 128
+// candidates at a time in registers (index with image bits, and the single-
+// precision position with the image shift applied) and test them against each
+// particle of a batch of up to NNS_PB, broadcast from the lane that holds it: a
+// single-precision distance test against a bound slightly above h^2, survivors
+// compacted with a ballot into the particle's shared list in stencil order.
+// Phase 2: the batch's lists are walked as one sequence, 32 candidates at a
+// time, with the reference's FP64 test exactly (d^2 = (dx*dx + dy*dy) + dz*dz <
+// h*h, no fused multiply-add) and W(r); real neighbours are appended (in order)
+// to the slot list, with their offsets, and images parked behind them, then
+// placed behind the real neighbours sorted by parent index.  Every count lives
+// on the lane of its particle and is kept with ballots.  The single-precision
+// test only decides which candidates phase 2 sees; it passes every neighbour
+// (its error is far below the bound's margin), so the lists are those of the
+// FP64 test alone.
+// Bound: the FP64 pipe (64 % active) and issue (45 %).  With the chunk staged in
+// shared memory and read back for every particle, counts in shared memory and a
+// loop over the particles for the images, this took 341 M warp instructions on
+// Sedov 64^3 and 4.48 ms on Sedov 128^3; now 218 M and 2.57 ms (64 KH members
+// 1015 -> 620 us, Sedov 33^3 168 -> 96, KH 24^2 38 -> 17).
 constexpr int NNS_WARPS = 8;
-constexpr int NNS_PB = 12;    // particles of a cell filtered per staged chunk
-constexpr int NNS_CH = 128;   // candidates per staged chunk
-// blocks of the neighbour search resident per SM: 3 caps it at 80 registers
-// and gives 24 warps per SM
+constexpr int NNS_PB = 12;    // particles of a cell per batch
+constexpr int NNS_REG = 4;    // candidates per lane held in registers (k_neighbours)
+constexpr int NNS_CH = 128;   // candidates per staged chunk (k_hsolve)
+// blocks of the neighbour search resident per SM: 4 caps it at 64 registers and
+// gives 32 warps per SM (Sedov 128^3: 2.57 ms, 2.91 at 3, 3.13 at 2)
 #ifndef MLH_NNS_MINB
-#define MLH_NNS_MINB 3
+#define MLH_NNS_MINB 4
 #endif
 
 struct NnsCells {
@@ -534,22 +542,23 @@ struct NnsCells {
     float shift[27][3];   // image shift of a wrapped axis (-L or +L, single precision), else 0
 };
 
-// shared memory of k_neighbours: NNS_WARPS NnsCells, then per warp the
-// staged chunk (NNS_CH float4 positions and entries), NNS_PB candidate lists
-// (K + 32 uint32 each), four NNS_PB int arrays (candidate counts, offsets in
-// the batch's sequence, real and image neighbour counts), image W (K doubles)
-// and image entries (K uint32), each rounded up to 16 bytes
+// shared memory of k_neighbours: NNS_WARPS NnsCells, then per warp NNS_PB
+// candidate lists (K + 32 uint32 each), the offsets of the lists in the batch's
+// sequence (NNS_PB ints), image W (K doubles) and image entries (K uint32), each
+// rounded up to 16 bytes
 __host__ __device__ constexpr size_t nns_cells_bytes() {
     return (sizeof(NnsCells) * NNS_WARPS + 15) / 16 * 16;
 }
 __host__ __device__ constexpr size_t nns_r16(size_t b) { return (b + 15) / 16 * 16; }
-// (with per-particle smoothing lengths also the staged chunk's h_j, NNS_CH
-// floats, at the end: without them the area of 8 warps stays within a third
-// of the SM's shared memory at K = 64, for 3 blocks per SM)
-__host__ __device__ constexpr size_t nns_warp_bytes(int K, bool adaptive = false) {
-    return (size_t)NNS_CH * 4 + (size_t)NNS_CH * 16 + nns_r16((size_t)NNS_PB * (K + 32) * 4) +
-           nns_r16((size_t)4 * NNS_PB * 4) + nns_r16((size_t)K * 8) + nns_r16((size_t)K * 4) +
-           (adaptive ? (size_t)NNS_CH * 4 : 0);
+__host__ __device__ constexpr size_t nns_warp_bytes(int K) {
+    return nns_r16((size_t)NNS_PB * (K + 32) * 4) + nns_r16((size_t)NNS_PB * 4) + nns_r16((size_t)K * 8) +
+           nns_r16((size_t)K * 4);
+}
+// bits [lo, hi) of a warp mask (any integers)
+__device__ __forceinline__ unsigned range_mask(int lo, int hi) {
+    lo = lo < 0 ? 0 : lo;
+    hi = hi > 32 ? 32 : hi;
+    return lo < hi ? (0xffffffffu >> (32 - (hi - lo))) << lo : 0u;
 }
 
 // The 3^D stencil cells of local cell ic in the reference's order
@@ -620,9 +629,9 @@ __device__ __forceinline__ int nns_cell_of(const NnsCells *cs, int t) {
     return k;
 }
 
-template <int D>
+template <int D, bool ADAPT>
 __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
-    Params p, const Member *__restrict__ members, const int *__restrict__ memberOf,
+    Params p, int nsplit, int pb, const Member *__restrict__ members, const int *__restrict__ memberOf,
     const GridInfo *__restrict__ grids, const double *__restrict__ x, const double *__restrict__ y,
     const double *__restrict__ z, const float4 *__restrict__ posf, const double *__restrict__ vx,
     const double *__restrict__ vy, const double *__restrict__ vz, const double *__restrict__ m,
@@ -630,6 +639,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
     const int *__restrict__ cellList, uint32_t *__restrict__ nbr, double *__restrict__ dd,
     double *__restrict__ ww, int *__restrict__ noi, int *__restrict__ noiImg, int *__restrict__ faceCnt,
     Prim *__restrict__ prim, Geo *__restrict__ geo, float4 *__restrict__ velf, unsigned *__restrict__ status) {
+    constexpr unsigned ALL = 0xffffffffu;
     const int K = p.K;
     const int CAP = K + 32;
     extern __shared__ __align__(16) unsigned char nns_smem[];
@@ -638,15 +648,11 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
     // per-warp shared areas; every sub-array starts on a 16-byte boundary
     // whatever K is (see nns_warp_bytes)
     NnsCells *cs = reinterpret_cast<NnsCells *>(nns_smem) + warp;
-    unsigned char *wbase = nns_smem + nns_cells_bytes() + (size_t)warp * nns_warp_bytes(K, p.adaptive_h);
-    float4 *stP = reinterpret_cast<float4 *>(wbase);                                  // staged positions
-    uint32_t *stE = reinterpret_cast<uint32_t *>(wbase + (size_t)NNS_CH * 16);        // staged entries
-    uint32_t *candq = stE + NNS_CH;                                                   // NNS_PB lists of CAP
-    int *ncq = reinterpret_cast<int *>(wbase + (size_t)NNS_CH * 20 + nns_r16((size_t)NNS_PB * CAP * 4));
-    int *offq = ncq + NNS_PB, *nrq = offq + NNS_PB, *niq = nrq + NNS_PB;
-    double *imgW = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(ncq) + nns_r16((size_t)4 * NNS_PB * 4));
-    uint32_t *imgE = reinterpret_cast<uint32_t *>(imgW + K);
-    float *stH = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(imgE) + nns_r16((size_t)K * 4));   // staged h_j
+    unsigned char *wbase = nns_smem + nns_cells_bytes() + (size_t)warp * nns_warp_bytes(K);
+    uint32_t *candq = reinterpret_cast<uint32_t *>(wbase);                            // NNS_PB lists of CAP
+    int *offq = reinterpret_cast<int *>(wbase + nns_r16((size_t)NNS_PB * CAP * 4));
+    double *imgW = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(offq) + nns_r16((size_t)NNS_PB * 4));
+    uint32_t *imgE = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(imgW) + nns_r16((size_t)K * 8));
 
     const double *X[3] = {x, y, z};
     // a binning that gave up a bounded wait left no valid cells
@@ -657,15 +663,15 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
     // lane): omega sums the stored W of the real neighbours in list order,
     // then W(0), then the images (Particles::compDensity, Particles.cpp:
     // 1151-1184, and its image part :2262-2290, in that order)
-    int bi = -1, bnr = 0, bni = 0, iter = 0;
+    int bi = -1, bnr = 0, bni = 0, filled = 0;   // filled: lanes 0 .. filled - 1 hold a particle
     double bw0 = 0.;
     auto finish = [&]() {
         if (bi < 0) return;
         const double *wb = ww + (size_t)bi * K;
         double bomega = 0.;
-        for (int s = 0; s < bnr; ++s) bomega += wb[s];
-        bomega += bw0;
-        for (int s = bnr; s < bnr + bni; ++s) bomega += wb[s];
+        for (int s = 0; s < bnr; ++s) bomega = addr(bomega, wb[s]);
+        bomega = addr(bomega, bw0);
+        for (int s = bnr; s < bnr + bni; ++s) bomega = addr(bomega, wb[s]);
         const double rho = m[bi] * bomega;
         const double P = (p.gamma - 1.) * rho * u[bi];
         // rho <= 0 and P <= 0 as sign tests on the bit patterns (a NaN with
@@ -690,225 +696,217 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
         velf[bi] = make_float4(__double2float_rn(pr.vx), __double2float_rn(pr.vy), __double2float_rn(pr.vz),
                                __double2float_rn(cs));
     };
-    const int ncells = *cellTotal;
-    for (int c = gw; c < ncells; c += nw) {
+    const int nunits = *cellTotal * nsplit;
+    for (int un = gw; un < nunits; un += nw) {
+        const int c = nsplit > 1 ? un / nsplit : un, part = nsplit > 1 ? un - c * nsplit : 0;
         const int c0 = cellStart[c], ncell = cellStart[c + 1] - c0;
-        if (ncell <= 0) continue;
+        if (ncell <= part * pb) continue;
         const int mi = memberOf ? memberOf[cellList[c0]] : 0;   // a cell holds one member's particles
-        const GridInfo g = grids[mi];
-        const Member mb = members[mi];
+        const GridInfo &g = grids[mi];
+        const Member &mb = members[mi];
         const int total = nns_stencil<D>(p, g, c - g.cell_base, cellStart, cs);
-        for (int b0 = 0; b0 < ncell; b0 += NNS_PB) {
-            const int nb = ncell - b0 < NNS_PB ? ncell - b0 : NNS_PB;
-            // --- phase 1 for the batch: particle q of the batch on lane q
-            int myI = -1;
+        for (int b0 = part * pb; b0 < ncell; b0 += nsplit * pb) {
+            const int nb = ncell - b0 < pb ? ncell - b0 : pb;
+            // --- phase 1: particle q of the batch and its candidate count on lane q
+            int myI = -1, myNc = 0;
             float4 myF = make_float4(0.f, 0.f, 0.f, 0.f);
             float myHf = 0.f;
             if (lane < nb) {
                 myI = cellList[c0 + b0 + lane];
                 myF = posf[myI];
-                if (p.adaptive_h) myHf = p.hpf[myI];
+                if (ADAPT) myHf = p.hpf[myI];
             }
-            if (lane < NNS_PB) ncq[lane] = 0;
-            __syncwarp();
-            for (int ch = 0; ch < total; ch += NNS_CH) {
-                const int cl = total - ch < NNS_CH ? total - ch : NNS_CH;
-                // stage candidates [ch, ch + cl) of the sequence
-                for (int t = lane; t < cl; t += 32) {
-                    const int k = nns_cell_of<D>(cs, ch + t);
-                    const int j = cellList[cs->start[k] + (ch + t - cs->excl[k])];
-                    const unsigned wr = cs->wrap[k];
-                    float4 fj = posf[j];
-                    if (wr) {
-                        fj.x += cs->shift[k][0];
-                        fj.y += cs->shift[k][1];
-                        if (D == 3) fj.z += cs->shift[k][2];
+            const float hsq_f = mb.hsq_f;
+            for (int ch = 0; ch < total; ch += 32 * NNS_REG) {
+                float cx[NNS_REG], cy[NNS_REG], cz[NNS_REG], chf[NNS_REG];
+                uint32_t ce[NNS_REG];
+#pragma unroll
+                for (int r = 0; r < NNS_REG; ++r) {
+                    const int t = ch + r * 32 + lane;
+                    cx[r] = FLT_INF_; cy[r] = 0.f; cz[r] = 0.f; chf[r] = 0.f; ce[r] = 0u;   // no candidate: infinitely far
+                    if (t < total) {
+                        const int k = nns_cell_of<D>(cs, t);
+                        const int j = cellList[cs->start[k] + (t - cs->excl[k])];
+                        const unsigned wr = cs->wrap[k];
+                        float4 fj = posf[j];
+                        if (wr) {
+                            fj.x += cs->shift[k][0];
+                            fj.y += cs->shift[k][1];
+                            if (D == 3) fj.z += cs->shift[k][2];
+                        }
+                        cx[r] = fj.x; cy[r] = fj.y; cz[r] = fj.z;
+                        ce[r] = (uint32_t)j | (wr << IMG_SHIFT);
+                        if (ADAPT) chf[r] = p.hpf[j];
                     }
-                    stP[t] = fj;
-                    stE[t] = (uint32_t)j | (wr << IMG_SHIFT);
-                    if (p.adaptive_h) stH[t] = p.hpf[j];
                 }
-                __syncwarp();
                 for (int q = 0; q < nb; ++q) {
-                    const uint32_t iq = (uint32_t)__shfl_sync(0xffffffffu, myI, q);
-                    const float fx = __shfl_sync(0xffffffffu, myF.x, q);
-                    const float fy = __shfl_sync(0xffffffffu, myF.y, q);
-                    const float fz = __shfl_sync(0xffffffffu, myF.z, q);
-                    const float hq = __shfl_sync(0xffffffffu, myHf, q);
-                    uint32_t *cq = candq + (size_t)q * CAP;
-                    int nq = ncq[q];
-                    for (int t0 = 0; t0 < cl; t0 += 32) {
-                        const int t = t0 + lane;
-                        bool pass = false;
-                        uint32_t ent = 0;
-                        if (t < cl) {
-                            ent = stE[t];
-                            if (ent != iq) {   // the particle itself (its images are candidates)
-                                const float4 fj = stP[t];
-                                const float dx = fj.x - fx, dy = fj.y - fy, dz = fj.z - fz;
-                                const float d2f = dx * dx + dy * dy + (D == 3 ? dz * dz : 0.f);
-                                // with per-particle smoothing lengths the pair needs
-                                // r < max(h_i, h_j): the same bound margin on the
-                                // rounded-up single-precision h
-                                float lim = mb.hsq_f;
-                                if (p.adaptive_h) {
-                                    const float m = fmaxf(hq, stH[t]);
-                                    lim = m * m * 1.001f;
-                                }
-                                pass = d2f <= lim;
-                            }
+                    const uint32_t iq = (uint32_t)__shfl_sync(ALL, myI, q);
+                    const float fx = __shfl_sync(ALL, myF.x, q), fy = __shfl_sync(ALL, myF.y, q);
+                    const float fz = D == 3 ? __shfl_sync(ALL, myF.z, q) : 0.f;
+                    const float hq = ADAPT ? __shfl_sync(ALL, myHf, q) : 0.f;
+                    int nq = __shfl_sync(ALL, myNc, q);
+                    uint32_t *cq = candq + q * CAP;
+#pragma unroll
+                    for (int r = 0; r < NNS_REG; ++r) {
+                        if (ch + r * 32 >= total) break;
+                        const float dx = cx[r] - fx, dy = cy[r] - fy, dz = cz[r] - fz;
+                        const float d2f = dx * dx + dy * dy + (D == 3 ? dz * dz : 0.f);
+                        // with per-particle smoothing lengths the pair needs
+                        // r < max(h_i, h_j): the same bound margin on the
+                        // rounded-up single-precision h
+                        float lim = hsq_f;
+                        if (ADAPT) {
+                            const float mh = fmaxf(hq, chf[r]);
+                            lim = mh * mh * 1.001f;
                         }
-                        const unsigned bal = __ballot_sync(0xffffffffu, pass);
-                        if (pass) {
-                            const int pos = nq + __popc(bal & lt_mask);
-                            if (pos < CAP) cq[pos] = ent;
-                        }
+                        // the particle itself is none (its images are candidates)
+                        const bool pass = d2f <= lim && ce[r] != iq;
+                        const unsigned bal = __ballot_sync(ALL, pass);
+                        const int pos = nq + __popc(bal & lt_mask);
+                        if (pass && pos < CAP) cq[pos] = ce[r];
                         nq += __popc(bal);
                     }
-                    __syncwarp();
-                    if (lane == 0) ncq[q] = nq;
-                    __syncwarp();
+                    if (lane == q) myNc = nq;
                 }
             }
-            // --- phase 2: exact FP64 test, r, W, over the candidate lists of
-            // the batch walked as one sequence, 32 candidates at a time (about
-            // 20 candidates per particle in 2D would leave a third of the lanes
-            // idle per particle).  With per-particle smoothing lengths the pair
-            // test is r^2 < max(h_i^2, h_j^2) and W uses h_i.  Particle q's
-            // position and kernel parameters live on lane q.  Real neighbours
-            // go to the front of the particle's slot row in candidate order,
-            // images to its back (slot K-1-t for the t-th), from where the
-            // per-particle step below sorts them behind the real ones.
-            {
-                const int myN = lane < nb ? (ncq[lane] < CAP ? ncq[lane] : CAP) : 0;
-                int myOff = myN;
+            // --- phase 2: exact FP64 test, offset, W.  With per-particle smoothing
+            // lengths the pair test is r^2 < max(h_i^2, h_j^2) and W uses h_i.
+            // Particle q's position, kernel parameters, list and counts live on
+            // lane q.  Real neighbours go to the front of the particle's slot row
+            // in candidate order, images to its back (slot K-1-t for the t-th),
+            // from where the step below sorts them behind the real ones.
+            const int myN = lane < nb ? (myNc < CAP ? myNc : CAP) : 0;
+            int myOff = myN;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, myOff, o);
-                    if (lane >= o) myOff += t;
-                }
-                const int seq = __shfl_sync(0xffffffffu, myOff, 31);
-                myOff -= myN;
-                if (lane < NNS_PB) { offq[lane] = myOff; nrq[lane] = 0; niq[lane] = 0; }
-                double myX[3] = {0., 0., 0.};
-                double myHsq = mb.hsq, myIh2 = mb.ih2, mySig = mb.sigma, mySig4 = 0.;
-                if (lane < nb) {
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(ALL, myOff, o);
+                if (lane >= o) myOff += t;
+            }
+            const int seq = __shfl_sync(ALL, myOff, 31);
+            myOff -= myN;
+            __syncwarp();   // the batch before has read offq
+            if (lane < NNS_PB) offq[lane] = lane < nb ? myOff : 0x7fffffff;
+            double myX[3] = {0., 0., 0.};
+            double myHsq = 0., myIh2 = 0., mySig = 0., mySig4 = 0., myW0 = 0.;
+            if (lane < nb) {
 #pragma unroll
-                    for (int a = 0; a < D; ++a) myX[a] = X[a][myI];
-                    if (p.adaptive_h) {
-                        const double hi_ = p.hp[myI];
-                        const double h2_i = hi_ / 2.;
-                        myHsq = __dmul_rn(hi_, hi_);
-                        myIh2 = 1. / h2_i;
-                        mySig = kernel_sigma<D>(h2_i);
-                    }
-                }
-                mySig4 = 0.25 * mySig;   // the outer piece's factor, once per particle (exact)
-                __syncwarp();
-                for (int t0 = 0; t0 < seq; t0 += 32) {
-                    const int gi = t0 + lane;
-                    const bool valid = gi < seq;
-                    // the particle of position gi: the last one whose list starts at
-                    // or before it (an empty list shares its offset with the next)
-                    int q = 0;
-#pragma unroll
-                    for (int l = 1; l < NNS_PB; ++l)
-                        if (l < nb && offq[l] <= gi) q = l;
-                    const int i = __shfl_sync(0xffffffffu, myI, q);
-                    double xi[3] = {0., 0., 0.};
-#pragma unroll
-                    for (int a = 0; a < D; ++a) xi[a] = __shfl_sync(0xffffffffu, myX[a], q);
-                    const double hsq_i = __shfl_sync(0xffffffffu, myHsq, q);
-                    const double ih2_i = __shfl_sync(0xffffffffu, myIh2, q);
-                    const double sigma_i = __shfl_sync(0xffffffffu, mySig, q);
-                    const double sigma4_i = __shfl_sync(0xffffffffu, mySig4, q);
-                    bool pass = false, img = false;
-                    uint32_t e = 0;
-                    double w = 0., ed[3] = {0., 0., 0.};
-                    if (valid) {
-                        e = candq[(size_t)q * CAP + (gi - offq[q])];
-                        const int j = (int)(e & IDX_MASK);
-                        const unsigned wr = e >> IMG_SHIFT;
-                        img = wr != 0;
-                        double xj[3];
-                        bool ok = true;
-#pragma unroll
-                        for (int a = 0; a < D; ++a) {
-                            xj[a] = X[a][j];
-                            if (wr & (1u << a)) {
-                                if (in_band(xj[a], g, a)) xj[a] = image_coord(xj[a], g, a);
-                                else ok = false;
-                            }
-                        }
-                        if (ok) {
-#pragma unroll
-                            for (int a = 0; a < D; ++a) ed[a] = subr(xj[a], xi[a]);
-                            double d2 = addr(mulr(ed[0], ed[0]), mulr(ed[1], ed[1]));
-                            if (D == 3) d2 = addr(d2, mulr(ed[2], ed[2]));
-                            // d2, h^2 >= 0: compared as bit patterns on the integer pipe
-                            double lim = mb.hsq;
-                            if (p.adaptive_h) {
-                                const double hj = p.hp[j];
-                                const double hsq_j = __dmul_rn(hj, hj);
-                                lim = __double_as_longlong(hsq_i) < __double_as_longlong(hsq_j) ? hsq_j : hsq_i;
-                            }
-                            pass = __double_as_longlong(d2) < __double_as_longlong(lim);
-                            if (pass) w = kernelW2(fsqrt_rn(d2), ih2_i, sigma_i, sigma4_i);
-                        }
-                    }
-                    // lanes of the same particle, and their ranks among its passes
-                    const unsigned grp = __match_any_sync(0xffffffffu, valid ? q : -1);
-                    const unsigned balR = __ballot_sync(0xffffffffu, pass && !img) & grp;
-                    const unsigned balI = __ballot_sync(0xffffffffu, pass && img) & grp;
-                    const int nr0 = nrq[q], ni0 = niq[q];
-                    const size_t base = (size_t)i * K;
-                    if (pass && !img) {
-                        const int pos = nr0 + __popc(balR & lt_mask);
-                        if (pos < K) {
-                            nbr[base + pos] = e;
-                            ww[base + pos] = w;
-#pragma unroll
-                            for (int a = 0; a < D; ++a) dd[(base + pos) * 3 + a] = ed[a];
-                        }
-                    }
-                    if (pass && img) {
-                        const int pos = ni0 + __popc(balI & lt_mask);
-                        if (pos < K) { nbr[base + K - 1 - pos] = e; ww[base + K - 1 - pos] = w; }
-                    }
-                    __syncwarp();
-                    if (valid && (grp & lt_mask) == 0) {   // first lane of each particle's group
-                        nrq[q] = nr0 + __popc(balR);
-                        niq[q] = ni0 + __popc(balI);
-                    }
-                    __syncwarp();
+                for (int a = 0; a < D; ++a) myX[a] = X[a][myI];
+                if (ADAPT) {
+                    const double hi_ = p.hp[myI];
+                    const double h2_i = hi_ / 2.;
+                    myHsq = __dmul_rn(hi_, hi_);
+                    myIh2 = 1. / h2_i;
+                    mySig = kernel_sigma<D>(h2_i);
+                    mySig4 = 0.25 * mySig;   // the outer piece's factor, once per particle (exact)
+                    myW0 = mySig;
                 }
             }
-            for (int q = 0; q < nb; ++q) {
-                const int i = __shfl_sync(0xffffffffu, myI, q);
-                bool overflow = ncq[q] > CAP;
-                int nr = nrq[q], ni = niq[q], fc = 0;
+            if (!ADAPT) { myIh2 = mb.ih2; mySig = mb.sigma; mySig4 = 0.25 * mySig; myW0 = mb.w0; }
+            const double hsq = mb.hsq;
+            __syncwarp();
+            int myNr = 0, myNi = 0, myFc = 0;
+            for (int t0 = 0; t0 < seq; t0 += 32) {
+                const int gi = t0 + lane;
+                const bool valid = gi < seq;
+                // the particle of position gi: the last one whose list starts at
+                // or before it (an empty list shares its offset with the next)
+                int q = 0;
+#pragma unroll
+                for (int l4 = 0; l4 < NNS_PB; l4 += 4) {
+                    const int4 o = *reinterpret_cast<const int4 *>(offq + l4);
+                    if (l4 > 0) q += o.x <= gi;
+                    q += (o.y <= gi) + (o.z <= gi) + (o.w <= gi);
+                }
+                const int i = __shfl_sync(ALL, myI, q), off = __shfl_sync(ALL, myOff, q), n_q = __shfl_sync(ALL, myN, q);
+                const int nr0 = __shfl_sync(ALL, myNr, q), ni0 = __shfl_sync(ALL, myNi, q);
+                double xi[3] = {0., 0., 0.};
+#pragma unroll
+                for (int a = 0; a < D; ++a) xi[a] = __shfl_sync(ALL, myX[a], q);
+                const double hsq_i = ADAPT ? __shfl_sync(ALL, myHsq, q) : hsq;
+                const double ih2_i = ADAPT ? __shfl_sync(ALL, myIh2, q) : myIh2;
+                const double sigma_i = ADAPT ? __shfl_sync(ALL, mySig, q) : mySig;
+                const double sigma4_i = ADAPT ? __shfl_sync(ALL, mySig4, q) : mySig4;
+                bool pass = false, img = false;
+                uint32_t e = 0;
+                double w = 0., ed[3] = {0., 0., 0.};
+                if (valid) {
+                    e = candq[q * CAP + (gi - off)];
+                    const int j = (int)(e & IDX_MASK);
+                    const unsigned wr = e >> IMG_SHIFT;
+                    img = wr != 0;
+                    double xj[3];
+                    bool ok = true;
+#pragma unroll
+                    for (int a = 0; a < D; ++a) {
+                        xj[a] = X[a][j];
+                        if (wr & (1u << a)) {
+                            if (in_band(xj[a], g, a)) xj[a] = image_coord(xj[a], g, a);
+                            else ok = false;
+                        }
+                    }
+                    if (ok) {
+#pragma unroll
+                        for (int a = 0; a < D; ++a) ed[a] = subr(xj[a], xi[a]);
+                        double d2 = addr(mulr(ed[0], ed[0]), mulr(ed[1], ed[1]));
+                        if (D == 3) d2 = addr(d2, mulr(ed[2], ed[2]));
+                        // d2, h^2 >= 0: compared as bit patterns on the integer pipe
+                        double lim = hsq;
+                        if (ADAPT) {
+                            const double hj = p.hp[j];
+                            const double hsq_j = __dmul_rn(hj, hj);
+                            lim = __double_as_longlong(hsq_i) < __double_as_longlong(hsq_j) ? hsq_j : hsq_i;
+                        }
+                        pass = __double_as_longlong(d2) < __double_as_longlong(lim);
+                        if (pass) w = kernelW2(fsqrt_rn(d2), ih2_i, sigma_i, sigma4_i);
+                    }
+                }
+                // ranks among the passes of the lane's particle, and the counts of
+                // the particle on this lane
+                const unsigned balR = __ballot_sync(ALL, pass && !img), balI = __ballot_sync(ALL, pass && img);
+                const unsigned balF = __ballot_sync(ALL, pass && (int)(e & IDX_MASK) > i);   // canonical faces
+                const unsigned grp = range_mask(off - t0, off - t0 + n_q) & lt_mask;
+                const unsigned own = range_mask(myOff - t0, myOff - t0 + myN);
                 const size_t base = (size_t)i * K;
-                double w0_i = mb.w0;
-                if (p.adaptive_h) w0_i = kernel_sigma<D>(p.hp[i] / 2.);
-                if (nr + ni > K || overflow) {
-                    overflow = true;
-                    if (nr > K) nr = K;
-                    if (ni > K - nr) ni = K - nr;
+                if (pass) {
+                    const int pos = img ? ni0 + __popc(balI & grp) : nr0 + __popc(balR & grp);
+                    if (pos < K) {
+                        const size_t sl = base + (img ? K - 1 - pos : pos);
+                        nbr[sl] = e;
+                        ww[sl] = w;
+                        if (!img) {
+#pragma unroll
+                            for (int a = 0; a < D; ++a) dd[sl * 3 + a] = ed[a];
+                        }
+                    }
                 }
+                myNr += __popc(balR & own);
+                myNi += __popc(balI & own);
+                myFc += __popc(balF & own);
+            }
+            __syncwarp();   // the slots written above are visible to every lane
+            // --- particles with images: behind the real neighbours, ordered by
+            // parent index (their offsets are formed again: few particles have
+            // images); particles that overflow their slots: clipped, and the step
+            // is repeated with more
+            const bool over = lane < nb && (myNc > CAP || myNr + myNi > K);
+            for (unsigned todo = __ballot_sync(ALL, lane < nb && (myNi > 0 || over)); todo; todo &= todo - 1u) {
+                const int q = __ffs((int)todo) - 1;
+                const int i = __shfl_sync(ALL, myI, q);
+                int nr = __shfl_sync(ALL, myNr, q), ni = __shfl_sync(ALL, myNi, q), fc = 0;
+                const size_t base = (size_t)i * K;
+                if (nr > K) nr = K;
+                if (ni > K - nr) ni = K - nr;
                 // images from the back of the row, in candidate order
                 for (int t = lane; t < ni; t += 32) {
                     imgE[t] = nbr[base + K - 1 - t];
                     imgW[t] = ww[base + K - 1 - t];
                 }
                 __syncwarp();
-                // --- images behind the real neighbours, ordered by parent index
-                // (their offsets are formed again: few particles have images, and
-                // a copy beside imgE and imgW would cost a resident block)
                 for (int t = lane; t < ni; t += 32) {
                     const uint32_t e = imgE[t];
                     const uint32_t id = e & IDX_MASK;
                     int rank = 0;
-                    for (int u = 0; u < ni; ++u) rank += (imgE[u] & IDX_MASK) < id;
+                    for (int v = 0; v < ni; ++v) rank += (imgE[v] & IDX_MASK) < id;
                     nbr[base + nr + rank] = e;
                     ww[base + nr + rank] = imgW[t];
 #pragma unroll
@@ -919,26 +917,39 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
                     }
                 }
                 __syncwarp();
-                // canonical faces among the stored slots (neighbour or parent > i);
-                // counted from the final list so that it matches k_link exactly
+                // canonical faces counted again from the final list, so that they
+                // match k_link_own where the list was clipped
                 for (int t = lane; t < nr + ni; t += 32) fc += (int)(nbr[base + t] & IDX_MASK) > i;
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) fc += __shfl_xor_sync(0xffffffffu, fc, o);
-                if (lane == 0) {
-                    if (overflow) flag(status, ST_NGB_OVERFLOW);
-                    if (nr + ni == 0) flag(status, ST_NO_NEIGHBOUR);
-                    noi[i] = nr;
-                    noiImg[i] = ni;
-                    faceCnt[i] = fc;
-                }
-                // the floating-point tail of every 32 particles of this warp runs
-                // once on all 32 lanes (lane k keeps the k-th particle); the stored
-                // slots are visible to every lane after the __syncwarp above
-                if (lane == (iter & 31)) { bi = i; bnr = nr; bni = ni; bw0 = w0_i; }
-                if ((iter & 31) == 31) { finish(); bi = -1; }
-                ++iter;
+                for (int o = 16; o > 0; o >>= 1) fc += __shfl_xor_sync(ALL, fc, o);
+                if (lane == q) { myNr = nr; myNi = ni; myFc = fc; }
                 __syncwarp();
-            }   // particles of the batch
+            }
+            if (lane < nb) {
+                noi[myI] = myNr;
+                noiImg[myI] = myNi;
+                faceCnt[myI] = myFc;
+                if (over) flag(status, ST_NGB_OVERFLOW);
+                if (myNr + myNi == 0) flag(status, ST_NO_NEIGHBOUR);
+            }
+            // the floating-point tail runs on all 32 lanes, once 32 particles of
+            // this warp are there: this batch's go to the lanes after the filled ones
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int src = lane - filled + 32 * half;   // the particle of the batch for this lane
+                const bool take = src >= 0 && src < nb;
+                const int ti = __shfl_sync(ALL, myI, src & 31), tr = __shfl_sync(ALL, myNr, src & 31);
+                const int tn = __shfl_sync(ALL, myNi, src & 31);
+                const double tw = ADAPT ? __shfl_sync(ALL, myW0, src & 31) : myW0;
+                if (take) { bi = ti; bnr = tr; bni = tn; bw0 = tw; }
+                if (half == 0) {
+                    if (filled + nb < 32) { filled += nb; break; }
+                    finish();
+                    bi = -1;
+                } else {
+                    filled += nb - 32;
+                }
+            }
         }   // batches of the cell
     }
     finish();
@@ -1252,8 +1263,8 @@ size_t hsolve_smem_bytes(int K) {
     return nns_cells_bytes() + (size_t)NNS_WARPS * hsolve_warp_bytes(K);
 }
 
-size_t nns_smem_bytes(int K, bool adaptive) {
-    return nns_cells_bytes() + (size_t)NNS_WARPS * nns_warp_bytes(K, adaptive);
+size_t nns_smem_bytes(int K) {
+    return nns_cells_bytes() + (size_t)NNS_WARPS * nns_warp_bytes(K);
 }
 
 // ------------------------------------------------------------------ dt
@@ -2266,14 +2277,31 @@ void launch_step(StepArgs &a) {
 
     tick(KT_NNS);
     {
-        const int warps_total = a.sm_count * a.tune.nns_warps_per_sm;   // grid-stride, one warp per cell
-        const int blocks = (warps_total + NNS_WARPS - 1) / NNS_WARPS;
-        const size_t smem = nns_smem_bytes(p.K, p.adaptive_h);
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(k_neighbours<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_neighbours<D><<<blocks, NNS_WARPS * 32, smem, s>>>(
-            p, a.members, a.memberOf, a.grids, a.x, a.y, a.z, a.posf, a.vx, a.vy, a.vz, a.m, a.u, a.cellTotal,
-            a.cellStart, a.cellList, a.nbr, a.psi, a.ww, a.noi, a.noiImg, a.faceCnt, a.prim, a.geo, a.velf, a.status);
+        const size_t smem = nns_smem_bytes(p.K);
+        // parts per cell: with fewer than two cells per resident warp a cell's
+        // particles go to several warps (each stages the candidates), in batches
+        // that split a mean cell evenly
+        const long long cells = a.cells_est > 0 ? a.cells_est : 1, resident = (long long)a.sm_count * NNS_WARPS * MLH_NNS_MINB;
+        long long nsplit = (2 * resident + cells - 1) / cells;
+        nsplit = nsplit < 1 ? 1 : nsplit > 8 ? 8 : nsplit;
+        if ((long long)p.ncells_cap * nsplit > 0x7fffffffll) nsplit = 1;
+        long long pb = nsplit > 1 ? (p.n + cells * nsplit - 1) / (cells * nsplit) : NNS_PB;
+        pb = pb < 1 ? 1 : pb > NNS_PB ? NNS_PB : pb;
+        // grid-stride over the units, in whole rounds of resident blocks
+        int per_sm = (a.tune.nns_warps_per_sm + NNS_WARPS - 1) / NNS_WARPS;
+        per_sm = (per_sm + MLH_NNS_MINB - 1) / MLH_NNS_MINB * MLH_NNS_MINB;
+        const long long most = ((long long)p.ncells_cap * nsplit + NNS_WARPS - 1) / NNS_WARPS;
+        const long long want = (long long)a.sm_count * per_sm;
+        const int blocks = (int)(want < most ? want : most < 1 ? 1 : most);
+        auto run = [&](auto kern) {
+            if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            kern<<<blocks, NNS_WARPS * 32, smem, s>>>(
+                p, (int)nsplit, (int)pb, a.members, a.memberOf, a.grids, a.x, a.y, a.z, a.posf, a.vx, a.vy, a.vz, a.m,
+                a.u, a.cellTotal, a.cellStart, a.cellList, a.nbr, a.psi, a.ww, a.noi, a.noiImg, a.faceCnt, a.prim,
+                a.geo, a.velf, a.status);
+        };
+        if (p.adaptive_h) run(k_neighbours<D, true>);
+        else run(k_neighbours<D, false>);
     }
     tock(KT_NNS);
 

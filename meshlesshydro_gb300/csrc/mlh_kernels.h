@@ -14,7 +14,7 @@ struct Tuning {
     int face_threads = 128;        // threads per block of k_faces
     int face_blocks_per_sm = 32;   // grid of the grid-stride face loop (32 against 8: -0.5 % on Sedov 128^3, -9 % on 16 blasts in 48^3, whose shocks fill a few blocks)
     int grad_threads = 128;        // threads per block of k_gradients
-    int nns_warps_per_sm = 64;     // warps (= particles in flight) of k_neighbours
+    int nns_warps_per_sm = 32;     // warps per SM of k_neighbours: one round of resident blocks
     int face_split = 0;            // plain root-solver step: 1 second Newton pass over a queue, 2 in-block, 0 none
     int link_overlap = 1;          // face links on the second stream beside the time step and gradients
     int persistent_binning = 0;    // the binning as one persistent cooperative kernel (k_binning)
@@ -56,6 +56,7 @@ struct StepArgs {
     // grids, one per member
     GridInfo *grids;
     int *cellTotal;
+    long long cells_est;       // cells of all grids when the context was created
     double *boundsPart;
     int *cell, *cellCount, *cellStart, *cellFill, *cellList;
     // neighbours
