@@ -528,8 +528,7 @@ __global__ void __launch_bounds__(PB_T) k_binning(const double *__restrict__ x, 
 // 1015 -> 620 us, Sedov 33^3 168 -> 96, KH 24^2 38 -> 17).
 constexpr int NNS_WARPS = 8;
 constexpr int NNS_PB = 12;    // particles of a cell per batch
-constexpr int NNS_REG = 4;    // candidates per lane held in registers (k_neighbours)
-constexpr int NNS_CH = 128;   // candidates per staged chunk (k_hsolve)
+constexpr int NNS_REG = 4;    // candidates per lane held in registers
 // blocks of the neighbour search resident per SM: 4 caps it at 64 registers and
 // gives 32 warps per SM (Sedov 128^3: 2.57 ms, 2.91 at 3, 3.13 at 2)
 #ifndef MLH_NNS_MINB
@@ -629,6 +628,34 @@ __device__ __forceinline__ int nns_cell_of(const NnsCells *cs, int t) {
     return k;
 }
 
+// Candidates [ch, ch + 32 NNS_REG) of the stencil's sequence, candidate ch + 32 r
+// + lane in element r: single-precision position with the image shift applied,
+// index with image bits.  Beyond the sequence: infinitely far.
+template <int D>
+__device__ __forceinline__ void nns_candidates(const NnsCells *cs, const float4 *__restrict__ posf,
+                                               const int *__restrict__ cellList, int ch, int total, float *cx,
+                                               float *cy, float *cz, uint32_t *ce) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < NNS_REG; ++r) {
+        const int t = ch + r * 32 + lane;
+        cx[r] = FLT_INF_; cy[r] = 0.f; cz[r] = 0.f; ce[r] = 0u;
+        if (t < total) {
+            const int k = nns_cell_of<D>(cs, t);
+            const int j = cellList[cs->start[k] + (t - cs->excl[k])];
+            const unsigned wr = cs->wrap[k];
+            float4 fj = posf[j];
+            if (wr) {
+                fj.x += cs->shift[k][0];
+                fj.y += cs->shift[k][1];
+                if (D == 3) fj.z += cs->shift[k][2];
+            }
+            cx[r] = fj.x; cy[r] = fj.y; cz[r] = fj.z;
+            ce[r] = (uint32_t)j | (wr << IMG_SHIFT);
+        }
+    }
+}
+
 template <int D, bool ADAPT>
 __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
     Params p, int nsplit, int pb, const Member *__restrict__ members, const int *__restrict__ memberOf,
@@ -720,25 +747,10 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
             for (int ch = 0; ch < total; ch += 32 * NNS_REG) {
                 float cx[NNS_REG], cy[NNS_REG], cz[NNS_REG], chf[NNS_REG];
                 uint32_t ce[NNS_REG];
+                nns_candidates<D>(cs, posf, cellList, ch, total, cx, cy, cz, ce);
 #pragma unroll
-                for (int r = 0; r < NNS_REG; ++r) {
-                    const int t = ch + r * 32 + lane;
-                    cx[r] = FLT_INF_; cy[r] = 0.f; cz[r] = 0.f; chf[r] = 0.f; ce[r] = 0u;   // no candidate: infinitely far
-                    if (t < total) {
-                        const int k = nns_cell_of<D>(cs, t);
-                        const int j = cellList[cs->start[k] + (t - cs->excl[k])];
-                        const unsigned wr = cs->wrap[k];
-                        float4 fj = posf[j];
-                        if (wr) {
-                            fj.x += cs->shift[k][0];
-                            fj.y += cs->shift[k][1];
-                            if (D == 3) fj.z += cs->shift[k][2];
-                        }
-                        cx[r] = fj.x; cy[r] = fj.y; cz[r] = fj.z;
-                        ce[r] = (uint32_t)j | (wr << IMG_SHIFT);
-                        if (ADAPT) chf[r] = p.hpf[j];
-                    }
-                }
+                for (int r = 0; r < NNS_REG; ++r)
+                    chf[r] = ADAPT && ch + r * 32 + lane < total ? p.hpf[ce[r] & IDX_MASK] : 0.f;
                 for (int q = 0; q < nb; ++q) {
                     const uint32_t iq = (uint32_t)__shfl_sync(ALL, myI, q);
                     const float fx = __shfl_sync(ALL, myF.x, q), fy = __shfl_sync(ALL, myF.y, q);
@@ -974,26 +986,28 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
 // iterations.  The CPU restatement performs the same operations in the same
 // order and gets the same bits.
 //
-// One warp per cell, as the neighbour search: the cell's candidate sequence
-// is staged in shared memory once and filtered for a batch of up to HS_PB of
-// its particles; the warp then computes their candidate distances and runs
-// their Newton iterations side by side: per iteration, the sums of each
-// unfinished particle of the batch (all lanes, the order above), then the
-// scalar updates of all of them at once, particle q on lane q, so that the
-// divisions and tests of an update are issued once per batch instead of once
-// per particle.
+// One warp per cell, as the neighbour search: the lanes hold the cell's
+// candidates in registers and filter them for a batch of up to HS_PB of its
+// particles; the warp then computes their candidate distances, the batch's lists
+// as one sequence, and runs their Newton iterations side by side: per
+// iteration, the sums of each unfinished particle of the batch (all lanes, the
+// order above), then the scalar updates of all of them at once, particle q on
+// lane q, so that the divisions and tests of an update are issued once per batch
+// instead of once per particle.  Bound: the FP64 pipe (58 % active) and latency
+// at 16 warps per SM; 61^3 with 32 neighbours: 1600 us with a staged chunk, FP64
+// products and __dsqrt_rn, 1020 us so.  80 or 64 registers for more warps: 1.10,
+// 1.22 ms.
 constexpr int HSOLVE_MAXIT = 50;
 constexpr int HS_PB = 8;
 // the reduce-scatter of the solve's sums maps the 2 HS_PB = 16 sums onto
 // the 32 lanes (sum k on lanes 2k and 2k + 1)
 static_assert(HS_PB == 8, "k_hsolve reduces exactly 16 sums per batch");
 
-// staged chunk (NNS_CH entries and positions), HS_PB candidate lists (K + 32
-// uint32) and their counts, HS_PB distance lists (K + 32 doubles) and their
-// counts, each rounded up to 16 bytes
+// HS_PB candidate lists (K + 32 uint32 each), their offsets in the batch's
+// sequence (HS_PB ints) and HS_PB distance lists (K + 32 doubles each), each
+// rounded up to 16 bytes
 __host__ __device__ constexpr size_t hsolve_warp_bytes(int K) {
-    return (size_t)NNS_CH * 20 + nns_r16((size_t)HS_PB * (K + 32) * 4) + nns_r16((size_t)HS_PB * 4) +
-           (size_t)HS_PB * (K + 32) * 8 + nns_r16((size_t)HS_PB * 4);
+    return nns_r16((size_t)HS_PB * (K + 32) * 4) + nns_r16((size_t)HS_PB * 4) + (size_t)HS_PB * (K + 32) * 8;
 }
 
 // Shape of the cubic spline and its scaled derivative for the smoothing-length
@@ -1005,30 +1019,32 @@ __host__ __device__ constexpr size_t hsolve_warp_bytes(int K) {
 // gets the same bits.  Both pieces run as the same operations with selected
 // operands (f = (t^2/4) t as fma(t^2/4, t, 0), the same rounded product), so
 // a warp whose candidates fall on both sides of q = 1 issues them once.
+// The products, of positive factors, on the integer pipe (xmul, the same bits).
 __device__ __forceinline__ void hsolve_shape_sel(double r, double ihh2, double &f, double &g) {
-    const double q = __dmul_rn(r, ihh2);
+    const double q = xmul(r, ihh2);
     const long long qb = __double_as_longlong(q);   // q >= 0: q <= 1 and q < 2 on the bits
     const bool inner = qb <= 0x3FF0000000000000ll, in = qb < 0x4000000000000000ll;
-    const double t = __dsub_rn(2., q);
+    const double t = subr(2., q);
     const double a = inner ? q : t;
-    const double a2 = __dmul_rn(a, a);
+    const double a2 = xmul(a, a);
     const double u = __fma_rn(0.75, q, -1.5);
     const double v = __fma_rn(-2.25, q, 3.);
     // a2 / 4 (exact) on the integer pipe
     const double f_ = __fma_rn(inner ? a2 : scale_down<2>(a2), inner ? u : t, inner ? 1. : 0.);
-    const double g_ = __dmul_rn(inner ? a2 : __dmul_rn(0.75, a2), inner ? v : q);
+    const double g_ = xmul(inner ? a2 : xmul(0.75, a2), inner ? v : q);
     f = in ? f_ : 0.;
     g = in ? g_ : 0.;
 }
 
 template <int D>
-__global__ void __launch_bounds__(NNS_WARPS * 32) k_hsolve(
+__global__ void __launch_bounds__(NNS_WARPS * 32, 2) k_hsolve(
     Params p, const Member *__restrict__ members, const int *__restrict__ memberOf,
     const GridInfo *__restrict__ grids, const double *__restrict__ x, const double *__restrict__ y,
     const double *__restrict__ z, const float4 *__restrict__ posf, const int *__restrict__ cellTotal,
     const int *__restrict__ cellStart, const int *__restrict__ cellList, double *__restrict__ hp,
     float *__restrict__ hpf, double *__restrict__ neff, unsigned long long *__restrict__ hstat,
     unsigned *__restrict__ status) {
+    constexpr unsigned ALL = 0xffffffffu;
     const int K = p.K;
     const int CAP = K + 32;
     extern __shared__ __align__(16) unsigned char hs_smem[];
@@ -1036,13 +1052,9 @@ __global__ void __launch_bounds__(NNS_WARPS * 32) k_hsolve(
     const unsigned lt_mask = (1u << lane) - 1u;
     NnsCells *cs = reinterpret_cast<NnsCells *>(hs_smem) + warp;
     unsigned char *wbase = hs_smem + nns_cells_bytes() + (size_t)warp * hsolve_warp_bytes(K);
-    float4 *stP = reinterpret_cast<float4 *>(wbase);
-    uint32_t *stE = reinterpret_cast<uint32_t *>(wbase + (size_t)NNS_CH * 16);
-    uint32_t *candq = stE + NNS_CH;                                                   // HS_PB lists of CAP
-    unsigned char *nb0 = wbase + (size_t)NNS_CH * 20 + nns_r16((size_t)HS_PB * CAP * 4);
-    int *ncq = reinterpret_cast<int *>(nb0);
-    double *rlq = reinterpret_cast<double *>(nb0 + nns_r16((size_t)HS_PB * 4));       // HS_PB lists of CAP
-    int *nrq = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(rlq) + (size_t)HS_PB * CAP * 8);
+    uint32_t *candq = reinterpret_cast<uint32_t *>(wbase);                            // HS_PB lists of CAP
+    int *offq = reinterpret_cast<int *>(wbase + nns_r16((size_t)HS_PB * CAP * 4));
+    double *rlq = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(offq) + nns_r16((size_t)HS_PB * 4));   // HS_PB lists of CAP
     constexpr double KD = D == 3 ? 32. / 3. : 40. / 7.;
     const double St = p.sngb_t;
     const double tolS = __dmul_rn(1e-12, St);
@@ -1057,114 +1069,110 @@ __global__ void __launch_bounds__(NNS_WARPS * 32) k_hsolve(
         const int c0 = cellStart[c], ncell = cellStart[c + 1] - c0;
         if (ncell <= 0) continue;
         const int mi = memberOf ? memberOf[cellList[c0]] : 0;
-        const GridInfo g = grids[mi];
-        const Member mb = members[mi];
+        const GridInfo &g = grids[mi];
+        const Member &mb = members[mi];
         const double H = mb.h;
         const int total = nns_stencil<D>(p, g, c - g.cell_base, cellStart, cs);
         for (int b0 = 0; b0 < ncell; b0 += HS_PB) {
             const int nb = ncell - b0 < HS_PB ? ncell - b0 : HS_PB;
-            int myI = -1;
+            // --- candidates of the batch within H, in stencil order: single-
+            // precision filter as in k_neighbours, particle q on lane q
+            int myI = -1, myNc = 0;
             float4 myF = make_float4(0.f, 0.f, 0.f, 0.f);
             if (lane < nb) { myI = cellList[c0 + b0 + lane]; myF = posf[myI]; }
-            if (lane < HS_PB) ncq[lane] = 0;
-            __syncwarp();
-            // --- candidates of the batch: staged chunks, single-precision filter
-            for (int ch = 0; ch < total; ch += NNS_CH) {
-                const int cl = total - ch < NNS_CH ? total - ch : NNS_CH;
-                for (int t = lane; t < cl; t += 32) {
-                    const int k = nns_cell_of<D>(cs, ch + t);
-                    const int j = cellList[cs->start[k] + (ch + t - cs->excl[k])];
-                    const unsigned wr = cs->wrap[k];
-                    float4 fj = posf[j];
-                    if (wr) {
-                        fj.x += cs->shift[k][0];
-                        fj.y += cs->shift[k][1];
-                        if (D == 3) fj.z += cs->shift[k][2];
-                    }
-                    stP[t] = fj;
-                    stE[t] = (uint32_t)j | (wr << IMG_SHIFT);
-                }
-                __syncwarp();
+            const float hsq_f = mb.hsq_f;
+            for (int ch = 0; ch < total; ch += 32 * NNS_REG) {
+                float cx[NNS_REG], cy[NNS_REG], cz[NNS_REG];
+                uint32_t ce[NNS_REG];
+                nns_candidates<D>(cs, posf, cellList, ch, total, cx, cy, cz, ce);
                 for (int q = 0; q < nb; ++q) {
-                    const uint32_t iq = (uint32_t)__shfl_sync(0xffffffffu, myI, q);
-                    const float fx = __shfl_sync(0xffffffffu, myF.x, q);
-                    const float fy = __shfl_sync(0xffffffffu, myF.y, q);
-                    const float fz = __shfl_sync(0xffffffffu, myF.z, q);
-                    uint32_t *cq = candq + (size_t)q * CAP;
-                    int nq = ncq[q];
-                    for (int t0 = 0; t0 < cl; t0 += 32) {
-                        const int t = t0 + lane;
-                        bool pass = false;
-                        uint32_t ent = 0;
-                        if (t < cl) {
-                            ent = stE[t];
-                            if (ent != iq) {
-                                const float4 fj = stP[t];
-                                const float dx = fj.x - fx, dy = fj.y - fy, dz = fj.z - fz;
-                                pass = dx * dx + dy * dy + (D == 3 ? dz * dz : 0.f) <= mb.hsq_f;
-                            }
-                        }
-                        const unsigned bal = __ballot_sync(0xffffffffu, pass);
-                        if (pass) {
-                            const int pos = nq + __popc(bal & lt_mask);
-                            if (pos < CAP) cq[pos] = ent;
-                        }
+                    const uint32_t iq = (uint32_t)__shfl_sync(ALL, myI, q);
+                    const float fx = __shfl_sync(ALL, myF.x, q), fy = __shfl_sync(ALL, myF.y, q);
+                    const float fz = D == 3 ? __shfl_sync(ALL, myF.z, q) : 0.f;
+                    int nq = __shfl_sync(ALL, myNc, q);
+                    uint32_t *cq = candq + q * CAP;
+#pragma unroll
+                    for (int r = 0; r < NNS_REG; ++r) {
+                        if (ch + r * 32 >= total) break;
+                        const float dx = cx[r] - fx, dy = cy[r] - fy, dz = cz[r] - fz;
+                        const bool pass = dx * dx + dy * dy + (D == 3 ? dz * dz : 0.f) <= hsq_f && ce[r] != iq;
+                        const unsigned bal = __ballot_sync(ALL, pass);
+                        const int pos = nq + __popc(bal & lt_mask);
+                        if (pass && pos < CAP) cq[pos] = ce[r];
                         nq += __popc(bal);
                     }
-                    __syncwarp();
-                    if (lane == 0) ncq[q] = nq;
-                    __syncwarp();
+                    if (lane == q) myNc = nq;
                 }
             }
-            // --- exact FP64 distances of the candidates within H, in order
-            for (int q = 0; q < nb; ++q) {
-                const int i = __shfl_sync(0xffffffffu, myI, q);
-                const int ncand = ncq[q];
-                int nr = 0;
-                if (ncand <= CAP) {
-                    const uint32_t *cand = candq + (size_t)q * CAP;
-                    double *rl = rlq + (size_t)q * CAP;
-                    double xi[3] = {0., 0., 0.};
+            // --- exact FP64 distances of the candidates within H, in order: the
+            // lists walked as one sequence, as in k_neighbours
+            const int myN = lane < nb && myNc <= CAP ? myNc : 0;
+            int myOff = myN;
 #pragma unroll
-                    for (int a = 0; a < D; ++a) xi[a] = X[a][i];
-                    for (int t0 = 0; t0 < ncand; t0 += 32) {
-                        const int t = t0 + lane;
-                        bool pass = false;
-                        double r = 0.;
-                        if (t < ncand) {
-                            const uint32_t e = cand[t];
-                            const int j = (int)(e & IDX_MASK);
-                            const unsigned wr = e >> IMG_SHIFT;
-                            double xj[3];
-                            bool ok = true;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(ALL, myOff, o);
+                if (lane >= o) myOff += t;
+            }
+            const int seq = __shfl_sync(ALL, myOff, 31);
+            myOff -= myN;
+            __syncwarp();
+            if (lane < HS_PB) offq[lane] = lane < nb ? myOff : 0x7fffffff;
+            double myX[3] = {0., 0., 0.};
+            if (lane < nb) {
 #pragma unroll
-                            for (int a = 0; a < D; ++a) {
-                                xj[a] = X[a][j];
-                                if (wr & (1u << a)) {
-                                    if (in_band(xj[a], g, a)) xj[a] = image_coord(xj[a], g, a);
-                                    else ok = false;
-                                }
-                            }
-                            if (ok) {
-                                double ex = __dsub_rn(xj[0], xi[0]), ey = __dsub_rn(xj[1], xi[1]);
-                                double d2 = __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey));
-                                if (D == 3) { double ez = __dsub_rn(xj[2], xi[2]); d2 = __dadd_rn(d2, __dmul_rn(ez, ez)); }
-                                pass = __double_as_longlong(d2) < __double_as_longlong(mb.hsq);   // d2 < H^2, both >= 0
-                                if (pass) r = fsqrt_rn(d2);
-                            }
+                for (int a = 0; a < D; ++a) myX[a] = X[a][myI];
+            }
+            const double hsq = mb.hsq;
+            __syncwarp();
+            int myNr = 0;
+            for (int t0 = 0; t0 < seq; t0 += 32) {
+                const int gi = t0 + lane;
+                int q = 0;
+#pragma unroll
+                for (int l4 = 0; l4 < HS_PB; l4 += 4) {
+                    const int4 o = *reinterpret_cast<const int4 *>(offq + l4);
+                    if (l4 > 0) q += o.x <= gi;
+                    q += (o.y <= gi) + (o.z <= gi) + (o.w <= gi);
+                }
+                const int off = __shfl_sync(ALL, myOff, q), n_q = __shfl_sync(ALL, myN, q), nr0 = __shfl_sync(ALL, myNr, q);
+                double xi[3] = {0., 0., 0.};
+#pragma unroll
+                for (int a = 0; a < D; ++a) xi[a] = __shfl_sync(ALL, myX[a], q);
+                bool pass = false;
+                double r = 0.;
+                if (gi < seq) {
+                    const uint32_t e = candq[q * CAP + (gi - off)];
+                    const int j = (int)(e & IDX_MASK);
+                    const unsigned wr = e >> IMG_SHIFT;
+                    double xj[3];
+                    bool ok = true;
+#pragma unroll
+                    for (int a = 0; a < D; ++a) {
+                        xj[a] = X[a][j];
+                        if (wr & (1u << a)) {
+                            if (in_band(xj[a], g, a)) xj[a] = image_coord(xj[a], g, a);
+                            else ok = false;
                         }
-                        const unsigned bal = __ballot_sync(0xffffffffu, pass);
-                        if (pass) rl[nr + __popc(bal & lt_mask)] = r;
-                        nr += __popc(bal);
                     }
-                } else {
-                    nr = -1;   // overflow: the host grows the slots and repeats
+                    if (ok) {
+                        double ed[3];
+#pragma unroll
+                        for (int a = 0; a < D; ++a) ed[a] = subr(xj[a], xi[a]);
+                        double d2 = addr(mulr(ed[0], ed[0]), mulr(ed[1], ed[1]));
+                        if (D == 3) d2 = addr(d2, mulr(ed[2], ed[2]));
+                        pass = __double_as_longlong(d2) < __double_as_longlong(hsq);   // d2 < H^2, both >= 0
+                        if (pass) r = fsqrt_rn(d2);
+                    }
                 }
-                if (lane == 0) nrq[q] = nr;
-                __syncwarp();
+                const unsigned bal = __ballot_sync(ALL, pass);
+                if (pass) rlq[(size_t)q * CAP + nr0 + __popc(bal & range_mask(off - t0, off - t0 + n_q) & lt_mask)] = r;
+                myNr += __popc(bal & range_mask(myOff - t0, myOff - t0 + myN));
             }
+            __syncwarp();
             // --- bracketed Newton on S(x) = St, particle q's state on lane q
-            const int mynr = lane < nb ? nrq[lane] : -1;
+            // (-1: no solve; more candidates than the list holds: the host grows the
+            // slots and repeats)
+            const int mynr = lane < nb && myNc <= CAP ? myNr : -1;
             if (lane < nb && mynr < 0) overflow_any = true;
             bool done = !(lane < nb) || mynr < 0;
             double xh = H, lo = 0., hi = H, S = 0., sfq = 0., sgq = 0.;
@@ -1192,8 +1200,8 @@ __global__ void __launch_bounds__(NNS_WARPS * 32) k_hsolve(
                         for (int t = lane; t < nrq_; t += 32) {
                             double f, gg;
                             hsolve_shape_sel(rl[t], ihq, f, gg);
-                            v[2 * q] = __dadd_rn(v[2 * q], f);
-                            v[2 * q + 1] = __dadd_rn(v[2 * q + 1], gg);
+                            v[2 * q] = addr(v[2 * q], f);
+                            v[2 * q + 1] = addr(v[2 * q + 1], gg);
                         }
                     }
                 }
@@ -1210,7 +1218,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32) k_hsolve(
                         if (j < m) {
                             const double send = upper ? v[j] : v[j + m];
                             const double keep = upper ? v[j + m] : v[j];
-                            v[j] = __dadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, d));
+                            v[j] = addr(keep, __shfl_xor_sync(0xffffffffu, send, d));
                         }
                     }
                 }
@@ -2248,8 +2256,12 @@ void launch_hsolve(StepArgs &a) {
     const Params &p = a.p;
     cudaStream_t s = a.stream;
     cudaMemsetAsync(a.hstat, 0, 2 * sizeof(unsigned long long), s);
-    const int warps_total = a.sm_count * a.tune.nns_warps_per_sm;
-    const int blocks = (warps_total + NNS_WARPS - 1) / NNS_WARPS;
+    // eight rounds of resident blocks: cells take uneven numbers of iterations
+    // (61^3: 1158 us at two rounds, 1020 at eight and more)
+    const int warps_total = 4 * a.sm_count * a.tune.nns_warps_per_sm;
+    const int most = (p.ncells_cap + NNS_WARPS - 1) / NNS_WARPS;
+    int blocks = (warps_total + NNS_WARPS - 1) / NNS_WARPS;
+    if (blocks > most) blocks = most;
     const size_t smem = hsolve_smem_bytes(p.K);
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_hsolve<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_hsolve<D><<<blocks, NNS_WARPS * 32, smem, s>>>(p, a.members, a.memberOf, a.grids, a.x, a.y, a.z, a.posf, a.cellTotal,
