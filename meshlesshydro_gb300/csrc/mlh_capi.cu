@@ -98,6 +98,7 @@ struct mlh_ctx {
     unsigned *status = nullptr;
     unsigned long long *dtbits = nullptr, *newtonSum = nullptr;
     double *dt = nullptr, *simTime = nullptr;
+    unsigned *arrived = nullptr;
     int *stepsDone = nullptr;
     int *scanTiles = nullptr, *scanTotal = nullptr;
     bool debug_arrays = true;
@@ -302,7 +303,7 @@ StepArgs make_args(mlh_ctx *c, double dt_max) {
     a.prim = c->prim; a.geo = c->geo; a.grad = c->grad; a.gradRaw = c->debug_arrays ? c->gradRaw : nullptr;
     a.Fface = c->Fface; a.fluxSums = c->debug_arrays ? c->fluxSums : nullptr;
     a.status = c->status; a.dtbits = c->dtbits; a.newtonSum = c->newtonSum;
-    a.dt = c->dt; a.simTime = c->simTime; a.stepsDone = c->stepsDone;
+    a.dt = c->dt; a.simTime = c->simTime; a.arrived = c->arrived; a.stepsDone = c->stepsDone;
     a.scanTiles = c->scanTiles; a.scanTotal = c->scanTotal;
     a.learned = (c->learned && c->tune.learned_guess) ? 1 : 0;
     a.fstate = c->fstate; a.feat = c->feat; a.yguess = c->yguess;
@@ -464,7 +465,7 @@ static int create_impl(const mlh_config *cfg, int nmembers, const mlh_member *md
     A(status, 1); A(dtbits, nm); A(newtonSum, 3); A(dt, nm); A(simTime, nm); A(stepsDone, 1);
     A(hp, n); A(neff, n); A(hstat, 2); A(hpf, n);
     A(scanTotal, 1);
-    A(bar, 2);
+    A(bar, 2); A(arrived, 1);
 #undef A
     if ((rc = alloc_cell_buffers(c))) return fail(rc);
     if ((rc = alloc_neighbour_buffers(c))) return fail(rc);
@@ -482,6 +483,7 @@ static int create_impl(const mlh_config *cfg, int nmembers, const mlh_member *md
     cudaMemsetAsync(c->dt, 0, sizeof(double) * nm, c->stream);
     cudaMemsetAsync(c->newtonSum, 0, 3 * sizeof(unsigned long long), c->stream);
     cudaMemsetAsync(c->stepsDone, 0, sizeof(int), c->stream);
+    cudaMemsetAsync(c->arrived, 0, sizeof(unsigned), c->stream);
     cudaMemsetAsync(c->neff, 0, sizeof(double) * n, c->stream);
     cudaMemsetAsync(c->hstat, 0, 2 * sizeof(unsigned long long), c->stream);
     // empty lists until the first search (kernels after a binning that gave
@@ -558,7 +560,7 @@ void mlh_destroy(mlh_ctx *c) {
                     c->cellTotal, c->boundsPart, c->cell, c->cellList, c->noi, c->noiImg, c->faceCnt, c->faceOff,
                     c->prim, c->geo, c->grad, c->gradRaw, c->fluxSums, c->status, c->dtbits, c->newtonSum, c->dt,
                     c->simTime, c->stepsDone, c->scanTiles, c->scanTotal, c->hp, c->neff, c->hstat, c->hpf, c->bar,
-                    c->velf, c->dtlo, c->dtcap};
+                    c->velf, c->dtlo, c->dtcap, c->arrived};
     for (void *q : ptrs) if (q) cudaFree(q);
     free_cell_buffers(c);
     free_neighbour_buffers(c);

@@ -259,6 +259,20 @@ __device__ __forceinline__ double fma_dotD(const double *a, const double *b, dou
     return r;
 }
 
+// True when the binning of this step is not valid: a bounded wait gave up
+// (ST_TIMEOUT), a particle fell outside the grid (ST_GRID: outside the box,
+// a NaN coordinate, or fewer than 3 cells on a periodic axis) or the cells
+// exceed their buffers (ST_CAPACITY, the step is repeated with more).  The
+// kernels that read the binning then skip their work: the step completes
+// nothing and reports the bits, and a NaN particle, which the grid clamps
+// into one cell, cannot make a cell of every particle whose sort and search
+// are quadratic in its size.  The value is the same for every thread of a
+// launch (the bits are set by earlier kernels or before a grid barrier; ST_CAPACITY also
+// by the face links beside the gradients, and then the step is repeated).
+__device__ __forceinline__ bool step_aborted(const unsigned *status) {
+    return (*(volatile const unsigned *)status & (ST_TIMEOUT | ST_GRID | ST_CAPACITY)) != 0u;
+}
+
 __device__ __forceinline__ void flag(unsigned *status, unsigned bits) {
     atomicOr(status, bits);
 }

@@ -374,6 +374,7 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
                                                unsigned *__restrict__ status, FaceQueue qa, FaceQueue qb,
                                                float4 *__restrict__ feat, const float *__restrict__ yguess,
                                                Harvest hv) {
+    if (step_aborted(status)) return;   // no valid faces
     int nf = *faceTotal < p.faces_cap ? *faceTotal : p.faces_cap;
     constexpr bool QUEUED = MODE == 2 || MODE == 4;   // passes over the queue
     if (QUEUED) {   // the queue holds min(count, capacity) faces; MODE 3 finished the rest itself
@@ -556,6 +557,7 @@ __global__ void MLH_FACE_BOUNDS k_faces_block(Params p, RiemannConsts rc, const 
     __shared__ int todo[FB_T];
     __shared__ int slist[LEARNED ? FB_T : 1];
     __shared__ int wcount[FB_T / 32];
+    if (step_aborted(status)) return;   // no valid faces
     const int nf = *faceTotal < p.faces_cap ? *faceTotal : p.faces_cap;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long iters_local = 0, fallback_local = 0, learned_local = 0;

@@ -127,7 +127,36 @@ __global__ void k_scan_apply(const int *__restrict__ in, int n, const int *__res
     if (write_total_at_n && blockIdx.x == 0 && threadIdx.x == 0) out[n] = *total;
 }
 
+// The same in one launch of one block, tile after tile, for few items: three
+// dependent launches take about 9 us whatever they do, a tile here about 1.5 us.
+__global__ void __launch_bounds__(SCAN_T) k_scan_one(const int *__restrict__ in, int n, int *__restrict__ out,
+                                                     int *__restrict__ total) {
+    __shared__ int smem[32];
+    int carry = 0;
+    for (int b = 0; b < n; b += SCAN_TILE) {
+        const int i0 = b + threadIdx.x * SCAN_I;
+        int v[SCAN_I], loc = 0, tot;
+#pragma unroll
+        for (int k = 0; k < SCAN_I; ++k) {
+            v[k] = i0 + k < n ? in[i0 + k] : 0;
+            loc += v[k];
+        }
+        int ex = carry + block_exclusive_scan(loc, smem, tot);
+#pragma unroll
+        for (int k = 0; k < SCAN_I; ++k) {
+            if (i0 + k < n) out[i0 + k] = ex;
+            ex += v[k];
+        }
+        carry += tot;
+    }
+    if (threadIdx.x == 0) { out[n] = carry; *total = carry; }
+}
+
 void exclusive_scan(const int *in, int n, int *out, int *tile_buf, int *total, cudaStream_t s) {
+    if (n <= 4 * SCAN_TILE) {
+        k_scan_one<<<1, SCAN_T, 0, s>>>(in, n, out, total);
+        return;
+    }
     int ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (ntiles < 1) ntiles = 1;
     k_scan_reduce<<<ntiles, SCAN_T, 0, s>>>(in, n, tile_buf);
@@ -193,91 +222,153 @@ __device__ __forceinline__ void bounds_partial_block(int vb, const double *__res
 template <int D>
 __global__ void k_bounds_partial(const double *__restrict__ x, const double *__restrict__ y,
                                  const double *__restrict__ z, Params p, const Member *__restrict__ members,
-                                 int bpm, double *__restrict__ part) {
+                                 int bpm, double *__restrict__ part, int *__restrict__ cellCount,
+                                 int *__restrict__ cellFill) {
+    // with the cell counters (a step's binning): cleared here
+    if (cellCount)
+        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= p.ncells_cap; k += gridDim.x * blockDim.x) {
+            cellCount[k] = 0;
+            cellFill[k] = 0;
+        }
     bounds_partial_block<D>(blockIdx.x, x, y, z, p, members, bpm, part);
 }
 
-// Final pass + Domain::createGrid (Domain.cpp:9-54) for every simulation,
-// then the cell numbering of the concatenated grids.  For periodic runs the
-// bounds are the configured box.
+// Domain::createGrid of one simulation; lo and mx1: the minima and the maxima
+// over i >= 1 of an open box's coordinates
+template <int D>
+__device__ __forceinline__ void bounds_grid(const double *const *X, const Params &p, const Member &mb, const double *lo,
+                                            const double *mx1, GridInfo *out, unsigned *status) {
+    GridInfo g;
+    for (int a = 0; a < 3; ++a) { g.lo[a] = 0.; g.hi[a] = 0.; g.cs[a] = 1.; g.cells[a] = 1; }
+    for (int a = 0; a < D; ++a) {
+        if (p.periodic) { g.lo[a] = mb.box_lo[a]; g.hi[a] = mb.box_hi[a]; continue; }
+        const double x0 = X[a][mb.first];
+        double hi;
+        if (mb.count < 2 || !(mx1[a] >= x0)) {
+            // sequential rule of the reference
+            double lo_s = DBL_MAX_, hi_s = DBL_MIN_;
+            for (int i = mb.first; i < mb.first + mb.count; ++i) {
+                double v = X[a][i];
+                if (v < lo_s) lo_s = v;
+                else if (v > hi_s) hi_s = v;
+            }
+            hi = hi_s;
+        } else {
+            hi = mx1[a] > DBL_MIN_ ? mx1[a] : DBL_MIN_;
+        }
+        g.lo[a] = lo[a];
+        g.hi[a] = hi;
+    }
+    // the product saturates at ncells_cap + 1 (each factor is below 2^31,
+    // so the product of the saturated value and one factor fits in 64 bits)
+    long long total = 1;
+    for (int a = 0; a < D; ++a) {
+        double c = floor((g.hi[a] - g.lo[a]) / mb.h);
+        int ci = (c >= 1. && c < 2147483647.) ? (int)c : 1;
+        if (!(c >= 1.)) flag(status, ST_GRID);
+        if (c >= 2147483647.) { flag(status, ST_CAPACITY); ci = 1; }
+        if (p.periodic && ci < 3) flag(status, ST_GRID);
+        g.cells[a] = ci;
+        total *= ci;
+        if (total > p.ncells_cap) total = (long long)p.ncells_cap + 1;
+    }
+    for (int a = 0; a < D; ++a) g.cs[a] = (g.hi[a] - g.lo[a]) / (double)g.cells[a];
+    for (int a = 0; a < 3; ++a) {
+        g.band_lo[a] = g.lo[a] + mb.h;
+        g.band_hi[a] = g.hi[a] - mb.h;
+        g.Lf[a] = (float)(g.hi[a] - g.lo[a]);
+    }
+    if (total > p.ncells_cap) { flag(status, ST_CAPACITY); total = 1; }
+    g.ncells = (int)total;
+    g.cell_base = 0;
+    *out = g;
+}
+
+// Final pass + Domain::createGrid (Domain.cpp:9-54) for every simulation: the
+// partials by a warp per simulation (one thread reading 304 of them one after
+// another took 145 us of an open 33^3 step), the grid by a thread per
+// simulation, then the cell numbering of the concatenated grids.  For periodic
+// runs the bounds are the configured box.
+// With dtbits, the time step's minima are set to their start too.
 template <int D>
 __device__ __forceinline__ void bounds_final_block(const double *__restrict__ x, const double *__restrict__ y,
                                                    const double *__restrict__ z, const double *__restrict__ part,
                                                    int bpm, const Params &p, const Member *__restrict__ members,
                                                    int nmembers, GridInfo *__restrict__ grids,
-                                                   int *__restrict__ cellTotal, unsigned *__restrict__ status) {
+                                                   int *__restrict__ cellTotal, unsigned *__restrict__ status,
+                                                   unsigned long long *__restrict__ dtbits,
+                                                   unsigned *__restrict__ dtcap) {
     const double *X[3] = {x, y, z};
-    for (int mi = threadIdx.x; mi < nmembers; mi += blockDim.x) {
-        const Member mb = members[mi];
-        GridInfo g;
-        for (int a = 0; a < 3; ++a) { g.lo[a] = 0.; g.hi[a] = 0.; g.cs[a] = 1.; g.cells[a] = 1; }
-        for (int a = 0; a < D; ++a) {
-            if (p.periodic) { g.lo[a] = mb.box_lo[a]; g.hi[a] = mb.box_hi[a]; continue; }
-            double mn = DBL_MAX_, mx1 = -DBL_MAX_;
-            for (int b = mi * bpm; b < (mi + 1) * bpm; ++b) {
-                mn = fmin(mn, part[(b * 3 + a) * 2]);
-                mx1 = fmax(mx1, part[(b * 3 + a) * 2 + 1]);
-            }
-            const double x0 = X[a][mb.first];
-            double hi;
-            if (mb.count < 2 || !(mx1 >= x0)) {
-                // sequential rule of the reference
-                double lo_s = DBL_MAX_, hi_s = DBL_MIN_;
-                for (int i = mb.first; i < mb.first + mb.count; ++i) {
-                    double v = X[a][i];
-                    if (v < lo_s) lo_s = v;
-                    else if (v > hi_s) hi_s = v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    __shared__ double lo_s[BOUNDS_T / 8][3], mx_s[BOUNDS_T / 8][3];
+    for (int m0 = 0; m0 < nmembers; m0 += BOUNDS_T / 8) {
+        const int here = nmembers - m0 < BOUNDS_T / 8 ? nmembers - m0 : BOUNDS_T / 8;
+        if (!p.periodic) {
+            for (int k = warp; k < here; k += nwarps) {
+#pragma unroll
+                for (int a = 0; a < D; ++a) {
+                    double mn = DBL_MAX_, mx = -DBL_MAX_;
+                    for (int b = (m0 + k) * bpm + lane; b < (m0 + k + 1) * bpm; b += 32) {
+                        mn = fmin(mn, part[(b * 3 + a) * 2]);
+                        mx = fmax(mx, part[(b * 3 + a) * 2 + 1]);
+                    }
+                    for (int o = 16; o > 0; o >>= 1) {
+                        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+                        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                    }
+                    if (lane == 0) { lo_s[k][a] = mn; mx_s[k][a] = mx; }
                 }
-                hi = hi_s;
-            } else {
-                hi = mx1 > DBL_MIN_ ? mx1 : DBL_MIN_;
             }
-            g.lo[a] = mn;
-            g.hi[a] = hi;
+            __syncthreads();
         }
-        // the product saturates at ncells_cap + 1 (each factor is below 2^31,
-        // so the product of the saturated value and one factor fits in 64 bits)
-        long long total = 1;
-        for (int a = 0; a < D; ++a) {
-            double c = floor((g.hi[a] - g.lo[a]) / mb.h);
-            int ci = (c >= 1. && c < 2147483647.) ? (int)c : 1;
-            if (!(c >= 1.)) flag(status, ST_GRID);
-            if (c >= 2147483647.) { flag(status, ST_CAPACITY); ci = 1; }
-            if (p.periodic && ci < 3) flag(status, ST_GRID);
-            g.cells[a] = ci;
-            total *= ci;
-            if (total > p.ncells_cap) total = (long long)p.ncells_cap + 1;
+        if ((int)threadIdx.x < here) {
+            const int mi = m0 + threadIdx.x;
+            const Member mb = members[mi];
+            bounds_grid<D>(X, p, mb, lo_s[threadIdx.x], mx_s[threadIdx.x], grids + mi, status);
         }
-        for (int a = 0; a < D; ++a) g.cs[a] = (g.hi[a] - g.lo[a]) / (double)g.cells[a];
-        for (int a = 0; a < 3; ++a) {
-            g.band_lo[a] = g.lo[a] + mb.h;
-            g.band_hi[a] = g.hi[a] - mb.h;
-            g.Lf[a] = (float)(g.hi[a] - g.lo[a]);
-        }
-        if (total > p.ncells_cap) { flag(status, ST_CAPACITY); total = 1; }
-        g.ncells = (int)total;
-        g.cell_base = 0;
-        grids[mi] = g;
+        __syncthreads();
     }
+    if (dtbits)
+        for (int mi = threadIdx.x; mi < nmembers; mi += blockDim.x) {
+            dtbits[mi] = ~0ull;
+            dtcap[mi] = 0x7f7f7f7fu;   // 3.4e38
+        }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        long long base = 0;
-        for (int mi = 0; mi < nmembers; ++mi) {
-            int nc = grids[mi].ncells;
-            if (base + nc > p.ncells_cap) { flag(status, ST_CAPACITY); nc = 0; grids[mi].ncells = 0; }
-            grids[mi].cell_base = (int)base;
-            base += nc;
+    // the cell numbering, in shared memory: a simulation that does not fit keeps no
+    // cells (the step is then repeated with more)
+    __shared__ int nc_s[BOUNDS_T], base_s[BOUNDS_T];
+    __shared__ long long next;
+    if (threadIdx.x == 0) next = 0;
+    for (int m0 = 0; m0 < nmembers; m0 += BOUNDS_T) {
+        const int here = nmembers - m0 < BOUNDS_T ? nmembers - m0 : BOUNDS_T;
+        const int mi = m0 + threadIdx.x;
+        if ((int)threadIdx.x < here) nc_s[threadIdx.x] = grids[mi].ncells;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            long long base = next;
+            for (int k = 0; k < here; ++k) {
+                int nc = nc_s[k];
+                if (base + nc > p.ncells_cap) { flag(status, ST_CAPACITY); nc = 0; }
+                nc_s[k] = nc;
+                base_s[k] = (int)base;
+                base += nc;
+            }
+            next = base;
         }
-        *cellTotal = (int)base;
+        __syncthreads();
+        if ((int)threadIdx.x < here) { grids[mi].ncells = nc_s[threadIdx.x]; grids[mi].cell_base = base_s[threadIdx.x]; }
+        __syncthreads();
     }
+    if (threadIdx.x == 0) *cellTotal = (int)next;
 }
 
 template <int D>
 __global__ void k_bounds_final(const double *__restrict__ x, const double *__restrict__ y,
                                const double *__restrict__ z, const double *__restrict__ part, int bpm, Params p,
                                const Member *__restrict__ members, int nmembers, GridInfo *__restrict__ grids,
-                               int *__restrict__ cellTotal, unsigned *__restrict__ status) {
-    bounds_final_block<D>(x, y, z, part, bpm, p, members, nmembers, grids, cellTotal, status);
+                               int *__restrict__ cellTotal, unsigned *__restrict__ status,
+                               unsigned long long *__restrict__ dtbits, unsigned *__restrict__ dtcap) {
+    bounds_final_block<D>(x, y, z, part, bpm, p, members, nmembers, grids, cellTotal, status, dtbits, dtcap);
 }
 
 // Particles::assignParticlesAndCells (Particles.cpp:270-322).
@@ -316,19 +407,6 @@ __global__ void k_assign(const double *__restrict__ x, const double *__restrict_
         assign_one<D>(i, x, y, z, memberOf, grids, cell, cellCount, status);
 }
 
-// True when the binning of this step is not valid: a bounded wait gave up
-// (ST_TIMEOUT), a particle fell outside the grid (ST_GRID: outside the box,
-// a NaN coordinate, or fewer than 3 cells on a periodic axis) or the cells
-// exceed their buffers (ST_CAPACITY, the step is repeated with more).  The
-// kernels that read the binning then skip their work: the step completes
-// nothing and reports the bits, and a NaN particle, which the grid clamps
-// into one cell, cannot make a cell of every particle whose sort and search
-// are quadratic in its size.  The value is the same for every thread of a
-// launch (the bits are set by earlier kernels or before a grid barrier).
-__device__ __forceinline__ bool step_aborted(const unsigned *status) {
-    return (*(volatile const unsigned *)status & (ST_TIMEOUT | ST_GRID | ST_CAPACITY)) != 0u;
-}
-
 __global__ void k_fill_cells(const int *__restrict__ cell, int n, const int *__restrict__ cellStart,
                              int *__restrict__ cellFill, int *__restrict__ cellList,
                              const unsigned *__restrict__ status) {
@@ -352,12 +430,36 @@ __device__ __forceinline__ void sort_cell(int c, const int *__restrict__ cellSta
     }
 }
 
-__global__ void k_sort_cells(const int *__restrict__ cellTotal, const int *__restrict__ cellStart,
-                             int *__restrict__ cellList, const unsigned *__restrict__ status) {
+// The same by a warp: up to 64 members on the lanes, each written at its rank (a
+// thread's insertion sort is one chain of dependent accesses: 33 us for the 10
+// members per cell of an open 33^3 step); larger cells by the first lane.
+__device__ __forceinline__ void sort_cell_warp(int c, const int *__restrict__ cellStart, int *__restrict__ cellList) {
+    const int lane = threadIdx.x & 31;
+    const int b = cellStart[c], n = cellStart[c + 1] - b;
+    if (n < 2) return;
+    if (n > 64) {
+        if (lane == 0) sort_cell(c, cellStart, cellList);
+        return;
+    }
+    const int v0 = lane < n ? cellList[b + lane] : 0x7fffffff, v1 = lane + 32 < n ? cellList[b + lane + 32] : 0x7fffffff;
+    int r0 = 0, r1 = 0;
+    for (int k = 0; k < n; ++k) {
+        const int w = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
+        r0 += w < v0;
+        r1 += w < v1;
+    }
+    __syncwarp();
+    if (lane < n) cellList[b + r0] = v0;
+    if (lane + 32 < n) cellList[b + r1] = v1;
+}
+
+__global__ void __launch_bounds__(256) k_sort_cells(const int *__restrict__ cellTotal,
+                                                    const int *__restrict__ cellStart, int *__restrict__ cellList,
+                                                    const unsigned *__restrict__ status) {
     if (step_aborted(status)) return;
     const int nc = *cellTotal;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x)
-        sort_cell(c, cellStart, cellList);
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nc; c += (gridDim.x * blockDim.x) >> 5)
+        sort_cell_warp(c, cellStart, cellList);
 }
 
 // ------------------------------------------------------------------ persistent binning
@@ -425,7 +527,8 @@ __global__ void __launch_bounds__(PB_T) k_binning(const double *__restrict__ x, 
                                                   int *__restrict__ cellStart, int *__restrict__ cellFill,
                                                   int *__restrict__ cellList, int *__restrict__ tileSums,
                                                   int *__restrict__ scanTotal, unsigned *__restrict__ status,
-                                                  GridBar bar) {
+                                                  unsigned long long *__restrict__ dtbits,
+                                                  unsigned *__restrict__ dtcap, GridBar bar) {
     __shared__ int smem[32];
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
     const int ncap = p.ncells_cap;
@@ -436,7 +539,7 @@ __global__ void __launch_bounds__(PB_T) k_binning(const double *__restrict__ x, 
     for (int k = tid; k <= ncap; k += nthr) { cellCount[k] = 0; cellFill[k] = 0; }
     if (!grid_sync(bar, status)) return;
     // 2: final bounds and Domain::createGrid (one block)
-    if (blockIdx.x == 0) bounds_final_block<D>(x, y, z, part, bpm, p, members, nmembers, grids, cellTotal, status);
+    if (blockIdx.x == 0) bounds_final_block<D>(x, y, z, part, bpm, p, members, nmembers, grids, cellTotal, status, dtbits, dtcap);
     if (!grid_sync(bar, status)) return;
     // 3: Particles::assignParticlesAndCells and the cell counts
     for (int i = tid; i < p.n; i += nthr) assign_one<D>(i, x, y, z, memberOf, grids, cell, cellCount, status);
@@ -492,7 +595,7 @@ __global__ void __launch_bounds__(PB_T) k_binning(const double *__restrict__ x, 
     }
     if (!grid_sync(bar, status)) return;
     const int nc = *cellTotal;
-    for (int c = tid; c < nc; c += nthr) sort_cell(c, cellStart, cellList);
+    for (int c = tid >> 5; c < nc; c += nthr >> 5) sort_cell_warp(c, cellStart, cellList);
 }
 
 // ------------------------------------------------------------------ neighbour search
@@ -1277,6 +1380,18 @@ size_t nns_smem_bytes(int K) {
 
 // ------------------------------------------------------------------ dt
 
+// dt of every simulation from its minimum (or the fixed time step), clamped; by
+// one block.  A step whose binning was given up keeps the dt of the last one.
+__device__ __forceinline__ void dt_final(const Params &p, int nmembers, const unsigned long long *dtbits, double dt_max,
+                                         double *__restrict__ dt_out) {
+    for (int mi = threadIdx.x; mi < nmembers; mi += blockDim.x) {
+        double dt = p.adaptive ? __longlong_as_double((long long)*(const volatile unsigned long long *)(dtbits + mi))
+                               : p.time_step;
+        if (dt_max > 0. && dt > dt_max) dt = dt_max;
+        dt_out[mi] = dt;
+    }
+}
+
 // c_i + c_j - min(0, v_ij . x_ij / r) as one fused multiply-add: 1/r only when
 // the dot product dv = v_ij . x_ij is negative, 0 otherwise; r as the neighbour
 // search takes it
@@ -1301,10 +1416,15 @@ __global__ void __launch_bounds__(256) k_timestep(Params p, const Member *__rest
                                                   const Geo *__restrict__ geo, const uint32_t *__restrict__ nbr,
                                                   const int *__restrict__ noi,
                                                   unsigned long long *__restrict__ dtbits,
-                                                  const float *__restrict__ dtlo, const unsigned *__restrict__ dtcap) {
+                                                  const float *__restrict__ dtlo, const unsigned *__restrict__ dtcap,
+                                                  int nmembers, double dt_max, double *__restrict__ dt_out,
+                                                  unsigned *__restrict__ arrived,
+                                                  const unsigned *__restrict__ status) {
     const int lane = threadIdx.x & 31;
+    // no valid lists after an aborted binning
+    const int n = step_aborted(status) ? 0 : p.n;
     // warp-uniform loop: every lane takes part in the reductions below
-    for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; i0 < p.n; i0 += gridDim.x * blockDim.x) {
+    for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; i0 < n; i0 += gridDim.x * blockDim.x) {
         const int i = i0 + lane;
         int mi = -1;
         double dti = DBL_MAX_;
@@ -1360,15 +1480,23 @@ __global__ void __launch_bounds__(256) k_timestep(Params p, const Member *__rest
             atomic_min_pos_double(dtbits + mi, dti);
         }
     }
+    // the last block to arrive holds every minimum
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(arrived, 1u) + 1u == gridDim.x;
+    __syncthreads();
+    if (last) {
+        if (threadIdx.x == 0) *arrived = 0u;   // for the next step
+        __threadfence();
+        if (n > 0) dt_final(p, nmembers, dtbits, dt_max, dt_out);
+    }
 }
 
+// dt of every simulation when no k_timestep follows the minima
 __global__ void k_dt_final(Params p, int nmembers, const unsigned long long *__restrict__ dtbits, double dt_max,
-                           double *__restrict__ dt_out) {
-    for (int mi = blockIdx.x * blockDim.x + threadIdx.x; mi < nmembers; mi += gridDim.x * blockDim.x) {
-        double dt = p.adaptive ? __longlong_as_double((long long)dtbits[mi]) : p.time_step;
-        if (dt_max > 0. && dt > dt_max) dt = dt_max;
-        dt_out[mi] = dt;
-    }
+                           double *__restrict__ dt_out, const unsigned *__restrict__ status) {
+    if (!step_aborted(status)) dt_final(p, nmembers, dtbits, dt_max, dt_out);
 }
 
 // ------------------------------------------------------------------ face links
@@ -1483,6 +1611,7 @@ __global__ void __launch_bounds__(256) k_link_own(Params p, const uint32_t *__re
                                                   const int *__restrict__ noi, const int *__restrict__ noiImg,
                                                   const int *__restrict__ faceOff, int *__restrict__ faceOf,
                                                   FaceRef *__restrict__ faces, unsigned *__restrict__ status) {
+    if (step_aborted(status)) return;   // no valid lists
     const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
     bool full = false;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < p.n; i += nw) {
@@ -1511,7 +1640,7 @@ __global__ void __launch_bounds__(256) k_link_own(Params p, const uint32_t *__re
 // other, so slot s of i's real part puts i near slot noi[j] - 1 - s of j's: the
 // search starts at that 4-entry chunk and widens to both sides.  Images are
 // ordered by parent index: that part is searched from its start.  Sedov 64^3 /
-// 128^3 / 64 KH members, with the scan of the face counts: 130 / 1015 / 276 us; a thread
+// 128^3 / 64 KH members, with the scan of the face counts: 130 / 966 / 265 us; a thread
 // per particle, searching four lists in lockstep from their ends (link_particle,
 // which the gradients kernel runs with link_overlap 2), took 288 / 1771 / 446 us,
 // 700 warp instructions per particle with 13 of 32 lanes active.
@@ -1519,6 +1648,7 @@ __global__ void __launch_bounds__(256) k_link(Params p, const uint32_t *__restri
                                               const int *__restrict__ noiImg, const int *__restrict__ faceTotal,
                                               int *__restrict__ faceOf, FaceRef *__restrict__ faces,
                                               unsigned *__restrict__ status) {
+    if (step_aborted(status)) return;
     const int nf = *faceTotal < p.faces_cap ? *faceTotal : p.faces_cap;
     bool lost = false;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
@@ -1644,6 +1774,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                                                    unsigned *__restrict__ dtcap) {
     constexpr int NF = D + 2;
     const int lane = threadIdx.x & 31;
+    if (step_aborted(status)) return;   // no valid lists
     // warp-uniform loop: every lane takes part in the time-step reduction
     for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; i0 < p.n; i0 += gridDim.x * blockDim.x) {
       const int i = i0 + lane;
@@ -2069,9 +2200,15 @@ __global__ void __launch_bounds__(256) k_update(Params p, const int *__restrict_
                                                 double *__restrict__ x, double *__restrict__ y, double *__restrict__ z,
                                                 double *__restrict__ vx, double *__restrict__ vy, double *__restrict__ vz,
                                                 double *__restrict__ m, double *__restrict__ u, float4 *__restrict__ posf,
-                                                double *__restrict__ fluxSums, unsigned *__restrict__ status) {
-    const unsigned st0 = *status;
+                                                double *__restrict__ fluxSums, unsigned *__restrict__ status,
+                                                int nmembers, double *__restrict__ simTime, int *__restrict__ stepsDone) {
+    // (the bits tested are not raised by this kernel: the same for every thread)
+    const unsigned st0 = *(volatile const unsigned *)status;
     if (st0 & (ST_NGB_OVERFLOW | ST_CAPACITY | ST_TIMEOUT | ST_GRID)) return;
+    if (blockIdx.x == 0) {   // simulation time of every member, the count of completed steps
+        for (int mi = threadIdx.x; mi < nmembers; mi += blockDim.x) simTime[mi] += dtp[mi];
+        if (threadIdx.x == 0) *stepsDone += 1;
+    }
     double *X[3] = {x, y, z};
     double *Vv[3] = {vx, vy, vz};
     unsigned st_local = 0;
@@ -2172,16 +2309,6 @@ __global__ void __launch_bounds__(256) k_update(Params p, const int *__restrict_
     if ((threadIdx.x & 31) == 0 && st_local) flag(status, st_local);
 }
 
-// Simulation time of every member and the count of completed steps (skipped,
-// like the update, when the step is to be repeated with more capacity).
-__global__ void k_advance_time(int nmembers, const double *__restrict__ dt, double *__restrict__ simTime,
-                               int *__restrict__ stepsDone, const unsigned *__restrict__ status) {
-    if (*status & (ST_NGB_OVERFLOW | ST_CAPACITY | ST_TIMEOUT | ST_GRID)) return;
-    for (int mi = blockIdx.x * blockDim.x + threadIdx.x; mi < nmembers; mi += gridDim.x * blockDim.x)
-        simTime[mi] += dt[mi];
-    if (blockIdx.x == 0 && threadIdx.x == 0) *stepsDone += 1;
-}
-
 template <int D>
 __global__ void k_pack_posf(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
                             int n, float4 *__restrict__ posf) {
@@ -2236,18 +2363,19 @@ void launch_binning(StepArgs &a) {
         cudaLaunchKernelEx(&cfg, k_binning<D>, (const double *)a.x, (const double *)a.y, (const double *)a.z, p,
                            (const Member *)a.members, a.memberOf, a.nmembers, a.bpm, a.boundsPart, a.grids,
                            a.cellTotal, a.cell, a.cellCount, a.cellStart, a.cellFill, a.cellList, a.scanTiles,
-                           a.scanTotal, a.status, bar);
+                           a.scanTotal, a.status, a.dtbits, a.dtcap, bar);
         return;
     }
-    k_bounds_partial<D><<<a.nmembers * a.bpm, BOUNDS_T, 0, s>>>(a.x, a.y, a.z, p, a.members, a.bpm, a.boundsPart);
-    k_bounds_final<D><<<1, 256, 0, s>>>(a.x, a.y, a.z, a.boundsPart, a.bpm, p, a.members, a.nmembers, a.grids,
-                                        a.cellTotal, a.status);
-    cudaMemsetAsync(a.cellCount, 0, sizeof(int) * (size_t)(p.ncells_cap + 1), s);
-    cudaMemsetAsync(a.cellFill, 0, sizeof(int) * (size_t)(p.ncells_cap + 1), s);
+    k_bounds_partial<D><<<a.nmembers * a.bpm, BOUNDS_T, 0, s>>>(a.x, a.y, a.z, p, a.members, a.bpm, a.boundsPart,
+                                                                a.cellCount, a.cellFill);
+    k_bounds_final<D><<<1, BOUNDS_T, 0, s>>>(a.x, a.y, a.z, a.boundsPart, a.bpm, p, a.members, a.nmembers, a.grids,
+                                             a.cellTotal, a.status, a.dtbits, a.dtcap);
     k_assign<D><<<blocksN, T, 0, s>>>(a.x, a.y, a.z, p.n, a.memberOf, a.grids, a.cell, a.cellCount, a.status);
     exclusive_scan(a.cellCount, p.ncells_cap, a.cellStart, a.scanTiles, a.scanTotal, s);
     k_fill_cells<<<blocksN, T, 0, s>>>(a.cell, p.n, a.cellStart, a.cellFill, a.cellList, a.status);
-    k_sort_cells<<<(p.ncells_cap + T - 1) / T, T, 0, s>>>(a.cellTotal, a.cellStart, a.cellList, a.status);
+    const long long sortBlocks = ((long long)p.ncells_cap + 7) / 8;
+    k_sort_cells<<<(int)(sortBlocks < a.sm_count * 8ll ? sortBlocks : a.sm_count * 8ll), 256, 0, s>>>(
+        a.cellTotal, a.cellStart, a.cellList, a.status);
 }
 
 // Smoothing lengths of every particle on the current grid (k_hsolve).
@@ -2325,8 +2453,8 @@ void launch_step(StepArgs &a) {
     // 0: in order
     const bool fused = a.tune.link_overlap == 2 && !a.stop_after_gradients;
     const bool overlap = !fused && a.stream2 && !a.timer && !a.stop_after_gradients && a.tune.link_overlap == 1;
-    auto grid_of = [&](long long threads) {   // blocks of 256 threads, at most 8 rounds of a full GPU
-        const long long b = (threads + 255) / 256, most = a.sm_count * 64ll;
+    auto grid_of = [&](long long threads) {   // blocks of 256 threads, at most one round of a full GPU
+        const long long b = (threads + 255) / 256, most = a.sm_count * 8ll;
         return (int)(b < 1 ? 1 : b < most ? b : most);
     };
     auto launch_links = [&](cudaStream_t ls) {
@@ -2347,18 +2475,16 @@ void launch_step(StepArgs &a) {
     // (k_gradients with dtbits; k_timestep, the separate kernel of the same
     // arithmetic, is the fallback when the time step is timed on its own)
     const int gT = a.tune.grad_threads;
-    cudaMemsetAsync(a.dtbits, 0xff, sizeof(unsigned long long) * (size_t)a.nmembers, s);
     // with the single-precision filters the gradients kernel bounds every
-    // particle's dt (dtlo, and the least upper bound per simulation in dtcap,
-    // 0x7F7F7F7F = 3.4e38 to start) and k_timestep evaluates v_sig in FP64
+    // particle's dt (dtlo, and the least upper bound per simulation in dtcap) and k_timestep evaluates v_sig in FP64
     // for the particles whose bound reaches it
     const bool dt_filter = p.adaptive && !a.separate_dt && (a.tune.fp32_filters & MLH_FILTER_TIMESTEP) && a.velf &&
                            a.dtlo && a.dtcap;
-    if (dt_filter) cudaMemsetAsync(a.dtcap, 0x7f, sizeof(unsigned) * (size_t)a.nmembers, s);
     if (a.separate_dt) {
         tick(KT_DT);
         k_timestep<D><<<(p.n + 255) / 256, 256, 0, s>>>(p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.noi,
-                                                        a.dtbits, nullptr, nullptr);
+                                                        a.dtbits, nullptr, nullptr, a.nmembers, a.dt_max, a.dt,
+                                                        a.arrived, a.status);
         tock(KT_DT);
     }
     tick(KT_GRAD);
@@ -2374,8 +2500,10 @@ void launch_step(StepArgs &a) {
                                                       a.dtcap);
     if (dt_filter)
         k_timestep<D><<<(p.n + 255) / 256, 256, 0, s>>>(p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.noi,
-                                                        a.dtbits, a.dtlo, a.dtcap);
-    k_dt_final<<<(a.nmembers + 127) / 128, 128, 0, s>>>(p, a.nmembers, a.dtbits, a.dt_max, a.dt);
+                                                        a.dtbits, a.dtlo, a.dtcap, a.nmembers, a.dt_max, a.dt,
+                                                        a.arrived, a.status);
+    else
+        k_dt_final<<<1, 128, 0, s>>>(p, a.nmembers, a.dtbits, a.dt_max, a.dt, a.status);
     tock(KT_GRAD);
     if (a.stop_after_gradients) return;
 
@@ -2395,8 +2523,8 @@ void launch_step(StepArgs &a) {
 
     tick(KT_UPDATE);
     k_update<D><<<blocksN, T, 0, s>>>(p, a.memberOf, a.grids, a.noi, a.noiImg, a.faceOf, a.Fface, a.dt, a.x, a.y,
-                                      a.z, a.vx, a.vy, a.vz, a.m, a.u, a.posf, a.fluxSums, a.status);
-    k_advance_time<<<(a.nmembers + 127) / 128, 128, 0, s>>>(a.nmembers, a.dt, a.simTime, a.stepsDone, a.status);
+                                      a.z, a.vx, a.vy, a.vz, a.m, a.u, a.posf, a.fluxSums, a.status, a.nmembers, a.simTime,
+                                      a.stepsDone);
     tock(KT_UPDATE);
 }
 
@@ -2405,11 +2533,13 @@ void launch_grid_bounds(const double *x, const double *y, const double *z, const
                         int *cellTotal, unsigned *status, cudaStream_t s) {
     const int blocks = nmembers * bpm;
     if (p.dim == 2) {
-        k_bounds_partial<2><<<blocks, BOUNDS_T, 0, s>>>(x, y, z, p, members, bpm, partials);
-        k_bounds_final<2><<<1, 256, 0, s>>>(x, y, z, partials, bpm, p, members, nmembers, grids, cellTotal, status);
+        k_bounds_partial<2><<<blocks, BOUNDS_T, 0, s>>>(x, y, z, p, members, bpm, partials, nullptr, nullptr);
+        k_bounds_final<2><<<1, BOUNDS_T, 0, s>>>(x, y, z, partials, bpm, p, members, nmembers, grids, cellTotal, status,
+                                                 nullptr, nullptr);
     } else {
-        k_bounds_partial<3><<<blocks, BOUNDS_T, 0, s>>>(x, y, z, p, members, bpm, partials);
-        k_bounds_final<3><<<1, 256, 0, s>>>(x, y, z, partials, bpm, p, members, nmembers, grids, cellTotal, status);
+        k_bounds_partial<3><<<blocks, BOUNDS_T, 0, s>>>(x, y, z, p, members, bpm, partials, nullptr, nullptr);
+        k_bounds_final<3><<<1, BOUNDS_T, 0, s>>>(x, y, z, partials, bpm, p, members, nmembers, grids, cellTotal, status,
+                                                 nullptr, nullptr);
     }
 }
 

@@ -73,6 +73,7 @@ struct StepArgs {
     unsigned *status;
     unsigned long long *dtbits, *newtonSum;
     double *dt, *simTime;
+    unsigned *arrived;         // blocks of k_timestep that are done (0 between steps)
     int *stepsDone;
     int *scanTiles, *scanTotal;
     // learned p* guess: queue of the faces handed to the network (face ids,
