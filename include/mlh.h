@@ -147,8 +147,10 @@ typedef struct mlh_tuning {
     int face_split;          /* faces Newton has not finished after one step:
                               * 1 go to a second, dense pass over a queue;
                               * 2 are continued inside the block by its first
-                              * threads; 0: one pass (the plain gamma = 5/3
-                              * step only) */
+                              * threads; 0: one pass.  The plain steps of
+                              * gamma = 5/3 and 7/5 with the first-order
+                              * quadrature point; the others run one pass.
+                              * Until set: 2 from 65536 particles, else 0 */
     int link_overlap;        /* 1: the face links run on a second stream beside
                               * the time step and the gradients; 2: inside the
                               * gradients kernel, each particle's links before

@@ -273,6 +273,15 @@ void collect_timers(mlh_ctx *c) {
     c->tid.clear();
 }
 
+// Structure of the plain face pass when neither the caller nor the autotuner
+// chose one: one pass (0) for few particles, where a block has one or two
+// rounds of faces and the in-block regrouping (2) only adds its barriers;
+// in-block above.  Pass times in us at 0 / 2: KH 24^2 20 / 24, KH 100^2 46 / 47,
+// Sedov 33^3 (36k particles) 226 / 236, KH 317^2 (100k) 326 / 324, 16 blasts in
+// 48^3 (110k) 846 / 817, Sedov 64^3 1710 / 1655, 128^3 13990 / 13200, 64 KH
+// members (1.2M) 2844 / 2625.
+int face_split_rule(size_t n) { return n < (size_t)1 << 16 ? 0 : 2; }
+
 StepArgs make_args(mlh_ctx *c, double dt_max) {
     StepArgs a{};   // zeroed pointers and counts, the tuning's defaults
     a.p = c->p;
@@ -306,6 +315,7 @@ StepArgs make_args(mlh_ctx *c, double dt_max) {
     a.dt = c->dt; a.simTime = c->simTime; a.arrived = c->arrived; a.stepsDone = c->stepsDone;
     a.scanTiles = c->scanTiles; a.scanTotal = c->scanTotal;
     a.learned = (c->learned && c->tune.learned_guess) ? 1 : 0;
+    if (a.tune.face_split < 0) a.tune.face_split = a.learned ? 1 : face_split_rule(c->n);
     a.fstate = c->fstate; a.feat = c->feat; a.yguess = c->yguess;
     a.queueFace = c->queueFace; a.queueCount = c->queueCount; a.mlp_packed = c->mlp_packed;
     a.fstate2 = c->fstate2; a.queueFace2 = c->queueFace2; a.queueCount2 = c->queueCount2;

@@ -86,9 +86,9 @@ struct Prim {       // positions, primitive state of this step
 };
 struct Grad {       // limited gradients: rho, vx, vy, vz, P (x,y,z each), div v
     double g[16];
-    // particle part of the half-step prediction of each field, in the order
-    // rho, P, vx, vy, vz: rho div v + v.grad rho, gamma P div v + v.grad P,
-    // (grad P)_a / rho + v.grad v_a (the face subtracts v_frame.grad f)
+    // source terms of the half-step prediction of each field, in the order
+    // rho, P, vx, vy, vz: rho div v, gamma P div v, (grad P)_a / rho (the face
+    // adds (v - v_frame) . grad f)
     double t[8];
 };
 struct Geo {        // E_i^{-1}, 1/omega_i, omega_i, sound speed, 1/rho_i
@@ -99,9 +99,9 @@ struct FaceRef {    // canonical face: owner i, slot index, reverse slot (images
     int i, slot, rslot, pad;
 };
 // Face-frame state of one deferred face between the two passes of the
-// learned-guess face pipeline: R[5], L[5], A[3], v_frame[3], A/|A| [3], p_TR
+// learned-guess face pipeline: R[5], L[5], A[3], v_frame[3], p_TR
 struct FaceState {
-    double v[20];
+    double v[17];
 };
 // A queue of faces for a second face pass: their face-frame states, face ids
 // and the number of faces offered (entries at or beyond cap were not stored).

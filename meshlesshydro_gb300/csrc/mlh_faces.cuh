@@ -120,7 +120,7 @@ __device__ __forceinline__ float4 pstar_features(const double *R, const double *
 // MODE 0.  MODE 2 (second pass, over the queue): reload the state, solve from
 // the network's guess, project the flux.  `harvest` (MODE 0) records network
 // inputs and targets log(p*/p_TR) of every `stride`-th face.
-// MODE 3 (plain first pass, gamma = 5/3): one Newton step from the
+// MODE 3 (plain first pass, root solver): one Newton step from the
 // two-rarefaction guess; faces that have not converged are queued with their
 // iterate, so that the warps of this pass do not all run the second step that
 // a fifth of the faces need (nearly every warp holds one).  MODE 4 (second
@@ -132,14 +132,18 @@ __device__ __forceinline__ float4 pstar_features(const double *R, const double *
 // A/|A|.  The one-dimensional problem reads only the first rotated velocity
 // component, and the first row of that rotation is hatA: u = hatA . v.  The
 // velocities themselves stay unrotated (see project_flux).
+struct FaceNormal {
+    double AA, iAN;     // |A|^2, 1 / |A|
+    double unR, unL;    // their velocity components along the normal A / |A|
+};
 template <int D>
-__device__ __forceinline__ void face_normal(const double *A, const double *R, const double *L, double *hatA,
-                                            double &unR, double &unL) {
-    const double iAN = frsqrt(dotD<D>(A, A));
-#pragma unroll
-    for (int a = 0; a < D; ++a) hatA[a] = mulr(iAN, A[a]);
-    unR = dotD<D>(hatA, R + 2);
-    unL = dotD<D>(hatA, L + 2);
+__device__ __forceinline__ FaceNormal face_normal(const double *A, const double *R, const double *L) {
+    FaceNormal fn;
+    fn.AA = dotD<D>(A, A);
+    fn.iAN = frsqrt(fn.AA);
+    fn.unR = mulr(fn.iAN, dotD<D>(A, R + 2));
+    fn.unL = mulr(fn.iAN, dotD<D>(A, L + 2));
+    return fn;
 }
 
 // Riemann::exact after the solve and rotateAndProjectFluxes2D/3D
@@ -147,33 +151,30 @@ __device__ __forceinline__ void face_normal(const double *A, const double *R, co
 // tangential components from the sampled side, is rotated back and boosted by
 // the frame velocity, and the flux is projected on A_ij.  Rotating a state
 // into the face frame, replacing its normal component by u* and rotating back
-// leaves its tangential part unchanged, so v* = v_side + (u* - u_side) hatA
-// (u* hatA for vacuum), without the rotation matrices.  R (particle i, the
+// leaves its tangential part unchanged, so v* = v_side + (u* - u_side) hatA,
+// without the rotation matrices.  R (particle i, the
 // left state) and L: [rho, P, v..] with unrotated velocities, unR/unL their
 // normal components.  Fo: [mass, energy, px, py, pz].  Returns ST_VACUUM
 // when the solution is vacuum, else 0.
 template <int D>
 __device__ __forceinline__ unsigned project_flux(const RiemannResult &rs, const double *R, const double *L,
-                                                 double unR, double unL, const double *hatA, const double *A,
-                                                 const double *vf, double inv_gm1, int mfm, double *Fo) {
+                                                 const FaceNormal &fn, const double *A, const double *vf,
+                                                 double inv_gm1, int mfm, double *Fo) {
     unsigned st = 0;
     double vSol[3] = {0., 0., 0.};
-    if (rs.flag == 1 || rs.flag == -1) {
-        const double *side = rs.flag == 1 ? L : R;
-        const double du = subr(rs.u, rs.flag == 1 ? unL : unR);
+    // v* = v_side + s A with s = (u* - u_side) / |A|, and A . v* = u* |A|; for
+    // vacuum v_side = 0 and u* = 0
+    const bool left = rs.flag == 1, vacuum = rs.flag != 1 && rs.flag != -1;
+    if (vacuum) st = ST_VACUUM;
+    const double sA = mulr(subr(rs.u, vacuum ? 0. : left ? fn.unL : fn.unR), fn.iAN);
 #pragma unroll
-        for (int a = 0; a < D; ++a) vSol[a] = fma(du, hatA[a], side[2 + a]);
-    } else {
-        st = ST_VACUUM;
-#pragma unroll
-        for (int a = 0; a < D; ++a) vSol[a] = mulr(rs.u, hatA[a]);
-    }
+    for (int a = 0; a < D; ++a) vSol[a] = fma(sA, A[a], vacuum ? 0. : left ? L[2 + a] : R[2 + a]);
     // F_m = rho* (A . v*), F_p = F_m v_lab + P* A,
     // F_E = (A . v*) (P*/(gamma-1) + rho*/2 |v_lab|^2) + P* (A . v_lab);
     // MESHLESS_FINITE_MASS keeps F_m and drops the advective terms
     const double rhoSol = rs.rho, PSol = rs.p;
     const double pe = xmul(PSol, inv_gm1);
-    const double Av = dotD<D>(A, vSol);
+    const double Av = mulr(rs.u, mulr(fn.AA, fn.iAN));
     double vLab[3] = {0., 0., 0.};
 #pragma unroll
     for (int a = 0; a < D; ++a) vLab[a] = addr(vSol[a], vf[a]);
@@ -189,17 +190,20 @@ __device__ __forceinline__ unsigned project_flux(const RiemannResult &rs, const 
 }
 
 // Register caps of the face kernels: with the roots and products on the integer
-// pipe the passes wait on latency at 16 warps per SM.  One pass over the Sedov
-// 128^3 faces at 128 / 104 / 96 / 80 registers (16 / 16 / 20 / 24 warps):
-// 14.3 / 14.2 / 13.9 / 14.2 ms; over those of 64 KH members at 128 / 96 / 80 /
-// 72 (28 warps): 2.96 / 2.87 / 2.83 / 2.85 ms.  The grid is a multiple of the blocks that
-// reside at once (face_blocks): at 96 registers 8 blocks per SM left the
-// second of two rounds 3/5 full, 16.4 ms.
+// pipe the passes wait on latency at 16 warps per SM.  The in-block pass over the
+// Sedov 128^3 faces at 104 / 96 / 88 / 80 / 72 registers (16 / 20 / 20 / 24 / 28
+// warps): 13.84 / 13.30 / 13.33 / 13.25 / 13.41 ms; over those of 64 KH members at
+// 80 / 72 / 64: 2.65 / 2.63 / 2.74 ms; of 16 blasts in 48^3 (3D) at 96 / 80 / 72:
+// 832 / 817 / 822 us.  The grid is a multiple of the blocks that reside at once
+// (face_blocks): 8 blocks per SM at 96 registers left the second of two rounds
+// 3/5 full, 16.4 ms.  What the pass does per face: 198 FP64 operations, the
+// FP64 pipe 84 % active; the relative velocities in the prediction and v* along
+// A instead of along A / |A| took 13 of 198 (13.64 -> 13.30 ms at 96 registers).
 #ifndef MLH_FACE_MAXREG_3D
-#define MLH_FACE_MAXREG_3D 96
+#define MLH_FACE_MAXREG_3D 80
 #endif
 #ifndef MLH_FACE_MAXREG_2D
-#define MLH_FACE_MAXREG_2D 80
+#define MLH_FACE_MAXREG_2D 72
 #endif
 #define MLH_FACE_BOUNDS __maxnreg__(D == 3 ? MLH_FACE_MAXREG_3D : MLH_FACE_MAXREG_2D)
 // The face-frame Riemann problem of canonical face f (i < j): effective face
@@ -222,8 +226,7 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
                                             const Grad *__restrict__ grad, const uint32_t *__restrict__ nbr,
                                             const double *__restrict__ psi, const FaceRef *__restrict__ faces,
                                             const double *__restrict__ dtp, int f, unsigned &st_local, double *R,
-                                            double *L, double *A, double *vf, double *hatA, double &unR,
-                                            double &unL) {
+                                            double *L, double *A, double *vf, FaceNormal &fn) {
     constexpr int NV = D + 2;
     const FaceRef fr = faces[f];
     if (fr.i < 0 || fr.slot < 0) {
@@ -241,19 +244,6 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
     double xi[3] = {pi.x, pi.y, pi.z}, xj[3];
     if (img) neighbour_pos<D>(e, pj, grids[mi], xj);
     else { xj[0] = pj.x; xj[1] = pj.y; xj[2] = pj.z; }
-    // --- effective face, from V_i psi~_j(x_i) of both slots
-    {
-        const double *ps_i = psi + si * 3;
-        if (fr.rslot >= 0) {
-            const double *ps_j = psi + ((size_t)j * p.K + fr.rslot) * 3;
-#pragma unroll
-            for (int a = 0; a < D; ++a) A[a] = subr(ps_i[a], ps_j[a]);
-        } else {
-            st_local |= ST_ASYMMETRIC;
-#pragma unroll
-            for (int a = 0; a < D; ++a) A[a] = ps_i[a];
-        }
-    }
     // --- states at the face
     double xijxi[3], xjxi[3], xijxj[3];
     const double hq = MID ? 0. : p.adaptive_h ? p.hp[i] : members[mi].h;   // quadrature-point radius
@@ -272,94 +262,107 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
         }
     }
     const double vi[3] = {pi.vx, pi.vy, pi.vz}, vj[3] = {pj.vx, pj.vy, pj.vz};
-    if (p.move) {
-        if (MID) {
+    // v_i - v_f and v_j - v_f; with the midpoint the frame moves with the mean, and
+    // they are (v_i - v_j) / 2 and its exact negation
+    double wi[3] = {0., 0., 0.}, wj[3] = {0., 0., 0.};
+    if (MID) {
 #pragma unroll
-            for (int a = 0; a < D; ++a) vf[a] = half_of(addr(vi[a], vj[a]));
-        } else {
+        for (int a = 0; a < D; ++a) {
+            const double mean = half_of(addr(vi[a], vj[a])), half = half_of(subr(vi[a], vj[a]));
+            vf[a] = p.move ? mean : 0.;
+            wi[a] = p.move ? half : vi[a];
+            wj[a] = p.move ? flip_if(half, true) : vj[a];
+        }
+    } else {
+        if (p.move) {
             const double dotProd = dotD<D>(xijxi, xjxi);
             const double dSqr = dotD<D>(xjxi, xjxi);
 #pragma unroll
             for (int a = 0; a < D; ++a) vf[a] = addr(vi[a], mulr(subr(vj[a], vi[a]), dotProd) / dSqr);
         }
+#pragma unroll
+        for (int a = 0; a < D; ++a) { wi[a] = subr(vi[a], vf[a]); wj[a] = subr(vj[a], vf[a]); }
     }
     const double *Gi = grad[i].g, *Gj = grad[j].g;
     // gradient blocks: 0 rho, 3 vx, 6 vy, 9 vz, 12 P
     R[0] = pi.rho; L[0] = pj.rho;
     R[1] = pi.P; L[1] = pj.P;
 #pragma unroll
-    for (int a = 0; a < D; ++a) { R[2 + a] = subr(vi[a], vf[a]); L[2 + a] = subr(vj[a], vf[a]); }
-    // W -= dt/2 (source + (v - v_frame) . grad W): the particle part,
-    // source + v . grad W, comes with the gradients (Grad::t); the face adds
-    // v_frame . grad W.  The reference uses vz[i] on the j side of the vx and
-    // vy terms in 3D (Particles.cpp:1717,1719): (vz_i - vf_z) = (vz_j - vq_z)
-    // with the shifted frame velocity vq_z = vf_z - (vz_i - vz_j).
-    const double hdt = half_of(dt), nhdt = flip_if(hdt, true);
+    for (int a = 0; a < D; ++a) { R[2 + a] = wi[a]; L[2 + a] = wj[a]; }
+    // W -= dt/2 (source + (v - v_frame) . grad W): the sources come with the
+    // gradients (Grad::t).  The reference uses vz[i] on the j side of the vx and
+    // vy terms in 3D (Particles.cpp:1717,1719).
+    const double nhdt = flip_if(half_of(dt), true);
     const double *Ti = grad[i].t, *Tj = grad[j].t;
     const int blk[5] = {0, 12, 3, 6, 9};   // gradient blocks: 0 rho, 3 vx, 6 vy, 9 vz, 12 P
-    const double vq2 = D == 3 ? subr(vf[2], subr(vi[2], vj[2])) : 0.;
     if (D == 2 && !p.pairwise) {
         // no limiter between reconstruction and prediction: one FMA chain per
-        // field and side, W - dt/2 T + grad W . (x_ij - x_side + dt/2 v_frame)
+        // field and side, W - dt/2 source + grad W . (x_ij - x_side - dt/2 (v - v_frame))
         // (a run-wide branch: with the limiter on, image faces that skip it
         // keep the other form, so that warps do not run both; 3D keeps the
         // other form, whose registers the 3D face kernels are tuned to)
-        double yi[3], yj[3], yq[3];
+        double yi[3], yj[3];
 #pragma unroll
         for (int a = 0; a < D; ++a) {
-            yi[a] = fma(hdt, vf[a], xijxi[a]);
-            yj[a] = fma(hdt, vf[a], xijxj[a]);
-            yq[a] = (D == 3 && a == 2) ? fma(hdt, vq2, xijxj[a]) : yj[a];
+            yi[a] = fma(nhdt, wi[a], xijxi[a]);
+            yj[a] = MID ? flip_if(yi[a], true) : fma(nhdt, wj[a], xijxj[a]);
+        }
+        if (MID && !p.move) {   // both sides advected with their own velocity
+#pragma unroll
+            for (int a = 0; a < D; ++a) yj[a] = fma(nhdt, wj[a], xijxj[a]);
         }
 #pragma unroll
         for (int f = 0; f < NV; ++f) {
             R[f] = fma_dotD<D>(Gi + blk[f], yi, fma(nhdt, Ti[f], R[f]));
-            const double *yy = (D == 3 && (f == 2 || f == 3)) ? yq : yj;
-            L[f] = fma_dotD<D>(Gj + blk[f], yy, fma(nhdt, Tj[f], L[f]));
+            L[f] = fma_dotD<D>(Gj + blk[f], yj, fma(nhdt, Tj[f], L[f]));
         }
     } else {
-        double Rb[5], Lb[5];
+        // image faces skip the limiter (Particles.cpp:2533-2683)
+        const bool limit = p.pairwise && (!img || p.img_pw);
+        // |x_ij - x_i| / |x_j - x_i| and |x_ij - x_j| / |x_j - x_i|: with the
+        // first-order quadrature point x_ij - x_i = (x_j - x_i) / 2 exactly,
+        // so both quotients are exactly 0.5
+        double ri = .5, rj = .5;
+        if (!MID && limit) {
+            double xijxi_abs = 0., xijxj_abs = 0., xjxi_abs = 0.;
 #pragma unroll
-        for (int k = 0; k < NV; ++k) { Rb[k] = R[k]; Lb[k] = L[k]; }
-        // W + grad W . (x_ij - x_side), one FMA chain from W per field
-#pragma unroll
-        for (int f = 0; f < NV; ++f) {
-            R[f] = fma_dotD<D>(Gi + blk[f], xijxi, R[f]);
-            L[f] = fma_dotD<D>(Gj + blk[f], xijxj, L[f]);
-        }
-        if (p.pairwise && (!img || p.img_pw)) {   // image faces skip it (Particles.cpp:2533-2683)
-            // |x_ij - x_i| / |x_j - x_i| and |x_ij - x_j| / |x_j - x_i|: with the
-            // first-order quadrature point x_ij - x_i = (x_j - x_i) / 2 exactly,
-            // so both quotients are exactly 0.5
-            double ri = .5, rj = .5;
-            if (!MID) {
-                double xijxi_abs = 0., xijxj_abs = 0., xjxi_abs = 0.;
-#pragma unroll
-                for (int a = 0; a < D; ++a) {
-                    xijxi_abs = fma(xijxi[a], xijxi[a], xijxi_abs);
-                    xijxj_abs = fma(xijxj[a], xijxj[a], xijxj_abs);
-                    xjxi_abs = fma(xjxi[a], xjxi[a], xjxi_abs);
-                }
-                xjxi_abs = sqrt(xjxi_abs);
-                ri = sqrt(xijxi_abs) / xjxi_abs;
-                rj = sqrt(xijxj_abs) / xjxi_abs;
+            for (int a = 0; a < D; ++a) {
+                xijxi_abs = fma(xijxi[a], xijxi[a], xijxi_abs);
+                xijxj_abs = fma(xijxj[a], xijxj[a], xijxj_abs);
+                xjxi_abs = fma(xjxi[a], xjxi[a], xjxi_abs);
             }
-#pragma unroll
-            for (int k = 0; k < NV; ++k) pairwise_limiter<MID>(p, R[k], L[k], Rb[k], Lb[k], ri, rj);
+            xjxi_abs = sqrt(xjxi_abs);
+            ri = sqrt(xijxi_abs) / xjxi_abs;
+            rj = sqrt(xijxj_abs) / xjxi_abs;
         }
-        // the prediction, one FMA chain per field and side from the limited value
-        const double nvf[3] = {flip_if(vf[0], true), flip_if(vf[1], true), flip_if(vf[2], true)};
-        const double nvq[3] = {nvf[0], nvf[1], flip_if(vq2, true)};
+        const double wq[3] = {wj[0], wj[1], wi[2]};
+        // field by field, so that one field's gradients and particle values are
+        // live at a time: W + grad W . (x_ij - x_side), one FMA chain from W; the
+        // limiter; the prediction, one FMA chain per side from the limited value
 #pragma unroll
         for (int f = 0; f < NV; ++f) {
-            R[f] = fma(nhdt, fma_dotD<D>(nvf, Gi + blk[f], Ti[f]), R[f]);
-            const double *nj = (D == 3 && (f == 2 || f == 3)) ? nvq : nvf;
-            L[f] = fma(nhdt, fma_dotD<D>(nj, Gj + blk[f], Tj[f]), L[f]);
+            double r = fma_dotD<D>(Gi + blk[f], xijxi, R[f]), l = fma_dotD<D>(Gj + blk[f], xijxj, L[f]);
+            if (limit) pairwise_limiter<MID>(p, r, l, R[f], L[f], ri, rj);
+            R[f] = fma(nhdt, fma_dotD<D>(wi, Gi + blk[f], Ti[f]), r);
+            L[f] = fma(nhdt, fma_dotD<D>((D == 3 && (f == 2 || f == 3)) ? wq : wj, Gj + blk[f], Tj[f]), l);
         }
     }
     if (dneg(R[1]) || dneg(L[1])) st_local |= ST_NEG_PRESSURE;
+    // --- effective face, from V_i psi~_j(x_i) of both slots
+    {
+        const double *ps_i = psi + si * 3;
+        if (fr.rslot >= 0) {
+            const double *ps_j = psi + ((size_t)j * p.K + fr.rslot) * 3;
+#pragma unroll
+            for (int a = 0; a < D; ++a) A[a] = subr(ps_i[a], ps_j[a]);
+        } else {
+            st_local |= ST_ASYMMETRIC;
+#pragma unroll
+            for (int a = 0; a < D; ++a) A[a] = ps_i[a];
+        }
+    }
     // --- Riemann problem in the face frame (i left, j right)
-    face_normal<D>(A, R, L, hatA, unR, unL);
+    fn = face_normal<D>(A, R, L);
     return true;
 }
 
@@ -387,23 +390,23 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nf; t += gridDim.x * blockDim.x) {
         // MODE 2 walks the queue: t is the queue position, f the face
         const int f = QUEUED ? qa.face[t] : t;
-        double R[5], L[5], A[3] = {0., 0., 0.}, vf[3] = {0., 0., 0.}, hatA[3] = {0., 0., 0.};
-        double unR = 0., unL = 0.;   // velocity components along the face normal
+        double R[5], L[5], A[3] = {0., 0., 0.}, vf[3] = {0., 0., 0.};
+        FaceNormal fn = {};
         double ptr_q = -1.;   // MODE 2: two-rarefaction guess found in MODE 1; MODE 4: Newton iterate
         if (QUEUED) {
             const FaceState &fs = qa.st[t];
-            ptr_q = fs.v[19];
+            ptr_q = fs.v[16];
 #pragma unroll
             for (int k = 0; k < 5; ++k) { R[k] = fs.v[k]; L[k] = fs.v[5 + k]; }
 #pragma unroll
-            for (int a = 0; a < 3; ++a) { A[a] = fs.v[10 + a]; vf[a] = fs.v[13 + a]; hatA[a] = fs.v[16 + a]; }
-            unR = dotD<D>(hatA, R + 2);
-            unL = dotD<D>(hatA, L + 2);
+            for (int a = 0; a < 3; ++a) { A[a] = fs.v[10 + a]; vf[a] = fs.v[13 + a]; }
+            fn = face_normal<D>(A, R, L);
         } else {
         if (!face_states<D, MID>(p, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, f, st_local, R, L, A,
-                            vf, hatA, unR, unL))
+                            vf, fn))
             continue;
         }   // !QUEUED
+        const double unR = fn.unR, unL = fn.unL;
         double guess = -1.;
         if (MODE == 2) {
             const float y = yguess[t];
@@ -428,8 +431,8 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
 #pragma unroll
                 for (int k = 0; k < 5; ++k) { fs.v[k] = R[k]; fs.v[5 + k] = L[k]; }
 #pragma unroll
-                for (int a = 0; a < 3; ++a) { fs.v[10 + a] = A[a]; fs.v[13 + a] = vf[a]; fs.v[16 + a] = hatA[a]; }
-                fs.v[19] = rs.pstar;   // the two-rarefaction guess (strong) or the Newton iterate
+                for (int a = 0; a < 3; ++a) { fs.v[10 + a] = A[a]; fs.v[13 + a] = vf[a]; }
+                fs.v[16] = rs.pstar;   // the two-rarefaction guess (strong) or the Newton iterate
                 fq.face[q] = f;
                 if (strong) feat[q] = pstar_features(R, L, unR, unL, gamma);
                 else iters_local += (unsigned long long)rs.iters;
@@ -473,7 +476,7 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
             iters_local += (unsigned long long)rs.iters;
         }
         double Fo[5];
-        st_local |= project_flux<D>(rs, R, L, unR, unL, hatA, A, vf, rc.inv_gm1, p.mfm, Fo);
+        st_local |= project_flux<D>(rs, R, L, fn, A, vf, rc.inv_gm1, p.mfm, Fo);
         // the face's Newton steps (the step of the first pass included in
         // MODE 4; -1: no convergence) in the record's sixth double, for parity
         // checks
@@ -498,7 +501,7 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
     }
 }
 
-// Plain gamma = 5/3 face pass with the faces that need more than one Newton
+// Plain root-solver face pass with the faces that need more than one Newton
 // step regrouped inside the block (face_split 2).  A warp issues every
 // instruction that any of its lanes needs, so the second Newton step of the
 // few faces that need it would hold the whole warp.  Instead: every face of
@@ -564,18 +567,18 @@ __global__ void MLH_FACE_BOUNDS k_faces_block(Params p, RiemannConsts rc, const 
     unsigned st_local = 0;
     for (int t0 = blockIdx.x * FB_T; t0 < nf; t0 += gridDim.x * FB_T) {
         const int f = t0 + threadIdx.x;
-        double R[5], L[5], A[3] = {0., 0., 0.}, vf[3] = {0., 0., 0.}, hatA[3] = {0., 0., 0.};
-        double unR = 0., unL = 0.;
+        double R[5], L[5], A[3] = {0., 0., 0.}, vf[3] = {0., 0., 0.};
+        FaceNormal fn = {};
         bool valid = f < nf;
         if (valid)
             valid = face_states<D, true>(p, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, f, st_local, R,
-                                   L, A, vf, hatA, unR, unL);
+                                   L, A, vf, fn);
         bool unfinished = false, strong = false;
         if (valid) {
             // strong shocks of the learned step stop before their first
             // Newton step: p_TR > PSTAR_HARD min(pL, pR) (min on the keys)
             const double defer = LEARNED ? PSTAR_HARD * (dlt(L[1], R[1]) ? L[1] : R[1]) : 0.;
-            const RootSolve s0 = riemann_root_begin<ROOT>(rc, R[0], unR, R[1], L[0], unL, L[1], -1., defer, 1);
+            const RootSolve s0 = riemann_root_begin<ROOT>(rc, R[0], fn.unR, R[1], L[0], fn.unL, L[1], -1., defer, 1);
             sv[threadIdx.x] = s0;
             unfinished = s0.stage == 2;
             strong = LEARNED && s0.stage == 3;
@@ -628,7 +631,7 @@ __global__ void MLH_FACE_BOUNDS k_faces_block(Params p, RiemannConsts rc, const 
             if (rs.iters < 0) st_local |= ST_NEWTON;
             else iters_local += (unsigned long long)rs.iters;
             double Fo[5];
-            st_local |= project_flux<D>(rs, R, L, unR, unL, hatA, A, vf, rc.inv_gm1, p.mfm, Fo);
+            st_local |= project_flux<D>(rs, R, L, fn, A, vf, rc.inv_gm1, p.mfm, Fo);
             const int face_iters = rs.iters < 0 ? -1 : rs.iters + (unfinished ? 1 : 0);
             double2 *dst = reinterpret_cast<double2 *>(Fface + (size_t)f * 6);
             dst[0] = make_double2(Fo[0], Fo[1]);
@@ -669,18 +672,19 @@ __global__ void __launch_bounds__(256) k_riemann_batch(int n, RiemannConsts rc, 
     unsigned st = 0;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < n; f += gridDim.x * blockDim.x) {
         double R[5] = {0., 0., 0., 0., 0.}, L[5] = {0., 0., 0., 0., 0.};
-        double A[3] = {0., 0., 0.}, vf[3] = {0., 0., 0.}, hatA[3], unR, unL;
+        double A[3] = {0., 0., 0.}, vf[3] = {0., 0., 0.};
 #pragma unroll
         for (int k = 0; k < NV; ++k) { R[k] = Wi[(size_t)f * NV + k]; L[k] = Wj[(size_t)f * NV + k]; }
 #pragma unroll
         for (int a = 0; a < D; ++a) { A[a] = Aij[(size_t)f * D + a]; vf[a] = vFrame[(size_t)f * D + a]; }
         if (R[1] < 0. || L[1] < 0.) st |= ST_NEG_PRESSURE;
-        face_normal<D>(A, R, L, hatA, unR, unL);
+        const FaceNormal fn = face_normal<D>(A, R, L);
+        const double unR = fn.unR, unL = fn.unL;
         const RiemannResult rs = ROOT ? riemann_exact_root<ROOT ? ROOT : 5>(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.)
                                        : riemann_exact(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.);
         if (rs.iters < 0) st |= ST_NEWTON;
         double Fo[5];
-        st |= project_flux<D>(rs, R, L, unR, unL, hatA, A, vf, rc.inv_gm1, mfm, Fo);
+        st |= project_flux<D>(rs, R, L, fn, A, vf, rc.inv_gm1, mfm, Fo);
 #pragma unroll
         for (int k = 0; k < NV; ++k) F[(size_t)f * NV + k] = Fo[k];
         if (iters) iters[f] = rs.iters;

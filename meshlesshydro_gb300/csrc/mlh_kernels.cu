@@ -2143,16 +2143,13 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
         }
         // div v of the limited gradients, in the face kernel's order
         go.g[15] = D == 3 ? (go.g[3] + go.g[7]) + go.g[11] : go.g[3] + go.g[7];
-        {   // the particle part of the half-step prediction (fma chains)
+        {   // the sources of the half-step prediction
             const double *G = go.g;
             const double div = go.g[15], irho = geo[i].irho;
-            const double v[3] = {pi.vx, pi.vy, pi.vz};
-            const double src[5] = {pi.rho * div, (p.gamma * pi.P) * div, G[12] * irho, G[13] * irho, G[14] * irho};
-            const int blk[5] = {0, 12, 3, 6, 9};
+            const double src[5] = {mulr(pi.rho, div), mulr(p.gamma * pi.P, div), mulr(G[12], irho), mulr(G[13], irho),
+                                   mulr(G[14], irho)};
 #pragma unroll
-            for (int f = 0; f < 8; ++f) go.t[f] = 0.;
-#pragma unroll
-            for (int f = 0; f < D + 2; ++f) go.t[f] = fma_dotD<D>(v, G + blk[f], src[f]);
+            for (int f = 0; f < 8; ++f) go.t[f] = f < D + 2 ? src[f < 5 ? f : 0] : 0.;
         }
         grad[i] = go;
       }   // i < p.n

@@ -15,7 +15,7 @@ struct Tuning {
     int face_blocks_per_sm = 32;   // grid of the grid-stride face loop (32 against 8: -0.5 % on Sedov 128^3, -9 % on 16 blasts in 48^3, whose shocks fill a few blocks)
     int grad_threads = 128;        // threads per block of k_gradients
     int nns_warps_per_sm = 32;     // warps per SM of k_neighbours: one round of resident blocks
-    int face_split = 0;            // plain root-solver step: 1 second Newton pass over a queue, 2 in-block, 0 none
+    int face_split = -1;           // plain root-solver step: 1 second Newton pass over a queue, 2 in-block, 0 none; -1: by size (mlh_capi.cu, face_split_rule)
     int link_overlap = 1;          // face links on the second stream beside the time step and gradients
     int persistent_binning = 0;    // the binning as one persistent cooperative kernel (k_binning)
     int fp32_filters = 3;          // bits: 1 slope-limiter extrema, 2 time step (FP64 only where a single-precision bound reaches the result)

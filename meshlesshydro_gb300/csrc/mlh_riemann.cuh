@@ -307,8 +307,8 @@ struct RootSolve {
 // p_TR (Toro eq. 4.46) of the sorted problem.
 template <int N>
 __device__ __forceinline__ double root_guess(const RiemannConsts &k, const RiemannSide &A, const RiemannSide &B,
-                                             double du) {
-    const double num = fma(-k.g7, du, addr(A.c, B.c));
+                                             double csum, double du) {
+    const double num = fma(-k.g7, du, csum);
     const double den = fma(A.c, rroot<N>(A.p), xmul(B.c, rroot<N>(B.p)));
     const double t = mulr(num, frcp(den));
     const double t2 = xmul(t, t), t4 = xmul(t2, t2);
@@ -331,7 +331,7 @@ __device__ __forceinline__ void riemann_root_newton(const RiemannConsts &k, Root
         if (attempt == 1) {
             if (!tried_guess) break;
             extra = k.max_iter;
-            p0 = root_guess<N>(k, A, B, du);
+            p0 = root_guess<N>(k, A, B, addr(A.c, B.c), du);
         }
         p = nn_le(p0, pfloor) ? pfloor : p0;
         for (int it = 1; it <= k.max_iter; ++it) {
@@ -381,7 +381,8 @@ __device__ __forceinline__ RootSolve riemann_root_begin(const RiemannConsts &k, 
     s.B = make_side(k, mir ? rhoL : rhoR, mir ? flip_if(uL, true) : uR, mir ? pL : pR);
     s.fAs = 0.; s.fBs = 0.; s.qAs = -1.; s.qBs = -1.; s.iters = 0; s.p = 0.;
     s.du = subr(s.B.u, s.A.u);
-    if (!dlt(s.du, addr(s.A.g4c, s.B.g4c))) {   // g4 cL + g4 cR <= uR - uL: vacuum
+    const double csum = addr(s.A.c, s.B.c);
+    if (!dlt(s.du, xmul(k.g4, csum))) {         // g4 (cL + cR) <= uR - uL: vacuum
         s.stage = 0;
         return s;
     }
@@ -390,7 +391,7 @@ __device__ __forceinline__ RootSolve riemann_root_begin(const RiemannConsts &k, 
     const bool tried_guess = __double_as_longlong(guess) > 0;   // guess > 0 (-1: none)
     if (tried_guess) p0 = guess;
     else {
-        p0 = root_guess<N>(k, s.A, s.B, s.du);
+        p0 = root_guess<N>(k, s.A, s.B, csum, s.du);
         // defer_above > 0 and p0 > defer_above, on the keys (see riemann_exact)
         if (ord_key(defer_above) > 0 && dlt(defer_above, p0)) {
             s.p = p0; s.stage = 3;
