@@ -42,6 +42,29 @@ cudaError_t dalloc(T **p, size_t count) {
     return cudaMalloc((void **)p, sizeof(T) * count);
 }
 
+// Arrays cut from one allocation on 256-byte boundaries: a context holds some
+// sixty arrays, and an allocation of its own for each made 0.7 ms of a small
+// context's creation.
+class Arena {
+public:
+    template <class T>
+    void add(T **p, size_t count) {
+        *p = nullptr;
+        want_.push_back({(void **)p, bytes_});
+        bytes_ += (sizeof(T) * (count ? count : 1) + 255) & ~(size_t)255;
+    }
+    cudaError_t alloc(char **base) {
+        const cudaError_t e = cudaMalloc((void **)base, bytes_);
+        if (e != cudaSuccess) { *base = nullptr; return e; }
+        for (const auto &w : want_) *w.first = *base + w.second;
+        return cudaSuccess;
+    }
+
+private:
+    std::vector<std::pair<void **, size_t>> want_;
+    size_t bytes_ = 0;
+};
+
 }  // namespace
 
 namespace mlh {
@@ -94,7 +117,14 @@ struct mlh_ctx {
     double *hp = nullptr, *neff = nullptr;
     float *hpf = nullptr;
     unsigned long long *hstat = nullptr;
-    // scalars
+    // allocations the arrays are cut from: sized by the particles and
+    // simulations, by the neighbour slots, by the cells
+    char *arena = nullptr, *ngbArena = nullptr, *cellArena = nullptr;
+    // scalars: newtonSum[3], status, stepsDone, dt and simTime of every
+    // simulation lie in one block, cleared and read back in one operation each
+    // per mlh_step; hscal is its pinned copy, with the number of faces behind
+    char *scal = nullptr;
+    char *hscal = nullptr;
     unsigned *status = nullptr;
     unsigned long long *dtbits = nullptr, *newtonSum = nullptr;
     double *dt = nullptr, *simTime = nullptr;
@@ -136,10 +166,8 @@ namespace {
 int round_slots(int k) { return (k + 3) & ~3; }
 
 void free_neighbour_buffers(mlh_ctx *c) {
-    cudaFree(c->nbr); cudaFree(c->ww); cudaFree(c->psi); cudaFree(c->faceOf); cudaFree(c->faces);
-    cudaFree(c->Fface);
-    cudaFree(c->fstate); cudaFree(c->feat); cudaFree(c->yguess); cudaFree(c->queueFace); cudaFree(c->queueCount);
-    cudaFree(c->fstate2); cudaFree(c->queueFace2); cudaFree(c->queueCount2);
+    cudaFree(c->ngbArena);
+    c->ngbArena = nullptr;
     c->queueFace = nullptr; c->queueCount = nullptr;
     c->fstate2 = nullptr; c->queueFace2 = nullptr; c->queueCount2 = nullptr;
     c->nbr = nullptr; c->ww = nullptr; c->psi = nullptr; c->faceOf = nullptr; c->faces = nullptr;
@@ -158,13 +186,14 @@ int alloc_neighbour_buffers(mlh_ctx *c) {
         g_last_error = "too many faces for 32-bit face ids (particles x neighbour slots / 2 above 2^31 - 1)";
         return MLH_ERR_CAPACITY;
     }
-    CK(dalloc(&c->nbr, slots));
-    CK(dalloc(&c->ww, slots));
-    CK(dalloc(&c->psi, slots * 3));
+    Arena ar;
+    ar.add(&c->nbr, slots);
+    ar.add(&c->ww, slots);
+    ar.add(&c->psi, slots * 3);
     c->faces_cap = faces;
-    CK(dalloc(&c->faceOf, slots));
-    CK(dalloc(&c->faces, faces));
-    CK(dalloc(&c->Fface, faces * 6));
+    ar.add(&c->faceOf, slots);
+    ar.add(&c->faces, faces);
+    ar.add(&c->Fface, faces * 6);
     // queues of faces for second face passes.  A: in the plain step the
     // faces Newton has not finished after one step (a fifth to two thirds of
     // them; faces_cap is about twice the faces of a step; a full queue
@@ -173,35 +202,39 @@ int alloc_neighbour_buffers(mlh_ctx *c) {
     // guess only): the faces Newton has not finished after one step.
     const size_t half = faces / 2 + 1024;
     c->queue_cap = c->learned ? faces : half;
-    CK(dalloc(&c->fstate, c->queue_cap));
-    CK(dalloc(&c->queueFace, c->queue_cap));
-    CK(dalloc(&c->queueCount, 1));
+    ar.add(&c->fstate, c->queue_cap);
+    ar.add(&c->queueFace, c->queue_cap);
+    ar.add(&c->queueCount, 1);
     c->queue_cap2 = 0;
     if (c->learned) {
-        CK(dalloc(&c->feat, faces));
-        CK(dalloc(&c->yguess, faces));
+        ar.add(&c->feat, faces);
+        ar.add(&c->yguess, faces);
         c->queue_cap2 = half;
-        CK(dalloc(&c->fstate2, half));
-        CK(dalloc(&c->queueFace2, half));
-        CK(dalloc(&c->queueCount2, 1));
+        ar.add(&c->fstate2, half);
+        ar.add(&c->queueFace2, half);
+        ar.add(&c->queueCount2, 1);
     }
+    CK(ar.alloc(&c->ngbArena));
     return 0;
 }
 
 void free_cell_buffers(mlh_ctx *c) {
-    cudaFree(c->cellCount); cudaFree(c->cellStart); cudaFree(c->cellFill);
+    cudaFree(c->cellArena);
+    c->cellArena = nullptr;
+    c->scanTiles = nullptr;
     c->cellCount = c->cellStart = c->cellFill = nullptr;
 }
 
 int alloc_cell_buffers(mlh_ctx *c) {
     size_t nc = (size_t)c->p.ncells_cap + 1;
-    CK(dalloc(&c->cellCount, nc));
-    CK(dalloc(&c->cellStart, nc + 1));
-    CK(dalloc(&c->cellFill, nc));
+    Arena ar;
+    ar.add(&c->cellCount, nc);
+    ar.add(&c->cellStart, nc + 1);
+    ar.add(&c->cellFill, nc);
     // tile sums of the scans over the cell counts and over the particles
-    cudaFree(c->scanTiles);
     const size_t m = nc > (size_t)c->n ? nc : (size_t)c->n;
-    CK(dalloc(&c->scanTiles, m / 4096 + 1024));
+    ar.add(&c->scanTiles, m / 4096 + 1024);
+    CK(ar.alloc(&c->cellArena));
     return 0;
 }
 
@@ -272,6 +305,11 @@ void collect_timers(mlh_ctx *c) {
     c->tev.clear();
     c->tid.clear();
 }
+
+// Layout of mlh_ctx::scal: counters (newtonSum[3], status, stepsDone), then dt
+// of the `nm` simulations, then simTime of the first `times`.
+constexpr size_t STEP_COUNTERS = 3 * sizeof(unsigned long long) + sizeof(unsigned) + sizeof(int);
+size_t step_scalars_bytes(size_t nm, size_t times) { return STEP_COUNTERS + sizeof(double) * (nm + times); }
 
 // Structure of the plain face pass when neither the caller nor the autotuner
 // chose one: one pass (0) for few particles, where a block has one or two
@@ -464,7 +502,8 @@ static int create_impl(const mlh_config *cfg, int nmembers, const mlh_member *md
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess)
         return fail(cuda_fail(cudaGetLastError(), "second stream"));
     size_t n = (size_t)c->n, nm = (size_t)nmembers;
-#define A(ptr, cnt) if (dalloc(&c->ptr, cnt) != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "cudaMalloc " #ptr))
+    Arena ar;
+#define A(ptr, cnt) ar.add(&c->ptr, cnt)
     A(x, n); A(y, n); A(z, n); A(vx, n); A(vy, n); A(vz, n); A(m, n); A(u, n);
     A(posf, n); A(velf, n); A(dtlo, n); A(dtcap, nm);
     A(members, nm); A(grids, nm); A(cellTotal, 1); A(boundsPart, nm * (size_t)c->bpm * 6);
@@ -472,11 +511,20 @@ static int create_impl(const mlh_config *cfg, int nmembers, const mlh_member *md
     A(cell, n); A(cellList, n);
     A(noi, n); A(noiImg, n); A(faceCnt, n); A(faceOff, n + 1);
     A(prim, n); A(geo, n); A(grad, n); A(gradRaw, n); A(fluxSums, n * 5);
-    A(status, 1); A(dtbits, nm); A(newtonSum, 3); A(dt, nm); A(simTime, nm); A(stepsDone, 1);
+    A(dtbits, nm);
+    A(scal, step_scalars_bytes(nm, nm));
     A(hp, n); A(neff, n); A(hstat, 2); A(hpf, n);
     A(scanTotal, 1);
     A(bar, 2); A(arrived, 1);
 #undef A
+    if (ar.alloc(&c->arena) != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "cudaMalloc"));
+    c->newtonSum = (unsigned long long *)c->scal;
+    c->status = (unsigned *)(c->scal + 3 * sizeof(unsigned long long));
+    c->stepsDone = (int *)(c->status + 1);
+    c->dt = (double *)(c->scal + STEP_COUNTERS);
+    c->simTime = c->dt + nm;
+    if (cudaMallocHost(&c->hscal, step_scalars_bytes(nm, 1) + sizeof(int)) != cudaSuccess)
+        return fail(cuda_fail(cudaGetLastError(), "cudaMallocHost"));
     if ((rc = alloc_cell_buffers(c))) return fail(rc);
     if ((rc = alloc_neighbour_buffers(c))) return fail(rc);
     if (cudaMemcpyAsync(c->members, mem.data(), sizeof(Member) * nm, cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
@@ -488,11 +536,7 @@ static int create_impl(const mlh_config *cfg, int nmembers, const mlh_member *md
         if (cudaMemcpy(c->memberOf, mo.data(), sizeof(int) * n, cudaMemcpyHostToDevice) != cudaSuccess)
             return fail(cuda_fail(cudaGetLastError(), "memberOf"));
     }
-    cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream);
-    cudaMemsetAsync(c->simTime, 0, sizeof(double) * nm, c->stream);
-    cudaMemsetAsync(c->dt, 0, sizeof(double) * nm, c->stream);
-    cudaMemsetAsync(c->newtonSum, 0, 3 * sizeof(unsigned long long), c->stream);
-    cudaMemsetAsync(c->stepsDone, 0, sizeof(int), c->stream);
+    cudaMemsetAsync(c->scal, 0, step_scalars_bytes(nm, nm), c->stream);
     cudaMemsetAsync(c->arrived, 0, sizeof(unsigned), c->stream);
     cudaMemsetAsync(c->neff, 0, sizeof(double) * n, c->stream);
     cudaMemsetAsync(c->hstat, 0, 2 * sizeof(unsigned long long), c->stream);
@@ -566,12 +610,8 @@ void mlh_destroy(mlh_ctx *c) {
     if (!c) return;
     if (c->stream) cudaStreamSynchronize(c->stream);
     drop_graph(c);
-    void *ptrs[] = {c->x, c->y, c->z, c->vx, c->vy, c->vz, c->m, c->u, c->posf, c->members, c->memberOf, c->grids,
-                    c->cellTotal, c->boundsPart, c->cell, c->cellList, c->noi, c->noiImg, c->faceCnt, c->faceOff,
-                    c->prim, c->geo, c->grad, c->gradRaw, c->fluxSums, c->status, c->dtbits, c->newtonSum, c->dt,
-                    c->simTime, c->stepsDone, c->scanTiles, c->scanTotal, c->hp, c->neff, c->hstat, c->hpf, c->bar,
-                    c->velf, c->dtlo, c->dtcap, c->arrived};
-    for (void *q : ptrs) if (q) cudaFree(q);
+    cudaFree(c->arena);
+    if (c->hscal) cudaFreeHost(c->hscal);
     free_cell_buffers(c);
     free_neighbour_buffers(c);
     if (c->mlp_w) cudaFree(c->mlp_w);
@@ -634,15 +674,14 @@ int mlh_step(mlh_ctx *c, int nsteps, double dt_max, mlh_step_stats *stats) {
     int done_total = 0;
     int remaining = nsteps;
     int retries = 0;
+    bool have_scalars = false;
     while (remaining > 0) {
         const bool use_graph = c->graph_mode && !c->timing;
         if (use_graph && (!c->graph_exec || c->graph_dt_max != dt_max)) {
             int rc = capture_step(c, dt_max);
             if (rc) return rc;
         }
-        CK(cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream));
-        CK(cudaMemsetAsync(c->stepsDone, 0, sizeof(int), c->stream));
-        CK(cudaMemsetAsync(c->newtonSum, 0, 3 * sizeof(unsigned long long), c->stream));
+        CK(cudaMemsetAsync(c->scal, 0, STEP_COUNTERS, c->stream));
         CK(cudaEventRecord(c->ev0, c->stream));
         if (use_graph) {
             for (int k = 0; k < remaining; ++k) CK(cudaGraphLaunch(c->graph_exec, c->stream));
@@ -652,25 +691,29 @@ int mlh_step(mlh_ctx *c, int nsteps, double dt_max, mlh_step_stats *stats) {
         }
         CK(cudaEventRecord(c->ev1, c->stream));
         CK(cudaGetLastError());
+        // counters, dt and time of the first simulation, and the last step's
+        // face count, waited for once
+        const size_t sb = step_scalars_bytes((size_t)c->nmembers, 1);
+        CK(cudaMemcpyAsync(c->hscal, c->scal, sb, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpyAsync(c->hscal + sb, c->faceOff + c->n, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         float ms = 0.f;
         cudaEventElapsedTime(&ms, c->ev0, c->ev1);
         dev_ms += ms;
         if (c->timing) collect_timers(c);
         unsigned st = 0;
-        int done = 0;
+        int done = 0, ftot = 0;
         unsigned long long nsum[3] = {0, 0, 0};
-        CK(cudaMemcpy(&st, c->status, sizeof(unsigned), cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(&done, c->stepsDone, sizeof(int), cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(nsum, c->newtonSum, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
+        std::memcpy(nsum, c->hscal, sizeof(nsum));
+        std::memcpy(&st, c->hscal + sizeof(nsum), sizeof(st));
+        std::memcpy(&done, c->hscal + sizeof(nsum) + sizeof(st), sizeof(done));
+        std::memcpy(&ftot, c->hscal + sb, sizeof(ftot));   // of the last step
+        have_scalars = true;
         newton += nsum[0];
         fallbacks += nsum[1];
         deferred += nsum[2];
         done_total += done;
         remaining -= done;
-        // per-step interaction counts of the last step
-        int ftot = 0;
-        CK(cudaMemcpy(&ftot, c->faceOff + c->n, sizeof(int), cudaMemcpyDeviceToHost));
         faces += (long long)ftot * done;
         pairs += 2ll * ftot * done;
         if (st & (MLH_ERR_NGB_OVERFLOW | ST_CAPACITY)) {
@@ -686,8 +729,13 @@ int mlh_step(mlh_ctx *c, int nsteps, double dt_max, mlh_step_stats *stats) {
     if (stats) {
         stats->steps = done_total;
         stats->status = accumulated;
-        cudaMemcpy(&stats->dt, c->dt, sizeof(double), cudaMemcpyDeviceToHost);
-        cudaMemcpy(&stats->time, c->simTime, sizeof(double), cudaMemcpyDeviceToHost);
+        if (have_scalars) {
+            std::memcpy(&stats->dt, c->hscal + STEP_COUNTERS, sizeof(double));
+            std::memcpy(&stats->time, c->hscal + STEP_COUNTERS + sizeof(double) * (size_t)c->nmembers, sizeof(double));
+        } else {
+            cudaMemcpy(&stats->dt, c->dt, sizeof(double), cudaMemcpyDeviceToHost);
+            cudaMemcpy(&stats->time, c->simTime, sizeof(double), cudaMemcpyDeviceToHost);
+        }
         stats->pair_interactions = pairs;
         stats->faces = faces;
         stats->newton_iterations = (long long)newton;
@@ -1053,15 +1101,14 @@ int mlh_riemann_fluxes(int dim, int n, const double *Wi, const double *Wj, const
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { g_last_error = "no CUDA device"; return MLH_ERR_NO_DEVICE; }
     const size_t NV = (size_t)dim + 2, nn = (size_t)n;
-    double *d = nullptr;
-    int *dit = nullptr;
-    unsigned *dst = nullptr;
+    // one allocation: cudaMalloc and cudaFree cost as much as the kernel
     const size_t doubles = nn * (3 * NV + 2 * dim);
-    CK(cudaMalloc(&d, sizeof(double) * doubles));
-    auto cleanup = [&]() { cudaFree(d); cudaFree(dit); cudaFree(dst); };
+    double *d = nullptr;
+    CK(cudaMalloc(&d, sizeof(double) * doubles + sizeof(int) * nn + sizeof(unsigned)));
     double *dWi = d, *dWj = d + nn * NV, *dv = d + 2 * nn * NV, *dA = dv + nn * dim, *dF = dA + nn * dim;
-    cudaError_t e = cudaMalloc(&dit, sizeof(int) * nn);
-    if (e == cudaSuccess) e = cudaMalloc(&dst, sizeof(unsigned));
+    int *dit = (int *)(d + doubles);
+    unsigned *dst = (unsigned *)(dit + nn);
+    cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = cudaMemset(dst, 0, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemcpy(dWi, Wi, sizeof(double) * nn * NV, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(dWj, Wj, sizeof(double) * nn * NV, cudaMemcpyHostToDevice);
@@ -1075,7 +1122,7 @@ int mlh_riemann_fluxes(int dim, int n, const double *Wi, const double *Wj, const
     if (e == cudaSuccess) e = cudaMemcpy(F, dF, sizeof(double) * nn * NV, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && iters) e = cudaMemcpy(iters, dit, sizeof(int) * nn, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(&st, dst, sizeof(unsigned), cudaMemcpyDeviceToHost);
-    cleanup();
+    cudaFree(d);
     if (e != cudaSuccess) return cuda_fail(e, "mlh_riemann_fluxes");
     return (int)st;
 }

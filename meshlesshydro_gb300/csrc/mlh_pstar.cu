@@ -352,7 +352,10 @@ struct DevBuf {
     ~DevBuf() { if (p) cudaFree(p); }
     cudaError_t alloc(size_t bytes) { return cudaMalloc(&p, bytes ? bytes : 16); }
     template <class T> T *as() const { return (T *)p; }
+    template <class T> T *at(size_t offset) const { return (T *)((char *)p + offset); }
 };
+
+size_t pad256(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
 
 int fail(cudaError_t e, const char *what) {
     std::string m = std::string(what) + ": " + cudaGetErrorString(e);
@@ -379,40 +382,43 @@ using namespace mlh;
 
 extern "C" int mlh_pstar_infer(const float *weights, const float *x, int n, float *y) {
     if (!weights || !x || !y || n < 1) return MLH_ERR_INVALID;
-    DevBuf w, pk, dx, dy;
-    PCK(w.alloc(sizeof(float) * PSTAR_PARAMS));
-    PCK(pk.alloc(pstar_packed_bytes()));
-    PCK(dx.alloc(sizeof(float) * 4 * (size_t)n));
-    PCK(dy.alloc(sizeof(float) * (size_t)n));
-    PCK(cudaMemcpy(w.p, weights, sizeof(float) * PSTAR_PARAMS, cudaMemcpyHostToDevice));
-    PCK(cudaMemcpy(dx.p, x, sizeof(float) * 4 * (size_t)n, cudaMemcpyHostToDevice));
-    pstar_pack(w.as<float>(), pk.p, 0);
-    pstar_infer(dx.as<float4>(), n, pk.p, dy.as<float>(), sm_count(), 0);
+    // one allocation, cut in 256-byte steps
+    const size_t bw = pad256(sizeof(float) * PSTAR_PARAMS), bp = pad256(pstar_packed_bytes());
+    const size_t bx = pad256(sizeof(float) * 4 * (size_t)n);
+    DevBuf all;
+    PCK(all.alloc(bw + bp + bx + sizeof(float) * (size_t)n));
+    float *w = all.at<float>(0), *dx = all.at<float>(bw + bp), *dy = all.at<float>(bw + bp + bx);
+    void *pk = all.at<char>(bw);
+    PCK(cudaMemcpy(w, weights, sizeof(float) * PSTAR_PARAMS, cudaMemcpyHostToDevice));
+    PCK(cudaMemcpy(dx, x, sizeof(float) * 4 * (size_t)n, cudaMemcpyHostToDevice));
+    pstar_pack(w, pk, 0);
+    pstar_infer((const float4 *)dx, n, pk, dy, sm_count(), 0);
     PCK(cudaGetLastError());
-    PCK(cudaMemcpy(y, dy.p, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost));
+    PCK(cudaMemcpy(y, dy, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost));
     return 0;
 }
 
 extern "C" int mlh_pstar_grad(const float *weights, const float *x, const float *t, int n, float *loss, float *grad) {
     if (!weights || !x || !t || !loss || !grad || n < 1) return MLH_ERR_INVALID;
     const int blocks = (n + 127) / 128;
-    DevBuf w, pk, dx, dt, part, g, l;
-    PCK(w.alloc(sizeof(float) * PSTAR_PARAMS));
-    PCK(pk.alloc(pstar_packed_bytes()));
-    PCK(dx.alloc(sizeof(float) * 4 * (size_t)n));
-    PCK(dt.alloc(sizeof(float) * (size_t)n));
-    PCK(part.alloc(sizeof(float) * (size_t)pstar_partial_floats() * blocks));
-    PCK(g.alloc(sizeof(float) * PSTAR_PARAMS));
-    PCK(l.alloc(sizeof(float)));
-    PCK(cudaMemcpy(w.p, weights, sizeof(float) * PSTAR_PARAMS, cudaMemcpyHostToDevice));
-    PCK(cudaMemcpy(dx.p, x, sizeof(float) * 4 * (size_t)n, cudaMemcpyHostToDevice));
-    PCK(cudaMemcpy(dt.p, t, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice));
-    pstar_pack(w.as<float>(), pk.p, 0);
-    pstar_train_batch(dx.as<float4>(), dt.as<float>(), nullptr, n, pk.p, part.as<float>(), g.as<float>(),
-                      l.as<float>(), 0);
+    // one allocation, cut in 256-byte steps
+    const size_t bw = pad256(sizeof(float) * PSTAR_PARAMS), bp = pad256(pstar_packed_bytes());
+    const size_t bx = pad256(sizeof(float) * 4 * (size_t)n), bt = pad256(sizeof(float) * (size_t)n);
+    const size_t bl = pad256(sizeof(float));
+    DevBuf all;
+    PCK(all.alloc(2 * bw + bp + bx + bt + bl + sizeof(float) * (size_t)pstar_partial_floats() * blocks));
+    float *w = all.at<float>(0), *g = all.at<float>(bw), *l = all.at<float>(2 * bw + bp);
+    void *pk = all.at<char>(2 * bw);
+    float *dx = all.at<float>(2 * bw + bp + bl), *dt = dx + bx / sizeof(float);
+    float *part = dt + bt / sizeof(float);
+    PCK(cudaMemcpy(w, weights, sizeof(float) * PSTAR_PARAMS, cudaMemcpyHostToDevice));
+    PCK(cudaMemcpy(dx, x, sizeof(float) * 4 * (size_t)n, cudaMemcpyHostToDevice));
+    PCK(cudaMemcpy(dt, t, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice));
+    pstar_pack(w, pk, 0);
+    pstar_train_batch((const float4 *)dx, dt, nullptr, n, pk, part, g, l, 0);
     PCK(cudaGetLastError());
-    PCK(cudaMemcpy(grad, g.p, sizeof(float) * PSTAR_PARAMS, cudaMemcpyDeviceToHost));
-    PCK(cudaMemcpy(loss, l.p, sizeof(float), cudaMemcpyDeviceToHost));
+    PCK(cudaMemcpy(grad, g, sizeof(float) * PSTAR_PARAMS, cudaMemcpyDeviceToHost));
+    PCK(cudaMemcpy(loss, l, sizeof(float), cudaMemcpyDeviceToHost));
     return 0;
 }
 
