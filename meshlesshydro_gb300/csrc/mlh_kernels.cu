@@ -1750,7 +1750,8 @@ __device__ __forceinline__ double field_of(const Prim &q, int f) {
 // 6.82 at 128 registers (a spill that 16 warps do not make up for), 7.21 at 200;
 // 64 KH members: 1.23 / 1.19 / 1.30 ms at 128 / 144 / 168.  The products of the offsets
 // on the integer pipe (xmul) made it slower, 7.34 ms: the chain per neighbour
-// gets longer.  Blocks of up to 256 threads.
+// gets longer.  Blocks of up to 256 threads.  L lanes share a particle: each takes
+// every L-th neighbour, sums and extrema are reduced across them (grad_lanes).
 #ifndef MLH_GRAD_MAXREG
 #define MLH_GRAD_MAXREG 168
 #endif
@@ -1758,7 +1759,14 @@ __device__ __forceinline__ double field_of(const Prim &q, int f) {
 #define MLH_GRAD_MAXREG_2D 144
 #endif
 #define MLH_GRAD_BOUNDS __maxnreg__(D == 3 ? MLH_GRAD_MAXREG : MLH_GRAD_MAXREG_2D)
-template <int D>
+// Reduction over the L lanes of a particle (the same bits on each of them).
+template <int L, class T, class F>
+__device__ __forceinline__ T lanes_reduce(unsigned mask, T v, F f) {
+#pragma unroll
+    for (int o = 1; o < L; o *= 2) v = f(v, __shfl_xor_sync(mask, v, o));
+    return v;
+}
+template <int D, int L>
 __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__ members,
                                                    const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
                                                    const Prim *__restrict__ prim, Geo *__restrict__ geo,
@@ -1773,11 +1781,12 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                                                    const float4 *__restrict__ velf, float *__restrict__ dtlo,
                                                    unsigned *__restrict__ dtcap) {
     constexpr int NF = D + 2;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, sub = lane & (L - 1);
+    const unsigned mates = L == 32 ? 0xffffffffu : ((1u << L) - 1u) << (lane - sub);   // the particle's lanes
     if (step_aborted(status)) return;   // no valid lists
     // warp-uniform loop: every lane takes part in the time-step reduction
-    for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; i0 < p.n; i0 += gridDim.x * blockDim.x) {
-      const int i = i0 + lane;
+    for (int i0 = ((blockIdx.x * blockDim.x + threadIdx.x) & ~31) / L; i0 < p.n; i0 += gridDim.x * blockDim.x / L) {
+      const int i = i0 + lane / L;
       int mi = -1;
       double dti = DBL_MAX_;
       float dthi = FLT_INF_;   // with dtlo: upper bound on the particle's dt
@@ -1785,7 +1794,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
         // with faceOff, the particle's face links first (link_particle):
         // integer searches whose load latency the other warps' FP64 work
         // hides, and whose registers are free again before the passes below
-        if (faceOff) link_particle(i, p, nbr, noi, noiImg, faceOff, faceOf, faces, status);
+        if (faceOff && sub == 0) link_particle(i, p, nbr, noi, noiImg, faceOff, faceOf, faces, status);
         mi = memberOf ? memberOf[i] : 0;
         const double hq = p.adaptive_h ? p.hp[i] : members[mi].h;   // quadrature-point radius
         const Prim pi = prim[i];
@@ -1820,17 +1829,17 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
 #pragma unroll
         for (int f = 0; f < NF; ++f) { mxN[f] = kmin; mnN[f] = kmax; }
         // the next neighbour's record is on its way while this one is summed
-        uint32_t en = tot > 0 ? nbr[base] : 0u, en2 = tot > 1 ? nbr[base + 1] : 0u;
+        uint32_t en = sub < tot ? nbr[base + sub] : 0u, en2 = sub + L < tot ? nbr[base + sub + L] : 0u;
         Prim pn = prim[en & IDX_MASK];
         float4 vn = want_dtf ? velf[en & IDX_MASK] : vif;
-        for (int s = 0; s < tot; ++s) {
+        for (int s = sub; s < tot; s += L) {
             const uint32_t e = en;
             const Prim pj = pn;
             const float4 vj = vn;
             en = en2;
             pn = prim[en & IDX_MASK];
             if (want_dtf) vn = velf[en & IDX_MASK];
-            en2 = s + 2 < tot ? nbr[base + s + 2] : 0u;
+            en2 = s + 2 * L < tot ? nbr[base + s + 2 * L] : 0u;
             const double wij = ww[base + s];
             const double *ds = psi + (base + s) * 3;
             double d[3], dp[3];
@@ -1879,6 +1888,30 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 vhi = fmaxf(vhi, vs + B);
             }
         }
+        const auto addD = [](double a, double b) { return addr(a, b); };
+        const auto maxF = [](float a, float b) { return fmaxf(a, b); };
+        const auto minF = [](float a, float b) { return fminf(a, b); };
+        const auto maxK = [](long long a, long long b) { return a < b ? b : a; };
+        const auto minK = [](long long a, long long b) { return b < a ? b : a; };
+        if (L > 1) {   // the lanes' sums, extrema and bounds
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+#pragma unroll
+                for (int b = a; b < D; ++b) E[D * a + b] = lanes_reduce<L>(mates, E[D * a + b], addD);
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+#pragma unroll
+                for (int a = 0; a < D; ++a) gr[f][a] = lanes_reduce<L>(mates, gr[f][a], addD);
+                mxN[f] = lanes_reduce<L>(mates, mxN[f], maxK);
+                mnN[f] = lanes_reduce<L>(mates, mnN[f], minK);
+            }
+            if (want_dt) vSig = lanes_reduce<L>(mates, vSig, [](double a, double b) { return dlt(a, b) ? b : a; });
+            if (want_dtf) {
+                vlo = lanes_reduce<L>(mates, vlo, maxF);
+                vhi = lanes_reduce<L>(mates, vhi, maxF);
+                dt_exact = (__ballot_sync(mates, dt_exact) & mates) != 0u;
+            }
+        }
         if (want_dt) dti = (p.adaptive_h ? p.cfl * p.hp[i] : members[mi].cfl_h) / vSig;
         if (want_dtf) {
             // dt = cfl_h / v_sig bounded below by the largest v_sig and above by
@@ -1892,7 +1925,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
             if (!(lo < 1e38f)) lo = 0.f;   // below any cap
             if (!dt_exact && nr > 0 && vlo > 0.f)
                 dthi = __fmul_ru(__fdiv_ru(ch, vlo), 1.f + 4.f * EPS32);
-            dtlo[i] = dt_exact ? 0.f : lo;
+            if (sub == 0) dtlo[i] = dt_exact ? 0.f : lo;
             if (dt_exact) dthi = FLT_INF_;
         }
         invert_symmetric<D>(E);
@@ -1909,7 +1942,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 gr[f][a] = t;
             }
         }
-        if (gradRaw) {
+        if (gradRaw && sub == 0) {
             Grad graw;
             for (int k = 0; k < 16; ++k) graw.g[k] = 0.;
             for (int k = 0; k < 8; ++k) graw.t[k] = 0.;
@@ -1926,7 +1959,8 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
         {
             const double omega_i = geo[i].omega, V_i = geo[i].V;
 #pragma unroll
-            for (int k = 0; k < D * D; ++k) geo[i].B[k] = mulr(E[k], omega_i);
+            for (int k = 0; k < D * D; ++k)
+                if (sub == 0) geo[i].B[k] = mulr(E[k], omega_i);
 #pragma unroll
             for (int a = 0; a < D; ++a)
 #pragma unroll
@@ -1983,7 +2017,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 }
             };
             if (!(fp32_filters & MLH_FILTER_SLOPE)) {
-                for (int s = 0; s < tot; ++s) {
+                for (int s = sub; s < tot; s += L) {
                     const double *ds = psi + (base + s) * 3;
                     const double d[3] = {ds[0], ds[1], D == 3 ? ds[2] : 0.};
                     exact_slot(d);
@@ -2021,7 +2055,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 float hiQ[NF], loQ[NF], dmax = 0.f;
 #pragma unroll
                 for (int f = 0; f < NF; ++f) { hiQ[f] = -FLT_MAX_; loQ[f] = FLT_MAX_; }
-                for (int s = 0; s < tot; ++s) {
+                for (int s = sub; s < tot; s += L) {
                     float df[3];
                     double d[3];
                     offset_f(s, df, d);
@@ -2032,6 +2066,14 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                         const float q = incr(f, df);
                         hiQ[f] = fmaxf(hiQ[f], q);
                         loQ[f] = fminf(loQ[f], q);
+                    }
+                }
+                if (L > 1) {
+                    dmax = lanes_reduce<L>(mates, dmax, maxF);
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        hiQ[f] = lanes_reduce<L>(mates, hiQ[f], maxF);
+                        loQ[f] = lanes_reduce<L>(mates, loQ[f], minF);
                     }
                 }
                 // B_f = 16 eps32 S (dmax + 1e-30) + 12 u64 (|f_i| + S dmax) with S = sum
@@ -2065,7 +2107,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 // (taken where they stand, some lane of the warp would want nearly
                 // every slot); slots from the 65th on are all candidates
                 unsigned long long cand = 0ull;
-                for (int s = 0; s < tot; ++s) {
+                for (int s = sub; s < tot; s += L) {
                     float df[3];
                     double d[3];
                     offset_f(s, df, d);
@@ -2099,6 +2141,13 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                         if (flat[f]) mxM[f] = mnM[f] = ord_key(fi[f]);
                 }
             }
+            if (L > 1) {
+#pragma unroll
+                for (int f = 0; f < NF; ++f) {
+                    mxM[f] = lanes_reduce<L>(mates, mxM[f], maxK);
+                    mnM[f] = lanes_reduce<L>(mates, mnM[f], minK);
+                }
+            }
             if (p.foqp) {
 #pragma unroll
                 for (int f = 0; f < NF; ++f)
@@ -2126,7 +2175,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
             }
         }
         else {
-            for (int s = 0; s < tot; ++s) {
+            for (int s = sub; s < tot; s += L) {
                 const double *ds = psi + (base + s) * 3;
                 const double d[3] = {ds[0], ds[1], D == 3 ? ds[2] : 0.};
                 store_psi(s, d);
@@ -2151,7 +2200,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
 #pragma unroll
             for (int f = 0; f < 8; ++f) go.t[f] = f < D + 2 ? src[f < 5 ? f : 0] : 0.;
         }
-        grad[i] = go;
+        if (sub == 0) grad[i] = go;
       }   // i < p.n
       if (dtlo) {
         // the least upper bound on dt of each simulation (positive floats
@@ -2181,6 +2230,20 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
         }
       }
     }
+}
+
+// Lanes per particle of k_gradients: more where the particles leave the SMs
+// short of warps and the passes wait on their loads, one once a lane each
+// fills them (the FP64 pipe then bounds them and the reductions only add to
+// it).  The lines lie at 5, 9 and 10 warps per SM with 8, 4 and 2 lanes.  Time
+// in us with 1 / 2 / 4 / 8 lanes (with the time step's kernel): KH 24^2 57 / 43 /
+// 35 / 31, 50^2 56 / 43 / 35 / 33, 71^2 56 / 41 / 35 / 41, 100^2 60 / 46 / 44 / 69,
+// 145^2 70 / 59 / 80 / 111, 180^2 77 / 75 / 105 / 157; Sedov 13^3 106 / 72 / 53 / 42,
+// 17^3 106 / 70 / 56 / 64, 21^3 107 / 74 / 66 / 104, 25^3 114 / 97 / 121 / 155, 31^3
+// 158 / 175 / 191 / 257.
+int grad_lanes(int n, int sm_count) {
+    const long long one = 32ll * sm_count;   // a warp per SM
+    return 8ll * n <= 5 * one ? 8 : 4ll * n <= 9 * one ? 4 : 2ll * n <= 10 * one ? 2 : 1;
 }
 
 // ------------------------------------------------------------------ gather + update
@@ -2471,7 +2534,6 @@ void launch_step(StepArgs &a) {
     // the time step runs inside the gradients' first neighbour pass
     // (k_gradients with dtbits; k_timestep, the separate kernel of the same
     // arithmetic, is the fallback when the time step is timed on its own)
-    const int gT = a.tune.grad_threads;
     // with the single-precision filters the gradients kernel bounds every
     // particle's dt (dtlo, and the least upper bound per simulation in dtcap) and k_timestep evaluates v_sig in FP64
     // for the particles whose bound reaches it
@@ -2489,12 +2551,20 @@ void launch_step(StepArgs &a) {
         exclusive_scan(a.faceCnt, p.n, a.faceOff, a.scanTiles, a.scanTotal, s);
         cudaMemsetAsync(a.faces, 0xff, sizeof(FaceRef) * a.faces_cap, s);
     }
-    k_gradients<D><<<(p.n + gT - 1) / gT, gT, 0, s>>>(p, a.members, a.memberOf, a.grids, a.prim, a.geo, a.nbr, a.ww,
-                                                      a.noi, a.noiImg, a.grad, a.gradRaw, a.psi,
-                                                      (p.adaptive && !a.separate_dt && !dt_filter) ? a.dtbits : nullptr,
-                                                      fused ? a.faceOff : nullptr, a.faceOf, a.faces, a.status,
-                                                      a.tune.fp32_filters, a.velf, dt_filter ? a.dtlo : nullptr,
-                                                      a.dtcap);
+    const int gl = grad_lanes(p.n, a.sm_count);
+    const int gT = gl > 1 && a.tune.grad_threads > 64 ? 64 : a.tune.grad_threads;   // few blocks: small ones spread evenly (KH 100^2: 49 -> 44 us)
+    const int gB = (int)(((long long)p.n * gl + gT - 1) / gT);
+#define MLH_GRADIENTS(LANES)                                                                                     \
+    k_gradients<D, LANES><<<gB, gT, 0, s>>>(p, a.members, a.memberOf, a.grids, a.prim, a.geo, a.nbr, a.ww,       \
+                                            a.noi, a.noiImg, a.grad, a.gradRaw, a.psi,                           \
+                                            (p.adaptive && !a.separate_dt && !dt_filter) ? a.dtbits : nullptr,   \
+                                            fused ? a.faceOff : nullptr, a.faceOf, a.faces, a.status,            \
+                                            a.tune.fp32_filters, a.velf, dt_filter ? a.dtlo : nullptr, a.dtcap)
+    if (gl == 8) MLH_GRADIENTS(8);
+    else if (gl == 4) MLH_GRADIENTS(4);
+    else if (gl == 2) MLH_GRADIENTS(2);
+    else MLH_GRADIENTS(1);
+#undef MLH_GRADIENTS
     if (dt_filter)
         k_timestep<D><<<(p.n + 255) / 256, 256, 0, s>>>(p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.noi,
                                                         a.dtbits, a.dtlo, a.dtcap, a.nmembers, a.dt_max, a.dt,
