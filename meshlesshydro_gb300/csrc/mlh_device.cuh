@@ -259,6 +259,14 @@ __device__ __forceinline__ double fma_dotD(const double *a, const double *b, dou
     return r;
 }
 
+// First statement of the kernels that launch_dep starts before their predecessor
+// on the stream has ended (programmatic dependent launch): wait for all of its
+// writes, then let the next kernel's blocks come up.  No effect in a kernel
+// launched in the ordinary way.
+__device__ __forceinline__ void step_begin() {
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // True when the binning of this step is not valid: a bounded wait gave up
 // (ST_TIMEOUT), a particle fell outside the grid (ST_GRID: outside the box,
 // a NaN coordinate, or fewer than 3 cells on a periodic axis) or the cells

@@ -72,6 +72,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *smem, int &total
 }
 
 __global__ void k_scan_reduce(const int *__restrict__ in, int n, int *__restrict__ tile_sums) {
+    step_begin();
     __shared__ int smem[32];
     long long base = (long long)blockIdx.x * SCAN_TILE;
     int s = 0;
@@ -90,6 +91,7 @@ __global__ void k_scan_reduce(const int *__restrict__ in, int n, int *__restrict
 }
 
 __global__ void k_scan_tiles(int *__restrict__ tile_sums, int ntiles, int *__restrict__ total_out) {
+    step_begin();
     __shared__ int smem[32];
     int carry = 0;
     for (int b = 0; b < ntiles; b += SCAN_T) {
@@ -105,6 +107,7 @@ __global__ void k_scan_tiles(int *__restrict__ tile_sums, int ntiles, int *__res
 
 __global__ void k_scan_apply(const int *__restrict__ in, int n, const int *__restrict__ tile_offsets,
                              int *__restrict__ out, const int *__restrict__ total, int write_total_at_n) {
+    step_begin();
     __shared__ int smem[32];
     long long base = (long long)blockIdx.x * SCAN_TILE;
     long long idx0 = base + (long long)threadIdx.x * SCAN_I;
@@ -131,6 +134,7 @@ __global__ void k_scan_apply(const int *__restrict__ in, int n, const int *__res
 // dependent launches take about 9 us whatever they do, a tile here about 1.5 us.
 __global__ void __launch_bounds__(SCAN_T) k_scan_one(const int *__restrict__ in, int n, int *__restrict__ out,
                                                      int *__restrict__ total) {
+    step_begin();
     __shared__ int smem[32];
     int carry = 0;
     for (int b = 0; b < n; b += SCAN_TILE) {
@@ -152,16 +156,41 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_one(const int *__restrict__ in,
     if (threadIdx.x == 0) { out[n] = carry; *total = carry; }
 }
 
-void exclusive_scan(const int *in, int n, int *out, int *tile_buf, int *total, cudaStream_t s) {
+// A kernel whose first statement is step_begin, launched so that its blocks come
+// up while its predecessor on the stream still runs: a step of few particles is
+// eleven kernels of a few microseconds each, and the gaps between them count.
+template <class... P, class... A>
+void launch_dep(void (*kernel)(P...), int blocks, int threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
+template <class... P, class... A>
+void launch_kernel(bool dep, void (*kernel)(P...), int blocks, int threads, size_t smem, cudaStream_t s, A... args) {
+    if (dep) launch_dep(kernel, blocks, threads, smem, s, args...);
+    else kernel<<<blocks, threads, smem, s>>>((P)args...);
+}
+
+// after_kernel: the operation before it on the stream is a kernel (not an event's wait)
+void exclusive_scan(const int *in, int n, int *out, int *tile_buf, int *total, cudaStream_t s, bool after_kernel) {
     if (n <= 4 * SCAN_TILE) {
-        k_scan_one<<<1, SCAN_T, 0, s>>>(in, n, out, total);
+        launch_kernel(after_kernel, k_scan_one, 1, SCAN_T, 0, s, in, n, out, total);
         return;
     }
     int ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (ntiles < 1) ntiles = 1;
-    k_scan_reduce<<<ntiles, SCAN_T, 0, s>>>(in, n, tile_buf);
-    k_scan_tiles<<<1, SCAN_T, 0, s>>>(tile_buf, ntiles, total);
-    k_scan_apply<<<ntiles, SCAN_T, 0, s>>>(in, n, tile_buf, out, total, 1);
+    launch_kernel(after_kernel, k_scan_reduce, ntiles, SCAN_T, 0, s, in, n, tile_buf);
+    launch_dep(k_scan_tiles, 1, SCAN_T, 0, s, tile_buf, ntiles, total);
+    launch_dep(k_scan_apply, ntiles, SCAN_T, 0, s, in, n, tile_buf, out, total, 1);
 }
 
 // ------------------------------------------------------------------ bounds + grid
@@ -224,6 +253,7 @@ __global__ void k_bounds_partial(const double *__restrict__ x, const double *__r
                                  const double *__restrict__ z, Params p, const Member *__restrict__ members,
                                  int bpm, double *__restrict__ part, int *__restrict__ cellCount,
                                  int *__restrict__ cellFill) {
+    step_begin();
     // with the cell counters (a step's binning): cleared here
     if (cellCount)
         for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= p.ncells_cap; k += gridDim.x * blockDim.x) {
@@ -368,6 +398,7 @@ __global__ void k_bounds_final(const double *__restrict__ x, const double *__res
                                const Member *__restrict__ members, int nmembers, GridInfo *__restrict__ grids,
                                int *__restrict__ cellTotal, unsigned *__restrict__ status,
                                unsigned long long *__restrict__ dtbits, unsigned *__restrict__ dtcap) {
+    step_begin();
     bounds_final_block<D>(x, y, z, part, bpm, p, members, nmembers, grids, cellTotal, status, dtbits, dtcap);
 }
 
@@ -403,6 +434,7 @@ template <int D>
 __global__ void k_assign(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
                          int n, const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
                          int *__restrict__ cell, int *__restrict__ cellCount, unsigned *__restrict__ status) {
+    step_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         assign_one<D>(i, x, y, z, memberOf, grids, cell, cellCount, status);
 }
@@ -410,6 +442,7 @@ __global__ void k_assign(const double *__restrict__ x, const double *__restrict_
 __global__ void k_fill_cells(const int *__restrict__ cell, int n, const int *__restrict__ cellStart,
                              int *__restrict__ cellFill, int *__restrict__ cellList,
                              const unsigned *__restrict__ status) {
+    step_begin();
     if (step_aborted(status)) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int c = cell[i];
@@ -456,6 +489,7 @@ __device__ __forceinline__ void sort_cell_warp(int c, const int *__restrict__ ce
 __global__ void __launch_bounds__(256) k_sort_cells(const int *__restrict__ cellTotal,
                                                     const int *__restrict__ cellStart, int *__restrict__ cellList,
                                                     const unsigned *__restrict__ status) {
+    step_begin();
     if (step_aborted(status)) return;
     const int nc = *cellTotal;
     for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nc; c += (gridDim.x * blockDim.x) >> 5)
@@ -769,6 +803,7 @@ __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
     const int *__restrict__ cellList, uint32_t *__restrict__ nbr, double *__restrict__ dd,
     double *__restrict__ ww, int *__restrict__ noi, int *__restrict__ noiImg, int *__restrict__ faceCnt,
     Prim *__restrict__ prim, Geo *__restrict__ geo, float4 *__restrict__ velf, unsigned *__restrict__ status) {
+    step_begin();
     constexpr unsigned ALL = 0xffffffffu;
     const int K = p.K;
     const int CAP = K + 32;
@@ -1420,6 +1455,7 @@ __global__ void __launch_bounds__(256) k_timestep(Params p, const Member *__rest
                                                   int nmembers, double dt_max, double *__restrict__ dt_out,
                                                   unsigned *__restrict__ arrived,
                                                   const unsigned *__restrict__ status) {
+    step_begin();
     const int lane = threadIdx.x & 31;
     // no valid lists after an aborted binning
     const int n = step_aborted(status) ? 0 : p.n;
@@ -1496,6 +1532,7 @@ __global__ void __launch_bounds__(256) k_timestep(Params p, const Member *__rest
 // dt of every simulation when no k_timestep follows the minima
 __global__ void k_dt_final(Params p, int nmembers, const unsigned long long *__restrict__ dtbits, double dt_max,
                            double *__restrict__ dt_out, const unsigned *__restrict__ status) {
+    step_begin();
     if (!step_aborted(status)) dt_final(p, nmembers, dtbits, dt_max, dt_out);
 }
 
@@ -1611,6 +1648,7 @@ __global__ void __launch_bounds__(256) k_link_own(Params p, const uint32_t *__re
                                                   const int *__restrict__ noi, const int *__restrict__ noiImg,
                                                   const int *__restrict__ faceOff, int *__restrict__ faceOf,
                                                   FaceRef *__restrict__ faces, unsigned *__restrict__ status) {
+    step_begin();
     if (step_aborted(status)) return;   // no valid lists
     const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
     bool full = false;
@@ -1648,6 +1686,7 @@ __global__ void __launch_bounds__(256) k_link(Params p, const uint32_t *__restri
                                               const int *__restrict__ noiImg, const int *__restrict__ faceTotal,
                                               int *__restrict__ faceOf, FaceRef *__restrict__ faces,
                                               unsigned *__restrict__ status) {
+    step_begin();
     if (step_aborted(status)) return;
     const int nf = *faceTotal < p.faces_cap ? *faceTotal : p.faces_cap;
     bool lost = false;
@@ -1780,6 +1819,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                                                    int fp32_filters,
                                                    const float4 *__restrict__ velf, float *__restrict__ dtlo,
                                                    unsigned *__restrict__ dtcap) {
+    step_begin();
     constexpr int NF = D + 2;
     const int lane = threadIdx.x & 31, sub = lane & (L - 1);
     const unsigned mates = L == 32 ? 0xffffffffu : ((1u << L) - 1u) << (lane - sub);   // the particle's lanes
@@ -2262,6 +2302,7 @@ __global__ void __launch_bounds__(256) k_update(Params p, const int *__restrict_
                                                 double *__restrict__ m, double *__restrict__ u, float4 *__restrict__ posf,
                                                 double *__restrict__ fluxSums, unsigned *__restrict__ status,
                                                 int nmembers, double *__restrict__ simTime, int *__restrict__ stepsDone) {
+    step_begin();
     // (the bits tested are not raised by this kernel: the same for every thread)
     const unsigned st0 = *(volatile const unsigned *)status;
     if (st0 & (ST_NGB_OVERFLOW | ST_CAPACITY | ST_TIMEOUT | ST_GRID)) return;
@@ -2426,16 +2467,15 @@ void launch_binning(StepArgs &a) {
                            a.scanTotal, a.status, a.dtbits, a.dtcap, bar);
         return;
     }
-    k_bounds_partial<D><<<a.nmembers * a.bpm, BOUNDS_T, 0, s>>>(a.x, a.y, a.z, p, a.members, a.bpm, a.boundsPart,
+    launch_dep(k_bounds_partial<D>, a.nmembers * a.bpm, BOUNDS_T, 0, s, a.x, a.y, a.z, p, a.members, a.bpm, a.boundsPart,
                                                                 a.cellCount, a.cellFill);
-    k_bounds_final<D><<<1, BOUNDS_T, 0, s>>>(a.x, a.y, a.z, a.boundsPart, a.bpm, p, a.members, a.nmembers, a.grids,
+    launch_dep(k_bounds_final<D>, 1, BOUNDS_T, 0, s, a.x, a.y, a.z, a.boundsPart, a.bpm, p, a.members, a.nmembers, a.grids,
                                              a.cellTotal, a.status, a.dtbits, a.dtcap);
-    k_assign<D><<<blocksN, T, 0, s>>>(a.x, a.y, a.z, p.n, a.memberOf, a.grids, a.cell, a.cellCount, a.status);
-    exclusive_scan(a.cellCount, p.ncells_cap, a.cellStart, a.scanTiles, a.scanTotal, s);
-    k_fill_cells<<<blocksN, T, 0, s>>>(a.cell, p.n, a.cellStart, a.cellFill, a.cellList, a.status);
+    launch_dep(k_assign<D>, blocksN, T, 0, s, a.x, a.y, a.z, p.n, a.memberOf, a.grids, a.cell, a.cellCount, a.status);
+    exclusive_scan(a.cellCount, p.ncells_cap, a.cellStart, a.scanTiles, a.scanTotal, s, true);
+    launch_dep(k_fill_cells, blocksN, T, 0, s, a.cell, p.n, a.cellStart, a.cellFill, a.cellList, a.status);
     const long long sortBlocks = ((long long)p.ncells_cap + 7) / 8;
-    k_sort_cells<<<(int)(sortBlocks < a.sm_count * 8ll ? sortBlocks : a.sm_count * 8ll), 256, 0, s>>>(
-        a.cellTotal, a.cellStart, a.cellList, a.status);
+    launch_dep(k_sort_cells, (int)(sortBlocks < a.sm_count * 8ll ? sortBlocks : a.sm_count * 8ll), 256, 0, s, a.cellTotal, a.cellStart, a.cellList, a.status);
 }
 
 // Smoothing lengths of every particle on the current grid (k_hsolve).
@@ -2475,6 +2515,13 @@ void launch_step(StepArgs &a) {
         tock(KT_HSOLVE);
     }
 
+    const int gl = grad_lanes(p.n, a.sm_count);
+    // Kernels started before their predecessors have ended (launch_dep): the
+    // binning always; the rest only where particles are few.  In full grids the
+    // early blocks take the SM slots that the links on the second stream fill
+    // (16 blasts in 48^3: 1543 us a step, 1600 with every kernel early, 1536 so).
+    // KH 24^2 113 -> 91 us a step, KH 100^2 165 -> 162, Sedov 33^3 557 -> 542.
+    const bool early = gl > 1;
     tick(KT_NNS);
     {
         const size_t smem = nns_smem_bytes(p.K);
@@ -2495,7 +2542,7 @@ void launch_step(StepArgs &a) {
         const int blocks = (int)(want < most ? want : most < 1 ? 1 : most);
         auto run = [&](auto kern) {
             if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<blocks, NNS_WARPS * 32, smem, s>>>(
+            launch_kernel(early, kern, blocks, NNS_WARPS * 32, smem, s,
                 p, (int)nsplit, (int)pb, a.members, a.memberOf, a.grids, a.x, a.y, a.z, a.posf, a.vx, a.vy, a.vz, a.m,
                 a.u, a.cellTotal, a.cellStart, a.cellList, a.nbr, a.psi, a.ww, a.noi, a.noiImg, a.faceCnt, a.prim,
                 a.geo, a.velf, a.status);
@@ -2541,7 +2588,7 @@ void launch_step(StepArgs &a) {
                            a.dtlo && a.dtcap;
     if (a.separate_dt) {
         tick(KT_DT);
-        k_timestep<D><<<(p.n + 255) / 256, 256, 0, s>>>(p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.noi,
+        launch_dep(k_timestep<D>, (p.n + 255) / 256, 256, 0, s, p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.noi,
                                                         a.dtbits, nullptr, nullptr, a.nmembers, a.dt_max, a.dt,
                                                         a.arrived, a.status);
         tock(KT_DT);
@@ -2551,26 +2598,23 @@ void launch_step(StepArgs &a) {
         exclusive_scan(a.faceCnt, p.n, a.faceOff, a.scanTiles, a.scanTotal, s);
         cudaMemsetAsync(a.faces, 0xff, sizeof(FaceRef) * a.faces_cap, s);
     }
-    const int gl = grad_lanes(p.n, a.sm_count);
     const int gT = gl > 1 && a.tune.grad_threads > 64 ? 64 : a.tune.grad_threads;   // few blocks: small ones spread evenly (KH 100^2: 49 -> 44 us)
     const int gB = (int)(((long long)p.n * gl + gT - 1) / gT);
-#define MLH_GRADIENTS(LANES)                                                                                     \
-    k_gradients<D, LANES><<<gB, gT, 0, s>>>(p, a.members, a.memberOf, a.grids, a.prim, a.geo, a.nbr, a.ww,       \
-                                            a.noi, a.noiImg, a.grad, a.gradRaw, a.psi,                           \
-                                            (p.adaptive && !a.separate_dt && !dt_filter) ? a.dtbits : nullptr,   \
-                                            fused ? a.faceOff : nullptr, a.faceOf, a.faces, a.status,            \
-                                            a.tune.fp32_filters, a.velf, dt_filter ? a.dtlo : nullptr, a.dtcap)
-    if (gl == 8) MLH_GRADIENTS(8);
-    else if (gl == 4) MLH_GRADIENTS(4);
-    else if (gl == 2) MLH_GRADIENTS(2);
-    else MLH_GRADIENTS(1);
-#undef MLH_GRADIENTS
+#define MLH_GRAD_ARGS                                                                                          \
+    a.members, a.memberOf, a.grids, a.prim, a.geo, a.nbr, a.ww, a.noi, a.noiImg, a.grad, a.gradRaw, a.psi,     \
+        (p.adaptive && !a.separate_dt && !dt_filter) ? a.dtbits : nullptr, fused ? a.faceOff : nullptr, a.faceOf, \
+        a.faces, a.status, a.tune.fp32_filters, a.velf, dt_filter ? a.dtlo : nullptr, a.dtcap
+    auto gradients = [&](auto kern) { launch_kernel(early, kern, gB, gT, 0, s, p, MLH_GRAD_ARGS); };
+    if (gl == 8) gradients(k_gradients<D, 8>);
+    else if (gl == 4) gradients(k_gradients<D, 4>);
+    else if (gl == 2) gradients(k_gradients<D, 2>);
+    else gradients(k_gradients<D, 1>);
+#undef MLH_GRAD_ARGS
     if (dt_filter)
-        k_timestep<D><<<(p.n + 255) / 256, 256, 0, s>>>(p, a.members, a.memberOf, a.prim, a.geo, a.nbr, a.noi,
-                                                        a.dtbits, a.dtlo, a.dtcap, a.nmembers, a.dt_max, a.dt,
-                                                        a.arrived, a.status);
+        launch_kernel(early, k_timestep<D>, (p.n + 255) / 256, 256, 0, s, p, a.members, a.memberOf, a.prim, a.geo,
+                      a.nbr, a.noi, a.dtbits, a.dtlo, a.dtcap, a.nmembers, a.dt_max, a.dt, a.arrived, a.status);
     else
-        k_dt_final<<<1, 128, 0, s>>>(p, a.nmembers, a.dtbits, a.dt_max, a.dt, a.status);
+        launch_kernel(early, k_dt_final, 1, 128, 0, s, p, a.nmembers, a.dtbits, a.dt_max, a.dt, a.status);
     tock(KT_GRAD);
     if (a.stop_after_gradients) return;
 
@@ -2589,7 +2633,7 @@ void launch_step(StepArgs &a) {
     tock(KT_FACES);
 
     tick(KT_UPDATE);
-    k_update<D><<<blocksN, T, 0, s>>>(p, a.memberOf, a.grids, a.noi, a.noiImg, a.faceOf, a.Fface, a.dt, a.x, a.y,
+    launch_kernel(early, k_update<D>, blocksN, T, 0, s, p, a.memberOf, a.grids, a.noi, a.noiImg, a.faceOf, a.Fface, a.dt, a.x, a.y,
                                       a.z, a.vx, a.vy, a.vz, a.m, a.u, a.posf, a.fluxSums, a.status, a.nmembers, a.simTime,
                                       a.stepsDone);
     tock(KT_UPDATE);
@@ -2600,12 +2644,12 @@ void launch_grid_bounds(const double *x, const double *y, const double *z, const
                         int *cellTotal, unsigned *status, cudaStream_t s) {
     const int blocks = nmembers * bpm;
     if (p.dim == 2) {
-        k_bounds_partial<2><<<blocks, BOUNDS_T, 0, s>>>(x, y, z, p, members, bpm, partials, nullptr, nullptr);
-        k_bounds_final<2><<<1, BOUNDS_T, 0, s>>>(x, y, z, partials, bpm, p, members, nmembers, grids, cellTotal, status,
+        launch_dep(k_bounds_partial<2>, blocks, BOUNDS_T, 0, s, x, y, z, p, members, bpm, partials, nullptr, nullptr);
+        launch_dep(k_bounds_final<2>, 1, BOUNDS_T, 0, s, x, y, z, partials, bpm, p, members, nmembers, grids, cellTotal, status,
                                                  nullptr, nullptr);
     } else {
-        k_bounds_partial<3><<<blocks, BOUNDS_T, 0, s>>>(x, y, z, p, members, bpm, partials, nullptr, nullptr);
-        k_bounds_final<3><<<1, BOUNDS_T, 0, s>>>(x, y, z, partials, bpm, p, members, nmembers, grids, cellTotal, status,
+        launch_dep(k_bounds_partial<3>, blocks, BOUNDS_T, 0, s, x, y, z, p, members, bpm, partials, nullptr, nullptr);
+        launch_dep(k_bounds_final<3>, 1, BOUNDS_T, 0, s, x, y, z, partials, bpm, p, members, nmembers, grids, cellTotal, status,
                                                  nullptr, nullptr);
     }
 }

@@ -128,7 +128,8 @@ void launch_grid_bounds(const double *x, const double *y, const double *z, const
                         const Member *members, int nmembers, int bpm, double *partials, GridInfo *grids,
                         int *cellTotal, unsigned *status, cudaStream_t s);
 void pack_posf(const double *x, const double *y, const double *z, int n, int dim, float4 *posf, cudaStream_t s);
-void exclusive_scan(const int *in, int n, int *out, int *tile_buf, int *total, cudaStream_t s);
+void exclusive_scan(const int *in, int n, int *out, int *tile_buf, int *total, cudaStream_t s,
+                    bool after_kernel = false);
 const char *kernel_timer_name(int id);
 // Riemann problems of n independent faces (device arrays; see k_riemann_batch)
 void riemann_batch(int dim, int n, double gamma, double rtol, int max_iter, int mfm, const double *Wi,
