@@ -51,47 +51,48 @@ WORKLOADS = {
 }
 METRIC = "particle-updates/s per MFV step on 1 GB300"
 # kernels launched by one plain mlh_step iteration (csrc/mlh_kernels.cu,
-# launch_step): binning (k_bounds_partial, k_bounds_final, k_assign, 3 scan
-# kernels, k_fill_cells, k_sort_cells), k_neighbours, face links (3 scan
-# kernels, k_link), k_timestep, k_dt_final, k_gradients, the face pass
-# (k_faces_block, or k_faces first pass + second Newton pass), k_update,
-# k_advance_time
-LAUNCHES_PER_STEP = 20
+# launch_step): binning (k_bounds_partial, k_bounds_final, k_assign, the scan,
+# k_fill_cells, k_sort_cells), k_neighbours, face links (the scan, k_link_own,
+# k_link), k_gradients, k_timestep, the face pass (k_faces_block or k_faces),
+# k_update; a scan is one kernel up to 16384 entries, three above
+def launches_per_step(n: int) -> int:
+    return 12 + (2 if n <= 16384 else 6)
+
 
 # What each kernel of the step executes per unit (particle, or canonical
 # face for the face pass), from ncu captures of the same kernels: FP64
 # operations (2 x DFMA + DADD + DMUL thread instructions per unit) and DRAM
 # bytes (read + write per unit); 3D on the 64^3 periodic Sedov step (the time
 # step's single-precision bounds inside the gradients' first pass and its FP64
-# v_sig for the few candidate particles in k_timestep, the face pass as its
-# first pass and the second Newton pass over the queue), 2D on the 256-member
-# Kelvin-Helmholtz ensemble (the face pass with the unfinished faces
-# continued inside the block).  These are executed, not
+# v_sig for the few candidate particles in k_timestep), 2D on the 256-member
+# Kelvin-Helmholtz ensemble; the face pass with the unfinished faces continued
+# inside the block.  Reciprocals, square roots, fifth roots and some products
+# run in 64-bit fixed point on the integer pipe and are not in the counts.  These are executed, not
 # algorithmic, operations: a kernel cannot execute more than the FP64 pipe
 # issues, so the rates they give are bounded by the pipe's peak.
 KERNEL_UNITS = {"neighbours_density": "particle", "timestep": "particle", "gradients_limiter": "particle",
                 "face_links": "particle", "faces_riemann": "face", "gather_update": "particle"}
 KERNEL_EXEC = {
-    3: {"neighbours_density": (1026.1, 870.9), "timestep": (0.0, 4.1), "gradients_limiter": (2906.7, 1803.9),
-        "face_links": (0.0, 1007.7), "faces_riemann": (537.7, 300.9), "gather_update": (212.0, 1534.5)},
-    2: {"neighbours_density": (592.7, 887.2), "timestep": (0.0, 8.5), "gradients_limiter": (1126.9, 2074.6),
-        "face_links": (0.0, 876.0), "faces_riemann": (344.3, 180.8), "gather_update": (120.0, 975.6)},
+    3: {"neighbours_density": (1007.2, 1633.5), "timestep": (0.0, 4.1), "gradients_limiter": (3173.3, 2591.1),
+        "face_links": (0.0, 1227.5), "faces_riemann": (371.1, 185.8), "gather_update": (206.0, 1305.9)},
+    2: {"neighbours_density": (510.1, 1871.6), "timestep": (0.0, 8.4), "gradients_limiter": (1210.0, 2471.1),
+        "face_links": (0.0, 1245.2), "faces_riemann": (213.4, 189.4), "gather_update": (114.0, 942.4)},
 }
 # FP64 thread instructions (DFMA + DADD + DMUL) per unit of the same
 # captures: what the FP64 pipe issues, each instruction one lane-slot
 KERNEL_FP64_INSTR = {
-    3: {"neighbours_density": 791.1, "timestep": 0.0, "gradients_limiter": 1845.3, "face_links": 0.0,
-        "faces_riemann": 353.5, "gather_update": 195.0},
-    2: {"neighbours_density": 441.7, "timestep": 0.0, "gradients_limiter": 747.7, "face_links": 0.0,
-        "faces_riemann": 244.4, "gather_update": 107.0},
+    3: {"neighbours_density": 526.2, "timestep": 0.0, "gradients_limiter": 1610.0, "face_links": 0.0,
+        "faces_riemann": 192.3, "gather_update": 192.0},
+    2: {"neighbours_density": 269.1, "timestep": 0.0, "gradients_limiter": 618.8, "face_links": 0.0,
+        "faces_riemann": 112.0, "gather_update": 104.0},
 }
 # FP64 pipe active (sm__pipe_fp64_cycles_active over elapsed cycles) of the
 # same captures
 KERNEL_FP64_PIPE = {
-    3: {"neighbours_density": 0.588, "timestep": 0.546, "gradients_limiter": 0.840, "faces_riemann": 0.878,
-        "gather_update": 0.764, "face_links": 0.0},
-    2: {"neighbours_density": 0.716, "timestep": 0.656, "gradients_limiter": 0.766, "faces_riemann": 0.858,
-        "gather_update": 0.840, "face_links": 0.0},
+    3: {"neighbours_density": 0.687, "timestep": 0.409, "gradients_limiter": 0.854, "faces_riemann": 0.768,
+        "gather_update": 0.761, "face_links": 0.0},
+    2: {"neighbours_density": 0.748, "timestep": 0.500, "gradients_limiter": 0.869, "faces_riemann": 0.680,
+        "gather_update": 0.837, "face_links": 0.0},
 }
 # Operations of the reference's method per unit, counted by the
 # operation-counting build of the oracle (oracle/flops.py; every addition,
@@ -802,7 +803,7 @@ def run_mlh(args):
             "newton_iterations_per_face": st.newton_iterations / max(st.faces, 1),
             "status": runtime.status_names(st.status),
             "wall_s_timed": wall,
-            "gpu_launches": LAUNCHES_PER_STEP * st.steps,
+            "gpu_launches": launches_per_step(n) * st.steps,
             "kernel_ms_per_step": per,
             "kernel_ms_source": "up to 3 further steps with per-kernel CUDA events, which serialise the face-link "
                                 "stream that the timed steps overlap with the time step and gradients",

@@ -287,7 +287,7 @@ __device__ __forceinline__ void pressure_fn_root(const RiemannSide &s, double p,
 // is the same double.  In the weak-wave faces that make up most of a step,
 // p* lies between pL and pR: A is a shock and B a rarefaction in nearly
 // every lane, where the unsorted problem splits each side's branch of
-// pressure_fn5 at random.  (2) The solution is sampled at S = 0 by the
+// pressure_fn_root at random.  (2) The solution is sampled at S = 0 by the
 // left-side logic only: on the left state as given when the contact moves
 // right (u* >= 0), on the mirror image of the right state otherwise.  Every
 // speed of the mirrored sampling is the exact negation of the right-side
