@@ -314,10 +314,10 @@ size_t step_scalars_bytes(size_t nm, size_t times) { return STEP_COUNTERS + size
 // Structure of the plain face pass when neither the caller nor the autotuner
 // chose one: one pass (0) for few particles, where a block has one or two
 // rounds of faces and the in-block regrouping (2) only adds its barriers;
-// in-block above.  Pass times in us at 0 / 2: KH 24^2 20 / 24, KH 100^2 46 / 47,
-// Sedov 33^3 (36k particles) 226 / 236, KH 317^2 (100k) 326 / 324, 16 blasts in
-// 48^3 (110k) 846 / 817, Sedov 64^3 1710 / 1655, 128^3 13990 / 13200, 64 KH
-// members (1.2M) 2844 / 2625.
+// in-block above.  Pass times in us at 0 / 2: KH 24^2 23 / 28, KH 100^2 47 / 43,
+// 180^2 111 / 121, 260^2 (68k) 206 / 214, 317^2 (100k) 326 / 326, 64 KH members (866k)
+// 2844 / 2480; Sedov 17^3 50 / 58, 33^3 (36k) 252 / 255, 40^3 (64k) 429 / 431, 44^3 583 /
+// 553, 128^3 13990 / 12470; 16 blasts in 48^3 (110k) 846 / 756.
 int face_split_rule(size_t n) { return n < (size_t)1 << 16 ? 0 : 2; }
 
 StepArgs make_args(mlh_ctx *c, double dt_max) {

@@ -190,20 +190,25 @@ __device__ __forceinline__ unsigned project_flux(const RiemannResult &rs, const 
 }
 
 // Register caps of the face kernels: with the roots and products on the integer
-// pipe the passes wait on latency at 16 warps per SM.  The in-block pass over the
-// Sedov 128^3 faces at 104 / 96 / 88 / 80 / 72 registers (16 / 20 / 20 / 24 / 28
-// warps): 13.84 / 13.30 / 13.33 / 13.25 / 13.41 ms; over those of 64 KH members at
-// 80 / 72 / 64: 2.65 / 2.63 / 2.74 ms; of 16 blasts in 48^3 (3D) at 96 / 80 / 72:
-// 832 / 817 / 822 us.  The grid is a multiple of the blocks that reside at once
+// pipe the passes wait on latency at 16 warps per SM.  k_faces_block: 80, three
+// blocks of 256 threads (24 warps) per SM.  With 128 threads the pass over the Sedov
+// 128^3 faces at 104 / 96 / 88 / 80 / 72 registers took 13.84 / 13.30 / 13.33 / 13.25 /
+// 13.41 ms, that over those of 64 KH members at 80 / 72 / 64 2.65 / 2.63 / 2.74 ms; with
+// 256 threads 12.47 at 80, 13.63 at 84 (two blocks), 2.52 and 2.47 ms (KH) at 72 and
+// 80.  k_faces in 2D: 72.  The grid is a multiple of the blocks that reside at once
 // (face_blocks): 8 blocks per SM at 96 registers left the second of two rounds
-// 3/5 full, 16.4 ms.  What the pass does per face: 198 FP64 operations, the
-// FP64 pipe 84 % active; the relative velocities in the prediction and v* along
-// A instead of along A / |A| took 13 of 198 (13.64 -> 13.30 ms at 96 registers).
+// 3/5 full, 16.4 ms.  What the pass does per face: 192 FP64 operations among 5400
+// instructions, more than the instruction cache holds (no-instruction stalls a
+// sixth of the time at 128 threads); a block's warps run in step between its
+// barriers and share what is fetched.
 #ifndef MLH_FACE_MAXREG_3D
 #define MLH_FACE_MAXREG_3D 80
 #endif
 #ifndef MLH_FACE_MAXREG_2D
 #define MLH_FACE_MAXREG_2D 72
+#endif
+#ifndef MLH_FACE_MAXREG_BLOCK
+#define MLH_FACE_MAXREG_BLOCK 80
 #endif
 #define MLH_FACE_BOUNDS __maxnreg__(D == 3 ? MLH_FACE_MAXREG_3D : MLH_FACE_MAXREG_2D)
 // The face-frame Riemann problem of canonical face f (i < j): effective face
@@ -519,11 +524,16 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
 // without strong shocks skips) and continues them from p_TR e^y together with
 // the other unfinished faces.  Nothing leaves the block: the plain and the
 // learned step differ only by that branch.
-constexpr int FB_T = 128;   // threads per block of k_faces_block
+// Threads per block of k_faces_block: 128 / 192 / 256: Sedov 128^3 13.2 / 13.1 / 12.5
+// ms, 64 KH members 2.63 / 2.66 / 2.47 ms, 16 blasts in 48^3 817 / 790 / 756 us.  The
+// barriers keep a block's warps in step, so that they share the instructions
+// that are fetched; with fewer of them (one count for a round instead of one per
+// warp, two barriers instead of four) 128 threads took 2.72 ms on the members.
+constexpr int FB_T = 256;
 
 // The network's guesses for the ns strong-shock faces of a round listed in
 // slist (their solver states in sv, s.p = p_TR): warp w takes the faces
-// w*16 .. w*16+15, then the next 64, and so on; s.p becomes p_TR e^y where
+// w*16 .. w*16+15, then the next FB_T / 2, and so on; s.p becomes p_TR e^y where
 // PSTAR_GATE < |y| < 30 (finite), and stays p_TR elsewhere.  Every lane of a
 // warp runs the MMAs (rows beyond ns are zero inputs whose outputs are
 // dropped).  Out of line, so that the rare branch that calls it does not shape
@@ -548,7 +558,7 @@ static __device__ __noinline__ void block_network_guess(const PackedMlp *__restr
 }
 
 template <int D, int ROOT, bool LEARNED>
-__global__ void MLH_FACE_BOUNDS k_faces_block(Params p, RiemannConsts rc, const Member *__restrict__ members,
+__global__ void __maxnreg__(MLH_FACE_MAXREG_BLOCK) k_faces_block(Params p, RiemannConsts rc, const Member *__restrict__ members,
                                               const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
                                               const Prim *__restrict__ prim, const Geo *__restrict__ geo,
                                               const Grad *__restrict__ grad, const uint32_t *__restrict__ nbr,
@@ -697,8 +707,7 @@ __global__ void __launch_bounds__(256) k_riemann_batch(int n, RiemannConsts rc, 
 // Blocks of a face pass: the tuned number per SM, raised to a multiple of the
 // blocks that an SM holds at once (the register cap's threads), and no more
 // than the faces that the table can hold need.
-inline int face_blocks(int dim, int threads, const StepArgs &a) {
-    const int cap = dim == 3 ? MLH_FACE_MAXREG_3D : MLH_FACE_MAXREG_2D;
+inline int face_blocks(int cap, int threads, const StepArgs &a) {
     int resident = 65536 / cap / threads;
     if (resident < 1) resident = 1;
     const int per_sm = (a.tune.face_blocks_per_sm + resident - 1) / resident * resident;
@@ -713,7 +722,8 @@ template <int D, int ROOT>
 void launch_faces(StepArgs &a) {
     const Params &p = a.p;
     cudaStream_t s = a.stream;
-    const int fT = a.tune.face_threads, fB = face_blocks(D, fT, a), fBb = face_blocks(D, FB_T, a);
+    const int fT = a.tune.face_threads, fBb = face_blocks(MLH_FACE_MAXREG_BLOCK, FB_T, a);
+    const int fB = face_blocks(D == 3 ? MLH_FACE_MAXREG_3D : MLH_FACE_MAXREG_2D, fT, a);
     Params pf = p;   // the face passes see the tuned split
     const RiemannConsts rc = make_riemann_consts(p.gamma, p.rtol, p.rmaxit);
     const FaceQueue qa{a.fstate, a.queueFace, a.queueCount, a.qcap};
