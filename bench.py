@@ -74,9 +74,9 @@ KERNEL_UNITS = {"neighbours_density": "particle", "timestep": "particle", "gradi
                 "face_links": "particle", "faces_riemann": "face", "gather_update": "particle"}
 KERNEL_EXEC = {
     3: {"neighbours_density": (1007.2, 1633.5), "timestep": (0.0, 4.1), "gradients_limiter": (3173.3, 2591.1),
-        "face_links": (0.0, 1227.5), "faces_riemann": (371.1, 185.8), "gather_update": (206.0, 1305.9)},
+        "face_links": (0.0, 1227.5), "faces_riemann": (371.1, 155.5), "gather_update": (206.0, 1305.9)},
     2: {"neighbours_density": (510.1, 1871.6), "timestep": (0.0, 8.4), "gradients_limiter": (1210.0, 2471.1),
-        "face_links": (0.0, 1245.2), "faces_riemann": (213.4, 189.4), "gather_update": (114.0, 942.4)},
+        "face_links": (0.0, 1245.2), "faces_riemann": (213.4, 170.4), "gather_update": (114.0, 942.4)},
 }
 # FP64 thread instructions (DFMA + DADD + DMUL) per unit of the same
 # captures: what the FP64 pipe issues, each instruction one lane-slot
@@ -89,9 +89,9 @@ KERNEL_FP64_INSTR = {
 # FP64 pipe active (sm__pipe_fp64_cycles_active over elapsed cycles) of the
 # same captures
 KERNEL_FP64_PIPE = {
-    3: {"neighbours_density": 0.687, "timestep": 0.409, "gradients_limiter": 0.854, "faces_riemann": 0.768,
+    3: {"neighbours_density": 0.687, "timestep": 0.409, "gradients_limiter": 0.854, "faces_riemann": 0.815,
         "gather_update": 0.761, "face_links": 0.0},
-    2: {"neighbours_density": 0.748, "timestep": 0.500, "gradients_limiter": 0.869, "faces_riemann": 0.680,
+    2: {"neighbours_density": 0.748, "timestep": 0.500, "gradients_limiter": 0.869, "faces_riemann": 0.693,
         "gather_update": 0.837, "face_links": 0.0},
 }
 # Operations of the reference's method per unit, counted by the

@@ -1780,7 +1780,7 @@ __device__ __forceinline__ double field_of(const Prim &q, int f) {
 // numeric_limits<double>::min(), the same expressions), on the positions and
 // velocities that pass loads anyway; the per-particle dt goes into the
 // per-member minimum (warp reduction, then one atomicMin on its bit pattern).
-// Bound: the FP64 pipe (79 % active on Sedov 64^3, 1625 instructions per
+// Bound: the FP64 pipe (85 % active on Sedov 64^3, 1610 instructions per
 // particle, 41 per neighbour) and, at 12 warps per SM, the latency of the
 // gathers.  One gather of the neighbours' records instead of three (the sums and
 // the neighbours' extrema), the next one's in flight while one is summed: Sedov
