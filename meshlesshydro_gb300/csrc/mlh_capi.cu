@@ -78,6 +78,7 @@ struct mlh_ctx {
     int n = 0;
     int device = 0;
     int sm_count = 152;
+    int smem_per_block = 0;   // the most shared memory that a block can ask for
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;              // face links, overlapped
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -484,6 +485,7 @@ static int create_impl(const mlh_config *cfg, int nmembers, const mlh_member *md
     c->bpm = nmembers >= BOUNDS_BLOCKS ? 1 : (BOUNDS_BLOCKS + nmembers - 1) / nmembers;
     cudaGetDevice(&c->device);
     cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
+    cudaDeviceGetAttribute(&c->smem_per_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
     fill_params(c);
     // slots per particle: a multiple of 4, so that every particle's list
     // starts on a 16-byte boundary (read as uint4 by k_link)
@@ -584,13 +586,34 @@ static void drop_graph(mlh_ctx *c) {
     c->graph_exec = nullptr;
 }
 
+static int too_many_neighbours(int most) {
+    g_last_error = "more neighbours than the search's shared memory lists (" + std::to_string(most) + " slots per particle)";
+    return MLH_ERR_CAPACITY;
+}
+
+// Before a launch sequence: 0 when every kernel of it can be launched.  A search
+// whose lists do not fit the shared memory fails to launch, and the kernels
+// behind it would read lists that nobody wrote; so would they in a context
+// whose buffers an earlier call failed to allocate.
+static int check_launchable(mlh_ctx *c, bool hsolve) {
+    if (!c->ngbArena || !c->cellArena) {
+        g_last_error = "the context has no buffers: an earlier allocation failed";
+        return MLH_ERR_CAPACITY;
+    }
+    const int most = most_slots((size_t)c->smem_per_block, hsolve);
+    return c->p.K > most ? too_many_neighbours(most) : 0;
+}
+
 // After a launch sequence reported a capacity overflow: 1.5x neighbour slots
-// (MLH_ERR_NGB_OVERFLOW) and/or 2x cells (ST_CAPACITY); the work is repeated
-// by the caller.
-static int grow_buffers(mlh_ctx *c, unsigned st) {
+// (MLH_ERR_NGB_OVERFLOW), at most those the kernels can be launched with, and/or
+// 2x cells (ST_CAPACITY); the work is repeated by the caller.
+static int grow_buffers(mlh_ctx *c, unsigned st, bool hsolve) {
     if (st & MLH_ERR_NGB_OVERFLOW) {
+        const int most = most_slots((size_t)c->smem_per_block, hsolve);
+        const int more = round_slots(c->p.K + c->p.K / 2), K = more < most ? more : most;
+        if (K <= c->p.K) return too_many_neighbours(most);
         free_neighbour_buffers(c);
-        c->p.K = round_slots(c->p.K + c->p.K / 2);
+        c->p.K = K;
         if (int rc = alloc_neighbour_buffers(c)) return rc;
     }
     if (st & ST_CAPACITY) {
@@ -667,6 +690,9 @@ static int capture_step(mlh_ctx *c, double dt_max) {
 
 int mlh_step(mlh_ctx *c, int nsteps, double dt_max, mlh_step_stats *stats) {
     if (!c || nsteps < 0) { g_last_error = "invalid argument"; return MLH_ERR_INVALID; }
+    const bool hsolve = c->cfg.adaptive_h != 0;
+    if (nsteps > 0)
+        if (int rc = check_launchable(c, hsolve)) return rc;
     unsigned accumulated = 0;
     long long pairs = 0, faces = 0;
     unsigned long long newton = 0, fallbacks = 0, deferred = 0;
@@ -718,7 +744,7 @@ int mlh_step(mlh_ctx *c, int nsteps, double dt_max, mlh_step_stats *stats) {
         pairs += 2ll * ftot * done;
         if (st & (MLH_ERR_NGB_OVERFLOW | ST_CAPACITY)) {
             if (++retries > 8) { accumulated |= st; g_last_error = "capacity retries exhausted"; break; }
-            if (int rc = grow_buffers(c, st)) return rc;
+            if (int rc = grow_buffers(c, st, hsolve)) return rc;
             // the step is repeated: faces recorded by the aborted attempt go
             if (c->harvest.count) CK(cudaMemsetAsync(c->harvest.count, 0, sizeof(int), c->stream));
             continue;
@@ -810,7 +836,7 @@ int mlh_autotune(mlh_ctx *c, int trial_steps, mlh_tuning *out) {
         mlh_step_stats st;
         int rc = mlh_step(c, trial_steps, 0., &st);
         c->timing = false;
-        if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID)) return rc;
+        if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID | MLH_ERR_CAPACITY)) return rc;
         ms = c->kt_ms[id];
         return 0;
     };
@@ -892,7 +918,7 @@ int mlh_autotune(mlh_ctx *c, int trial_steps, mlh_tuning *out) {
                         if ((rc = restore())) goto done;
                         mlh_step_stats st;
                         rc = mlh_step(c, trial_steps, 0., &st);
-                        if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID)) goto done;
+                        if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID | MLH_ERR_CAPACITY)) goto done;
                         rc = 0;
                         if (st.device_ms < best_step) { best_step = st.device_ms; best.link_overlap = ov; }
                     }
@@ -907,7 +933,7 @@ int mlh_autotune(mlh_ctx *c, int trial_steps, mlh_tuning *out) {
                         if ((rc = restore())) goto done;
                         mlh_step_stats st;
                         rc = mlh_step(c, trial_steps, 0., &st);
-                        if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID | MLH_ERR_TIMEOUT)) goto done;
+                        if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID | MLH_ERR_CAPACITY | MLH_ERR_TIMEOUT)) goto done;
                         rc = 0;
                         if (st.device_ms < best_step) { best_step = st.device_ms; best.persistent_binning = pb; }
                     }
@@ -924,7 +950,7 @@ int mlh_autotune(mlh_ctx *c, int trial_steps, mlh_tuning *out) {
                         if ((rc = restore())) goto done;
                         mlh_step_stats st;
                         rc = mlh_step(c, trial_steps, 0., &st);
-                        if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID | MLH_ERR_TIMEOUT)) goto done;
+                        if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID | MLH_ERR_CAPACITY | MLH_ERR_TIMEOUT)) goto done;
                         rc = 0;
                         if (st.device_ms < best_step) { best_step = st.device_ms; best.fp32_filters = sf; }
                     }
@@ -937,7 +963,7 @@ int mlh_autotune(mlh_ctx *c, int trial_steps, mlh_tuning *out) {
                 if ((rc = restore())) goto done;
                 mlh_step_stats st;
                 rc = mlh_step(c, trial_steps, 0., &st);
-                if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID | MLH_ERR_TIMEOUT)) goto done;
+                if (rc & (MLH_ERR_CUDA | MLH_ERR_INVALID | MLH_ERR_CAPACITY | MLH_ERR_TIMEOUT)) goto done;
                 rc = 0;
                 if (st.device_ms < pipe_ms) pipe_ms = st.device_ms;
             }
@@ -1042,6 +1068,7 @@ int mlh_smoothing_lengths(mlh_ctx *c, double n_ngb, double *h_out, double *n_eff
         g_last_error = "n_ngb must exceed the particle's own count (32/3 in 3D, 40/7 in 2D)";
         return MLH_ERR_INVALID;
     }
+    if (int rc = check_launchable(c, true)) return rc;
     for (int retries = 0;; ++retries) {
         StepArgs a = make_args(c, 0.);
         a.p.sngb_t = sngb_target(c->cfg.dim, n_ngb);
@@ -1053,7 +1080,7 @@ int mlh_smoothing_lengths(mlh_ctx *c, double n_ngb, double *h_out, double *n_eff
         CK(cudaStreamSynchronize(c->stream));
         if (st & (MLH_ERR_NGB_OVERFLOW | ST_CAPACITY)) {
             if (retries >= 8) { g_last_error = "capacity retries exhausted"; return (int)st; }
-            if (int rc = grow_buffers(c, st)) return rc;
+            if (int rc = grow_buffers(c, st, true)) return rc;
             continue;
         }
         if (st) return (int)st;
@@ -1072,6 +1099,8 @@ int mlh_smoothing_lengths(mlh_ctx *c, double n_ngb, double *h_out, double *n_eff
 
 int mlh_prepare(mlh_ctx *c, double dt_max) {
     if (!c) { g_last_error = "null context"; return MLH_ERR_INVALID; }
+    const bool hsolve = c->cfg.adaptive_h != 0;
+    if (int rc = check_launchable(c, hsolve)) return rc;
     for (int retries = 0;; ++retries) {
         StepArgs a = make_args(c, dt_max);
         a.stop_after_gradients = 1;
@@ -1084,7 +1113,7 @@ int mlh_prepare(mlh_ctx *c, double dt_max) {
         CK(cudaStreamSynchronize(c->stream));
         if (st & (MLH_ERR_NGB_OVERFLOW | ST_CAPACITY)) {
             if (retries >= 8) { g_last_error = "capacity retries exhausted"; return (int)st; }
-            if (int rc = grow_buffers(c, st)) return rc;
+            if (int rc = grow_buffers(c, st, hsolve)) return rc;
             continue;
         }
         return (int)st;

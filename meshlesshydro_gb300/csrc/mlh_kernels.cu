@@ -1413,6 +1413,13 @@ size_t nns_smem_bytes(int K) {
     return nns_cells_bytes() + (size_t)NNS_WARPS * nns_warp_bytes(K);
 }
 
+// Both kernels list a particle's candidates in shared memory, K + 32 of them.
+int most_slots(size_t smem_per_block, bool hsolve) {
+    int K = 0;
+    while (nns_smem_bytes(K + 4) <= smem_per_block && (!hsolve || hsolve_smem_bytes(K + 4) <= smem_per_block)) K += 4;
+    return K;
+}
+
 // ------------------------------------------------------------------ dt
 
 // dt of every simulation from its minimum (or the fixed time step), clamped; by

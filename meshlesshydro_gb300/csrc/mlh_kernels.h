@@ -119,6 +119,10 @@ constexpr int BOUNDS_BLOCKS = 304;
 void step(StepArgs &a);
 // blocks of the persistent binning kernel resident at once (0: none)
 int binning_blocks(int dim, int sm_count);
+// Most neighbour slots per particle (a multiple of 4) with which the neighbour
+// search, and with `hsolve` the smoothing-length solve, fit the shared memory
+// that a block can have.
+int most_slots(size_t smem_per_block, bool hsolve);
 // binning and the smoothing-length solve alone, on the current positions
 void smoothing_lengths(StepArgs &a);
 // Particles::getDomainLimits + Domain::createGrid alone: per-block partial
