@@ -71,7 +71,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *smem, int &total
     return base + x - v;
 }
 
-__global__ void k_scan_reduce(const int *__restrict__ in, int n, int *__restrict__ tile_sums) {
+__global__ void k_scan_reduce(const int *in, int n, int *tile_sums) {
     step_begin();
     __shared__ int smem[32];
     long long base = (long long)blockIdx.x * SCAN_TILE;
@@ -90,7 +90,7 @@ __global__ void k_scan_reduce(const int *__restrict__ in, int n, int *__restrict
     }
 }
 
-__global__ void k_scan_tiles(int *__restrict__ tile_sums, int ntiles, int *__restrict__ total_out) {
+__global__ void k_scan_tiles(int *tile_sums, int ntiles, int *total_out) {
     step_begin();
     __shared__ int smem[32];
     int carry = 0;
@@ -105,8 +105,8 @@ __global__ void k_scan_tiles(int *__restrict__ tile_sums, int ntiles, int *__res
     if (threadIdx.x == 0) *total_out = carry;
 }
 
-__global__ void k_scan_apply(const int *__restrict__ in, int n, const int *__restrict__ tile_offsets,
-                             int *__restrict__ out, const int *__restrict__ total, int write_total_at_n) {
+__global__ void k_scan_apply(const int *in, int n, const int *tile_offsets,
+                             int *out, const int *total, int write_total_at_n) {
     step_begin();
     __shared__ int smem[32];
     long long base = (long long)blockIdx.x * SCAN_TILE;
@@ -132,8 +132,8 @@ __global__ void k_scan_apply(const int *__restrict__ in, int n, const int *__res
 
 // The same in one launch of one block, tile after tile, for few items: three
 // dependent launches take about 9 us whatever they do, a tile here about 1.5 us.
-__global__ void __launch_bounds__(SCAN_T) k_scan_one(const int *__restrict__ in, int n, int *__restrict__ out,
-                                                     int *__restrict__ total) {
+__global__ void __launch_bounds__(SCAN_T) k_scan_one(const int *in, int n, int *out,
+                                                     int *total) {
     step_begin();
     __shared__ int smem[32];
     int carry = 0;
@@ -249,10 +249,10 @@ __device__ __forceinline__ void bounds_partial_block(int vb, const double *__res
 }
 
 template <int D>
-__global__ void k_bounds_partial(const double *__restrict__ x, const double *__restrict__ y,
-                                 const double *__restrict__ z, Params p, const Member *__restrict__ members,
-                                 int bpm, double *__restrict__ part, int *__restrict__ cellCount,
-                                 int *__restrict__ cellFill) {
+__global__ void k_bounds_partial(const double *x, const double *y,
+                                 const double *z, Params p, const Member *__restrict__ members,
+                                 int bpm, double *part, int *cellCount,
+                                 int *cellFill) {
     step_begin();
     // with the cell counters (a step's binning): cleared here
     if (cellCount)
@@ -393,11 +393,11 @@ __device__ __forceinline__ void bounds_final_block(const double *__restrict__ x,
 }
 
 template <int D>
-__global__ void k_bounds_final(const double *__restrict__ x, const double *__restrict__ y,
-                               const double *__restrict__ z, const double *__restrict__ part, int bpm, Params p,
-                               const Member *__restrict__ members, int nmembers, GridInfo *__restrict__ grids,
-                               int *__restrict__ cellTotal, unsigned *__restrict__ status,
-                               unsigned long long *__restrict__ dtbits, unsigned *__restrict__ dtcap) {
+__global__ void k_bounds_final(const double *x, const double *y,
+                               const double *z, const double *part, int bpm, Params p,
+                               const Member *__restrict__ members, int nmembers, GridInfo *grids,
+                               int *cellTotal, unsigned *status,
+                               unsigned long long *dtbits, unsigned *dtcap) {
     step_begin();
     bounds_final_block<D>(x, y, z, part, bpm, p, members, nmembers, grids, cellTotal, status, dtbits, dtcap);
 }
@@ -431,17 +431,17 @@ __device__ __forceinline__ void assign_one(int i, const double *__restrict__ x, 
 }
 
 template <int D>
-__global__ void k_assign(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
-                         int n, const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
-                         int *__restrict__ cell, int *__restrict__ cellCount, unsigned *__restrict__ status) {
+__global__ void k_assign(const double *x, const double *y, const double *z,
+                         int n, const int *__restrict__ memberOf, const GridInfo *grids,
+                         int *cell, int *cellCount, unsigned *status) {
     step_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         assign_one<D>(i, x, y, z, memberOf, grids, cell, cellCount, status);
 }
 
-__global__ void k_fill_cells(const int *__restrict__ cell, int n, const int *__restrict__ cellStart,
-                             int *__restrict__ cellFill, int *__restrict__ cellList,
-                             const unsigned *__restrict__ status) {
+__global__ void k_fill_cells(const int *cell, int n, const int *cellStart,
+                             int *cellFill, int *cellList,
+                             const unsigned *status) {
     step_begin();
     if (step_aborted(status)) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -486,9 +486,9 @@ __device__ __forceinline__ void sort_cell_warp(int c, const int *__restrict__ ce
     if (lane + 32 < n) cellList[b + r1] = v1;
 }
 
-__global__ void __launch_bounds__(256) k_sort_cells(const int *__restrict__ cellTotal,
-                                                    const int *__restrict__ cellStart, int *__restrict__ cellList,
-                                                    const unsigned *__restrict__ status) {
+__global__ void __launch_bounds__(256) k_sort_cells(const int *cellTotal,
+                                                    const int *cellStart, int *cellList,
+                                                    const unsigned *status) {
     step_begin();
     if (step_aborted(status)) return;
     const int nc = *cellTotal;
@@ -796,13 +796,13 @@ __device__ __forceinline__ void nns_candidates(const NnsCells *cs, const float4 
 template <int D, bool ADAPT>
 __global__ void __launch_bounds__(NNS_WARPS * 32, MLH_NNS_MINB) k_neighbours(
     Params p, int nsplit, int pb, const Member *__restrict__ members, const int *__restrict__ memberOf,
-    const GridInfo *__restrict__ grids, const double *__restrict__ x, const double *__restrict__ y,
-    const double *__restrict__ z, const float4 *__restrict__ posf, const double *__restrict__ vx,
-    const double *__restrict__ vy, const double *__restrict__ vz, const double *__restrict__ m,
-    const double *__restrict__ u, const int *__restrict__ cellTotal, const int *__restrict__ cellStart,
-    const int *__restrict__ cellList, uint32_t *__restrict__ nbr, double *__restrict__ dd,
-    double *__restrict__ ww, int *__restrict__ noi, int *__restrict__ noiImg, int *__restrict__ faceCnt,
-    Prim *__restrict__ prim, Geo *__restrict__ geo, float4 *__restrict__ velf, unsigned *__restrict__ status) {
+    const GridInfo *grids, const double *x, const double *y,
+    const double *z, const float4 *posf, const double *vx,
+    const double *vy, const double *vz, const double *m,
+    const double *u, const int *cellTotal, const int *cellStart,
+    const int *cellList, uint32_t *nbr, double *dd,
+    double *ww, int *noi, int *noiImg, int *faceCnt,
+    Prim *prim, Geo *geo, float4 *velf, unsigned *status) {
     step_begin();
     constexpr unsigned ALL = 0xffffffffu;
     const int K = p.K;
@@ -1454,14 +1454,14 @@ __device__ __forceinline__ double signal_speed(double dv, const double *xij, dou
 // (positive) per-particle dt is deterministic.
 template <int D>
 __global__ void __launch_bounds__(256) k_timestep(Params p, const Member *__restrict__ members,
-                                                  const int *__restrict__ memberOf, const Prim *__restrict__ prim,
-                                                  const Geo *__restrict__ geo, const uint32_t *__restrict__ nbr,
-                                                  const int *__restrict__ noi,
-                                                  unsigned long long *__restrict__ dtbits,
-                                                  const float *__restrict__ dtlo, const unsigned *__restrict__ dtcap,
-                                                  int nmembers, double dt_max, double *__restrict__ dt_out,
-                                                  unsigned *__restrict__ arrived,
-                                                  const unsigned *__restrict__ status) {
+                                                  const int *__restrict__ memberOf, const Prim *prim,
+                                                  const Geo *geo, const uint32_t *nbr,
+                                                  const int *noi,
+                                                  unsigned long long *dtbits,
+                                                  const float *dtlo, const unsigned *dtcap,
+                                                  int nmembers, double dt_max, double *dt_out,
+                                                  unsigned *arrived,
+                                                  const unsigned *status) {
     step_begin();
     const int lane = threadIdx.x & 31;
     // no valid lists after an aborted binning
@@ -1537,8 +1537,8 @@ __global__ void __launch_bounds__(256) k_timestep(Params p, const Member *__rest
 }
 
 // dt of every simulation when no k_timestep follows the minima
-__global__ void k_dt_final(Params p, int nmembers, const unsigned long long *__restrict__ dtbits, double dt_max,
-                           double *__restrict__ dt_out, const unsigned *__restrict__ status) {
+__global__ void k_dt_final(Params p, int nmembers, const unsigned long long *dtbits, double dt_max,
+                           double *dt_out, const unsigned *status) {
     step_begin();
     if (!step_aborted(status)) dt_final(p, nmembers, dtbits, dt_max, dt_out);
 }
@@ -1651,10 +1651,10 @@ __device__ __forceinline__ void link_particle(int i, const Params &p, const uint
 // per slot: a slot with j > i owns face faceOff[i] + its rank among i's
 // canonical slots (a ballot); the other slots are set to 0 until their face
 // finds them.
-__global__ void __launch_bounds__(256) k_link_own(Params p, const uint32_t *__restrict__ nbr,
-                                                  const int *__restrict__ noi, const int *__restrict__ noiImg,
-                                                  const int *__restrict__ faceOff, int *__restrict__ faceOf,
-                                                  FaceRef *__restrict__ faces, unsigned *__restrict__ status) {
+__global__ void __launch_bounds__(256) k_link_own(Params p, const uint32_t *nbr,
+                                                  const int *noi, const int *noiImg,
+                                                  const int *faceOff, int *faceOf,
+                                                  FaceRef *faces, unsigned *status) {
     step_begin();
     if (step_aborted(status)) return;   // no valid lists
     const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
@@ -1689,10 +1689,10 @@ __global__ void __launch_bounds__(256) k_link_own(Params p, const uint32_t *__re
 // per particle, searching four lists in lockstep from their ends (link_particle,
 // which the gradients kernel runs with link_overlap 2), took 288 / 1771 / 446 us,
 // 700 warp instructions per particle with 13 of 32 lanes active.
-__global__ void __launch_bounds__(256) k_link(Params p, const uint32_t *__restrict__ nbr, const int *__restrict__ noi,
-                                              const int *__restrict__ noiImg, const int *__restrict__ faceTotal,
-                                              int *__restrict__ faceOf, FaceRef *__restrict__ faces,
-                                              unsigned *__restrict__ status) {
+__global__ void __launch_bounds__(256) k_link(Params p, const uint32_t *nbr, const int *noi,
+                                              const int *noiImg, const int *faceTotal,
+                                              int *faceOf, FaceRef *faces,
+                                              unsigned *status) {
     step_begin();
     if (step_aborted(status)) return;
     const int nf = *faceTotal < p.faces_cap ? *faceTotal : p.faces_cap;
@@ -1814,18 +1814,18 @@ __device__ __forceinline__ T lanes_reduce(unsigned mask, T v, F f) {
 }
 template <int D, int L>
 __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__ members,
-                                                   const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
-                                                   const Prim *__restrict__ prim, Geo *__restrict__ geo,
-                                                   const uint32_t *__restrict__ nbr, const double *__restrict__ ww,
-                                                   const int *__restrict__ noi, const int *__restrict__ noiImg,
-                                                   Grad *__restrict__ grad, Grad *__restrict__ gradRaw,
-                                                   double *__restrict__ psi,
-                                                   unsigned long long *__restrict__ dtbits,
-                                                   const int *__restrict__ faceOff, int *__restrict__ faceOf,
-                                                   FaceRef *__restrict__ faces, unsigned *__restrict__ status,
+                                                   const int *__restrict__ memberOf, const GridInfo *grids,
+                                                   const Prim *prim, Geo *geo,
+                                                   const uint32_t *nbr, const double *ww,
+                                                   const int *noi, const int *noiImg,
+                                                   Grad *grad, Grad *gradRaw,
+                                                   double *psi,
+                                                   unsigned long long *dtbits,
+                                                   const int *faceOff, int *faceOf,
+                                                   FaceRef *faces, unsigned *status,
                                                    int fp32_filters,
-                                                   const float4 *__restrict__ velf, float *__restrict__ dtlo,
-                                                   unsigned *__restrict__ dtcap) {
+                                                   const float4 *velf, float *dtlo,
+                                                   unsigned *dtcap) {
     step_begin();
     constexpr int NF = D + 2;
     const int lane = threadIdx.x & 31, sub = lane & (L - 1);
@@ -2301,14 +2301,14 @@ int grad_lanes(int n, int sm_count) {
 // more slots.
 template <int D>
 __global__ void __launch_bounds__(256) k_update(Params p, const int *__restrict__ memberOf,
-                                                const GridInfo *__restrict__ grids, const int *__restrict__ noi,
-                                                const int *__restrict__ noiImg, const int *__restrict__ faceOf,
-                                                const double *__restrict__ Fface, const double *__restrict__ dtp,
-                                                double *__restrict__ x, double *__restrict__ y, double *__restrict__ z,
-                                                double *__restrict__ vx, double *__restrict__ vy, double *__restrict__ vz,
-                                                double *__restrict__ m, double *__restrict__ u, float4 *__restrict__ posf,
-                                                double *__restrict__ fluxSums, unsigned *__restrict__ status,
-                                                int nmembers, double *__restrict__ simTime, int *__restrict__ stepsDone) {
+                                                const GridInfo *grids, const int *noi,
+                                                const int *noiImg, const int *faceOf,
+                                                const double *Fface, const double *dtp,
+                                                double *x, double *y, double *z,
+                                                double *vx, double *vy, double *vz,
+                                                double *m, double *u, float4 *posf,
+                                                double *fluxSums, unsigned *status,
+                                                int nmembers, double *simTime, int *stepsDone) {
     step_begin();
     // (the bits tested are not raised by this kernel: the same for every thread)
     const unsigned st0 = *(volatile const unsigned *)status;
