@@ -767,7 +767,9 @@ __device__ __forceinline__ int nns_cell_of(const NnsCells *cs, int t) {
 
 // Candidates [ch, ch + 32 NNS_REG) of the stencil's sequence, candidate ch + 32 r
 // + lane in element r: single-precision position with the image shift applied,
-// index with image bits.  Beyond the sequence: infinitely far.
+// index with image bits.  Beyond the sequence: NaN, which is within no distance (an
+// infinite distance would be within the bound h^2 of a kernelSize above 1.8e19,
+// which is infinite in single precision).
 template <int D>
 __device__ __forceinline__ void nns_candidates(const NnsCells *cs, const float4 *__restrict__ posf,
                                                const int *__restrict__ cellList, int ch, int total, float *cx,
@@ -776,7 +778,7 @@ __device__ __forceinline__ void nns_candidates(const NnsCells *cs, const float4 
 #pragma unroll
     for (int r = 0; r < NNS_REG; ++r) {
         const int t = ch + r * 32 + lane;
-        cx[r] = FLT_INF_; cy[r] = 0.f; cz[r] = 0.f; ce[r] = 0u;
+        cx[r] = __int_as_float(0x7fffffff); cy[r] = 0.f; cz[r] = 0.f; ce[r] = 0u;
         if (t < total) {
             const int k = nns_cell_of<D>(cs, t);
             const int j = cellList[cs->start[k] + (t - cs->excl[k])];
