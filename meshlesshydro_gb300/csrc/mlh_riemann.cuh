@@ -380,7 +380,9 @@ __device__ __forceinline__ RootSolve riemann_root_begin(const RiemannConsts &k, 
     s.A = make_side(k, mir ? rhoR : rhoL, mir ? flip_if(uR, true) : uL, mir ? pR : pL);
     s.B = make_side(k, mir ? rhoL : rhoR, mir ? flip_if(uL, true) : uR, mir ? pL : pR);
     s.fAs = 0.; s.fBs = 0.; s.qAs = -1.; s.qBs = -1.; s.iters = 0; s.p = 0.;
-    s.du = subr(s.B.u, s.A.u);
+    // the sorted problem's uB - uA, from the given velocities: flips on the
+    // integer pipe would turn a NaN's sign, which the vacuum test's order reads
+    s.du = subr(uR, uL);
     const double csum = addr(s.A.c, s.B.c);
     if (!dlt(s.du, xmul(k.g4, csum))) {         // g4 (cL + cR) <= uR - uL: vacuum
         s.stage = 0;
