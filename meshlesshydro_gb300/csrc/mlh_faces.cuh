@@ -371,6 +371,37 @@ __device__ __forceinline__ bool face_states(const Params &p, const Member *__res
     return true;
 }
 
+// The faces of a thread's rounds (f0, f0 + stride, ..) that the root solver does not
+// take, by riemann_exact: set up again, after the kernel's own loop, which skipped
+// them, so that the powers' calls shape no register of it (in the loop they cost the
+// pass 2-6 % at gamma = 7/5, also where every face is taken).
+template <int D, int ROOT, bool MID>
+__device__ __forceinline__ void general_faces(const Params &p, const RiemannConsts &rc, const Member *__restrict__ members,
+                                              const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
+                                              const Prim *__restrict__ prim, const Geo *__restrict__ geo,
+                                              const Grad *__restrict__ grad, const uint32_t *__restrict__ nbr,
+                                              const double *__restrict__ psi, const FaceRef *__restrict__ faces,
+                                              const double *__restrict__ dtp, double *__restrict__ Fface, int f0, int nf,
+                                              int stride, unsigned &st_local, unsigned long long &iters_local) {
+    for (int f = f0; f < nf; f += stride) {
+        double R[5], L[5], A[3] = {0., 0., 0.}, vf[3] = {0., 0., 0.};
+        FaceNormal fn = {};
+        if (!face_states<D, MID>(p, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, f, st_local, R, L, A,
+                                 vf, fn) ||
+            root_takes<ROOT>(R[0], fn.unR, R[1], L[0], fn.unL, L[1]))
+            continue;
+        const RiemannResult rs = riemann_exact(rc, R[0], fn.unR, R[1], L[0], fn.unL, L[1]);
+        if (rs.iters < 0) st_local |= ST_NEWTON;
+        else iters_local += (unsigned long long)rs.iters;
+        double Fo[5];
+        st_local |= project_flux<D>(rs, R, L, fn, A, vf, rc.inv_gm1, p.mfm, Fo);
+        double2 *dst = reinterpret_cast<double2 *>(Fface + (size_t)f * 6);
+        dst[0] = make_double2(Fo[0], Fo[1]);
+        dst[1] = make_double2(Fo[2], Fo[3]);
+        dst[2] = make_double2(Fo[4], (double)rs.iters);
+    }
+}
+
 template <int D, int ROOT, int MODE, bool MID>
 __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member *__restrict__ members,
                                                const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
@@ -385,6 +416,8 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
     if (step_aborted(status)) return;   // no valid faces
     int nf = *faceTotal < p.faces_cap ? *faceTotal : p.faces_cap;
     constexpr bool QUEUED = MODE == 2 || MODE == 4;   // passes over the queue
+    constexpr bool SOME = ROOT == 7 && !QUEUED;       // the solver does not take every face
+    bool general = false;
     if (QUEUED) {   // the queue holds min(count, capacity) faces; MODE 3 finished the rest itself
         const int qn = *qa.count < qa.cap ? *qa.count : qa.cap;
         nf = qn < nf ? qn : nf;
@@ -410,6 +443,7 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
         if (!face_states<D, MID>(p, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, f, st_local, R, L, A,
                             vf, fn))
             continue;
+        if (SOME && !root_takes<ROOT ? ROOT : 5>(R[0], fn.unR, R[1], L[0], fn.unL, L[1])) { general = true; continue; }
         }   // !QUEUED
         const double unR = fn.unR, unL = fn.unL;
         double guess = -1.;
@@ -491,6 +525,10 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
         dst[1] = make_double2(Fo[2], Fo[3]);
         dst[2] = make_double2(Fo[4], (double)face_iters);
     }
+    if (SOME && general)
+        general_faces<D, ROOT ? ROOT : 5, MID>(p, rc, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, Fface,
+                                               blockIdx.x * blockDim.x + threadIdx.x, nf, gridDim.x * blockDim.x, st_local,
+                                               iters_local);
     // block-level accumulation of the counters
     for (int o = 16; o > 0; o >>= 1) {
         iters_local += __shfl_xor_sync(0xffffffffu, iters_local, o);
@@ -565,7 +603,8 @@ __global__ void __maxnreg__(MLH_FACE_MAXREG_BLOCK) k_faces_block(Params p, Riema
                                               const double *__restrict__ psi, const int *__restrict__ faceTotal,
                                               const FaceRef *__restrict__ faces, const double *__restrict__ dtp,
                                               double *__restrict__ Fface, unsigned long long *__restrict__ newtonSum,
-                                              unsigned *__restrict__ status, const PackedMlp *__restrict__ mlp) {
+                                              unsigned *__restrict__ status, const PackedMlp *__restrict__ mlp,
+                                              int *__restrict__ generalCount) {
     __shared__ RootSolve sv[FB_T];
     __shared__ int todo[FB_T];
     __shared__ int slist[LEARNED ? FB_T : 1];
@@ -583,6 +622,10 @@ __global__ void __maxnreg__(MLH_FACE_MAXREG_BLOCK) k_faces_block(Params p, Riema
         if (valid)
             valid = face_states<D, true>(p, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, f, st_local, R,
                                    L, A, vf, fn);
+        if (ROOT == 7 && valid && !root_takes<ROOT>(R[0], fn.unR, R[1], L[0], fn.unL, L[1])) {
+            *generalCount = 1;   // left to k_faces_general
+            valid = false;
+        }
         bool unfinished = false, strong = false;
         if (valid) {
             // strong shocks of the learned step stop before their first
@@ -666,6 +709,29 @@ __global__ void __maxnreg__(MLH_FACE_MAXREG_BLOCK) k_faces_block(Params p, Riema
     }
 }
 
+// The faces that k_faces_block left to riemann_exact, when there are any
+// (generalCount).  A kernel of its own, for gamma = 7/5 alone: at the end of
+// k_faces_block the same code took registers from its loop (640^2 particles: 1277 us
+// without, 1343 there, 1291 so; the clear and this launch are 7 us of it).
+template <int D, int ROOT>
+__global__ void MLH_FACE_BOUNDS k_faces_general(Params p, RiemannConsts rc, const Member *__restrict__ members,
+                                                const int *__restrict__ memberOf, const GridInfo *__restrict__ grids,
+                                                const Prim *__restrict__ prim, const Geo *__restrict__ geo,
+                                                const Grad *__restrict__ grad, const uint32_t *__restrict__ nbr,
+                                                const double *__restrict__ psi, const int *__restrict__ faceTotal,
+                                                const FaceRef *__restrict__ faces, const double *__restrict__ dtp,
+                                                double *__restrict__ Fface, unsigned long long *__restrict__ newtonSum,
+                                                unsigned *__restrict__ status, const int *__restrict__ generalCount) {
+    if (*generalCount == 0 || step_aborted(status)) return;
+    const int nf = *faceTotal < p.faces_cap ? *faceTotal : p.faces_cap;
+    unsigned long long iters_local = 0;
+    unsigned st_local = 0;
+    general_faces<D, ROOT, true>(p, rc, members, memberOf, grids, prim, geo, grad, nbr, psi, faces, dtp, Fface,
+                                 blockIdx.x * blockDim.x + threadIdx.x, nf, gridDim.x * blockDim.x, st_local, iters_local);
+    if (iters_local) atomicAdd(newtonSum, iters_local);
+    if (st_local) flag(status, st_local);
+}
+
 // Riemann::Riemann + Riemann::exact (demonstrator/src/Riemann.cpp:7-229) for a
 // batch of independent faces: per face the left state Wi (particle i) and the
 // right state Wj (neighbour j), each [rho, P, v_x, v_y(, v_z)], the frame
@@ -690,8 +756,11 @@ __global__ void __launch_bounds__(256) k_riemann_batch(int n, RiemannConsts rc, 
         if (R[1] < 0. || L[1] < 0.) st |= ST_NEG_PRESSURE;
         const FaceNormal fn = face_normal<D>(A, R, L);
         const double unR = fn.unR, unL = fn.unL;
-        const RiemannResult rs = ROOT ? riemann_exact_root<ROOT ? ROOT : 5>(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.)
-                                       : riemann_exact(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.);
+        RiemannResult rs;
+        if (ROOT == 0) rs = riemann_exact(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.);
+        else if (!root_takes<ROOT ? ROOT : 5>(R[0], unR, R[1], L[0], unL, L[1]))
+            rs = riemann_exact_call(rc.gamma, rc.tol, rc.max_iter, R[0], unR, R[1], L[0], unL, L[1]);
+        else rs = riemann_exact_root<ROOT ? ROOT : 5>(rc, R[0], unR, R[1], L[0], unL, L[1], -1., 0.);
         if (rs.iters < 0) st |= ST_NEWTON;
         double Fo[5];
         st |= project_flux<D>(rs, R, L, fn, A, vf, rc.inv_gm1, mfm, Fo);
@@ -737,6 +806,13 @@ void launch_faces(StepArgs &a) {
         if (p.foqp) MLH_FACES(MODE, true, QA, QB);      \
         else MLH_FACES(MODE, false, QA, QB);            \
     } while (0)
+#define MLH_FACES_GENERAL()                                                                                       \
+    do {                                                                                                          \
+        if constexpr (ROOT == 7)                                                                                  \
+            k_faces_general<D, ROOT><<<fB, fT, 0, s>>>(pf, rc, a.members, a.memberOf, a.grids, a.prim, a.geo,     \
+                                                       a.grad, a.nbr, a.psi, a.faceOff + p.n, a.faces, a.dt,      \
+                                                       a.Fface, a.newtonSum, a.status, a.queueCount);             \
+    } while (0)
     // the structures that regroup unfinished faces (face_split 1, 2) are built
     // for the midpoint quadrature point; with the other one a step runs the one
     // pass (the same bits)
@@ -752,7 +828,8 @@ void launch_faces(StepArgs &a) {
                 // the network's guess evaluated there
                 k_faces_block<D, ROOT, true><<<fBb, FB_T, 0, s>>>(pf, rc, a.members, a.memberOf, a.grids, a.prim, a.geo, a.grad,
                                                            a.nbr, a.psi, a.faceOff + p.n, a.faces, a.dt, a.Fface,
-                                                           a.newtonSum, a.status, (const PackedMlp *)a.mlp_packed);
+                                                           a.newtonSum, a.status, (const PackedMlp *)a.mlp_packed, a.queueCount);
+                MLH_FACES_GENERAL();
             } else {
                 MLH_FACES_MID(1, qa, qb);
                 pstar_infer_dev(a.feat, a.queueCount, (int)a.faces_cap, a.mlp_packed, a.yguess, a.sm_count, s);
@@ -761,9 +838,11 @@ void launch_faces(StepArgs &a) {
             }
         } else if (a.harvest.stride == 0 && split == 2) {
             // unconverged faces after one Newton step continued inside the block
+            if (ROOT == 7) cudaMemsetAsync(a.queueCount, 0, sizeof(int), s);
             k_faces_block<D, ROOT, false><<<fBb, FB_T, 0, s>>>(pf, rc, a.members, a.memberOf, a.grids, a.prim, a.geo, a.grad, a.nbr,
                                                         a.psi, a.faceOff + p.n, a.faces, a.dt, a.Fface, a.newtonSum,
-                                                        a.status, nullptr);
+                                                        a.status, nullptr, a.queueCount);
+            MLH_FACES_GENERAL();
         } else if (a.fstate && a.harvest.stride == 0 && split) {
             // unconverged faces after one Newton step go to a second, dense pass
             cudaMemsetAsync(a.queueCount, 0, sizeof(int), s);
@@ -783,6 +862,7 @@ void launch_faces(StepArgs &a) {
             MLH_FACES_MID(0, qa, qb);
         }
     }
+#undef MLH_FACES_GENERAL
 #undef MLH_FACES_MID
 #undef MLH_FACES
 }

@@ -368,6 +368,27 @@ __device__ __forceinline__ void riemann_root_newton(const RiemannConsts &k, Root
     s.stage = 1;
 }
 
+// Whether the root solver takes a problem.  At gamma = 7/5 only one with densities
+// and pressures in 2^-400 .. 2^400 and finite velocities, where its products and
+// roots stay normal; the rest (cold gas with p = 0 above all, and states that are
+// no physical ones) goes to riemann_exact, as with any other gamma: the root solver
+// calls a side without pressure a vacuum.  At gamma = 5/3 it takes every problem.
+template <int N>
+__device__ __forceinline__ bool root_takes(double rhoL, double uL, double pL, double rhoR, double uR, double pR) {
+    if (N == 5) return true;
+    auto off = [](double x) { return (uint32_t)__double2hiint(x) - (623u << 20) >= 800u << 20; };
+    auto infinite = [](double x) { return ((uint32_t)__double2hiint(x) & 0x7fffffffu) >= 0x7ff00000u; };
+    return !(off(rhoL) | off(pL) | off(rhoR) | off(pR) | infinite(uL) | infinite(uR));
+}
+
+// riemann_exact out of line, from scalars (a reference to a kernel's constants would
+// be a copy on the stack)
+static __device__ __noinline__ RiemannResult riemann_exact_call(double gamma, double tol, int max_iter, double rhoL,
+                                                                double uL, double pL, double rhoR, double uR,
+                                                                double pR) {
+    return riemann_exact(make_riemann_consts(gamma, tol, max_iter), rhoL, uL, pL, rhoR, uR, pR);
+}
+
 // The sides, the vacuum test, the start (the given guess, or p_TR) and the
 // Newton iteration of riemann_exact_root, up to its optional stops.
 template <int N>

@@ -42,3 +42,73 @@ def test_nan_velocity_does_not_depend_on_the_sides(gamma):
     up, down = p[0] < p[1], p[0] > p[1]
     assert up.any() and down.any()
     assert len(set(it[up]) | set(it[down])) == 1
+
+
+def cold_one(rho, p, v):
+    p[1] = 0.0
+
+
+def cold_both(rho, p, v):
+    p[:] = 0.0
+
+
+def tiny_p(rho, p, v):
+    p *= 1e-300
+
+
+def huge_p(rho, p, v):
+    p *= 1e130
+
+
+def infinite_p(rho, p, v):
+    p[0] = np.inf
+
+
+def no_density(rho, p, v):
+    rho[1] = 0.0
+
+
+# gamma = 7/5 next to a gamma that has always taken the general solver: what the root
+# solver does not take (p = 0 and pressures outside 1e-120 .. 1e120 first of all) is
+# solved as there
+@pytest.mark.parametrize("edge", [cold_one, cold_both, tiny_p, huge_p, infinite_p, no_density])
+@pytest.mark.parametrize("gamma", [7.0 / 5.0, 1.3])
+def test_states_past_the_root_solver(oracle_mod, gamma, edge):
+    rho, p, v, A, vf = problems(500, 5)
+    edge(rho, p, v)
+    W = [np.concatenate([rho[k][:, None], p[k][:, None], v[k]], axis=1) for k in (0, 1)]
+    Fo, ito, sto = oracle_mod.riemann_fluxes(*W, vf, A, gamma=gamma)
+    F, it, st = solve(rho, p, v, A, vf, gamma)
+    assert np.array_equal(it < 0, ito < 0)
+    finite = np.isfinite(Fo).all(axis=1)
+    assert np.array_equal(np.isfinite(F).all(axis=1), finite)
+    ok = finite & (it >= 0)
+    # 1e-12 of the largest flux, the gate of the other flux tests
+    scale = np.maximum(np.max(np.abs(Fo[ok]), axis=0, initial=0.0), 1e-300)
+    assert np.max(np.abs(F[ok] - Fo[ok]) / scale, initial=0.0) <= 1e-12
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_cold_gas_steps_are_the_same_in_every_structure(dim):
+    """Half of the particles without pressure, gamma = 7/5: one pass, the queue and the
+    in-block regrouping give the same bits and Newton counts, with and without graph."""
+    from meshlesshydro_gb300 import build, ic, runtime
+    from meshlesshydro_gb300.config import MFVConfig
+    build.build()
+    p = ic.kelvin_helmholtz(n_side=30, seed=6, gamma=1.4) if dim == 2 else ic.sedov(n_side=12, seed=6, gamma=1.4)
+    p.u[::2] = 0.0
+    cfg = MFVConfig.kelvin_helmholtz(p) if dim == 2 else MFVConfig.sedov(p)
+    got = []
+    for split, graph in ((0, False), (1, False), (2, False), (2, True), (1, True)):
+        s = runtime.Simulation(cfg, p)
+        s.set_tuning({"face_threads": 128, "face_blocks_per_sm": 3, "grad_threads": 64, "nns_warps_per_sm": 32,
+                      "face_split": split})
+        s.set_graph_mode(graph)
+        st = s.step(2, check=False)
+        got.append((s.get_state(), st.newton_iterations, st.status))
+        s.close()
+    assert got[0][1] > 0
+    for state, newton, status in got[1:]:
+        assert (newton, status) == got[0][1:]
+        for k in state:
+            np.testing.assert_array_equal(state[k], got[0][0][k], err_msg=k)
