@@ -1763,14 +1763,28 @@ __device__ __forceinline__ void invert_symmetric(double *A) {
     }
 }
 
-// x in single precision, the mantissa truncated (error below 2^-23 |x|, or
-// 2^-126 where it flushes to zero), on the integer pipe
-__device__ __forceinline__ float trunc_f32(double x) {
+// x 2^(1023 - 127 - base / 2^20) in single precision, the mantissa truncated (error
+// below 2^-23 of the result, or 2^-126 where it flushes to zero), on the integer
+// pipe: the exponent is rebased on the way.  base: a biased double exponent less
+// 127, in place; 896 << 20 takes x as it is.
+__device__ __forceinline__ float trunc_f32(double x, int base) {
     const uint32_t h = __double2hiint(x), l = __double2loint(x);
-    const uint32_t m = (h & 0x7fffffffu) - (896u << 20);      // rebased exponent and the mantissa's top
+    const uint32_t m = (h & 0x7fffffffu) - (uint32_t)base;    // rebased exponent and the mantissa's top
     const uint32_t v = __funnelshift_l(l, m, 3);
     return __uint_as_float(((int)m < (1 << 20) ? 0u : (int)m >= (255 << 20) ? 0x7f800000u : v & 0x7fffffffu) | (h & 0x80000000u));
 }
+// the exponent field (in place) of the largest of D numbers' magnitudes, and the
+// base that takes it to 1 in single precision
+template <int D>
+__device__ __forceinline__ int top_exponent(const double *x) {
+    int e = 0;
+#pragma unroll
+    for (int a = 0; a < D; ++a) e = max(e, __double2hiint(x[a]) & 0x7ff00000);
+    return e;
+}
+__device__ __forceinline__ int f32_base(int exponent) { return max(exponent - (127 << 20), 0); }
+
+constexpr int AS_IS = 896 << 20;
 
 template <int D>
 __device__ __forceinline__ double field_of(const Prim &q, int f) {
@@ -1921,7 +1935,8 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 // most eps (2 (c_i + c_j) + 2 vs + 12 V) with V = |v_i|_1 + |v_j|_1
                 // (an offset that flushes to zero is below 2^-126, and r above 1e-30);
                 // B is twice eps (2 (c_i + c_j) + 2 vs + 16 V)
-                const float dx = trunc_f32(d[0]), dy = trunc_f32(d[1]), dz = D == 3 ? trunc_f32(d[2]) : 0.f;
+                const float dx = trunc_f32(d[0], AS_IS), dy = trunc_f32(d[1], AS_IS),
+                            dz = D == 3 ? trunc_f32(d[2], AS_IS) : 0.f;
                 const float wx = __fsub_rn(vif.x, vj.x), wy = __fsub_rn(vif.y, vj.y),
                             wz = D == 3 ? __fsub_rn(vif.z, vj.z) : 0.f;
                 const float dvd = __fmaf_rn(wz, dz, __fmaf_rn(wy, dy, __fmul_rn(wx, dx)));   // v_ij . (x_j - x_i)
@@ -2084,16 +2099,20 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 // chain runs only over the neighbours inside those windows (a
                 // handful; every lane of a warp walks its own list): the same
                 // extrema, bit for bit.  A field whose gradient is zero has
-                // f_ij = f_i at every neighbour.
+                // f_ij = f_i at every neighbour.  q_j and its bounds are in units of the
+                // field's gradient, so that a gradient below the normal range of single
+                // precision (a density in g/cm^3 over 10^18 cm) keeps its bits.
                 float gf[NF][3];
 #pragma unroll
-                for (int f = 0; f < NF; ++f)
+                for (int f = 0; f < NF; ++f) {
+                    const int gb = f32_base(top_exponent<D>(gr[f]));
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) gf[f][a] = a < D ? __double2float_rn(gr[f][a]) : 0.f;
+                    for (int a = 0; a < 3; ++a) gf[f][a] = a < D ? trunc_f32(gr[f][a], gb) : 0.f;
+                }
                 auto offset_f = [&](int s, float *df, double *d) {
                     const double *ds = psi + (base + s) * 3;
 #pragma unroll
-                    for (int a = 0; a < D; ++a) { d[a] = ds[a]; df[a] = trunc_f32(d[a]); }
+                    for (int a = 0; a < D; ++a) { d[a] = ds[a]; df[a] = trunc_f32(d[a], AS_IS); }
                 };
                 auto incr = [&](int f, const float *d) {
                     float q = __fmul_rn(gf[f][0], d[0]);
@@ -2127,8 +2146,8 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 }
                 // B_f = 16 eps32 S (dmax + 1e-30) + 12 u64 (|f_i| + S dmax) with S = sum
                 // |c grad f| and dmax = max |x_j - x_i|: more than twice the sum of the
-                // single-precision error, at most 6 eps32 S dmax (2 from the offset's
-                // truncation, 1 from the gradient, 3 from the chain) and 2^-126 S for
+                // single-precision error, at most 7 eps32 S dmax (2 from the offset's
+                // truncation, 2 from the gradient's, 3 from the chain) and 2^-126 S for
                 // offsets flushed to zero, and the FP64 chain's, at most 4 u64 (|f_i| +
                 // S dmax)
                 constexpr float EPS32 = 5.9604645e-8f, U64 = 1.1102230e-16f;
@@ -2145,7 +2164,9 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                         S += fabsf(gf[f][a]);
                     }
                     flat[f] = z;
-                    const float fa = fabsf(__double2float_rn(fi[f]));
+                    const int ge = top_exponent<D>(gr[f]);
+                    ok = ok && ge < 0x7ff00000;   // no infinity or NaN among the gradients
+                    const float fa = z ? 0.f : fabsf(trunc_f32(fi[f], f32_base(ge))) * (1.f + 4.f * EPS32);
                     const float SR = S * R;
                     ok = ok && SR < 1e36f && S < 1e36f && fa < 1e36f;   // false for NaN and infinity
                     const float B = 16.f * EPS32 * SR + 12.f * U64 * (fa + SR) + 1e-36f;

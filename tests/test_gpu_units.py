@@ -62,3 +62,42 @@ def test_smoothing_lengths(scale):
         sim.close()
     for a, b in zip(*got):
         np.testing.assert_array_equal(a, b)
+
+
+# cgs-like units among them: lengths of 1e18, densities of 1e-24, so that gradients of
+# the density (1e-41) are below the normal range of single precision.  Powers of 2^10
+# keep fifth roots of pressures exact as well.
+UNITS = [(2.0 ** 60, 1.0), (2.0 ** 60, 2.0 ** -80), (2.0 ** 60, 2.0 ** -100), (TWO67, 2.0 ** -80), (1 / TWO40, 2.0 ** 40),
+         (2.0 ** -60, 1.0), (1 / TWO67, 2.0 ** 80)]
+
+
+def state_after(cfg, p, steps, s, r, filters):
+    from meshlesshydro_gb300 import runtime
+    sim = runtime.Simulation(cfg, p)
+    sim.set_tuning({"face_threads": 128, "face_blocks_per_sm": 8, "grad_threads": 128, "nns_warps_per_sm": 32,
+                    "face_split": 0, "fp32_filters": filters})
+    sim.step(steps)
+    out = sim.get_state()
+    for k in "xyz":
+        if k in out:
+            out[k] = out[k] / s
+    out["m"] = out["m"] / (s ** p.dim * r)
+    out["time"] = sim.member_times()[1] / s
+    sim.close()
+    return out
+
+
+@pytest.mark.parametrize("s,r", UNITS)
+@pytest.mark.parametrize("dim", [2, 3])
+def test_steps(dim, s, r):
+    p, config = setup(dim)
+    rng = np.random.default_rng(8)
+    p.u *= rng.uniform(0.5, 2.0, p.n)       # fields without symmetry or flat parts
+    p.m *= rng.uniform(0.8, 1.25, p.n)
+    q = scaled(p, s)
+    q.m = q.m * r
+    want = state_after(config(p), p, 3, 1.0, 1.0, 3)
+    for filters in (0, 1, 2, 3):
+        got = state_after(config(q), q, 3, s, r, filters)
+        for k in want:
+            np.testing.assert_array_equal(got[k], want[k], err_msg=f"{k}, filters {filters}")
