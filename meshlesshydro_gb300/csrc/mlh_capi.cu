@@ -411,6 +411,12 @@ void fill_params(mlh_ctx *c) {
     // single-precision pre-filter bound: positions rounded to float move a
     // distance of ~1e-7 relative to the box; 1e-3 relative on h^2 is ample
     p.hsq_f = (float)(p.hsq * (1. + 1e-3));
+    {
+        double h = 0.;
+        for (const Member &mb : c->hmembers) h = h < mb.h ? mb.h : h;
+        const int e = std::isfinite(h) ? std::ilogb(h) + 1023 - 127 : 1920;   // h > 0
+        p.f32_base = (e < 0 ? 0 : e) << 20;
+    }
     p.adaptive_h = f.adaptive_h;
     p.cfl = f.cfl;
     p.sngb_t = sngb_target(f.dim, f.n_ngb);

@@ -1932,11 +1932,14 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
             if (want_dtf && s < nr) {
                 // |vs - vs64| <= B: the inputs' roundings (eps |c|, eps |v|, 2 eps |d|
                 // per offset), the estimate's own and the FP64 expression's, at
-                // most eps (2 (c_i + c_j) + 2 vs + 12 V) with V = |v_i|_1 + |v_j|_1
-                // (an offset that flushes to zero is below 2^-126, and r above 1e-30);
-                // B is twice eps (2 (c_i + c_j) + 2 vs + 16 V)
-                const float dx = trunc_f32(d[0], AS_IS), dy = trunc_f32(d[1], AS_IS),
-                            dz = D == 3 ? trunc_f32(d[2], AS_IS) : 0.f;
+                // most eps (2 (c_i + c_j) + 2 vs + 12 V) with V = |v_i|_1 + |v_j|_1;
+                // B is twice eps (2 (c_i + c_j) + 2 vs + 16 V).  Offsets are in units
+                // of kernelSize, so that the unit of length does not matter (only
+                // their direction does): an r above 1e-12 and a B above 1e-31 leave
+                // what flushes to zero (2^-126 of an offset, 2^-149 of a product)
+                // far below B.
+                const float dx = trunc_f32(d[0], p.f32_base), dy = trunc_f32(d[1], p.f32_base),
+                            dz = D == 3 ? trunc_f32(d[2], p.f32_base) : 0.f;
                 const float wx = __fsub_rn(vif.x, vj.x), wy = __fsub_rn(vif.y, vj.y),
                             wz = D == 3 ? __fsub_rn(vif.z, vj.z) : 0.f;
                 const float dvd = __fmaf_rn(wz, dz, __fmaf_rn(wy, dy, __fmul_rn(wx, dx)));   // v_ij . (x_j - x_i)
@@ -1947,7 +1950,7 @@ __global__ void MLH_GRAD_BOUNDS k_gradients(Params p, const Member *__restrict__
                 const float V = fabsf(vif.x) + fabsf(vif.y) + fabsf(vif.z) + fabsf(vj.x) + fabsf(vj.y) + fabsf(vj.z);
                 constexpr float EPS32 = 5.9604645e-8f;
                 const float B = 2.f * EPS32 * (2.f * (vif.w + vj.w) + 2.f * vs + 16.f * V);
-                dt_exact = dt_exact || !(r > 1e-15f) || !(r < 1e15f) || !(B < 1e30f);
+                dt_exact = dt_exact || !(r > 1e-12f) || !(r < 1e15f) || !(B > 1e-31f) || !(B < 1e30f);
                 vlo = fmaxf(vlo, vs - B);
                 vhi = fmaxf(vhi, vs + B);
             }

@@ -101,3 +101,27 @@ def test_steps(dim, s, r):
         got = state_after(config(q), q, 3, s, r, filters)
         for k in want:
             np.testing.assert_array_equal(got[k], want[k], err_msg=f"{k}, filters {filters}")
+
+
+def test_time_step_costs_the_same():
+    """The time step's filter works in units of kernelSize: in a large unit of length it
+    used to give up, and v_sig of every particle was evaluated in FP64 (the gradients
+    and the time step of KH 100^2: 103 us instead of 42)."""
+    from meshlesshydro_gb300 import build, ic, runtime
+    from meshlesshydro_gb300.config import MFVConfig
+    build.build()
+    p = ic.kelvin_helmholtz(n_side=100, seed=3)
+    ms = []
+    for s in (1.0, 2.0 ** 60, 2.0 ** -60):
+        q = scaled(p, s)
+        sim = runtime.Simulation(MFVConfig.kelvin_helmholtz(q), q)
+        sim.step(2)
+        sim.set_kernel_timing(True)
+        best = np.inf
+        for _ in range(5):
+            sim.reset_kernel_times()
+            sim.step(2)
+            best = min(best, sim.kernel_times()["gradients_limiter"][1])
+        ms.append(best)
+        sim.close()
+    assert max(ms) < 1.5 * min(ms), ms

@@ -61,3 +61,35 @@ def test_candidates_hold_the_extrema_at_every_scale():
         assert np.any(fij[cand] == fij.max()) and np.any(fij[cand] == fij.min())
         kept += 1
     assert kept > 5000
+
+
+def test_signal_speed_bound_in_units_of_kernel_size():
+    rng = np.random.default_rng(2)
+    used = 0
+    for t in range(6000):
+        D, n = 2 + t % 2, int(rng.integers(1, 40))
+        h = 10.0 ** rng.uniform(-200, 200)
+        d = (rng.random((n, D)) * 2 - 1) * h / np.sqrt(D) * 10.0 ** -rng.integers(0, 9)
+        if t % 7 == 0:
+            d[::2, 0] = rng.choice([0.0, 1e-45 * h, -1e-40 * h, 1e-60 * h], d[::2, 0].shape)
+        r = np.sqrt(np.sum((d / h) ** 2, axis=1)) * h
+        scale = 10.0 ** rng.integers(-26, 26)
+        vi = rng.standard_normal(D) * scale
+        vj = vi + rng.standard_normal((n, D)) * scale * (0.0 if t % 9 == 0 else 1.0)
+        ci, cj = abs(rng.standard_normal()) * scale, np.abs(rng.standard_normal(n)) * scale
+        dv = np.sum((vi - vj) * -(d / h), axis=1)
+        with np.errstate(all="ignore"):
+            vs = np.where(dv < 0, ci + cj - dv / (r / h), ci + cj)
+        df, vif, vjf = trunc_f32(d, base_of([h])), vi.astype(f32), vj.astype(f32)
+        with np.errstate(all="ignore"):
+            w = (vif - vjf).astype(f32)
+            dvd = np.sum((w * df).astype(f32), axis=1, dtype=f32)
+            rf = np.sqrt(np.sum((df * df).astype(f32), axis=1, dtype=f32)).astype(f32)
+            T = np.where(dvd > 0, (dvd / rf).astype(f32), f32(0))
+            vsf = (f32(ci) + cj.astype(f32) + T).astype(f32)
+            V = (np.abs(vif).sum() + np.abs(vjf).sum(axis=1)).astype(f32)
+            B = f32(2) * EPS32 * (f32(2) * (f32(ci) + cj.astype(f32)) + f32(2) * vsf + f32(16) * V)
+        ok = (rf > f32(1e-12)) & (rf < f32(1e15)) & (B > f32(1e-31)) & (B < f32(1e30))
+        assert np.all(np.abs(vsf.astype(np.float64) - vs)[ok] <= B[ok]), t
+        used += ok.mean()
+    assert used > 5500
