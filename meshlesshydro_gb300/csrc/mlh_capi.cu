@@ -628,6 +628,9 @@ static int grow_buffers(mlh_ctx *c, unsigned st, bool hsolve) {
             return MLH_ERR_CAPACITY;
         }
         free_cell_buffers(c);
+        // the grids hold more cells than that: the search's parts per cell are
+        // chosen by it
+        if (c->cells_est < c->p.ncells_cap) c->cells_est = c->p.ncells_cap;
         c->p.ncells_cap = c->p.ncells_cap * 2;
         if (int rc = alloc_cell_buffers(c)) return rc;
     }

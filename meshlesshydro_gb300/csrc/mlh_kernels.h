@@ -56,7 +56,7 @@ struct StepArgs {
     // grids, one per member
     GridInfo *grids;
     int *cellTotal;
-    long long cells_est;       // cells of all grids when the context was created
+    long long cells_est;       // cells of all grids when the context was created, or its buffers last grew
     double *boundsPart;
     int *cell, *cellCount, *cellStart, *cellFill, *cellList;
     // neighbours
