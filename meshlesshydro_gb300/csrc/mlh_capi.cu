@@ -122,10 +122,10 @@ struct mlh_ctx {
     // simulations, by the neighbour slots, by the cells
     char *arena = nullptr, *ngbArena = nullptr, *cellArena = nullptr;
     // scalars: newtonSum[3], status, stepsDone, dt and simTime of every
-    // simulation lie in one block, cleared and read back in one operation each
-    // per mlh_step; hscal is its pinned copy, with the number of faces behind
+    // simulation lie in one block, cleared in one operation per mlh_step; the
+    // number of faces (faceOff[n]) lies before it, and hscal is the copy of both
     char *scal = nullptr;
-    char *hscal = nullptr;
+    std::vector<char> hscal;
     unsigned *status = nullptr;
     unsigned long long *dtbits = nullptr, *newtonSum = nullptr;
     double *dt = nullptr, *simTime = nullptr;
@@ -311,6 +311,8 @@ void collect_timers(mlh_ctx *c) {
 // of the `nm` simulations, then simTime of the first `times`.
 constexpr size_t STEP_COUNTERS = 3 * sizeof(unsigned long long) + sizeof(unsigned) + sizeof(int);
 size_t step_scalars_bytes(size_t nm, size_t times) { return STEP_COUNTERS + sizeof(double) * (nm + times); }
+// the block in its host copy, behind the number of faces
+const char *step_scalars(const mlh_ctx *c) { return c->hscal.data() + (c->scal - (char *)(c->faceOff + c->n)); }
 
 // Structure of the plain face pass when neither the caller nor the autotuner
 // chose one: one pass (0) for few particles, where a block has one or two
@@ -517,10 +519,10 @@ static int create_impl(const mlh_config *cfg, int nmembers, const mlh_member *md
     A(members, nm); A(grids, nm); A(cellTotal, 1); A(boundsPart, nm * (size_t)c->bpm * 6);
     if (nmembers > 1) A(memberOf, n);
     A(cell, n); A(cellList, n);
-    A(noi, n); A(noiImg, n); A(faceCnt, n); A(faceOff, n + 1);
+    A(noi, n); A(noiImg, n); A(faceCnt, n);
     A(prim, n); A(geo, n); A(grad, n); A(gradRaw, n); A(fluxSums, n * 5);
     A(dtbits, nm);
-    A(scal, step_scalars_bytes(nm, nm));
+    A(faceOff, n + 1); A(scal, step_scalars_bytes(nm, nm));   // read back together
     A(hp, n); A(neff, n); A(hstat, 2); A(hpf, n);
     A(scanTotal, 1);
     A(bar, 2); A(arrived, 1);
@@ -531,8 +533,7 @@ static int create_impl(const mlh_config *cfg, int nmembers, const mlh_member *md
     c->stepsDone = (int *)(c->status + 1);
     c->dt = (double *)(c->scal + STEP_COUNTERS);
     c->simTime = c->dt + nm;
-    if (cudaMallocHost(&c->hscal, step_scalars_bytes(nm, 1) + sizeof(int)) != cudaSuccess)
-        return fail(cuda_fail(cudaGetLastError(), "cudaMallocHost"));
+    c->hscal.resize(c->scal - (char *)(c->faceOff + n) + step_scalars_bytes(nm, 1));
     if ((rc = alloc_cell_buffers(c))) return fail(rc);
     if ((rc = alloc_neighbour_buffers(c))) return fail(rc);
     if (cudaMemcpyAsync(c->members, mem.data(), sizeof(Member) * nm, cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
@@ -643,7 +644,6 @@ void mlh_destroy(mlh_ctx *c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     drop_graph(c);
     cudaFree(c->arena);
-    if (c->hscal) cudaFreeHost(c->hscal);
     free_cell_buffers(c);
     free_neighbour_buffers(c);
     if (c->mlp_w) cudaFree(c->mlp_w);
@@ -728,9 +728,9 @@ int mlh_step(mlh_ctx *c, int nsteps, double dt_max, mlh_step_stats *stats) {
         CK(cudaGetLastError());
         // counters, dt and time of the first simulation, and the last step's
         // face count, waited for once
-        const size_t sb = step_scalars_bytes((size_t)c->nmembers, 1);
-        CK(cudaMemcpyAsync(c->hscal, c->scal, sb, cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaMemcpyAsync(c->hscal + sb, c->faceOff + c->n, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        // (in pageable memory: a pinned block cost a small context a quarter of its
+        // creation, 100 us, and as much in mlh_destroy)
+        CK(cudaMemcpyAsync(c->hscal.data(), c->faceOff + c->n, c->hscal.size(), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         float ms = 0.f;
         cudaEventElapsedTime(&ms, c->ev0, c->ev1);
@@ -739,10 +739,11 @@ int mlh_step(mlh_ctx *c, int nsteps, double dt_max, mlh_step_stats *stats) {
         unsigned st = 0;
         int done = 0, ftot = 0;
         unsigned long long nsum[3] = {0, 0, 0};
-        std::memcpy(nsum, c->hscal, sizeof(nsum));
-        std::memcpy(&st, c->hscal + sizeof(nsum), sizeof(st));
-        std::memcpy(&done, c->hscal + sizeof(nsum) + sizeof(st), sizeof(done));
-        std::memcpy(&ftot, c->hscal + sb, sizeof(ftot));   // of the last step
+        const char *hs = step_scalars(c);
+        std::memcpy(nsum, hs, sizeof(nsum));
+        std::memcpy(&st, hs + sizeof(nsum), sizeof(st));
+        std::memcpy(&done, hs + sizeof(nsum) + sizeof(st), sizeof(done));
+        std::memcpy(&ftot, c->hscal.data(), sizeof(ftot));   // of the last step
         have_scalars = true;
         newton += nsum[0];
         fallbacks += nsum[1];
@@ -765,8 +766,8 @@ int mlh_step(mlh_ctx *c, int nsteps, double dt_max, mlh_step_stats *stats) {
         stats->steps = done_total;
         stats->status = accumulated;
         if (have_scalars) {
-            std::memcpy(&stats->dt, c->hscal + STEP_COUNTERS, sizeof(double));
-            std::memcpy(&stats->time, c->hscal + STEP_COUNTERS + sizeof(double) * (size_t)c->nmembers, sizeof(double));
+            std::memcpy(&stats->dt, step_scalars(c) + STEP_COUNTERS, sizeof(double));
+            std::memcpy(&stats->time, step_scalars(c) + STEP_COUNTERS + sizeof(double) * (size_t)c->nmembers, sizeof(double));
         } else {
             cudaMemcpy(&stats->dt, c->dt, sizeof(double), cudaMemcpyDeviceToHost);
             cudaMemcpy(&stats->time, c->simTime, sizeof(double), cudaMemcpyDeviceToHost);
