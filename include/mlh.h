@@ -311,6 +311,11 @@ int mlh_probe_scale2(int n, const double *x, double *half, double *quarter, doub
  * x^(-1/5), x^(1/7), x^(-1/7). */
 int mlh_probe_int_math(int n, const double *x, const double *y, double *out);
 
+/* TEST HOOK.  The kernels' quotients for n pairs of host values: out holds four
+ * arrays of n, 1/b correctly rounded, a/b correctly rounded, 1/b and 1/sqrt(b)
+ * within 0.52 ulp. */
+int mlh_probe_quotients(int n, const double *a, const double *b, double *out);
+
 /* TEST HOOK.  The grid barriers of the persistent binning wait for
  * `extra_arrivals` more blocks than the launch holds (nonzero: every wait runs
  * out, which no correct launch can make happen) and give up after

@@ -93,22 +93,44 @@ __device__ __forceinline__ uint32_t frac24(float y) {
     return (__float_as_uint(fmaxf(fminf(y, 0.99999994f), 0.5f)) & 0x7fffffu) | 0x800000u;
 }
 
-// 1/x.  Units: e in 2^-76, y e and y e^2 in 2^-76, the result in 2^-63.
-__device__ __forceinline__ double frcp(double x) {
-    const uint32_t xh = __double2hiint(x), xl = __double2loint(x);
-    // exponent field in [2, 2044]: 1/x normal
-    if ((xh & 0x7fffffffu) - 0x00200000u >= 0x7fb00000u) return rcp_fp64(x);
+// 1/x as a fixed-point number, R / 2^63 in [2^62, 2^63] up to its own error (below
+// 2^-9 of the result's last place).  Units: e in 2^-76, y e and y e^2 in 2^-76.
+__device__ __forceinline__ uint64_t rcp_fixed(uint32_t xl, uint32_t xh) {
     float yf;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(mant_f32(xl, xh)));
     const uint32_t Y = frac24(yf), Mh = (xh & 0xfffffu) | 0x100000u;
     const int64_t E = -(int64_t)(mul_wide(xl, Y) + ((uint64_t)(Mh * Y) << 32));   // 2^76 - M Y, mod 2^64
     int64_t T = mul_hi32(E << 8, Y);
     T += ((int64_t)(int32_t)(E >> 23) * (int32_t)(T >> 23)) >> 30;
-    const uint64_t r = (uint64_t)(((int64_t)Y << 39) + (T >> 13) + 512) >> 10;
+    return (uint64_t)(((int64_t)Y << 39) + (T >> 13));
+}
+// r / 2^53 with the sign and the exponent of 1/x
+__device__ __forceinline__ double rcp_pack(uint64_t r, uint32_t xh) {
     const uint32_t rh = hi_word(r) + (0x7fc00000u - (xh & 0x7ff00000u));
     return __hiloint2double(rh | (xh & 0x80000000u), (uint32_t)r);
 }
+
+// 1/x, within 0.52 ulp
+__device__ __forceinline__ double frcp(double x) {
+    const uint32_t xh = __double2hiint(x), xl = __double2loint(x);
+    // exponent field in [2, 2044]: 1/x normal
+    if ((xh & 0x7fffffffu) - 0x00200000u >= 0x7fb00000u) return rcp_fp64(x);
+    return rcp_pack((rcp_fixed(xl, xh) + 512) >> 10, xh);
+}
 __device__ __forceinline__ double fdiv(double a, double b) { return a * frcp(b); }
+
+// 1/x correctly rounded, for exponent fields in [2, 2044]: s the truncated
+// reciprocal, raised by one when M (2 s + 1), M the mantissa, is below 2^106, that
+// is when 1/x lies above the midpoint s + 1/2 (never on it: 2 s + 1 is odd).  The
+// comparison mod 2^64: the two differ by less than 2^55.  The fixed point's error may
+// put s one place above the floor (1/x is then next to s, and stays) or, next to
+// s + 1, one below (and is raised).
+__device__ __forceinline__ double frcp_rn(double x) {
+    const uint32_t xh = __double2hiint(x), xl = __double2loint(x), Mh = (xh & 0xfffffu) | 0x100000u;
+    const uint64_t s = rcp_fixed(xl, xh) >> 10, m = 2 * s + 1;
+    const uint64_t t = mul_wide((uint32_t)m, xl) + ((uint64_t)((uint32_t)m * Mh + hi_word(m) * xl) << 32);
+    return rcp_pack(s + ((int64_t)t < 0), xh);
+}
 
 // 1/sqrt(x): z = x 4^-q in [1, 4).  Units: e in 2^-68, y e in 2^-75.
 __device__ __forceinline__ double frsqrt(double x) {
@@ -315,13 +337,19 @@ __device__ __forceinline__ double xmul_z(double a, double b) {
 }
 
 static __device__ __noinline__ double div_fp64(double a, double b) { return a / b; }
-// a / b: the quotient by the reciprocal and its remainder's correction, three
-// FP64 instructions (90 SM cycles per warp for a / b); zero, subnormal,
-// infinite and NaN operands and those outside the window by a / b
+// a / b correctly rounded: the quotient by the reciprocal r and its remainder's
+// correction, three FP64 instructions (90 SM cycles per warp for a / b).  With r
+// correctly rounded this is the IEEE quotient (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990): beside a
+// midpoint of two doubles the estimate q is one of the two, half an ulp off, so the
+// corrected value is off by half an ulp times |b r - 1| <= 2^-54 b (b in [1, 2)), less
+// than the distance of any quotient from a midpoint, half an ulp times 2^-52 / b.
+// Zero, subnormal, infinite and NaN operands and
+// those outside the window, by a / b.
 __device__ __forceinline__ double fdiv_rn(double a, double b) {
     const uint32_t ah = __double2hiint(a), bh = __double2hiint(b);
     if ((out_of_window(ah) | out_of_window(bh)) & 0xe0000000u) return div_fp64(a, b);
-    const double r = frcp(b), q = mulr(a, r);
+    const double r = frcp_rn(b), q = mulr(a, r);
     return fma(fma(-q, b, a), r, q);
 }
 

@@ -114,6 +114,13 @@ __global__ void k_int_math(int n, const double *__restrict__ x, const double *__
     }
 }
 
+__global__ void k_quotients(int n, const double *__restrict__ a, const double *__restrict__ b, double *__restrict__ o) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double v[4] = {mlh::frcp_rn(b[i]), mlh::fdiv_rn(a[i], b[i]), mlh::frcp(b[i]), mlh::frsqrt(b[i])};
+        for (int k = 0; k < 4; ++k) o[(size_t)k * n + i] = v[k];
+    }
+}
+
 __global__ void k_scale2(int n, const double *__restrict__ x, double *__restrict__ half, double *__restrict__ quarter,
                          double *__restrict__ twice) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -160,6 +167,25 @@ extern "C" int mlh_probe_int_math(int n, const double *x, const double *y, doubl
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 9 * b, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? 0 : MLH_ERR_CUDA;
+}
+
+// Reciprocals, quotients and the reciprocal square root of mlh_intmath.cuh of host
+// values (4 arrays of n in out), for checking them against IEEE operations.
+extern "C" int mlh_probe_quotients(int n, const double *a, const double *b, double *out) {
+    if (n < 0 || (n > 0 && (!a || !b || !out))) return MLH_ERR_INVALID;
+    if (n == 0) return 0;
+    double *d = nullptr;
+    if (cudaMalloc(&d, sizeof(double) * 6 * (size_t)n) != cudaSuccess) return MLH_ERR_CUDA;
+    const size_t bytes = sizeof(double) * (size_t)n;
+    cudaError_t e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_quotients<<<(n + 255) / 256, 256>>>(n, d, d + n, d + 2 * (size_t)n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 4 * bytes, cudaMemcpyDeviceToHost);
     cudaFree(d);
     return e == cudaSuccess ? 0 : MLH_ERR_CUDA;
 }

@@ -68,7 +68,7 @@ EXPORTS = ["mlh_abi_version", "mlh_last_error", "mlh_create", "mlh_destroy", "ml
            "mlh_grid_bounds_noalloc", "mlh_ensemble_create", "mlh_member_times", "mlh_set_graph_mode",
            "mlh_autotune", "mlh_set_tuning", "mlh_pstar_infer", "mlh_pstar_grad", "mlh_pstar_train", "mlh_set_pstar_weights",
            "mlh_pstar_harvest", "mlh_pstar_harvest_strong", "mlh_smoothing_lengths", "mlh_prepare", "mlh_riemann_fluxes",
-           "mlh_probe_fast_math", "mlh_probe_scale2", "mlh_probe_int_math", "mlh_probe_fp64_lanes", "mlh_test_binning_barrier"]
+           "mlh_probe_fast_math", "mlh_probe_scale2", "mlh_probe_int_math", "mlh_probe_quotients", "mlh_probe_fp64_lanes", "mlh_test_binning_barrier"]
 
 _lib = None
 
@@ -149,6 +149,8 @@ def load(path: str = LIB_PATH):
     L.mlh_probe_fast_math.restype = ctypes.c_int
     L.mlh_probe_int_math.argtypes = [ctypes.c_int] + [dp] * 3
     L.mlh_probe_int_math.restype = ctypes.c_int
+    L.mlh_probe_quotients.argtypes = [ctypes.c_int] + [dp] * 3
+    L.mlh_probe_quotients.restype = ctypes.c_int
     L.mlh_probe_scale2.argtypes = [ctypes.c_int] + [dp] * 4
     L.mlh_probe_scale2.restype = ctypes.c_int
     L.mlh_probe_fp64_lanes.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
