@@ -326,15 +326,6 @@ __device__ __forceinline__ double xmul(double a, double b) {
     if ((out_of_window(ah) | out_of_window(bh)) & 0xe0000000u) return mul_fp64(a, b);
     return mul_mantissas(ah, al, bh, bl);
 }
-// the same where a may be zero (an offset along an axis of a lattice): zeros
-// stay on the straight path
-__device__ __forceinline__ double xmul_z(double a, double b) {
-    const uint32_t ah = __double2hiint(a), al = __double2loint(a), bh = __double2hiint(b), bl = __double2loint(b);
-    const bool zero = ((ah << 1) | al) == 0u;
-    if (((zero ? 0u : out_of_window(ah)) | out_of_window(bh)) & 0xe0000000u) return mul_fp64(a, b);
-    const double r = mul_mantissas(ah, al, bh, bl);
-    return zero ? __hiloint2double((ah ^ bh) & 0x80000000u, 0) : r;
-}
 
 static __device__ __noinline__ double div_fp64(double a, double b) { return a / b; }
 // a / b correctly rounded: the quotient by the reciprocal r and its remainder's
