@@ -789,7 +789,7 @@ int mlh_set_tuning(mlh_ctx *c, const mlh_tuning *t) {
     auto threads_ok = [](int v) { return v == 64 || v == 128 || v == 256; };
     if (!c || !t || !threads_ok(t->face_threads) || !threads_ok(t->grad_threads) || t->face_blocks_per_sm < 1 ||
         t->face_blocks_per_sm > 32 || t->nns_warps_per_sm < 8 || t->nns_warps_per_sm > 256 ||
-        t->face_split < 0 || t->face_split > 2 || t->link_overlap < 0 || t->link_overlap > 2 ||
+        t->face_split < -1 || t->face_split > 2 || t->link_overlap < 0 || t->link_overlap > 2 ||
         t->persistent_binning < 0 || t->persistent_binning > 1 || (t->persistent_binning && c->bin_blocks < 1) ||
         t->fp32_filters < 0 || t->fp32_filters > 3 || t->learned_guess < 0 || t->learned_guess > 1) {
         g_last_error = "invalid tuning";
