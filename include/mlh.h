@@ -150,9 +150,9 @@ typedef struct mlh_tuning {
                               * threads; 0: one pass.  The plain steps of
                               * gamma = 5/3 and 7/5 with the first-order
                               * quadrature point; the others run one pass.
-                              * -1, and until set: by size, 2 from 65536
-                              * particles, else 0, and 1 with star-pressure
-                              * weights */
+                              * -1, and until set: by size, 2 from a million
+                              * faces (65536 particles in 3D, 104858 in 2D),
+                              * else 0, and 1 with star-pressure weights */
     int link_overlap;        /* 1: the face links run on a second stream beside
                               * the time step and the gradients; 2: inside the
                               * gradients kernel, each particle's links before

@@ -315,13 +315,16 @@ size_t step_scalars_bytes(size_t nm, size_t times) { return STEP_COUNTERS + size
 const char *step_scalars(const mlh_ctx *c) { return c->hscal.data() + (c->scal - (char *)(c->faceOff + c->n)); }
 
 // Structure of the plain face pass when neither the caller nor the autotuner
-// chose one: one pass (0) for few particles, where a block has one or two
-// rounds of faces and the in-block regrouping (2) only adds its barriers;
-// in-block above.  Pass times in us at 0 / 2: KH 24^2 23 / 28, KH 100^2 47 / 43,
-// 180^2 111 / 121, 260^2 (68k) 206 / 214, 317^2 (100k) 326 / 326, 64 KH members (866k)
-// 2844 / 2480; Sedov 17^3 50 / 58, 33^3 (36k) 252 / 255, 40^3 (64k) 429 / 431, 44^3 583 /
-// 553, 128^3 13990 / 12470; 16 blasts in 48^3 (110k) 846 / 756.
-int face_split_rule(size_t n) { return n < (size_t)1 << 16 ? 0 : 2; }
+// chose one: one pass (0) for few faces, where a block has one or two rounds of
+// them and the in-block regrouping (2) only adds its barriers; in-block above a
+// million faces, 10 per particle in 2D and 16 in 3D.  Pass times in us at 0 / 2, by
+// thousands of faces: KH 24^2 (6) 23 / 27, 50^2 (25) 25 / 27, 180^2 (324) 111 / 121,
+// 260^2 (676) 205 / 215, 290^2 (841) 258 / 259, 317^2 (1005) 306 / 308, 360^2 (1296)
+// 389 / 383, 400^2 (1600) 492 / 465, 640^2 (4096) 1293 / 1186; Sedov 17^3 (79) 47 / 57,
+// 33^3 (575) 251 / 252, 36^3 (747) 320 / 325, 40^3 (1024) 426 / 426, 44^3 (1363) 574 /
+// 548, 64^3 (4194) 1792 / 1639; only KH 100^2 (100), 46 / 43, is off the line.  At
+// gamma = 7/5 (with k_faces_general) 317^2 316 / 338, 640^2 1340 / 1291, 64^3 1790 / 1743.
+int face_split_rule(size_t n, int dim) { return n * (dim == 3 ? 16 : 10) < (size_t)1 << 20 ? 0 : 2; }
 
 StepArgs make_args(mlh_ctx *c, double dt_max) {
     StepArgs a{};   // zeroed pointers and counts, the tuning's defaults
@@ -356,7 +359,7 @@ StepArgs make_args(mlh_ctx *c, double dt_max) {
     a.dt = c->dt; a.simTime = c->simTime; a.arrived = c->arrived; a.stepsDone = c->stepsDone;
     a.scanTiles = c->scanTiles; a.scanTotal = c->scanTotal;
     a.learned = (c->learned && c->tune.learned_guess) ? 1 : 0;
-    if (a.tune.face_split < 0) a.tune.face_split = a.learned ? 1 : face_split_rule(c->n);
+    if (a.tune.face_split < 0) a.tune.face_split = a.learned ? 1 : face_split_rule(c->n, c->cfg.dim);
     a.fstate = c->fstate; a.feat = c->feat; a.yguess = c->yguess;
     a.queueFace = c->queueFace; a.queueCount = c->queueCount; a.mlp_packed = c->mlp_packed;
     a.fstate2 = c->fstate2; a.queueFace2 = c->queueFace2; a.queueCount2 = c->queueCount2;

@@ -42,3 +42,24 @@ def test_rule_by_size_can_be_set():
     for other in states[1:]:
         for k in states[0]:
             np.testing.assert_array_equal(states[0][k], other[k])
+
+
+# both sides of the rule's line, a million faces: 10 per particle in 2D, 16 in 3D
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,n_side", [(2, 323), (2, 324), (3, 40), (3, 41)])
+def test_structures_beside_the_line(dim, n_side):
+    from meshlesshydro_gb300 import build, ic, runtime
+    from meshlesshydro_gb300.config import MFVConfig
+    build.build()
+    p = ic.kelvin_helmholtz(n_side=n_side, seed=2) if dim == 2 else ic.sedov(n_side=n_side, seed=2)
+    cfg = MFVConfig.kelvin_helmholtz(p) if dim == 2 else MFVConfig.sedov(p)
+    states = []
+    for split in (-1, 0, 2):
+        s = runtime.Simulation(cfg, p)
+        s.set_tuning(dict(SHAPES, face_split=split))
+        s.step(2)
+        states.append(s.get_state())
+        s.close()
+    for other in states[1:]:
+        for k in states[0]:
+            np.testing.assert_array_equal(states[0][k], other[k])
