@@ -141,9 +141,13 @@ int mlh_member_times(mlh_ctx *ctx, double *dt, double *time, int nmembers);
 /* Launch shapes of the step's main kernels. */
 typedef struct mlh_tuning {
     int face_threads;        /* threads per block, Riemann face kernel */
-    int face_blocks_per_sm;  /* blocks per SM of its grid-stride loop */
-    int grad_threads;        /* threads per block, gradient/limiter kernel */
-    int nns_warps_per_sm;    /* warps per SM of the neighbour search */
+    int face_blocks_per_sm;  /* blocks per SM of its grid-stride loop, raised to
+                              * whole rounds of the blocks that an SM holds,
+                              * and at most what the faces need */
+    int grad_threads;        /* threads per block, gradient/limiter kernel; 64
+                              * where several lanes share a particle */
+    int nns_warps_per_sm;    /* warps per SM of the neighbour search, raised to
+                              * whole rounds (multiples of 32) */
     int face_split;          /* faces Newton has not finished after one step:
                               * 1 go to a second, dense pass over a queue;
                               * 2 are continued inside the block by its first

@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -873,16 +874,23 @@ int mlh_autotune(mlh_ctx *c, int trial_steps, mlh_tuning *out) {
             {
                 const int cand_t[] = {64, 128, 256};
                 const int cand_b[] = {2, 4, 8, 16, 32};
+                std::set<int> grids;   // launches timed
                 Tuning best = c->tune;
                 double best_ms = 1e300;
                 // the face passes: one (0), a second over a queue (1) or the
                 // unfinished faces continued inside the block (2), each over the
                 // candidate grids (the structures favour different grids); which
                 // pays depends on how many faces need a second Newton step
+                // (where only one structure is built, the one pass alone; grids
+                // that are the same launch, once)
+                const StepArgs now = make_args(c, 0.);
                 for (int split : {1, 2, 0}) {
+                    if (split && !(now.root && now.p.foqp)) continue;
+                    grids.clear();
                     for (int b : cand_b) {
                         c->tune.face_split = split;
                         c->tune.face_blocks_per_sm = b;
+                        if (!grids.insert(face_grid(make_args(c, 0.), split)).second) continue;
                         double ms;
                         if ((rc = trial(KT_FACES, ms))) goto done;
                         if (ms < best_ms) { best_ms = ms; best.face_split = split; best.face_blocks_per_sm = b; }
@@ -891,31 +899,39 @@ int mlh_autotune(mlh_ctx *c, int trial_steps, mlh_tuning *out) {
                 c->tune.face_split = best.face_split;
                 c->tune.face_blocks_per_sm = best.face_blocks_per_sm;
                 for (int t : cand_t) {
+                    if (best.face_split == 2) break;   // has a block size of its own
                     c->tune.face_threads = t;
                     double ms;
                     if ((rc = trial(KT_FACES, ms))) goto done;
                     if (ms < best_ms) { best_ms = ms; best.face_threads = t; }
                 }
                 c->tune.face_threads = best.face_threads;
+                grids.clear();
                 for (int b : cand_b) {   // the grid again, for the chosen block size
+                    if (best.face_split == 2) break;
                     c->tune.face_blocks_per_sm = b;
+                    if (!grids.insert(face_grid(make_args(c, 0.), best.face_split)).second) continue;
                     double ms;
                     if ((rc = trial(KT_FACES, ms))) goto done;
                     if (ms < best_ms) { best_ms = ms; best.face_blocks_per_sm = b; }
                 }
                 c->tune.face_blocks_per_sm = best.face_blocks_per_sm;
                 best_ms = 1e300;
+                grids.clear();
                 for (int t : cand_t) {
                     c->tune.grad_threads = t;
+                    if (!grids.insert(gradients_threads(make_args(c, 0.))).second) continue;
                     double ms;
                     if ((rc = trial(KT_GRAD, ms))) goto done;
                     if (ms < best_ms) { best_ms = ms; best.grad_threads = t; }
                 }
                 c->tune.grad_threads = best.grad_threads;
                 best_ms = 1e300;
-                const int cand_w[] = {16, 32, 64, 128};
+                const int cand_w[] = {32, 64, 128};   // fewer are raised to 32
+                grids.clear();
                 for (int w : cand_w) {
                     c->tune.nns_warps_per_sm = w;
+                    if (!grids.insert(search_shape(make_args(c, 0.)).blocks).second) continue;
                     double ms;
                     if ((rc = trial(KT_NNS, ms))) goto done;
                     if (ms < best_ms) { best_ms = ms; best.nns_warps_per_sm = w; }

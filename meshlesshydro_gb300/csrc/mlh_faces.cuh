@@ -189,7 +189,7 @@ __device__ __forceinline__ unsigned project_flux(const RiemannResult &rs, const 
     return st;
 }
 
-// Register caps of the face kernels: with the roots and products on the integer
+// Register caps of the face kernels (MLH_FACE_MAXREG_*): with the roots and products on the integer
 // pipe the passes wait on latency at 16 warps per SM.  k_faces_block: 80, three
 // blocks of 256 threads (24 warps) per SM.  With 128 threads the pass over the Sedov
 // 128^3 faces at 104 / 96 / 88 / 80 / 72 registers took 13.84 / 13.30 / 13.33 / 13.25 /
@@ -201,15 +201,6 @@ __device__ __forceinline__ unsigned project_flux(const RiemannResult &rs, const 
 // instructions, more than the instruction cache holds (no-instruction stalls a
 // sixth of the time at 128 threads); a block's warps run in step between its
 // barriers and share what is fetched.
-#ifndef MLH_FACE_MAXREG_3D
-#define MLH_FACE_MAXREG_3D 80
-#endif
-#ifndef MLH_FACE_MAXREG_2D
-#define MLH_FACE_MAXREG_2D 72
-#endif
-#ifndef MLH_FACE_MAXREG_BLOCK
-#define MLH_FACE_MAXREG_BLOCK 80
-#endif
 #define MLH_FACE_BOUNDS __maxnreg__(D == 3 ? MLH_FACE_MAXREG_3D : MLH_FACE_MAXREG_2D)
 // The face-frame Riemann problem of canonical face f (i < j): effective face
 // A_ij = psi~_j(x_i)/omega_i - psi~_i(x_j)/omega_j from the psi~ of both
@@ -562,12 +553,6 @@ __global__ void MLH_FACE_BOUNDS k_faces(Params p, RiemannConsts rc, const Member
 // without strong shocks skips) and continues them from p_TR e^y together with
 // the other unfinished faces.  Nothing leaves the block: the plain and the
 // learned step differ only by that branch.
-// Threads per block of k_faces_block: 128 / 192 / 256: Sedov 128^3 13.2 / 13.1 / 12.5
-// ms, 64 KH members 2.63 / 2.66 / 2.47 ms, 16 blasts in 48^3 817 / 790 / 756 us.  The
-// barriers keep a block's warps in step, so that they share the instructions
-// that are fetched; with fewer of them (one count for a round instead of one per
-// warp, two barriers instead of four) 128 threads took 2.72 ms on the members.
-constexpr int FB_T = 256;
 
 // The network's guesses for the ns strong-shock faces of a round listed in
 // slist (their solver states in sv, s.p = p_TR): warp w takes the faces
@@ -773,26 +758,13 @@ __global__ void __launch_bounds__(256) k_riemann_batch(int n, RiemannConsts rc, 
 
 // ------------------------------------------------------------------ launchers
 
-// Blocks of a face pass: the tuned number per SM, raised to a multiple of the
-// blocks that an SM holds at once (the register cap's threads), and no more
-// than the faces that the table can hold need.
-inline int face_blocks(int cap, int threads, const StepArgs &a) {
-    int resident = 65536 / cap / threads;
-    if (resident < 1) resident = 1;
-    const int per_sm = (a.tune.face_blocks_per_sm + resident - 1) / resident * resident;
-    const size_t most = (a.faces_cap + threads - 1) / threads;
-    const size_t want = (size_t)a.sm_count * per_sm;
-    return (int)(want < most ? want : most);
-}
-
 // The face passes of a step: the structure that the tuning chose, of the solver
 // for ROOT = 2 gamma / (gamma - 1) (5, 7, or 0: any gamma, one pass).
 template <int D, int ROOT>
 void launch_faces(StepArgs &a) {
     const Params &p = a.p;
     cudaStream_t s = a.stream;
-    const int fT = a.tune.face_threads, fBb = face_blocks(MLH_FACE_MAXREG_BLOCK, FB_T, a);
-    const int fB = face_blocks(D == 3 ? MLH_FACE_MAXREG_3D : MLH_FACE_MAXREG_2D, fT, a);
+    const int fT = a.tune.face_threads, fB = face_grid(a, 0), fBb = face_grid(a, 2);
     Params pf = p;   // the face passes see the tuned split
     const RiemannConsts rc = make_riemann_consts(p.gamma, p.rtol, p.rmaxit);
     const FaceQueue qa{a.fstate, a.queueFace, a.queueCount, a.qcap};

@@ -2543,6 +2543,31 @@ void launch_hsolve(StepArgs &a) {
                                                      a.cellStart, a.cellList, a.hp, a.hpf, a.neff, a.hstat, a.status);
 }
 
+// The neighbour search's split and grid.  Parts per cell: with fewer than two cells
+// per resident warp a cell's particles go to several warps (each takes the candidates
+// again), in batches that split a mean cell evenly.  The grid: the tuned warps per SM
+// in whole rounds of resident blocks, grid-stride over the units.
+SearchShape search_shape(const StepArgs &a) {
+    const Params &p = a.p;
+    const long long cells = a.cells_est > 0 ? a.cells_est : 1, resident = (long long)a.sm_count * NNS_WARPS * MLH_NNS_MINB;
+    long long nsplit = (2 * resident + cells - 1) / cells;
+    nsplit = nsplit < 1 ? 1 : nsplit > 8 ? 8 : nsplit;
+    if ((long long)p.ncells_cap * nsplit > 0x7fffffffll) nsplit = 1;
+    long long pb = nsplit > 1 ? (p.n + cells * nsplit - 1) / (cells * nsplit) : NNS_PB;
+    pb = pb < 1 ? 1 : pb > NNS_PB ? NNS_PB : pb;
+    int per_sm = (a.tune.nns_warps_per_sm + NNS_WARPS - 1) / NNS_WARPS;
+    per_sm = (per_sm + MLH_NNS_MINB - 1) / MLH_NNS_MINB * MLH_NNS_MINB;
+    const long long most = ((long long)p.ncells_cap * nsplit + NNS_WARPS - 1) / NNS_WARPS;
+    const long long want = (long long)a.sm_count * per_sm;
+    return {(int)nsplit, (int)pb, (int)(want < most ? want : most < 1 ? 1 : most)};
+}
+
+// Threads per block of the gradients: with several lanes per particle there are few
+// blocks, and small ones spread evenly (KH 100^2: 49 -> 44 us).
+int gradients_threads(const StepArgs &a) {
+    return grad_lanes(a.p.n, a.sm_count) > 1 && a.tune.grad_threads > 64 ? 64 : a.tune.grad_threads;
+}
+
 template <int D>
 void launch_step(StepArgs &a) {
     const Params &p = a.p;
@@ -2572,25 +2597,11 @@ void launch_step(StepArgs &a) {
     tick(KT_NNS);
     {
         const size_t smem = nns_smem_bytes(p.K);
-        // parts per cell: with fewer than two cells per resident warp a cell's
-        // particles go to several warps (each stages the candidates), in batches
-        // that split a mean cell evenly
-        const long long cells = a.cells_est > 0 ? a.cells_est : 1, resident = (long long)a.sm_count * NNS_WARPS * MLH_NNS_MINB;
-        long long nsplit = (2 * resident + cells - 1) / cells;
-        nsplit = nsplit < 1 ? 1 : nsplit > 8 ? 8 : nsplit;
-        if ((long long)p.ncells_cap * nsplit > 0x7fffffffll) nsplit = 1;
-        long long pb = nsplit > 1 ? (p.n + cells * nsplit - 1) / (cells * nsplit) : NNS_PB;
-        pb = pb < 1 ? 1 : pb > NNS_PB ? NNS_PB : pb;
-        // grid-stride over the units, in whole rounds of resident blocks
-        int per_sm = (a.tune.nns_warps_per_sm + NNS_WARPS - 1) / NNS_WARPS;
-        per_sm = (per_sm + MLH_NNS_MINB - 1) / MLH_NNS_MINB * MLH_NNS_MINB;
-        const long long most = ((long long)p.ncells_cap * nsplit + NNS_WARPS - 1) / NNS_WARPS;
-        const long long want = (long long)a.sm_count * per_sm;
-        const int blocks = (int)(want < most ? want : most < 1 ? 1 : most);
+        const SearchShape sh = search_shape(a);
         auto run = [&](auto kern) {
             if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            launch_kernel(early, kern, blocks, NNS_WARPS * 32, smem, s,
-                p, (int)nsplit, (int)pb, a.members, a.memberOf, a.grids, a.x, a.y, a.z, a.posf, a.vx, a.vy, a.vz, a.m,
+            launch_kernel(early, kern, sh.blocks, NNS_WARPS * 32, smem, s,
+                p, sh.nsplit, sh.batch, a.members, a.memberOf, a.grids, a.x, a.y, a.z, a.posf, a.vx, a.vy, a.vz, a.m,
                 a.u, a.cellTotal, a.cellStart, a.cellList, a.nbr, a.psi, a.ww, a.noi, a.noiImg, a.faceCnt, a.prim,
                 a.geo, a.velf, a.status);
         };
@@ -2645,7 +2656,7 @@ void launch_step(StepArgs &a) {
         exclusive_scan(a.faceCnt, p.n, a.faceOff, a.scanTiles, a.scanTotal, s);
         cudaMemsetAsync(a.faces, 0xff, sizeof(FaceRef) * a.faces_cap, s);
     }
-    const int gT = gl > 1 && a.tune.grad_threads > 64 ? 64 : a.tune.grad_threads;   // few blocks: small ones spread evenly (KH 100^2: 49 -> 44 us)
+    const int gT = gradients_threads(a);
     const int gB = (int)(((long long)p.n * gl + gT - 1) / gT);
 #define MLH_GRAD_ARGS                                                                                          \
     a.members, a.memberOf, a.grids, a.prim, a.geo, a.nbr, a.ww, a.noi, a.noiImg, a.grad, a.gradRaw, a.psi,     \

@@ -116,6 +116,46 @@ struct StepArgs {
 // holds 6 doubles per block
 constexpr int BOUNDS_BLOCKS = 304;
 
+// Launch shapes as the tuned numbers give them; mlh_autotune leaves out candidates
+// that give a launch it has timed.
+struct SearchShape {
+    int nsplit, batch, blocks;   // warps per cell, particles per batch, blocks
+};
+SearchShape search_shape(const StepArgs &a);
+int gradients_threads(const StepArgs &a);
+// register caps of the face kernels (mlh_faces.cuh gives the times they were chosen by)
+#ifndef MLH_FACE_MAXREG_3D
+#define MLH_FACE_MAXREG_3D 80
+#endif
+#ifndef MLH_FACE_MAXREG_2D
+#define MLH_FACE_MAXREG_2D 72
+#endif
+#ifndef MLH_FACE_MAXREG_BLOCK
+#define MLH_FACE_MAXREG_BLOCK 80
+#endif
+// Threads per block of k_faces_block: 128 / 192 / 256: Sedov 128^3 13.2 / 13.1 / 12.5
+// ms, 64 KH members 2.63 / 2.66 / 2.47 ms, 16 blasts in 48^3 817 / 790 / 756 us.  The
+// barriers keep a block's warps in step, so that they share the instructions
+// that are fetched; with fewer of them (one count for a round instead of one per
+// warp, two barriers instead of four) 128 threads took 2.72 ms on the members.
+constexpr int FB_T = 256;
+// Blocks of a face pass: the tuned number per SM, raised to a multiple of the
+// blocks that an SM holds at once (the register cap's threads), and no more
+// than the faces that the table can hold need.
+inline int face_blocks(int cap, int threads, const StepArgs &a) {
+    int resident = 65536 / cap / threads;
+    if (resident < 1) resident = 1;
+    const int per_sm = (a.tune.face_blocks_per_sm + resident - 1) / resident * resident;
+    const size_t most = (a.faces_cap + threads - 1) / threads;
+    const size_t want = (size_t)a.sm_count * per_sm;
+    return (int)(want < most ? want : most);
+}
+// the grid of the face pass with structure `split` (0, 1, 2)
+inline int face_grid(const StepArgs &a, int split) {
+    if (split == 2) return face_blocks(MLH_FACE_MAXREG_BLOCK, FB_T, a);
+    return face_blocks(a.p.dim == 3 ? MLH_FACE_MAXREG_3D : MLH_FACE_MAXREG_2D, a.tune.face_threads, a);
+}
+
 void step(StepArgs &a);
 // blocks of the persistent binning kernel resident at once (0: none)
 int binning_blocks(int dim, int sm_count);
