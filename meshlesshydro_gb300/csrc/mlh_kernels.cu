@@ -13,9 +13,14 @@
 //                        solveRiemannProblems (one thread per canonical face)
 //   gather + kick/drift  collectFluxes + updateStateAndPosition
 //
-// Determinism: no floating-point atomics.  Every per-particle sum runs over the
-// neighbour list in the reference's order; each face flux is computed once,
-// from the side of the lower particle index, and gathered with sign.
+// Determinism: no floating-point atomics; each face flux is computed once, from the
+// side of the lower particle index, and gathered with sign; densities and flux sums
+// run over the neighbour list in the reference's order.  The sums of the least-squares
+// matrix and the gradients run in that order with one lane per particle; where few
+// particles in all leave the GPU short of warps, 2, 4 or 8 lanes sum every 2nd, 4th or
+// 8th neighbour each (grad_lanes, by the particles of the context and the SMs of the
+// GPU).  So one context gives the same bits on every run, graph or not, but a member of
+// a large ensemble may differ in rounding from the same simulation alone.
 #include "mlh_device.cuh"
 #include "mlh_riemann.cuh"
 #include "mlh_kernels.h"
