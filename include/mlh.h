@@ -56,7 +56,10 @@ typedef struct mlh_config {
                                    abs(double) when no <math.h>/<stdlib.h> is seen */
     int image_pairwise_limiter; /* pairwise limiter also on periodic-image faces */
     int riemann_max_iter;       /* Newton iteration cap */
-    int max_neighbours;         /* slots per particle; 0 = automatic */
+    int max_neighbours;         /* slots per particle to start with (they grow);
+                                 * 0 = automatic.  The search lists at most
+                                 * 444, 260 with smoothing lengths: a particle
+                                 * with more is MLH_ERR_CAPACITY */
     double box_lo[3];           /* periodicBoxLimits lowerX/Y/Z */
     double box_hi[3];           /* periodicBoxLimits upperX/Y/Z */
     double kernel_size;         /* kernelSize (support radius h) */
