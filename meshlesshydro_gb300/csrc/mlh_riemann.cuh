@@ -185,6 +185,11 @@ __device__ inline RiemannResult riemann_exact(const RiemannConsts &c, double rho
 // are ordered as the values.
 __device__ __forceinline__ bool nn_le(double a, double b) { return __double_as_longlong(a) <= __double_as_longlong(b); }
 
+// x < 0, false for NaN of either sign (dneg goes by the sign bit)
+__device__ __forceinline__ bool below_zero(double x) {
+    return (unsigned long long)__double_as_longlong(x) - 0x8000000000000001ull <= 0x7fefffffffffffffull;
+}
+
 // The multiplies, adds and fused multiply-adds of the fast path are written
 // out (mulr, addr, subr, fma): left to the compiler, their fusing would depend
 // on the basic blocks around them and so on the kernel that inlines the
@@ -508,7 +513,8 @@ __device__ inline RiemannResult riemann_root_finish(const RiemannConsts &k, cons
     } else {                                      // shock on side s
         const double pm = xmul(pstar, invp_s);
         const double sl = __fma_rn(-c_s, fsqrt_rn(fma(k.g2, pm, k.g1)), u_s);   // shock speed
-        if (!dneg(sl)) { rho = rho_s; u = u_s; pp = p_s; }
+        // NaN: p_s < 0 (a reconstructed pressure of cold gas), the side's state
+        if (!below_zero(sl)) { rho = rho_s; u = u_s; pp = p_s; }
         else { rho = xmul(rho_s, xmul(addr(pm, k.g6), frcp(fma(pm, k.g6, 1.)))); u = ustar_s; pp = pstar; }
     }
     res.flag = right ? 1 : -1;
